@@ -25,7 +25,8 @@ int maxSmemOptin() {
 // (14 level-0 Krylov arrays plus the AMG coarse levels), and leaving the unified
 // L1/shared storage to the L1 cache measured faster (1536 cells: 537 us per outer
 // iteration without an arena against 656 us with the largest one).
-int arenaDoublesFor(long wsDoubles, int knobKb, int nmax) {
+// The exchange vectors of the resident solvers come first, whatever the knob says.
+int arenaDoublesFor(long wsDoubles, int knobKb, int nmax, long resident) {
     const long shared = static_cast<long>(rq::solveSharedBytes());
     const long optin = maxSmemOptin();
     long bytes;
@@ -36,6 +37,7 @@ int arenaDoublesFor(long wsDoubles, int knobKb, int nmax) {
     else
         bytes = 0;
     bytes = std::max<long>(0, std::min(bytes, wsDoubles * 8));
+    bytes = std::min(std::max(bytes, resident * 8), optin - shared);
     return static_cast<int>(bytes / 8 / 32 * 32);
 }
 
@@ -55,12 +57,14 @@ int chooseArena(const std::vector<const rq_problem *> &probs) {
     long ws = 0;
     int knob = -1;
     int nmax = 0;
+    long resident = 0;
     for (const auto *p : probs) {
+        resident = std::max(resident, rq::residentDoubles(p->cls));
         ws = std::max(ws, static_cast<long>(p->cls.wsDoubles));
         knob = std::max(knob, p->arenaKb);
         nmax = std::max(nmax, p->mesh.n);
     }
-    return arenaDoublesFor(ws, knob, nmax);
+    return arenaDoublesFor(ws, knob, nmax, resident);
 }
 
 } // namespace rqc
@@ -264,6 +268,15 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
     if (h.coarseN() > rq::kMaxCoarse)
         throw RqError(RQ_E_UNSUPPORTED, "coarsest AMG level above 128 rows");
     C.nlev = L;
+    C.resAmg = h.sweeps == 1 && m.n <= 65535;
+    // 16-bit columns (padding: column 0), packed into the int32 upload
+    auto addH = [&](const uint16_t **slot, const std::vector<int> &v) {
+        std::vector<int32_t> packed((v.size() + 1) / 2, 0);
+        uint16_t *q = reinterpret_cast<uint16_t *>(packed.data());
+        for (size_t k = 0; k < v.size(); ++k)
+            q[k] = static_cast<uint16_t>(std::max(v[k], 0));
+        addI(reinterpret_cast<const int32_t **>(slot), packed);
+    };
     // ELL slots of levels >= 1: CSR entry k of row i -> (k - ptr[i]) * n + i
     std::vector<std::vector<int>> slotOf(L), entryOf(L);
     std::vector<int> width(L, 0);
@@ -298,6 +311,8 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
             for (int i = 0; i < Lv.n; ++i)
                 dpos[i] = slotOf[l][Lv.diagPos[i]];
             addI(&dl.ecol, ecol);
+            if (C.resAmg)
+                addH(&dl.ecol16, ecol);
             addI(&dl.diagPos, dpos);
         }
         if (l > 0 || L == 1)
@@ -326,6 +341,10 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
             addI(&dl.pcol, pc);
             addD(&dl.pval, pv);
             addI(&dl.rcol, rc);
+            if (C.resAmg) {
+                addH(&dl.pcol16, pc);
+                addH(&dl.rcol16, rc);
+            }
             addD(&dl.rval, rv);
             // gather lists in the next level's slot order; sources of level >= 1 as slots
             const int ns = width[l + 1] * nc;
@@ -375,11 +394,12 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
     check(cudaMemcpy(P.dCls.p, &C, sizeof(rq::DevClass), cudaMemcpyHostToDevice), "upload");
 }
 
-// CTA size of a class, measured per outer iteration on a B200 (FP64): 512 threads
-// for up to 1024 cells (384 cells: 153 us at 512, 182 us at 768; 768 cells: equal),
-// 768 threads above (1536 cells: 431 us at 768, 465 us at 512, 567 us at 1024 --
-// two cells per thread; 1024 threads cap registers at 64 and spill).
-int defaultBlock(int nCells) { return nCells > 1024 ? 768 : 512; }
+// CTA size of a class, measured per outer iteration on a B200 (FP64): 512 threads up to
+// 1536 cells, where the resident solvers hold three cells per thread in 128 registers
+// (1536 cells over the first 400 iterations: 332 us; 397 us with 768 threads, whose 80
+// registers leave only the general solvers), 768 threads above (200 x 100 bump, general
+// solvers: 12.4 ms against 17.0 ms with 512).
+int defaultBlock(int nCells) { return nCells > 1536 ? 768 : 512; }
 
 
 
@@ -616,7 +636,8 @@ int rq_problem_set_launch(rq_problem *p, const rq_launch_shape *shape) {
         if (shape->arena_kb < -1)
             throw std::invalid_argument("arena_kb must be -1 (default rule), 0 or positive");
         std::lock_guard<std::mutex> lock(p->mu);
-        const int arena = arenaDoublesFor(p->cls.wsDoubles, shape->arena_kb, p->mesh.n);
+        const int arena = arenaDoublesFor(p->cls.wsDoubles, shape->arena_kb, p->mesh.n,
+                                         rq::residentDoubles(p->cls));
         if (rq::solveBlocksPerSM(shape->block_threads, arena) < 1)
             throw std::invalid_argument("this launch shape does not fit on an SM");
         p->block = shape->block_threads;
@@ -687,7 +708,8 @@ int rq_problem_tune(rq_problem *p, const double *theta, int32_t iters,
             c.us_per_iteration = -1.0;
             if (!rq::launchVariantExists(c.block_threads) || c.arena_kb < -1)
                 continue;
-            const int arena = arenaDoublesFor(p->cls.wsDoubles, c.arena_kb, p->mesh.n);
+            const int arena = arenaDoublesFor(p->cls.wsDoubles, c.arena_kb, p->mesh.n,
+                                             rq::residentDoubles(p->cls));
             if (rq::solveBlocksPerSM(c.block_threads, arena) < 1)
                 continue;
             check(cudaMemset(dCounter.p, 0, sizeof(int)), "counter");
@@ -967,7 +989,7 @@ int rq_evaluate_noalloc(rq_problem *p, const double *theta_dev, rq_row_out *row_
         job.row = reinterpret_cast<rq::RowOut *>(row_dev);
         job.pred = predictions_dev;
         // shared-memory arena as the batch path sizes it for one class
-        const int arena = arenaDoublesFor(need, p->arenaKb, p->mesh.n);
+        const int arena = arenaDoublesFor(need, p->arenaKb, p->mesh.n, rq::residentDoubles(p->cls));
         check(rq::launchSolveNoAlloc(job, p->noallocScratch, p->block, arena,
                                      static_cast<cudaStream_t>(stream)),
               "allocation-free solve launch");

@@ -149,7 +149,7 @@ struct DeviceScope {
 void runOneJob(rq_problem &p, const rq::DevJob &job);
 int maxSmemOptin();
 // shared-memory arena (doubles) of a launch of these classes
-int arenaDoublesFor(long wsDoubles, int knobKb, int nmax);
+int arenaDoublesFor(long wsDoubles, int knobKb, int nmax, long resident);
 int chooseArena(const std::vector<const rq_problem *> &probs);
 inline rq_row_out toRow(const rq::RowOut &o) {
     return rq_row_out{o.status, o.iterations, o.stalled, o.converged, o.loglik, o.finalWorst,

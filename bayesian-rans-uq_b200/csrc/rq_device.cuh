@@ -42,6 +42,8 @@ struct DevAmgLevel {
     const int32_t *ecol, *diagPos;       // ELL columns (-1: padding); slot of the diagonal
     const int32_t *pcol, *rcol;          // prolongation / restriction ELL columns
     const double *pval, *rval;           // and weights
+    const uint16_t *ecol16, *pcol16, *rcol16; // the same columns in 16 bits, padding as column
+                                              // 0 (its values are 0); classes with resAmg
     const int32_t *gPtr, *gSrc;          // next-level value slot -> entries of this level
     const double *gW;                    // each entry's weight P_iI P_jJ in the Galerkin sum
 };
@@ -67,7 +69,8 @@ struct DevClass {
     DevAmgLevel lev[kMaxLevels];
     double amgW, amgAlpha;     // V-cycle smoother weight, coarse-correction scale
     int32_t amgVals, amgVecs;  // per-solve doubles for coarse values / vectors
-    int32_t amgSweeps, pad4;   // damped-Jacobi sweeps before and after each coarse correction
+    int32_t resAmg;            // the resident V-cycle applies: one sweep, 16-bit columns set
+    int32_t amgSweeps;   // damped-Jacobi sweeps before and after each coarse correction
     int64_t wsDoubles;         // per-solve workspace
     // InferenceParameterSet: active indices, the coefficients filling the rest,
     // and the admission bounds (core/include/InferenceParameters.hpp:67-77, 127-165)

@@ -7,6 +7,9 @@
 namespace rq {
 
 size_t solveSharedBytes();
+// Doubles at the start of the arena that the resident inner solvers of a class need (0:
+// the class is too large for them, rq_resident.cuh).
+long residentDoubles(const DevClass &C);
 // Persistent CTAs: each pulls job indices from *nextJob (zeroed by the caller)
 // until njobs are taken; ws is grid x wsStride doubles of per-CTA workspace.
 // arenaDoubles: shared-memory arena per CTA for the hot arrays (0 = all global).

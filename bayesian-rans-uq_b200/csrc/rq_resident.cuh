@@ -1,0 +1,623 @@
+// Inner linear solvers of the small mesh classes (n <= kResCells x the CTA's threads,
+// FP64 form): the recurrences of bicgstabT and pcgT (rq_solver.cu) with every vector and
+// the matrix rows in registers. A group of ceil(n / 96) warps works, three cells per
+// thread; only the vectors that a neighbour reads pass through shared memory. The other
+// warps of the CTA join for the coarse levels of the V-cycle and wait otherwise.
+//
+// What bounds them: latency. One BiCGSTAB iteration is a chain of two matrix products,
+// three block sums and FP64 divisions; at 384 cells the operands of all of it are 30 KB,
+// so neither memory nor the FP64 pipe is near its limit. Cycles per iteration in isolation
+// on a B200, by cells per thread: 384 cells 3147 / 2568 / 2677 / 3033 (1 / 2 / 3 / 4),
+// 1536 cells - / - / 4916 / 5450: few warps make the block sums cheap, and four cells (11
+// doubles of state each) spill out of 128 registers. With the sums on the tensor cores and
+// the branch-free quotients below: 1766 at 384 cells, 2550 at 768, 4234 at 1536.
+#pragma once
+
+// Threads of the working group, and the zero slot of an exchange vector: entries
+// n .. 3T - 1 belong to no cell and hold zero, entry 3T stands for absent neighbours.
+__host__ __device__ inline int resThreads(long n) {
+    return static_cast<int>((n + 32 * kResCells - 1) / (32 * kResCells)) * 32;
+}
+// Doubles of the two exchange vectors, which start the arena; the level vectors of the
+// V-cycle follow them.
+__host__ __device__ inline long resExchange(long n) {
+    return 2 * ((kResCells * resThreads(n) + 1L + 31) / 32 * 32);
+}
+
+extern __shared__ __align__(16) unsigned char rqSmem[];
+
+__device__ __forceinline__ void groupSync(int threads) {
+    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
+
+// D = A B of one FP64 m8n8k4 product: a is this lane's A[lane / 4][lane % 4], b its
+// B[lane % 4][lane / 4]; d0, d1 receive D[lane / 4][2 (lane % 4) + 0, 1].
+__device__ __forceinline__ void mma884(double &d0, double &d1, double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%4};"
+        : "=d"(d0), "=d"(d1)
+        : "d"(a), "d"(b), "d"(0.0));
+}
+
+// Sums of K values over the working group (nw warps), the same bits in every thread. A
+// warp adds its lanes with two FP64 matrix products: ones times the lanes' values gives
+// column sums of four lanes, of which each lane adds two and which a second product with
+// ones adds up for all lanes. Five shuffle steps in their place cost 160 to 240 cycles
+// (a 64-bit shuffle takes 24, 32 with 16 warps: the SM has one shuffle unit), and a
+// BiCGSTAB iteration with them 2677 instead of 1925 cycles at 384 cells. The warps'
+// partials are added by every thread (four at most) or once more by a product. Partials of
+// warps beyond nw are zero (resClear).
+template <int K> __device__ __forceinline__ void sumRes(double (&v)[K], int &rp, int nw) {
+    ResShared &R = reinterpret_cast<Shared *>(rqSmem)->R;
+    double u[K], w[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        mma884(u[k], w[k], 1.0, v[k]);
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        mma884(v[k], w[k], u[k] + w[k], 1.0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            R.red[rp][k][warp] = v[k];
+    groupSync(nw * 32);
+    const int q = nw <= 4 ? 0 : 4 * (lane & 3);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const double2 a = *reinterpret_cast<const double2 *>(&R.red[rp][k][q]);
+        const double2 b = *reinterpret_cast<const double2 *>(&R.red[rp][k][q + 2]);
+        v[k] = (a.x + b.x) + (a.y + b.y);
+    }
+    if (nw > 4)
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            mma884(v[k], w[k], v[k], 1.0);
+    rp ^= 1;
+}
+
+// a / b by Newton-Raphson iteration from the hardware's approximate reciprocal, and one
+// correction of the quotient: within one unit in the last place for operands and quotients
+// of normal size (the solvers' guards keep |b| above 1e-30). Unlike the division operator
+// it has no branch, so its latency overlaps the block sum beside it (85 cycles each, four
+// per BiCGSTAB iteration).
+__device__ __forceinline__ double recip(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = fma(y, fma(-b, y, 1.0), y);
+    y = fma(y, fma(-b, y, 1.0), y);
+    return y;
+}
+__device__ __forceinline__ double quot(double a, double b) {
+    const double y = recip(b), q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+
+// Whether the square sum q passes sqrt(q) / r0n < tol: decided by q against the squared
+// bound, and by the quotient itself only where rounding could matter (a square root and a
+// division cost 190 cycles, twice per iteration).
+__device__ __forceinline__ bool dropped(double q, double bound2, double r0n, double tol) {
+    if (fabs(q - bound2) > 1e-12 * bound2)
+        return q < bound2;
+    return sqrt(q) / r0n < tol;
+}
+
+// A thread's rows of the 5-point system: coefficients (x neighbours in face order) and
+// the exchange entries of the neighbours, packed in pairs. A row beyond n is the identity.
+struct ResRows {
+    double d[kResCells], a1[kResCells], a2[kResCells], aS[kResCells], aN[kResCells];
+    double rd[kResCells];
+    unsigned ix[kResCells], iy[kResCells];
+
+    __device__ __forceinline__ void load(const DevClass &C, const KW<double> &K, int T) {
+        const unsigned zero = kResCells * T;
+#pragma unroll
+        for (int k = 0; k < kResCells; ++k) {
+            const int c = threadIdx.x + k * T;
+            d[k] = rd[k] = 1.0;
+            a1[k] = a2[k] = aS[k] = aN[k] = 0.0;
+            ix[k] = iy[k] = zero | (zero << 16);
+            if (c < C.n) {
+                const Cell q = cellOf(C, c);
+                d[k] = K.d[c];
+                const double w = K.aW[c], e = K.aE[c];
+                a1[k] = q.xEfirst ? e : w;
+                a2[k] = q.xEfirst ? w : e;
+                ix[k] = static_cast<unsigned>(q.xEfirst ? q.E : q.W) |
+                        (static_cast<unsigned>(q.xEfirst ? q.W : q.E) << 16);
+                const unsigned s = q.south ? c - C.nx : zero, nn = q.north ? c + C.nx : zero;
+                iy[k] = s | (nn << 16);
+                aS[k] = q.south ? K.aS[c] : 0.0;
+                aN[k] = q.north ? K.aN[c] : 0.0;
+                rd[k] = (fabs(d[k]) > 1e-30) ? 1.0 / d[k] : 1.0; // jacobiPrecond as a product
+            }
+        }
+    }
+    // row k times the exchanged vector e, whose entry at the own cell is xc
+    __device__ __forceinline__ double times(int k, double xc, const double *e) const {
+        return d[k] * xc + a1[k] * e[ix[k] & 0xffffu] + a2[k] * e[ix[k] >> 16] +
+               aS[k] * e[iy[k] & 0xffffu] + aN[k] * e[iy[k] >> 16];
+    }
+};
+
+// Zero partials of absent warps and the zero slots; complete after the next group barrier.
+__device__ __forceinline__ void resClear(Shared &S, double *e0, double *e1, int T) {
+    for (int t = threadIdx.x; t < 2 * kResSums * kResMaxWarps; t += T)
+        if ((t & (kResMaxWarps - 1)) >= T / 32)
+            (&S.R.red[0][0][0])[t] = 0.0;
+    if (threadIdx.x == 0)
+        e0[kResCells * T] = e1[kResCells * T] = 0.0;
+}
+
+// Right-Jacobi BiCGSTAB (LinearSolver.hpp:251-345) on the rows K.d, K.aW .. K.aN;
+// K.r holds b - A x0 and r0n its norm; x is updated in place. Called by the working group
+// only; the caller's next CTA barrier makes x and *out visible. (s, s) is summed together
+// with (t, t) and (t, s): one block sum fewer per iteration for at most one matrix product
+// more per solve.
+__device__ __noinline__ void bicgstabRes(double *x, double r0n, int maxIter, double tol,
+                                         LinRes *out) {
+    Shared &S = *reinterpret_cast<Shared *>(rqSmem);
+    const DevClass &C = S.C;
+    const int n = C.n, nw = S.resWarps, T = nw * 32;
+    double *e0 = reinterpret_cast<double *>(rqSmem + kSharedBytes);
+    double *e1 = e0 + resExchange(n) / 2;
+    LinRes res{0, 0.0, r0n, false};
+    if (r0n < 1e-30) {
+        res.converged = true;
+        if (threadIdx.x == 0)
+            *out = res;
+        return;
+    }
+    ResRows A;
+    double r[kResCells], rh[kResCells], p[kResCells], v[kResCells], xv[kResCells];
+    A.load(C, S.K64, T);
+    double acc[1] = {0.0};
+#pragma unroll
+    for (int k = 0; k < kResCells; ++k) {
+        const int c = threadIdx.x + k * T;
+        p[k] = v[k] = 0.0;
+        r[k] = c < n ? S.K64.r[c] : 0.0;
+        xv[k] = c < n ? x[c] : 0.0;
+        rh[k] = r[k];
+        acc[0] += r[k] * r[k];
+    }
+    resClear(S, e0, e1, T);
+    int rp = 0;
+    sumRes<1>(acc, rp, nw);
+    const double bound2 = (tol * r0n) * (tol * r0n);
+    double rhoN = acc[0], rhoInv = 1, alphaOm = 1, omega = 1;
+    double last = r0n * r0n;
+    for (int it = 0; it < maxIter; ++it) {
+        if (fabs(rhoN) < 1e-30)
+            break;
+        const double beta = (rhoN * rhoInv) * alphaOm;
+#pragma unroll
+        for (int k = 0; k < kResCells; ++k) {
+            p[k] = r[k] + beta * (p[k] - omega * v[k]);
+            e0[threadIdx.x + k * T] = p[k] * A.rd[k];
+        }
+        groupSync(T);
+        double s1[1] = {0.0};
+#pragma unroll
+        for (int k = 0; k < kResCells; ++k) {
+            v[k] = A.times(k, p[k] * A.rd[k], e0);
+            s1[0] += rh[k] * v[k];
+        }
+        rhoInv = recip(rhoN + 1e-30);
+        sumRes<1>(s1, rp, nw);
+        if (fabs(s1[0]) < 1e-30)
+            break;
+        const double alpha = quot(rhoN, s1[0]);
+        double s3[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < kResCells; ++k) { // r holds s until the iteration's end
+            r[k] -= alpha * v[k];
+            e1[threadIdx.x + k * T] = r[k] * A.rd[k];
+            s3[2] += r[k] * r[k];
+        }
+        groupSync(T);
+        double t[kResCells];
+#pragma unroll
+        for (int k = 0; k < kResCells; ++k) {
+            t[k] = A.times(k, r[k] * A.rd[k], e1);
+            s3[0] += t[k] * t[k];
+            s3[1] += t[k] * r[k];
+        }
+        sumRes<3>(s3, rp, nw);
+        res.iterations = it + 1;
+        last = s3[2];
+        if (dropped(s3[2], bound2, r0n, tol)) {
+#pragma unroll
+            for (int k = 0; k < kResCells; ++k)
+                xv[k] += alpha * (p[k] * A.rd[k]);
+            res.converged = true;
+            break;
+        }
+        omega = (s3[0] > 1e-30) ? quot(s3[1], s3[0]) : 0.0;
+        double s4[2] = {0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < kResCells; ++k) {
+            xv[k] += alpha * (p[k] * A.rd[k]) + omega * (r[k] * A.rd[k]);
+            r[k] -= omega * t[k];
+            s4[0] += r[k] * r[k];
+            s4[1] += rh[k] * r[k];
+        }
+        alphaOm = quot(alpha, omega + 1e-30);
+        sumRes<2>(s4, rp, nw);
+        last = s4[0];
+        if (dropped(s4[0], bound2, r0n, tol)) {
+            res.converged = true;
+            break;
+        }
+        if (fabs(omega) < 1e-30)
+            break;
+        rhoN = s4[1];
+    }
+#pragma unroll
+    for (int k = 0; k < kResCells; ++k) {
+        const int c = threadIdx.x + k * T;
+        if (c < n)
+            x[c] = xv[k];
+    }
+    if (threadIdx.x == 0) {
+        res.finalRes = sqrt(last) / r0n;
+        *out = res;
+    }
+}
+
+// Levels of the resident V-cycle (thread 0, from carve): vectors in the arena, operator
+// values where the refresh writes them, and the constant tables and the coarsest inverse
+// in the arena as far as place() finds room, in the order of their use per byte.
+template <typename Place> __device__ void resPlace(Shared &S, Place place) {
+    const DevClass &C = S.C;
+    const int L = C.nlev;
+    for (int l = 0; l < L; ++l) {
+        const DevAmgLevel &F = C.lev[l];
+        ResLevel &R = S.RL[l];
+        double *v = S.W.amgVec + F.vecOff;
+        R.n = F.n;
+        R.sh = 0;
+        while (R.sh < 5 && (2 << R.sh) * F.n <= static_cast<int>(blockDim.x) &&
+               (2 << R.sh) <= F.n)
+            ++R.sh;
+        R.b = v;
+        R.x = v + F.n;
+        R.r = v + 3 * F.n;
+        R.rd = v + 4 * F.n;
+        R.aw = F.width;
+        R.av = S.W.amgVal + F.valOff;
+        R.ac = F.ecol16;
+        R.pw = l + 1 < L ? F.pw : 0;
+        R.pc = F.pcol16;
+        R.pv = F.pval;
+        R.rw = l > 0 ? C.lev[l - 1].rw : 0;
+        R.rc = l > 0 ? C.lev[l - 1].rcol16 : nullptr;
+        R.rv = l > 0 ? C.lev[l - 1].rval : nullptr;
+    }
+    auto put16 = [&](const uint16_t *&p, int cnt) {
+        if (double *q = place((cnt + 3) / 4))
+            p = reinterpret_cast<const uint16_t *>(q);
+    };
+    auto put = [&](const double *&p, int cnt) {
+        if (double *q = place(cnt))
+            p = q;
+    };
+    for (int l = L - 2; l >= 1; --l)
+        put16(S.RL[l].ac, S.RL[l].aw * S.RL[l].n);
+    for (int l = L - 1; l >= 0; --l) {
+        ResLevel &R = S.RL[l];
+        if (l > 0) {
+            put16(R.rc, R.rw * R.n);
+            put(R.rv, R.rw * R.n);
+        }
+        if (l + 1 < L) {
+            put16(R.pc, R.pw * R.n);
+            put(R.pv, R.pw * R.n);
+        }
+    }
+    const int m = S.RL[L - 1].n, seg = 1 << S.RL[L - 1].sh;
+    S.resInv = place(static_cast<long>((m + seg - 1) / seg) * m * seg);
+}
+
+// Copies the constant tables that resPlace put into the arena (all threads).
+__device__ __noinline__ void resTables(Shared &S) {
+    const DevClass &C = S.C;
+    const int L = C.nlev, t0 = threadIdx.x, ts = blockDim.x;
+    auto copy = [&](auto *dst, const auto *src, int cnt) {
+        if (dst != src)
+            for (int e = t0; e < cnt; e += ts)
+                const_cast<std::remove_const_t<std::remove_reference_t<decltype(*dst)>> *>(dst)[e] =
+                    src[e];
+    };
+    for (int l = 0; l < L; ++l) {
+        const ResLevel &R = S.RL[l];
+        const DevAmgLevel &F = C.lev[l];
+        if (l > 0 && l + 1 < L)
+            copy(R.ac, F.ecol16, R.aw * R.n);
+        if (l + 1 < L) {
+            copy(R.pc, F.pcol16, R.pw * R.n);
+            copy(R.pv, F.pval, R.pw * R.n);
+        }
+        if (l > 0) {
+            copy(R.rc, C.lev[l - 1].rcol16, R.rw * R.n);
+            copy(R.rv, C.lev[l - 1].rval, R.rw * R.n);
+        }
+    }
+    __syncthreads();
+}
+
+// The inverse of the coarsest level (amgRefreshT) in the order in which coarseRes reads
+// it: entry u * (m seg) + t is row t / seg, column t % seg + u seg.
+__device__ __noinline__ void denseOrder(Shared &S) {
+    const ResLevel &R = S.RL[S.C.nlev - 1];
+    const int m = R.n, seg = 1 << R.sh, w = m * seg;
+    const double *inv = m <= 32 ? S.coarse : S.W.dense0 + m;
+    const int ld = m <= 32 ? m : 2 * m;
+    for (int e = threadIdx.x; e < (m + seg - 1) / seg * w; e += blockDim.x) {
+        const int u = e / w, t = e - u * w, i = t >> R.sh, k = t - (i << R.sh) + u * seg;
+        if (k < m)
+            S.resInv[e] = inv[i * ld + k];
+    }
+    __syncthreads();
+}
+
+// One row of an ELL table (column-major, 16-bit columns) times the gathered vector; padding
+// entries have value 0 and column 0. Columns and values of up to eight entries are loaded
+// before the first of them is used.
+template <int W>
+__device__ __forceinline__ double rowFix(const uint16_t *cols, const double *val,
+                                         const double *vec, unsigned stride, unsigned row) {
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int k = 0; k < W; k += 8) {
+        unsigned c[8];
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8 && k + u < W; ++u) {
+            c[u] = cols[(k + u) * stride + row];
+            v[u] = val[(k + u) * stride + row];
+        }
+#pragma unroll
+        for (int u = 0; u < 8 && k + u < W; ++u)
+            (u & 1 ? s1 : s0) += v[u] * vec[c[u]];
+    }
+    return s0 + s1;
+}
+// The widths of the hierarchies of 3 to 5 cells' periodic width get code of their own: a
+// phase of the V-cycle is bound by the instructions it issues, and a loop with a run-time
+// width and bounds checks takes 5 times as many (1600 cycles for 192 rows of 11 entries).
+__device__ __forceinline__ double rowRes(const uint16_t *cols, const double *val,
+                                         const double *vec, int width, unsigned stride,
+                                         unsigned row) {
+    switch (width) {
+    case 2: return rowFix<2>(cols, val, vec, stride, row);
+    case 4: return rowFix<4>(cols, val, vec, stride, row);
+    case 11: return rowFix<11>(cols, val, vec, stride, row);
+    case 15: return rowFix<15>(cols, val, vec, stride, row);
+    default: break;
+    }
+    double s = 0.0;
+    int k = 0;
+    for (; k + 4 <= width; k += 4)
+        s += rowFix<4>(cols + k * stride, val + k * stride, vec, stride, row);
+    for (; k < width; ++k)
+        s += val[k * stride + row] * vec[cols[k * stride + row]];
+    return s;
+}
+
+// The coarse levels of one V-cycle with one damped-Jacobi sweep (vcycleT): the level-0
+// residual in rr0 is restricted, and level 1's solution is left in its x. All threads of
+// the CTA take part; the caller's barrier precedes.
+__device__ __forceinline__ void coarseRes(Shared &S, const double *rr0) {
+    const DevClass &C = S.C;
+    const int L = C.nlev;
+    const double om = C.amgW, al = C.amgAlpha;
+    const double *fr = rr0; // residual of the level above
+    const int t0 = threadIdx.x, ts = blockDim.x;
+    for (int l = 1; l + 1 < L; ++l) {
+        const ResLevel R = S.RL[l];
+        for (int i = t0; i < R.n; i += ts) {
+            const double bi = rowRes(R.rc, R.rv, fr, R.rw, R.n, i);
+            R.b[i] = bi;
+            R.x[i] = om * bi * R.rd[i];
+        }
+        __syncthreads();
+        for (int i = t0; i < R.n; i += ts)
+            R.r[i] = R.b[i] - rowRes(R.ac, R.av, R.x, R.aw, R.n, i);
+        __syncthreads();
+        fr = R.r;
+    }
+    {
+        const ResLevel R = S.RL[L - 1];
+        for (int i = t0; i < R.n; i += ts)
+            R.b[i] = L == 1 ? rr0[i] : rowRes(R.rc, R.rv, fr, R.rw, R.n, i);
+        __syncthreads();
+        // 1 << sh threads per row of the dense inverse
+        const int seg = 1 << R.sh, w = R.n << R.sh, j = t0 & (seg - 1);
+        for (int base = 0; base < w; base += ts) {
+            const int t = base + t0;
+            double s0 = 0.0, s1 = 0.0;
+            if (t < w) {
+                const double *q = S.resInv + t, *v = R.b + j;
+                int k = j;
+                for (; k + 7 * seg < R.n; k += 8 * seg, q += 8 * w, v += 8 * seg) {
+                    double a[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        a[u] = q[u * w];
+#pragma unroll
+                    for (int u = 0; u < 8; u += 2) {
+                        s0 += a[u] * v[u * seg];
+                        s1 += a[u + 1] * v[(u + 1) * seg];
+                    }
+                }
+                for (; k < R.n; k += seg, q += w, v += seg)
+                    s0 += q[0] * v[0];
+            }
+            s0 += s1;
+            for (int o = seg >> 1; o > 0; o >>= 1)
+                s0 += __shfl_xor_sync(FULL, s0, o);
+            if (j == 0 && t < w)
+                R.x[t >> R.sh] = s0;
+        }
+        __syncthreads();
+    }
+    for (int l = L - 2; l >= 1; --l) {
+        const ResLevel R = S.RL[l];
+        const double *xc = S.RL[l + 1].x;
+        for (int i = t0; i < R.n; i += ts)
+            R.r[i] = R.x[i] + al * rowRes(R.pc, R.pv, xc, R.pw, R.n, i);
+        __syncthreads();
+        for (int i = t0; i < R.n; i += ts)
+            R.x[i] = R.r[i] + om * (R.b[i] - rowRes(R.ac, R.av, R.r, R.aw, R.n, i)) * R.rd[i];
+        __syncthreads();
+    }
+}
+
+// PCG (LinearSolver.hpp:184-246 / :908-982) from x = 0, with the V-cycle of one sweep per
+// level or the Jacobi preconditioner; K64.r holds b and r0n its norm. The working group
+// holds the finest level in registers; all threads of the CTA run the coarse levels. The
+// caller's next CTA barrier makes x and *out visible.
+// What bounds it: the instructions that each of its 13 to 21 phases issues. Measured on a
+// B200, cycles of the pressure solve per PCG iteration: 19 800 / 39 200 / 62 900 at 384 /
+// 768 / 1536 cells, against 23 900 / 53 500 / 95 000 of pcgT and vcycleT.
+template <bool AMG>
+__device__ __noinline__ void pcgRes(double *x, double r0n, int maxIter, double tol, LinRes *out) {
+    Shared &S = *reinterpret_cast<Shared *>(rqSmem);
+    const DevClass &C = S.C;
+    const int n = C.n, nw = S.resWarps, T = nw * 32;
+    double *e0 = reinterpret_cast<double *>(rqSmem + kSharedBytes);
+    double *e1 = e0 + resExchange(n) / 2;
+    LinRes res{0, 0.0, r0n, false};
+    const bool mine = static_cast<int>(threadIdx.x) < T;
+    if (r0n < 1e-30) {
+        res.converged = true;
+        if (threadIdx.x == 0)
+            *out = res;
+        return;
+    }
+    const int L = C.nlev;
+    const double om = C.amgW, al = C.amgAlpha;
+    const double bound2 = (tol * r0n) * (tol * r0n);
+    ResRows A;
+    double r[kResCells], p[kResCells], xv[kResCells];
+    int rp = 0;
+    double rz = 0.0;
+    if (mine) {
+        A.load(C, S.K64, T);
+#pragma unroll
+        for (int k = 0; k < kResCells; ++k) {
+            const int c = threadIdx.x + k * T;
+            r[k] = c < n ? S.K64.r[c] : 0.0;
+            p[k] = xv[k] = 0.0;
+        }
+        resClear(S, e0, e1, T);
+    }
+    for (int it = 0;; ++it) {
+        double z[kResCells], q[1] = {0.0};
+        if constexpr (AMG) {
+            if (mine && L > 1) {
+#pragma unroll
+                for (int k = 0; k < kResCells; ++k)
+                    e0[threadIdx.x + k * T] = om * r[k] * A.rd[k];
+                groupSync(T);
+#pragma unroll
+                for (int k = 0; k < kResCells; ++k)
+                    e1[threadIdx.x + k * T] = r[k] - A.times(k, om * r[k] * A.rd[k], e0);
+            } else if (mine) {
+#pragma unroll
+                for (int k = 0; k < kResCells; ++k)
+                    e1[threadIdx.x + k * T] = r[k];
+            }
+            __syncthreads();
+            coarseRes(S, e1);
+        }
+        if (mine) {
+            if (AMG && L > 1) {
+                const ResLevel &R = S.RL[0];
+                const double *xc = S.RL[1].x;
+#pragma unroll
+                for (int k = 0; k < kResCells; ++k) {
+                    const int c = threadIdx.x + k * T;
+                    z[k] = c < n ? rowRes(R.pc, R.pv, xc, R.pw, n, c) : 0.0;
+                }
+#pragma unroll
+                for (int k = 0; k < kResCells; ++k) {
+                    z[k] = om * r[k] * A.rd[k] + al * z[k];
+                    e0[threadIdx.x + k * T] = z[k];
+                }
+                groupSync(T);
+#pragma unroll
+                for (int k = 0; k < kResCells; ++k) {
+                    z[k] += om * (r[k] - A.times(k, z[k], e0)) * A.rd[k];
+                    q[0] += r[k] * z[k];
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < kResCells; ++k) {
+                    const int c = threadIdx.x + k * T;
+                    z[k] = AMG ? (c < n ? S.RL[0].x[c] : 0.0) : r[k] * A.rd[k];
+                    q[0] += r[k] * z[k];
+                }
+            }
+            sumRes<1>(q, rp, nw);
+            const double beta = it == 0 ? 0.0 : q[0] / (rz + 1e-30);
+            rz = q[0];
+            q[0] = 0.0;
+#pragma unroll
+            for (int k = 0; k < kResCells; ++k) {
+                p[k] = z[k] + beta * p[k];
+                e1[threadIdx.x + k * T] = p[k];
+            }
+            groupSync(T);
+            double Ap[kResCells];
+#pragma unroll
+            for (int k = 0; k < kResCells; ++k) {
+                Ap[k] = A.times(k, p[k], e1);
+                q[0] += p[k] * Ap[k];
+            }
+            sumRes<1>(q, rp, nw);
+            bool done = false;
+            if (fabs(q[0]) < 1e-30) {
+                res.breakdown = true;
+                done = true;
+            } else {
+                const double alpha = quot(rz, q[0]);
+                q[0] = 0.0;
+#pragma unroll
+                for (int k = 0; k < kResCells; ++k) {
+                    xv[k] += alpha * p[k];
+                    r[k] -= alpha * Ap[k];
+                    q[0] += r[k] * r[k];
+                }
+                sumRes<1>(q, rp, nw);
+                res.iterations = it + 1;
+                res.finalRes = q[0]; // its square until the end
+                res.converged = dropped(q[0], bound2, r0n, tol);
+                done = res.converged || it + 1 >= maxIter;
+            }
+            if (threadIdx.x == 0)
+                S.resDone = done;
+            if (!AMG && done)
+                break;
+        }
+        if constexpr (AMG) {
+            __syncthreads();
+            if (S.resDone)
+                break;
+        } else if (!mine) {
+            break;
+        }
+    }
+    if (!mine)
+        return;
+#pragma unroll
+    for (int k = 0; k < kResCells; ++k) {
+        const int c = threadIdx.x + k * T;
+        if (c < n)
+            x[c] = xv[k];
+    }
+    if (threadIdx.x == 0) {
+        res.finalRes = sqrt(res.finalRes) / r0n;
+        *out = res;
+    }
+}

@@ -73,6 +73,27 @@ struct LoopState {
     bool established, converged, diverged;
 };
 
+// Shared memory of the resident solvers (rq_resident.cuh): block sums in alternating
+// buffers, up to three values of up to 16 warps.
+constexpr int kResCells = 3;        // cells per thread
+constexpr int kResMaxThreads = 512; // CTA size up to which a thread has 128 registers
+constexpr int kResMaxWarps = 16;
+constexpr int kResSums = 3;
+struct alignas(16) ResShared {
+    double red[2][kResSums][kResMaxWarps];
+};
+
+// One level of the resident V-cycle: its rows, the threads per row of the dense coarsest
+// solve (1 << sh), its operator, the prolongation to it from the next level and the restriction of the
+// level above (widths, 16-bit columns and values in ELL form), and its vectors.
+struct ResLevel {
+    int n, sh, aw, pw, rw, pad;
+    const uint16_t *ac, *pc, *rc;
+    const double *av, *pv, *rv;
+    double *b, *x, *r;
+    const double *rd;
+};
+
 struct Shared {
     DevClass C;
     Work W;
@@ -94,7 +115,16 @@ struct Shared {
                       // on a cold start, the cached solve's on a warm one, then b1)
     double coarse[32 * 32];               // in-place inverse of a coarsest level of <= 32 rows
     LoopState L;                          // the outer loop's scalars (runSolve)
+    ResShared R;                          // block sums of the resident solvers
+    int resWarps;                         // their working warps, 0: the general solvers
+    int resAmg;                           // the V-cycle too (one sweep per level)
+    double *resInv;                       // the coarsest inverse in coarseRes's order
+    int resDone;                          // a PCG solve has ended
+    ResLevel RL[kMaxLevels];              // levels of the resident V-cycle
 };
+
+// dynamic shared memory of every solve kernel: Shared, then the arena
+constexpr size_t kSharedBytes = (sizeof(Shared) + 15) / 16 * 16;
 
 // stage timers, as the reference's momentum / pressure / turbulence timers
 // (rans-uq/include/SIMPLESolver.hpp:293-305): 0 set-up, 1 closure, 2 momentum,
@@ -896,6 +926,8 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
     return rz;
 }
 
+#include "rq_resident.cuh"
+
 // The sweeps of one PCG iteration as functions of their own, so that the PCG loop
 // itself keeps only a few scalars live across the V-cycle call (every value live
 // across a call is saved to and reloaded from local memory around it).
@@ -1192,12 +1224,19 @@ __device__ __noinline__ LinRes mixedSolve(Shared &S, int &rp, double *x64, doubl
     return out;
 }
 
-// Linear-solve dispatch for the precision of the class.
-__device__ __forceinline__ LinRes solveBicg(Shared &S, int &rp, double *x, double r0n, int maxIter,
-                                            double tol) {
-    if (S.C.st.precision == kMixed)
-        return mixedSolve(S, rp, x, r0n, maxIter, tol, kPBicgstab, false);
-    return bicgstabT<double>(S, rp, S.K64, x, r0n, maxIter, tol);
+// Linear-solve dispatch: the resident form where carve() set it up, else by the
+// precision of the class. The result is complete in `out` (shared memory) after the
+// caller's next barrier.
+__device__ __forceinline__ void solveBicg(Shared &S, int &rp, double *x, double r0n, int maxIter,
+                                          double tol, LinRes *out) {
+    if (S.resWarps) {
+        if (static_cast<int>(threadIdx.x) < 32 * S.resWarps)
+            bicgstabRes(x, r0n, maxIter, tol, out);
+        return;
+    }
+    *out = S.C.st.precision == kMixed
+               ? mixedSolve(S, rp, x, r0n, maxIter, tol, kPBicgstab, false)
+               : bicgstabT<double>(S, rp, S.K64, x, r0n, maxIter, tol);
 }
 
 // The AMG coarse values (Galerkin products and the coarsest inverse) are refreshed
@@ -1216,7 +1255,22 @@ __device__ __forceinline__ LinRes solvePressure(Shared &S, int &rp, double *x, d
     const bool refresh = amg && needRefresh;
     LinRes res;
     const bool mixed = S.C.st.precision == kMixed;
-    if (kind == kPBicgstab)
+    if (S.resWarps && (!amg || S.resAmg)) { // the resident forms
+        if (refresh && r0n >= 1e-30) {
+            mark(S, 4);
+            amgRefreshT(S, S.K64);
+            denseOrder(S);
+            mark(S, 5);
+        }
+        if (amg)
+            pcgRes<true>(x, r0n, maxIter, tol, &S.L.resP);
+        else if (kind == kPPcg)
+            pcgRes<false>(x, r0n, maxIter, tol, &S.L.resP);
+        else if (static_cast<int>(threadIdx.x) < 32 * S.resWarps)
+            bicgstabRes(x, r0n, maxIter, tol, &S.L.resP);
+        __syncthreads();
+        res = S.L.resP;
+    } else if (kind == kPBicgstab)
         res = mixed ? mixedSolve(S, rp, x, r0n, maxIter, tol, kind, refresh)
                     : bicgstabT<double>(S, rp, S.K64, x, r0n, maxIter, tol);
     else if (mixed) // FP64 PCG, FP32 AMG V-cycle
@@ -1293,6 +1347,16 @@ __device__ void carve(Shared &S, double *ws, double *arena, long arenaDoubles) {
     Work &W = S.W;
     double *g = ws;
     long used = 0;
+    // the resident solvers where a thread can hold its cells in registers
+    S.resWarps = 0;
+    if (C.st.precision == kFP64 && static_cast<int>(blockDim.x) <= kResMaxThreads &&
+        n <= static_cast<long>(kResCells) * blockDim.x && resExchange(n) <= arenaDoubles) {
+        used = resExchange(n); // the exchange vectors start the arena
+        S.resWarps = resThreads(n) / 32;
+    }
+    // and their V-cycle, whose level vectors come next
+    const long vecs = (C.amgVecs + 31) / 32 * 32;
+    S.resAmg = S.resWarps && C.resAmg && used + vecs <= arenaDoubles;
     auto take = [&](long cnt) {
         const long sz = (cnt + 31) / 32 * 32;
         double *gp = g;
@@ -1302,6 +1366,18 @@ __device__ void carve(Shared &S, double *ws, double *arena, long arenaDoubles) {
             used += sz;
             return sp;
         }
+        return gp;
+    };
+    double *resVec = arena + used;
+    if (S.resAmg)
+        used += vecs;
+    // the general solvers' vectors: never touched where the resident forms cover all solves
+    const bool covered = S.resWarps && (S.resAmg || C.st.pSolver != kPAmg);
+    auto cold = [&](long cnt) {
+        if (!covered)
+            return take(cnt);
+        double *gp = g;
+        g += (cnt + 31) / 32 * 32;
         return gp;
     };
     auto takeF = [&](long cnt) { return reinterpret_cast<float *>(take((cnt + 1) / 2)); };
@@ -1344,22 +1420,32 @@ __device__ void carve(Shared &S, double *ws, double *arena, long arenaDoubles) {
         W.z = take(n);
         W.rd = take(n);
     } else {
-        W.pv = take(n);
-        W.v = take(n);
-        W.ph = take(n);
-        W.s = take(n);
-        W.sh = take(n);
-        W.t = take(n);
-        W.rh = take(n);
-        W.rd = take(n);
+        W.pv = cold(n);
+        W.v = cold(n);
+        W.ph = cold(n);
+        W.s = cold(n);
+        W.sh = cold(n);
+        W.t = cold(n);
+        W.rh = cold(n);
+        W.rd = cold(n);
         // the pressure PCG / V-cycle vectors share storage with the BiCGSTAB-only
         // vectors: the two solvers never run at the same time
         W.z = W.s;
         W.xa = W.t;
         W.xb = W.sh;
         W.rr = W.rh;
-        W.amgVec = take(C.amgVecs); // tier 2: AMG (vectors first: touched more often)
+        // tier 2: AMG (vectors first: touched more often)
+        W.amgVec = S.resAmg ? resVec : take(C.amgVecs);
         W.amgVal = take(C.amgVals);
+        if (S.resAmg)
+            resPlace(S, [&](long cnt) {
+                const long sz = (cnt + 31) / 32 * 32;
+                if (used + sz > arenaDoubles)
+                    return static_cast<double *>(nullptr);
+                double *sp = arena + used;
+                used += sz;
+                return sp;
+            });
     }
     // tier 3: solved fields and assembly inputs
     W.pp = take(n);
@@ -1399,6 +1485,8 @@ __device__ void carve(Shared &S, double *ws, double *arena, long arenaDoubles) {
     W.wOld = take(n);
     W.dense0 = take(2L * m * m); // [A | I] ping-pong of a coarsest level above 32 rows
     W.dense1 = take(2L * m * m);
+    if (S.resAmg && !S.resInv)
+        S.resInv = W.dense1;
     if (mixed) {
         W.ph = W.s = W.sh = W.t = W.rh = nullptr;
         W.xa = W.xb = W.rr = W.amgVec = W.amgVal = nullptr;
@@ -2326,7 +2414,7 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
             momRes = comp == 0 ? acc[0] : dmax(momRes, acc[0]);
             if (comp == 0)
                 momScale = acc[2];
-            resU[comp] = solveBicg(S, rp, U, sqrt(acc[1]), st.innerIter, st.innerTol);
+            solveBicg(S, rp, U, sqrt(acc[1]), st.innerIter, st.innerTol, &resU[comp]);
             if (threadIdx.x == 0)
                 S.innerKrylov += resU[comp].iterations;
             __syncthreads();
@@ -2374,11 +2462,8 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
                 // so the in-place update below cannot race with a neighbour's read)
                 phTurbResidual(S, eq, acc);
                 blockSum<1>(acc, S, rp);
-                LinRes rr = solveBicg(S, rp, X, sqrt(acc[0]), st.innerIter, st.innerTol);
-                if (eq == 0)
-                    resK = rr;
-                else
-                    resW = rr;
+                LinRes &rr = eq == 0 ? resK : resW;
+                solveBicg(S, rp, X, sqrt(acc[0]), st.innerIter, st.innerTol, &rr);
                 if (threadIdx.x == 0)
                     S.innerKrylov += rr.iterations;
                 __syncthreads();
@@ -2621,6 +2706,8 @@ __device__ void runJob(Shared &S, const DevJob &job, double *ws, double *arena, 
             carve(S, ws, arena, arenaDoubles);
     }
     __syncthreads();
+    if (S.admitted && S.resAmg)
+        resTables(S);
     if (S.admitted) {
         runSolve(S, job);
     } else {
@@ -2660,7 +2747,7 @@ __global__ void __launch_bounds__(NT) solveKernel(const DevJob *jobs, int njobs,
                                                   double *wsBase, long wsStride, int arenaDoubles) {
     extern __shared__ __align__(16) unsigned char smemRaw[];
     Shared &S = *reinterpret_cast<Shared *>(smemRaw);
-    double *arena = reinterpret_cast<double *>(smemRaw + ((sizeof(Shared) + 15) / 16) * 16);
+    double *arena = reinterpret_cast<double *>(smemRaw + kSharedBytes);
     double *ws = wsBase + wsStride * blockIdx.x;
     for (;;) {
         if (threadIdx.x == 0)
@@ -2688,7 +2775,7 @@ __global__ void __launch_bounds__(NT) serveKernel(ServeQueue q, double *wsBase, 
                                                   int arenaDoubles) {
     extern __shared__ __align__(16) unsigned char smemRaw[];
     Shared &S = *reinterpret_cast<Shared *>(smemRaw);
-    double *arena = reinterpret_cast<double *>(smemRaw + ((sizeof(Shared) + 15) / 16) * 16);
+    double *arena = reinterpret_cast<double *>(smemRaw + kSharedBytes);
     double *ws = wsBase + wsStride * blockIdx.x;
     for (;;) {
         if (threadIdx.x == 0) {
@@ -2735,50 +2822,72 @@ __global__ void __launch_bounds__(NT) serveKernel(ServeQueue q, double *wsBase, 
 }
 
 // ---------------------------------------------------------------- allocation-free single solve
-// Workspace of rq_evaluate_noalloc: one solve's scratch in a fixed device array
-// that the module owns, so that the call itself needs no device allocation. It
-// lives on every GPU that loads this library until the process exits.
-constexpr long kNoAllocScratchDoubles = 1L << 20; // 8 MiB
-static __device__ __align__(256) double g_noallocScratch[kNoAllocScratchDoubles];
-
 // One job passed by value (no job array, no queue counter), solved by one CTA in
 // the scratch array.
 template <int NT>
 __global__ void __launch_bounds__(NT) solveOneKernel(DevJob job, double *ws, int arenaDoubles) {
     extern __shared__ __align__(16) unsigned char smemRaw[];
     Shared &S = *reinterpret_cast<Shared *>(smemRaw);
-    double *arena = reinterpret_cast<double *>(smemRaw + ((sizeof(Shared) + 15) / 16) * 16);
+    double *arena = reinterpret_cast<double *>(smemRaw + kSharedBytes);
     if (threadIdx.x == 0)
         S.jd = job;
     __syncthreads();
     runJob(S, S.jd, ws, arena, arenaDoubles);
 }
 
-size_t solveSharedBytes() { return ((sizeof(Shared) + 15) / 16) * 16; }
+// The kernels of one CTA size. This file is compiled once per CTA size with RQ_CTA set
+// (the phases are separate functions that ptxas allocates for each kernel's register
+// budget, so one object for all sizes would compile serially), and once without for the
+// host entry points.
+enum SolveEntry { kEntrySolve = 0, kEntryServe = 1, kEntryOne = 2 };
+template <int NT> void *solveEntry(int kind);
+
+#ifdef RQ_CTA
+template <> void *solveEntry<RQ_CTA>(int kind) {
+    switch (kind) {
+    case kEntrySolve: return reinterpret_cast<void *>(&solveKernel<RQ_CTA>);
+#if RQ_CTA >= 256
+    case kEntryServe: return reinterpret_cast<void *>(&serveKernel<RQ_CTA>);
+#endif
+    case kEntryOne: return reinterpret_cast<void *>(&solveOneKernel<RQ_CTA>);
+    default: return nullptr;
+    }
+}
+#else
+template <> void *solveEntry<64>(int);
+template <> void *solveEntry<128>(int);
+template <> void *solveEntry<256>(int);
+template <> void *solveEntry<512>(int);
+template <> void *solveEntry<768>(int);
+template <> void *solveEntry<1024>(int);
+
+// Workspace of rq_evaluate_noalloc: one solve's scratch in a fixed device array
+// that the module owns, so that the call itself needs no device allocation. It
+// lives on every GPU that loads this library until the process exits.
+constexpr long kNoAllocScratchDoubles = 1L << 20; // 8 MiB
+static __device__ __align__(256) double g_noallocScratch[kNoAllocScratchDoubles];
+
+size_t solveSharedBytes() { return kSharedBytes; }
+long residentDoubles(const DevClass &C) {
+    if (C.n > kResCells * kResMaxThreads)
+        return 0;
+    return resExchange(C.n) + (C.resAmg ? (C.amgVecs + 31) / 32 * 32 : 0);
+}
 
 namespace {
-template <int NT> void *kernelFor() { return reinterpret_cast<void *>(&solveKernel<NT>); }
-template <int NT> void *serveFor() { return reinterpret_cast<void *>(&serveKernel<NT>); }
-void *pick(int block) {
+void *entryOf(int kind, int block) {
     switch (block) {
-    case 64: return kernelFor<64>();
-    case 128: return kernelFor<128>();
-    case 256: return kernelFor<256>();
-    case 512: return kernelFor<512>();
-    case 768: return kernelFor<768>();
-    case 1024: return kernelFor<1024>();
+    case 64: return solveEntry<64>(kind);
+    case 128: return solveEntry<128>(kind);
+    case 256: return solveEntry<256>(kind);
+    case 512: return solveEntry<512>(kind);
+    case 768: return solveEntry<768>(kind);
+    case 1024: return solveEntry<1024>(kind);
     default: return nullptr;
     }
 }
-void *pickServe(int block) {
-    switch (block) {
-    case 256: return serveFor<256>();
-    case 512: return serveFor<512>();
-    case 768: return serveFor<768>();
-    case 1024: return serveFor<1024>();
-    default: return nullptr;
-    }
-}
+void *pick(int block) { return entryOf(kEntrySolve, block); }
+void *pickServe(int block) { return entryOf(kEntryServe, block); }
 } // namespace
 
 bool launchVariantExists(int block) { return pick(block) != nullptr; }
@@ -2853,21 +2962,6 @@ int serveBlocksPerSM(int block, int arenaDoubles) {
 
 long noAllocScratchDoubles() { return kNoAllocScratchDoubles; }
 
-namespace {
-template <int NT> void *oneFor() { return reinterpret_cast<void *>(&solveOneKernel<NT>); }
-void *pickOne(int block) {
-    switch (block) {
-    case 64: return oneFor<64>();
-    case 128: return oneFor<128>();
-    case 256: return oneFor<256>();
-    case 512: return oneFor<512>();
-    case 768: return oneFor<768>();
-    case 1024: return oneFor<1024>();
-    default: return nullptr;
-    }
-}
-} // namespace
-
 // The device address of the scratch array on the current device. The host-side name
 // of a __device__ array is only a stand-in, not an address a kernel may use, so it is
 // looked up with cudaGetSymbolAddress (no allocation; the first lookup on a device
@@ -2887,7 +2981,7 @@ cudaError_t launchSolveNoAlloc(const DevJob &job, double *scratch, int block, in
     if (!scratch)
         return cudaErrorInvalidDevicePointer;
     double *ws = scratch;
-    void *fn = pickOne(block);
+    void *fn = entryOf(kEntryOne, block);
     if (!fn)
         return cudaErrorInvalidConfiguration;
     const size_t smem = solveSharedBytes() + sizeof(double) * static_cast<size_t>(arenaDoubles);
@@ -2902,5 +2996,7 @@ cudaError_t launchSolveNoAlloc(const DevJob &job, double *scratch, int block, in
         return e;
     return cudaGetLastError();
 }
+
+#endif // RQ_CTA
 
 } // namespace rq
