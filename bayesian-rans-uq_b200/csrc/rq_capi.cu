@@ -42,15 +42,55 @@ int arenaDoublesFor(long wsDoubles, int knobKb, int nmax, long resident) {
 }
 
 void runOneJob(rq_problem &p, const rq::DevJob &job) {
-    const int arena = chooseArena({&p});
     p.dJobs.ensure(sizeof(rq::DevJob));
     p.dWs.ensure(sizeof(double) * p.cls.wsDoubles);
     p.dCounter.ensure(sizeof(int));
     check(cudaMemcpy(p.dJobs.p, &job, sizeof(rq::DevJob), cudaMemcpyHostToDevice), "job");
     check(cudaMemset(p.dCounter.p, 0, sizeof(int)), "counter");
     check(rq::launchSolve(p.dJobs.as<rq::DevJob>(), 1, p.dCounter.as<int>(), p.dWs.as<double>(),
-                          p.cls.wsDoubles, 1, p.block, arena, nullptr),
+                          p.cls.wsDoubles, 1, shapeOf(p, p.block, p.arenaKb), nullptr),
           "solve launch");
+}
+
+// Shared-memory arena of a cluster's CTA, in doubles: the vectors of the levels that it runs
+// whole, their tables and operator values, and the coarsest inverse (resPlace), as far as
+// they fit.
+long clusterArena(const rq::DevClass &C) {
+    long need = pad32(C.locDoubles);
+    auto table = [&](int width, int rows) {
+        const long cnt = width * pad32(rows);
+        need += pad32((cnt + 3) / 4) + pad32(cnt);
+    };
+    for (int l = C.locLevel; l < C.nlev; ++l) {
+        table(C.lev[l].width, C.lev[l].n);
+        if (l > 0)
+            table(C.lev[l - 1].rw, C.lev[l].n);
+        if (l + 1 < C.nlev)
+            table(C.lev[l].pw, C.lev[l].n);
+    }
+    const long m = C.lev[C.nlev - 1].n;
+    need += pad32(2 * m * m);
+    return std::min(need, (maxSmemOptin() - static_cast<long>(rq::clusterSharedBytes())) / 256 * 32);
+}
+
+// CTAs per solve, by the class's size alone, so that a row's result does not depend on the
+// batch it is solved in. Classes above 1536 cells at the default CTA size and arena rule
+// take a cluster of 4 (8 from 32768 cells). Measured on a B200, ms per call with 4 / 8 CTAs
+// per solve (one CTA: 92, 171): 8 draws of 100 x 50 cells 45 / 38, 8 draws of 200 x 100
+// 38 / 28, but 32 draws of 200 x 100 51 / 85: 36 clusters of 4 fit the GPU at once, only 14
+// of 8. 400 x 200 cells: 14.5 / 8.8 ms per outer iteration.
+int clusterOf(const rq_problem &p, int block, int arenaKb) {
+    if (p.mesh.n <= 1536 || block != 768 || arenaKb >= 0 || p.cls.locDoubles > clusterArena(p.cls))
+        return 1;
+    return p.mesh.n < 32768 ? 4 : 8;
+}
+
+rq::LaunchShape shapeOf(const rq_problem &p, int block, int arenaKb) {
+    const int cluster = clusterOf(p, block, arenaKb);
+    if (cluster > 1)
+        return {block, static_cast<int>(clusterArena(p.cls)), cluster};
+    return {block,
+            arenaDoublesFor(p.cls.wsDoubles, arenaKb, p.mesh.n, rq::residentDoubles(p.cls)), 1};
 }
 
 int chooseArena(const std::vector<const rq_problem *> &probs) {
@@ -268,7 +308,7 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
     if (h.coarseN() > rq::kMaxCoarse)
         throw RqError(RQ_E_UNSUPPORTED, "coarsest AMG level above 128 rows");
     C.nlev = L;
-    C.resAmg = h.sweeps == 1 && m.n <= 65535;
+    C.resAmg = m.n <= 65535;
     // 16-bit columns (padding: column 0), packed into the int32 upload
     auto addH = [&](const uint16_t **slot, const std::vector<int> &v) {
         std::vector<int32_t> packed((v.size() + 1) / 2, 0);
@@ -277,7 +317,7 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
             q[k] = static_cast<uint16_t>(std::max(v[k], 0));
         addI(reinterpret_cast<const int32_t **>(slot), packed);
     };
-    // ELL slots of levels >= 1: CSR entry k of row i -> (k - ptr[i]) * n + i
+    // ELL slots of levels >= 1 (DevAmgLevel): CSR entry k of row i
     std::vector<std::vector<int>> slotOf(L), entryOf(L);
     std::vector<int> width(L, 0);
     for (int l = 1; l < L; ++l) {
@@ -285,10 +325,10 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
         for (int i = 0; i < Lv.n; ++i)
             width[l] = std::max(width[l], Lv.ptr[i + 1] - Lv.ptr[i]);
         slotOf[l].resize(Lv.col.size());
-        entryOf[l].assign(static_cast<size_t>(width[l]) * Lv.n, -1);
+        entryOf[l].assign(static_cast<size_t>(width[l]) * pad32(Lv.n), -1);
         for (int i = 0; i < Lv.n; ++i)
             for (int k = Lv.ptr[i]; k < Lv.ptr[i + 1]; ++k) {
-                const int slot = (k - Lv.ptr[i]) * Lv.n + i;
+                const int slot = rq::ellRow(i, width[l]) + 32 * (k - Lv.ptr[i]);
                 slotOf[l][k] = slot;
                 entryOf[l][slot] = k;
             }
@@ -299,7 +339,7 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
         rq::DevAmgLevel &dl = C.lev[l];
         dl.n = Lv.n;
         dl.width = l > 0 ? width[l] : 0;
-        dl.nnz = l > 0 ? width[l] * Lv.n : 0;
+        dl.nnz = l > 0 ? width[l] * static_cast<int>(pad32(Lv.n)) : 0;
         dl.valOff = valOff;
         dl.vecOff = vecOff;
         if (l > 0) {
@@ -318,19 +358,19 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
         if (l > 0 || L == 1)
             vecOff += static_cast<int>(pad32(5L * Lv.n)); // b, xa, xb, r, 1/diag
         if (l + 1 < L) {
-            // transfer operators as ELL (slot k * rows + row, -1 padding)
+            // transfer operators as ELL (the same slots, -1 padding)
             auto ell = [](const std::vector<int> &ptr, const std::vector<int> &col,
                           const std::vector<double> &val, int rows, int &w,
                           std::vector<int> &ec, std::vector<double> &ev) {
                 w = 0;
                 for (int r = 0; r < rows; ++r)
                     w = std::max(w, ptr[r + 1] - ptr[r]);
-                ec.assign(static_cast<size_t>(w) * rows, -1);
-                ev.assign(static_cast<size_t>(w) * rows, 0.0);
+                ec.assign(static_cast<size_t>(w) * pad32(rows), -1);
+                ev.assign(static_cast<size_t>(w) * pad32(rows), 0.0);
                 for (int r = 0; r < rows; ++r)
                     for (int k = ptr[r]; k < ptr[r + 1]; ++k) {
-                        ec[static_cast<size_t>(k - ptr[r]) * rows + r] = col[k];
-                        ev[static_cast<size_t>(k - ptr[r]) * rows + r] = val[k];
+                        ec[rq::ellRow(r, w) + 32 * (k - ptr[r])] = col[k];
+                        ev[rq::ellRow(r, w) + 32 * (k - ptr[r])] = val[k];
                     }
             };
             const int nc = h.lev[l + 1].n;
@@ -347,7 +387,7 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
             }
             addD(&dl.rval, rv);
             // gather lists in the next level's slot order; sources of level >= 1 as slots
-            const int ns = width[l + 1] * nc;
+            const int ns = width[l + 1] * static_cast<int>(pad32(nc));
             std::vector<int> gp(ns + 1, 0), gs;
             std::vector<double> gw;
             for (int slot = 0; slot < ns; ++slot) {
@@ -369,6 +409,10 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
     C.amgSweeps = h.sweeps;
     C.amgVals = valOff;
     C.amgVecs = vecOff;
+    C.locLevel = L;
+    while (C.locLevel > 1 && C.lev[C.locLevel - 1].n <= rq::kLocalRows)
+        --C.locLevel;
+    C.locDoubles = C.locLevel < L ? vecOff - C.lev[C.locLevel].vecOff : 0;
     C.nActive = static_cast<int32_t>(P.active.size());
     for (int a = 0; a < 11; ++a) {
         C.active[a] = a < C.nActive ? P.active[a] : 0;
@@ -424,14 +468,14 @@ void launchClass(rq_problem &P, const std::vector<int> &rows, const double *thet
         j.clock = clockDev ? clockDev + 12L * r : nullptr;
     }
     const long wsStride = P.cls.wsDoubles;
-    const int arena = chooseArena({&P});
+    const rq::LaunchShape shape = shapeOf(P, P.block, P.arenaKb);
     int dev = 0, sms = 1;
     check(cudaGetDevice(&dev), "cudaGetDevice");
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attribute");
-    const int perSM = rq::solveBlocksPerSM(P.block, arena);
-    if (perSM < 1)
+    const int atOnce = rq::concurrentSolves(shape, sms);
+    if (atOnce < 1)
         throw RqError(RQ_E_CUDA, "solve kernel does not fit on an SM with this arena");
-    const int grid = std::max(1, std::min(n, sms * perSM));
+    const int grid = std::max(1, std::min(n, atOnce));
     P.dJobs.ensure(sizeof(rq::DevJob) * n);
     P.dWs.ensure(sizeof(double) * wsStride * grid);
     P.dCounter.ensure(sizeof(int));
@@ -439,7 +483,7 @@ void launchClass(rq_problem &P, const std::vector<int> &rows, const double *thet
                           stream), "jobs");
     check(cudaMemsetAsync(P.dCounter.p, 0, sizeof(int), stream), "counter");
     check(rq::launchSolve(P.dJobs.as<rq::DevJob>(), n, P.dCounter.as<int>(), P.dWs.as<double>(),
-                          wsStride, grid, P.block, arena, stream),
+                          wsStride, grid, shape, stream),
           "solve launch");
 }
 
@@ -636,9 +680,7 @@ int rq_problem_set_launch(rq_problem *p, const rq_launch_shape *shape) {
         if (shape->arena_kb < -1)
             throw std::invalid_argument("arena_kb must be -1 (default rule), 0 or positive");
         std::lock_guard<std::mutex> lock(p->mu);
-        const int arena = arenaDoublesFor(p->cls.wsDoubles, shape->arena_kb, p->mesh.n,
-                                         rq::residentDoubles(p->cls));
-        if (rq::solveBlocksPerSM(shape->block_threads, arena) < 1)
+        if (rq::concurrentSolves(shapeOf(*p, shape->block_threads, shape->arena_kb), 1) < 1)
             throw std::invalid_argument("this launch shape does not fit on an SM");
         p->block = shape->block_threads;
         p->arenaKb = shape->arena_kb;
@@ -708,13 +750,12 @@ int rq_problem_tune(rq_problem *p, const double *theta, int32_t iters,
             c.us_per_iteration = -1.0;
             if (!rq::launchVariantExists(c.block_threads) || c.arena_kb < -1)
                 continue;
-            const int arena = arenaDoublesFor(p->cls.wsDoubles, c.arena_kb, p->mesh.n,
-                                             rq::residentDoubles(p->cls));
-            if (rq::solveBlocksPerSM(c.block_threads, arena) < 1)
+            const rq::LaunchShape shape = shapeOf(*p, c.block_threads, c.arena_kb);
+            if (rq::concurrentSolves(shape, 1) < 1)
                 continue;
             check(cudaMemset(dCounter.p, 0, sizeof(int)), "counter");
             check(rq::launchSolve(dJob.as<rq::DevJob>(), 1, dCounter.as<int>(), dWs.as<double>(),
-                                  p->cls.wsDoubles, 1, c.block_threads, arena, nullptr),
+                                  p->cls.wsDoubles, 1, shape, nullptr),
                   "tuning launch");
             check(cudaDeviceSynchronize(), "tuning solve");
             long long clk[12];
@@ -988,9 +1029,8 @@ int rq_evaluate_noalloc(rq_problem *p, const double *theta_dev, rq_row_out *row_
         job.theta = theta_dev;
         job.row = reinterpret_cast<rq::RowOut *>(row_dev);
         job.pred = predictions_dev;
-        // shared-memory arena as the batch path sizes it for one class
-        const int arena = arenaDoublesFor(need, p->arenaKb, p->mesh.n, rq::residentDoubles(p->cls));
-        check(rq::launchSolveNoAlloc(job, p->noallocScratch, p->block, arena,
+        // the batch path's launch shape of the class
+        check(rq::launchSolveNoAlloc(job, p->noallocScratch, shapeOf(*p, p->block, p->arenaKb),
                                      static_cast<cudaStream_t>(stream)),
               "allocation-free solve launch");
     });

@@ -151,6 +151,8 @@ int maxSmemOptin();
 // shared-memory arena (doubles) of a launch of these classes
 int arenaDoublesFor(long wsDoubles, int knobKb, int nmax, long resident);
 int chooseArena(const std::vector<const rq_problem *> &probs);
+// the launch shape of one class for a CTA size and arena knob
+rq::LaunchShape shapeOf(const rq_problem &p, int block, int arenaKb);
 inline rq_row_out toRow(const rq::RowOut &o) {
     return rq_row_out{o.status, o.iterations, o.stalled, o.converged, o.loglik, o.finalWorst,
                       o.contractionRate};

@@ -9,6 +9,7 @@
 namespace rq {
 
 constexpr int kMaxLevels = 12;    // AMG levels (the reference allows 20; meshes here need <= 8)
+constexpr int kLocalRows = 1536;  // rows of an AMG level that every CTA of a cluster runs whole
 constexpr int kMaxCoarse = 128;   // rows of the dense coarsest AMG level
 constexpr int kMaxProbes = 64;    // observations per problem
 constexpr int kWindowCap = 64;    // 2 * convergenceWindow samples kept per estimator
@@ -27,15 +28,22 @@ struct DevSettings {
     double kMin, kMax, wMin;
 };
 
-// Levels >= 1 are stored in ELL form: value slot k*n + i holds the k-th entry of
-// row i in column order (a warp reading slot k of 32 consecutive rows touches
-// consecutive addresses); shorter rows are padded with column -1. The transfer
-// operators between level l and level l+1 (nc rows) are ELL too: the prolongation
-// P (slot k*n + i: the k-th coarse row of fine row i and its weight) and the
-// restriction P^T (slot k*nc + I: the k-th fine row of coarse row I and its
+// Levels >= 1 are stored in ELL form in slices of 32 rows: entry k of row i, in column
+// order, is at slot ellRow(i, width) + 32 k (a warp reading entry k of 32 consecutive rows
+// touches consecutive addresses, and the entries of a row lie at constant distances, which
+// the load instructions hold as immediates); shorter rows and the rows that fill the last
+// slice are padded with column -1. The transfer operators between level l and level l+1
+// (nc rows) are ELL too: the prolongation P (entry k of fine row i: its k-th coarse row and
+// the weight) and the restriction P^T (entry k of coarse row I: its k-th fine row and the
 // weight), padded with -1.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int ellRow(int i, int width) {
+    return (i >> 5) * (width << 5) + (i & 31);
+}
 struct DevAmgLevel {
-    int32_t n, nnz;             // rows; value slots (levels >= 1: width x n)
+    int32_t n, nnz;             // rows; value slots (levels >= 1)
     int32_t valOff, vecOff;     // per-solve value / vector offsets (levels >= 1)
     int32_t width, pad;         // ELL width (levels >= 1)
     int32_t pw, rw;             // prolongation / restriction ELL widths (all but the last level)
@@ -69,7 +77,9 @@ struct DevClass {
     DevAmgLevel lev[kMaxLevels];
     double amgW, amgAlpha;     // V-cycle smoother weight, coarse-correction scale
     int32_t amgVals, amgVecs;  // per-solve doubles for coarse values / vectors
-    int32_t resAmg;            // the resident V-cycle applies: one sweep, 16-bit columns set
+    int32_t resAmg;            // the 16-bit columns are set: coarseRes runs the FP64 V-cycle
+    int32_t locLevel, locDoubles; // first level of at most kLocalRows rows (cluster solves run
+                                  // it and the coarser ones per CTA), and their vectors
     int32_t amgSweeps;   // damped-Jacobi sweeps before and after each coarse correction
     int64_t wsDoubles;         // per-solve workspace
     // InferenceParameterSet: active indices, the coefficients filling the rest,

@@ -6,18 +6,23 @@
 
 namespace rq {
 
-size_t solveSharedBytes();
+size_t solveSharedBytes();   // fixed shared memory of a CTA
+size_t clusterSharedBytes(); // the same of the cluster kernels
 // Doubles at the start of the arena that the resident inner solvers of a class need (0:
 // the class is too large for them, rq_resident.cuh).
 long residentDoubles(const DevClass &C);
-// Persistent CTAs: each pulls job indices from *nextJob (zeroed by the caller)
-// until njobs are taken; ws is grid x wsStride doubles of per-CTA workspace.
-// arenaDoubles: shared-memory arena per CTA for the hot arrays (0 = all global).
-// block: a compiled CTA size (64, 128, 256, 512 or 1024).
+// Launch shape of a solve: CTA size (64, 128, 256, 512, 768 or 1024), shared-memory arena
+// per CTA in doubles for the hot arrays (0 = all global), and CTAs per solve (above 1: a
+// thread-block cluster of 768-thread CTAs whose arena holds the small AMG levels).
+struct LaunchShape {
+    int block, arenaDoubles, cluster;
+};
+// Persistent solves: each pulls job indices from *nextJob (zeroed by the caller)
+// until njobs are taken; ws is solves x wsStride doubles of per-solve workspace.
 cudaError_t launchSolve(const DevJob *jobs, int njobs, int *nextJob, double *ws, long wsStride,
-                        int grid, int block, int arenaDoubles, cudaStream_t stream);
-// CTAs of the variant with the given arena that fit on one SM at once (0: does not fit).
-int solveBlocksPerSM(int block, int arenaDoubles);
+                        int solves, const LaunchShape &sh, cudaStream_t stream);
+// Solves of the shape that run at once on a GPU of `sms` SMs (0: does not fit).
+int concurrentSolves(const LaunchShape &sh, int sms);
 bool launchVariantExists(int block);
 // The serving loop (serveKernel): grid persistent CTAs of `block` threads (256, 512
 // or 1024) serving q until it is closed and drained, or until q.idleNs passes
@@ -29,10 +34,10 @@ int normalizeBlock(int block);
 // One solve of one job in the module's fixed scratch array (no device allocation):
 // capacity in doubles, the array's device address on the current device (looked up
 // by cudaGetSymbolAddress at every call of noAllocScratch, which allocates nothing),
-// and the launch (grid of one CTA of `block` threads) on that address.
+// and the launch (one solve of the given shape) on that address.
 long noAllocScratchDoubles();
 cudaError_t noAllocScratch(double **out);
-cudaError_t launchSolveNoAlloc(const DevJob &job, double *scratch, int block, int arenaDoubles,
+cudaError_t launchSolveNoAlloc(const DevJob &job, double *scratch, const LaunchShape &sh,
                                cudaStream_t stream);
 // Posterior weights (rq_stats.cu): one CTA; out = {max, sum of exp, non-finite count}.
 cudaError_t launchWeights(const double *ll, const double *lq, int64_t n, double *w, double *out,

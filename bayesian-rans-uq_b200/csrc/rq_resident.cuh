@@ -264,7 +264,9 @@ __device__ __noinline__ void bicgstabRes(double *x, double r0n, int maxIter, dou
     }
 }
 
-// Levels of the resident V-cycle (thread 0, from carve): vectors in the arena, operator
+__device__ __forceinline__ int up32(int n) { return (n + 31) & ~31; }
+
+// Levels of the V-cycle (thread 0, from carve): vectors, operator
 // values where the refresh writes them, and the constant tables and the coarsest inverse
 // in the arena as far as place() finds room, in the order of their use per byte.
 template <typename Place> __device__ void resPlace(Shared &S, Place place) {
@@ -273,14 +275,16 @@ template <typename Place> __device__ void resPlace(Shared &S, Place place) {
     for (int l = 0; l < L; ++l) {
         const DevAmgLevel &F = C.lev[l];
         ResLevel &R = S.RL[l];
-        double *v = S.W.amgVec + F.vecOff;
+        double *v = localLevel(S, l) ? levelVec<double>(S, S.K64, l) : S.W.amgVec + F.vecOff;
         R.n = F.n;
         R.sh = 0;
         while (R.sh < 5 && (2 << R.sh) * F.n <= static_cast<int>(blockDim.x) &&
                (2 << R.sh) <= F.n)
             ++R.sh;
+        R.vOff = static_cast<int>(reinterpret_cast<unsigned char *>(v) - rqSmem);
         R.b = v;
-        R.x = v + F.n;
+        R.xa = v + F.n;
+        R.x = v + 2 * F.n;
         R.r = v + 3 * F.n;
         R.rd = v + 4 * F.n;
         R.aw = F.width;
@@ -301,21 +305,28 @@ template <typename Place> __device__ void resPlace(Shared &S, Place place) {
         if (double *q = place(cnt))
             p = q;
     };
-    for (int l = L - 2; l >= 1; --l)
-        put16(S.RL[l].ac, S.RL[l].aw * S.RL[l].n);
-    for (int l = L - 1; l >= 0; --l) {
+    // a cluster's CTAs place the levels they run whole, with copies of the operator values
+    const int first = kCluster ? C.locLevel : 0;
+    for (int l = L - 2; l >= 1 && l >= first; --l) {
+        ResLevel &R = S.RL[l];
+        put16(R.ac, R.aw * up32(R.n));
+        if (kCluster)
+            put(R.av, R.aw * up32(R.n));
+    }
+    for (int l = L - 1; l >= first; --l) {
         ResLevel &R = S.RL[l];
         if (l > 0) {
-            put16(R.rc, R.rw * R.n);
-            put(R.rv, R.rw * R.n);
+            put16(R.rc, R.rw * up32(R.n));
+            put(R.rv, R.rw * up32(R.n));
         }
         if (l + 1 < L) {
-            put16(R.pc, R.pw * R.n);
-            put(R.pv, R.pw * R.n);
+            put16(R.pc, R.pw * up32(R.n));
+            put(R.pv, R.pw * up32(R.n));
         }
     }
     const int m = S.RL[L - 1].n, seg = 1 << S.RL[L - 1].sh;
     S.resInv = place(static_cast<long>((m + seg - 1) / seg) * m * seg);
+    S.ownInv = S.resInv != nullptr;
 }
 
 // Copies the constant tables that resPlace put into the arena (all threads).
@@ -332,149 +343,224 @@ __device__ __noinline__ void resTables(Shared &S) {
         const ResLevel &R = S.RL[l];
         const DevAmgLevel &F = C.lev[l];
         if (l > 0 && l + 1 < L)
-            copy(R.ac, F.ecol16, R.aw * R.n);
+            copy(R.ac, F.ecol16, R.aw * up32(R.n));
         if (l + 1 < L) {
-            copy(R.pc, F.pcol16, R.pw * R.n);
-            copy(R.pv, F.pval, R.pw * R.n);
+            copy(R.pc, F.pcol16, R.pw * up32(R.n));
+            copy(R.pv, F.pval, R.pw * up32(R.n));
         }
         if (l > 0) {
-            copy(R.rc, C.lev[l - 1].rcol16, R.rw * R.n);
-            copy(R.rv, C.lev[l - 1].rval, R.rw * R.n);
+            copy(R.rc, C.lev[l - 1].rcol16, R.rw * up32(R.n));
+            copy(R.rv, C.lev[l - 1].rval, R.rw * up32(R.n));
         }
     }
     __syncthreads();
 }
 
-// The inverse of the coarsest level (amgRefreshT) in the order in which coarseRes reads
-// it: entry u * (m seg) + t is row t / seg, column t % seg + u seg.
+// After a refresh: the inverse of the coarsest level in the order in which coarseRes reads
+// it (entry u * (m seg) + t is row t / seg, column t % seg + u seg), and a cluster's copies
+// of the operator values.
 __device__ __noinline__ void denseOrder(Shared &S) {
-    const ResLevel &R = S.RL[S.C.nlev - 1];
-    const int m = R.n, seg = 1 << R.sh, w = m * seg;
-    const double *inv = m <= 32 ? S.coarse : S.W.dense0 + m;
-    const int ld = m <= 32 ? m : 2 * m;
-    for (int e = threadIdx.x; e < (m + seg - 1) / seg * w; e += blockDim.x) {
-        const int u = e / w, t = e - u * w, i = t >> R.sh, k = t - (i << R.sh) + u * seg;
-        if (k < m)
-            S.resInv[e] = inv[i * ld + k];
+    const DevClass &C = S.C;
+    if (S.ownInv || ctaRank() == 0) {
+        const ResLevel &R = S.RL[C.nlev - 1];
+        const int m = R.n, seg = 1 << R.sh, w = m * seg;
+        const double *inv = m <= 32 ? S.coarse : S.W.dense0 + m;
+        const int ld = m <= 32 ? m : 2 * m;
+        for (int e = threadIdx.x; e < (m + seg - 1) / seg * w; e += blockDim.x) {
+            const int u = e / w, t = e - u * w, i = t >> R.sh, k = t - (i << R.sh) + u * seg;
+            if (k < m)
+                S.resInv[e] = inv[i * ld + k];
+        }
     }
-    __syncthreads();
+    if constexpr (kCluster)
+        for (int l = C.locLevel; l + 1 < C.nlev; ++l) {
+            const ResLevel &R = S.RL[l];
+            const double *from = S.W.amgVal + C.lev[l].valOff;
+            double *to = const_cast<double *>(R.av);
+            if (to != from)
+                for (int e = threadIdx.x; e < R.aw * up32(R.n); e += blockDim.x)
+                    to[e] = from[e];
+        }
+    SYNC();
 }
 
-// One row of an ELL table (column-major, 16-bit columns) times the gathered vector; padding
-// entries have value 0 and column 0. Columns and values of up to eight entries are loaded
+// One row of an ELL table (16-bit columns) times the gathered vector; padding
+// entries have value 0 and column 0. Columns and values of up to eleven entries are loaded
 // before the first of them is used.
 template <int W>
 __device__ __forceinline__ double rowFix(const uint16_t *cols, const double *val,
-                                         const double *vec, unsigned stride, unsigned row) {
+                                         const double *vec) {
+    constexpr int B = W <= 11 ? W : 8;
     double s0 = 0.0, s1 = 0.0;
 #pragma unroll
-    for (int k = 0; k < W; k += 8) {
-        unsigned c[8];
-        double v[8];
+    for (int k = 0; k < W; k += B) {
+        unsigned c[B];
+        double v[B];
 #pragma unroll
-        for (int u = 0; u < 8 && k + u < W; ++u) {
-            c[u] = cols[(k + u) * stride + row];
-            v[u] = val[(k + u) * stride + row];
+        for (int u = 0; u < B && k + u < W; ++u) {
+            c[u] = cols[32 * (k + u)];
+            v[u] = val[32 * (k + u)];
         }
 #pragma unroll
-        for (int u = 0; u < 8 && k + u < W; ++u)
+        for (int u = 0; u < B && k + u < W; ++u)
             (u & 1 ? s1 : s0) += v[u] * vec[c[u]];
     }
     return s0 + s1;
 }
-// The widths of the hierarchies of 3 to 5 cells' periodic width get code of their own: a
-// phase of the V-cycle is bound by the instructions it issues, and a loop with a run-time
-// width and bounds checks takes 5 times as many (1600 cycles for 192 rows of 11 entries).
+// The usual widths (channels of 3 to 5 cells: 2, 4, 11, 15; bump meshes: 1, 4, 9, 11) get
+// code of their own: a phase of the V-cycle is bound by the instructions it issues, and a
+// loop with a run-time width and bounds checks takes 5 times as many (1600 cycles for 192
+// rows of 11 entries).
 __device__ __forceinline__ double rowRes(const uint16_t *cols, const double *val,
-                                         const double *vec, int width, unsigned stride,
-                                         unsigned row) {
+                                         const double *vec, int width, int row) {
+    cols += ellRow(row, width);
+    val += ellRow(row, width);
     switch (width) {
-    case 2: return rowFix<2>(cols, val, vec, stride, row);
-    case 4: return rowFix<4>(cols, val, vec, stride, row);
-    case 11: return rowFix<11>(cols, val, vec, stride, row);
-    case 15: return rowFix<15>(cols, val, vec, stride, row);
+    case 1: return rowFix<1>(cols, val, vec);
+    case 2: return rowFix<2>(cols, val, vec);
+    case 4: return rowFix<4>(cols, val, vec);
+    case 9: return rowFix<9>(cols, val, vec);
+    case 11: return rowFix<11>(cols, val, vec);
+    case 15: return rowFix<15>(cols, val, vec);
     default: break;
     }
     double s = 0.0;
     int k = 0;
     for (; k + 4 <= width; k += 4)
-        s += rowFix<4>(cols + k * stride, val + k * stride, vec, stride, row);
+        s += rowFix<4>(cols + 32 * k, val + 32 * k, vec);
     for (; k < width; ++k)
-        s += val[k * stride + row] * vec[cols[k * stride + row]];
+        s += val[32 * k] * vec[cols[32 * k]];
     return s;
 }
 
-// The coarse levels of one V-cycle with one damped-Jacobi sweep (vcycleT): the level-0
-// residual in rr0 is restricted, and level 1's solution is left in its x. All threads of
-// the CTA take part; the caller's barrier precedes.
-__device__ __forceinline__ void coarseRes(Shared &S, const double *rr0) {
-    const DevClass &C = S.C;
-    const int L = C.nlev;
-    const double om = C.amgW, al = C.amgAlpha;
-    const double *fr = rr0; // residual of the level above
-    const int t0 = threadIdx.x, ts = blockDim.x;
-    for (int l = 1; l + 1 < L; ++l) {
-        const ResLevel R = S.RL[l];
-        for (int i = t0; i < R.n; i += ts) {
-            const double bi = rowRes(R.rc, R.rv, fr, R.rw, R.n, i);
-            R.b[i] = bi;
-            R.x[i] = om * bi * R.rd[i];
-        }
-        __syncthreads();
-        for (int i = t0; i < R.n; i += ts)
-            R.r[i] = R.b[i] - rowRes(R.ac, R.av, R.x, R.aw, R.n, i);
-        __syncthreads();
-        fr = R.r;
+// The coarse levels of one V-cycle (vcycleT): the level-0 residual in rr0 is restricted,
+// and level 1's solution is left in its x. All threads take part (levelThreads); the
+// caller's barrier precedes.
+// With Resident the vectors are known to be in shared memory (and loaded as such: 32-bit
+// addresses).
+template <bool Resident> __device__ __forceinline__ ResLevel levelOf(const Shared &S, int l) {
+    ResLevel R = S.RL[l];
+    if constexpr (Resident) {
+        double *v = reinterpret_cast<double *>(rqSmem + R.vOff);
+        R.b = v;
+        R.xa = v + R.n;
+        R.x = v + 2 * R.n;
+        R.r = v + 3 * R.n;
+        R.rd = v + 4 * R.n;
     }
-    {
-        const ResLevel R = S.RL[L - 1];
-        for (int i = t0; i < R.n; i += ts)
-            R.b[i] = L == 1 ? rr0[i] : rowRes(R.rc, R.rv, fr, R.rw, R.n, i);
-        __syncthreads();
-        // 1 << sh threads per row of the dense inverse
-        const int seg = 1 << R.sh, w = R.n << R.sh, j = t0 & (seg - 1);
-        for (int base = 0; base < w; base += ts) {
-            const int t = base + t0;
-            double s0 = 0.0, s1 = 0.0;
-            if (t < w) {
-                const double *q = S.resInv + t, *v = R.b + j;
-                int k = j;
-                for (; k + 7 * seg < R.n; k += 8 * seg, q += 8 * w, v += 8 * seg) {
-                    double a[8];
+    return R;
+}
+// out = x + om (b - A x) / diag on level l
+template <bool SH>
+__device__ __forceinline__ void smoothRes(const Shared &S, int l, const ResLevel &R,
+                                          const double *x, double *out) {
+    const double om = S.C.amgW;
+    const int ts = levelThreads(S, l);
+    for (int i = levelTid(S, l); i < R.n; i += ts)
+        out[i] = x[i] + om * (R.b[i] - rowRes(R.ac, R.av, x, R.aw, i)) * R.rd[i];
+    levelSync(S, l);
+}
+// level l on the way down: right-hand side from the residual fr above, pre-smoothing from
+// zero, residual
+template <bool SH>
+__device__ __forceinline__ void downRes(const Shared &S, int l, const double *fr) {
+    const ResLevel R = levelOf<SH>(S, l);
+    const bool two = S.C.amgSweeps >= 2;
+    const double om = S.C.amgW;
+    const int t0 = levelTid(S, l), ts = levelThreads(S, l);
+    for (int i = t0; i < R.n; i += ts) {
+        const double bi = rowRes(R.rc, R.rv, fr, R.rw, i);
+        R.b[i] = bi;
+        R.xa[i] = om * bi * R.rd[i];
+    }
+    levelSync(S, l);
+    if (two)
+        smoothRes<SH>(S, l, R, R.xa, R.x);
+    const double *x = two ? R.x : R.xa;
+    for (int i = t0; i < R.n; i += ts)
+        R.r[i] = R.b[i] - rowRes(R.ac, R.av, x, R.aw, i);
+    levelSync(S, l);
+}
+// and on the way up: the correction xc of the level below, post-smoothing; the solution in x
+template <bool SH>
+__device__ __forceinline__ void upRes(const Shared &S, int l, const double *xc) {
+    const ResLevel R = levelOf<SH>(S, l);
+    const bool two = S.C.amgSweeps >= 2;
+    const double al = S.C.amgAlpha, *x = two ? R.x : R.xa;
+    const int ts = levelThreads(S, l);
+    for (int i = levelTid(S, l); i < R.n; i += ts)
+        R.r[i] = x[i] + al * rowRes(R.pc, R.pv, xc, R.pw, i);
+    levelSync(S, l);
+    smoothRes<SH>(S, l, R, R.r, two ? R.xa : R.x);
+    if (two)
+        smoothRes<SH>(S, l, R, R.xa, R.x);
+}
+// levels l0 .. L - 1, all with vectors in shared memory (SH) or wherever they are
+template <bool SH>
+__device__ __forceinline__ void levelsRes(Shared &S, int l0, const double *fr) {
+    const int L = S.C.nlev;
+    for (int l = l0; l + 1 < L; ++l) {
+        downRes<SH>(S, l, fr);
+        fr = levelOf<SH>(S, l).r;
+    }
+    const int l = L - 1;
+    const ResLevel R = levelOf<SH>(S, l);
+    const int t0 = levelTid(S, l), ts = levelThreads(S, l);
+    for (int i = t0; i < R.n; i += ts)
+        R.b[i] = L == 1 ? fr[i] : rowRes(R.rc, R.rv, fr, R.rw, i);
+    levelSync(S, l);
+    // 1 << sh threads per row of the dense inverse
+    const int seg = 1 << R.sh, w = R.n << R.sh, j = t0 & (seg - 1);
+    for (int base = 0; base < w; base += ts) {
+        const int t = base + t0;
+        double s0 = 0.0, s1 = 0.0;
+        if (t < w) {
+            const double *q = S.resInv + t, *v = R.b + j;
+            int k = j;
+            for (; k + 7 * seg < R.n; k += 8 * seg, q += 8 * w, v += 8 * seg) {
+                double a[8];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        a[u] = q[u * w];
+                for (int u = 0; u < 8; ++u)
+                    a[u] = q[u * w];
 #pragma unroll
-                    for (int u = 0; u < 8; u += 2) {
-                        s0 += a[u] * v[u * seg];
-                        s1 += a[u + 1] * v[(u + 1) * seg];
-                    }
+                for (int u = 0; u < 8; u += 2) {
+                    s0 += a[u] * v[u * seg];
+                    s1 += a[u + 1] * v[(u + 1) * seg];
                 }
-                for (; k < R.n; k += seg, q += w, v += seg)
-                    s0 += q[0] * v[0];
             }
-            s0 += s1;
-            for (int o = seg >> 1; o > 0; o >>= 1)
-                s0 += __shfl_xor_sync(FULL, s0, o);
-            if (j == 0 && t < w)
-                R.x[t >> R.sh] = s0;
+            for (; k < R.n; k += seg, q += w, v += seg)
+                s0 += q[0] * v[0];
         }
-        __syncthreads();
+        s0 += s1;
+        for (int o = seg >> 1; o > 0; o >>= 1)
+            s0 += __shfl_xor_sync(FULL, s0, o);
+        if (j == 0 && t < w)
+            R.x[t >> R.sh] = s0;
     }
-    for (int l = L - 2; l >= 1; --l) {
-        const ResLevel R = S.RL[l];
-        const double *xc = S.RL[l + 1].x;
-        for (int i = t0; i < R.n; i += ts)
-            R.r[i] = R.x[i] + al * rowRes(R.pc, R.pv, xc, R.pw, R.n, i);
-        __syncthreads();
-        for (int i = t0; i < R.n; i += ts)
-            R.x[i] = R.r[i] + om * (R.b[i] - rowRes(R.ac, R.av, R.r, R.aw, R.n, i)) * R.rd[i];
-        __syncthreads();
+    levelSync(S, l);
+    for (int k = L - 2; k >= l0; --k)
+        upRes<SH>(S, k, levelOf<SH>(S, k + 1).x);
+}
+// rr0: the level-0 residual
+template <bool Resident>
+__device__ __forceinline__ void coarseRes(Shared &S, const double *rr0) {
+    if constexpr (kCluster) {
+        const int loc = S.C.locLevel;
+        const double *fr = rr0;
+        for (int l = 1; l < loc; ++l) {
+            downRes<false>(S, l, fr);
+            fr = S.RL[l].r;
+        }
+        levelsRes<true>(S, loc, fr);
+        for (int l = loc - 1; l >= 1; --l)
+            upRes<false>(S, l, S.RL[l + 1].x);
+    } else {
+        levelsRes<Resident>(S, S.C.nlev > 1 ? 1 : 0, rr0);
     }
 }
 
-// PCG (LinearSolver.hpp:184-246 / :908-982) from x = 0, with the V-cycle of one sweep per
-// level or the Jacobi preconditioner; K64.r holds b and r0n its norm. The working group
+// PCG (LinearSolver.hpp:184-246 / :908-982) from x = 0, with the V-cycle or the Jacobi
+// preconditioner; K64.r holds b and r0n its norm. The working group
 // holds the finest level in registers; all threads of the CTA run the coarse levels. The
 // caller's next CTA barrier makes x and *out visible.
 // What bounds it: the instructions that each of its 13 to 21 phases issues. Measured on a
@@ -496,6 +582,7 @@ __device__ __noinline__ void pcgRes(double *x, double r0n, int maxIter, double t
         return;
     }
     const int L = C.nlev;
+    const bool two = AMG && C.amgSweeps >= 2;
     const double om = C.amgW, al = C.amgAlpha;
     const double bound2 = (tol * r0n) * (tol * r0n);
     ResRows A;
@@ -515,40 +602,70 @@ __device__ __noinline__ void pcgRes(double *x, double r0n, int maxIter, double t
     for (int it = 0;; ++it) {
         double z[kResCells], q[1] = {0.0};
         if constexpr (AMG) {
-            if (mine && L > 1) {
+            if (mine && L > 1) { // pre-smoothed iterate in z, the residual in e1
 #pragma unroll
-                for (int k = 0; k < kResCells; ++k)
-                    e0[threadIdx.x + k * T] = om * r[k] * A.rd[k];
+                for (int k = 0; k < kResCells; ++k) {
+                    z[k] = om * r[k] * A.rd[k];
+                    e0[threadIdx.x + k * T] = z[k];
+                }
                 groupSync(T);
+                if (two) {
+#pragma unroll
+                    for (int k = 0; k < kResCells; ++k) {
+                        z[k] += om * (r[k] - A.times(k, z[k], e0)) * A.rd[k];
+                        e1[threadIdx.x + k * T] = z[k];
+                    }
+                    groupSync(T);
+                }
+                const double *e = two ? e1 : e0;
+                double rr[kResCells];
 #pragma unroll
                 for (int k = 0; k < kResCells; ++k)
-                    e1[threadIdx.x + k * T] = r[k] - A.times(k, om * r[k] * A.rd[k], e0);
+                    rr[k] = r[k] - A.times(k, z[k], e);
+                if (two)
+                    groupSync(T); // e1 is read until here
+#pragma unroll
+                for (int k = 0; k < kResCells; ++k)
+                    e1[threadIdx.x + k * T] = rr[k];
             } else if (mine) {
 #pragma unroll
                 for (int k = 0; k < kResCells; ++k)
                     e1[threadIdx.x + k * T] = r[k];
             }
             __syncthreads();
-            coarseRes(S, e1);
+            coarseRes<true>(S, e1);
         }
         if (mine) {
             if (AMG && L > 1) {
                 const ResLevel &R = S.RL[0];
-                const double *xc = S.RL[1].x;
+                const double *xc = levelOf<true>(S, 1).x;
+                double pz[kResCells];
 #pragma unroll
                 for (int k = 0; k < kResCells; ++k) {
                     const int c = threadIdx.x + k * T;
-                    z[k] = c < n ? rowRes(R.pc, R.pv, xc, R.pw, n, c) : 0.0;
+                    pz[k] = c < n ? rowRes(R.pc, R.pv, xc, R.pw, c) : 0.0;
                 }
 #pragma unroll
                 for (int k = 0; k < kResCells; ++k) {
-                    z[k] = om * r[k] * A.rd[k] + al * z[k];
+                    z[k] += al * pz[k];
                     e0[threadIdx.x + k * T] = z[k];
                 }
                 groupSync(T);
+                if (two) {
+#pragma unroll
+                    for (int k = 0; k < kResCells; ++k)
+                        pz[k] = z[k] + om * (r[k] - A.times(k, z[k], e0)) * A.rd[k];
+#pragma unroll
+                    for (int k = 0; k < kResCells; ++k) {
+                        z[k] = pz[k];
+                        e1[threadIdx.x + k * T] = z[k];
+                    }
+                    groupSync(T);
+                }
+                const double *e = two ? e1 : e0;
 #pragma unroll
                 for (int k = 0; k < kResCells; ++k) {
-                    z[k] += om * (r[k] - A.times(k, z[k], e0)) * A.rd[k];
+                    z[k] += om * (r[k] - A.times(k, z[k], e)) * A.rd[k];
                     q[0] += r[k] * z[k];
                 }
             } else {

@@ -30,6 +30,49 @@ namespace rq {
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
+
+// A solve runs on one CTA, or (objects compiled with RQ_CLUSTER) on a thread-block cluster
+// whose CTAs share the workspace in global memory: cells, faces and rows are dealt out
+// over all threads of the cluster, SYNC is its barrier, and block sums end in an exchange
+// of the CTAs' sums through distributed shared memory. Each CTA keeps its own copy of the
+// shared-memory state (Shared) and derives the same values in it.
+#ifdef RQ_CLUSTER
+constexpr bool kCluster = true;
+#else
+constexpr bool kCluster = false;
+#endif
+constexpr int kMaxCluster = 16;
+__device__ __forceinline__ int ctaRank() {
+    unsigned r = 0;
+    if constexpr (kCluster)
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return static_cast<int>(r);
+}
+__device__ __forceinline__ int ctaCount() {
+    unsigned r = 1;
+    if constexpr (kCluster)
+        asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r));
+    return static_cast<int>(r);
+}
+__device__ __forceinline__ int gTid() { return ctaRank() * blockDim.x + threadIdx.x; }
+__device__ __forceinline__ int gThreads() { return ctaCount() * blockDim.x; }
+__device__ __forceinline__ void SYNC() {
+    if constexpr (kCluster)
+        asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    else
+        __syncthreads();
+}
+// stores v at the address that p has in the shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ void putRemote(double *p, double v, int rank) {
+    const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(p));
+    asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\t"
+                 "st.shared::cluster.f64 [r], %2;\n\t}" ::"r"(a), "r"(rank), "d"(v) : "memory");
+}
+__device__ __forceinline__ void putRemote(int *p, int v, int rank) {
+    const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(p));
+    asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\t"
+                 "st.shared::cluster.s32 [r], %2;\n\t}" ::"r"(a), "r"(rank), "r"(v) : "memory");
+}
 constexpr int kRedSlots = 8;             // values per block reduction
 
 struct Work {
@@ -83,14 +126,15 @@ struct alignas(16) ResShared {
     double red[2][kResSums][kResMaxWarps];
 };
 
-// One level of the resident V-cycle: its rows, the threads per row of the dense coarsest
-// solve (1 << sh), its operator, the prolongation to it from the next level and the restriction of the
-// level above (widths, 16-bit columns and values in ELL form), and its vectors.
+// One level of the FP64 V-cycle (coarseRes): its rows, the threads per row of the dense
+// coarsest solve (1 << sh), its operator, the prolongation to it from the next level and
+// the restriction of the level above (widths, 16-bit columns and values in ELL form), and
+// its vectors: right-hand side, iterate, solution, residual, 1/diag.
 struct ResLevel {
-    int n, sh, aw, pw, rw, pad;
+    int n, sh, aw, pw, rw, vOff; // vOff: byte offset of the vectors in shared memory
     const uint16_t *ac, *pc, *rc;
     const double *av, *pv, *rv;
-    double *b, *x, *r;
+    double *b, *xa, *x, *r;
     const double *rd;
 };
 
@@ -101,6 +145,7 @@ struct Shared {
     KW<float> K32;
     double coeff[11];
     double red[2][kRedSlots][32];
+    double cred[2][kRedSlots][kCluster ? kMaxCluster : 1]; // the cluster's CTA sums
     double ring[4][kWindowCap];  // U, k, omega, Q change samples
     int cnt[4];
     double q[kMaxProbes], qPrev[kMaxProbes];
@@ -118,9 +163,12 @@ struct Shared {
     ResShared R;                          // block sums of the resident solvers
     int resWarps;                         // their working warps, 0: the general solvers
     int resAmg;                           // the V-cycle too (one sweep per level)
-    double *resInv;                       // the coarsest inverse in coarseRes's order
+    double *resInv;                       // the coarsest inverse in coarseRes's order,
+    int ownInv;                           // a CTA's own copy in shared memory
     int resDone;                          // a PCG solve has ended
-    ResLevel RL[kMaxLevels];              // levels of the resident V-cycle
+    ResLevel RL[kMaxLevels];              // levels of the FP64 V-cycle, filled where lean is set
+    int lean;                             // coarseRes runs the coarse levels
+    double *locVec;                       // vectors of a cluster's CTA-local levels
 };
 
 // dynamic shared memory of every solve kernel: Shared, then the arena
@@ -165,6 +213,20 @@ __device__ __forceinline__ void blockSum(double (&v)[K], Shared &S, int &rp) {
             s += __shfl_down_sync(FULL, s, o);
         v[k] = __shfl_sync(FULL, s, 0);
     }
+    if constexpr (kCluster) { // every CTA adds the CTA sums in the order of the ranks
+        const int nc = ctaCount(), rank = ctaRank();
+        if (static_cast<int>(threadIdx.x) < nc)
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                putRemote(&S.cred[rp][k][rank], v[k], threadIdx.x);
+        SYNC();
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            v[k] = S.cred[rp][k][0];
+            for (int c = 1; c < nc; ++c)
+                v[k] += S.cred[rp][k][c];
+        }
+    }
     rp ^= 1;
 }
 
@@ -186,6 +248,18 @@ __device__ __forceinline__ void blockMax(double (&v)[K], Shared &S, int &rp) {
         for (int o = 16; o > 0; o >>= 1)
             s = fmax(s, __shfl_xor_sync(FULL, s, o));
         v[k] = s;
+    }
+    if constexpr (kCluster) {
+        const int nc = ctaCount(), rank = ctaRank();
+        if (static_cast<int>(threadIdx.x) < nc)
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                putRemote(&S.cred[rp][k][rank], v[k], threadIdx.x);
+        SYNC();
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            for (int c = 0; c < nc; ++c)
+                v[k] = fmax(v[k], S.cred[rp][k][c]);
     }
     rp ^= 1;
 }
@@ -323,7 +397,7 @@ __device__ __forceinline__ double jac(double r, double d) {
 // thread measured 12 % slower per outer iteration at 1536 cells). Every per-cell
 // loop of a solve uses this one assignment, so a thread may read its own writes of
 // an earlier loop without a barrier.
-#define FOR_OWN(c, count) for (int c = threadIdx.x; c < (count); c += blockDim.x)
+#define FOR_OWN(c, count) for (int c = gTid(), ts_ = gThreads(); c < (count); c += ts_)
 #define FOR_CELLS(c) FOR_OWN(c, n)
 
 // ---------------------------------------------------------------- inner linear solvers
@@ -389,7 +463,7 @@ __device__ __noinline__ LinRes bicgstabT(Shared &S, int &rp, const KW<T> &K, T *
             p[c] = pc;
             ph[c] = pc * rd[c];
         }
-        __syncthreads();
+        SYNC();
         double a1[1] = {0.0};
         FOR_CELLS(c) {
             const Cell q = cellOf(C, c);
@@ -413,7 +487,7 @@ __device__ __noinline__ LinRes bicgstabT(Shared &S, int &rp, const KW<T> &K, T *
         const double sn = sqrt(a2[0]);
         if (sn / r0n < tol) {
             FOR_CELLS(c) x[c] += T(alpha) * ph[c];
-            __syncthreads();
+            SYNC();
             res.iterations = it + 1;
             res.finalRes = sn / r0n;
             res.converged = true;
@@ -451,7 +525,7 @@ __device__ __noinline__ LinRes bicgstabT(Shared &S, int &rp, const KW<T> &K, T *
         rho = rhoN;
         rhoN = a4[1];
     }
-    __syncthreads();
+    SYNC();
     return res;
 }
 
@@ -460,6 +534,33 @@ template <typename T> __device__ __forceinline__ T level0EntryT(const KW<T> &K, 
     const int slot = e / n, c = e - slot * n;
     const T *a = slot == 0 ? K.d : slot == 1 ? K.aW : slot == 2 ? K.aE : slot == 3 ? K.aS : K.aN;
     return a[c];
+}
+
+// The levels of at most kLocalRows rows: every CTA of a cluster runs them whole, on vectors
+// of its own in shared memory and with its own barrier (a cluster barrier costs about 520
+// cycles, a CTA barrier 60). The threads that share a level, and a level's vectors (b, xa,
+// xb, r, 1/diag).
+__device__ __forceinline__ bool localLevel(const Shared &S, int l) {
+    return kCluster && l >= S.C.locLevel;
+}
+__device__ __forceinline__ int levelTid(const Shared &S, int l) {
+    return localLevel(S, l) ? threadIdx.x : gTid();
+}
+__device__ __forceinline__ int levelThreads(const Shared &S, int l) {
+    return localLevel(S, l) ? blockDim.x : gThreads();
+}
+__device__ __forceinline__ void levelSync(const Shared &S, int l) {
+    if (localLevel(S, l))
+        __syncthreads();
+    else
+        SYNC();
+}
+template <typename T>
+__device__ __forceinline__ T *levelVec(const Shared &S, const KW<T> &K, int l) {
+    const int off = S.C.lev[l].vecOff;
+    if (localLevel(S, l))
+        return reinterpret_cast<T *>(S.locVec) + (off - S.C.lev[S.C.locLevel].vecOff);
+    return K.amgVec + off;
 }
 
 // Galerkin values of every coarse level from the current pressure system, the
@@ -481,7 +582,7 @@ template <typename T> __device__ __noinline__ void amgRefreshT(Shared &S, const 
         const T *fv = K.amgVal + F.valOff;
         // the first Galerkin sums cancel strongly (diagonal against off-diagonals of
         // one aggregate), so they are always formed from the FP64 finest matrix
-        for (int e = threadIdx.x; e < Q.nnz; e += blockDim.x) {
+        FOR_OWN(e, Q.nnz) {
             double s = 0.0;
             for (int k = __ldg(F.gPtr + e); k < __ldg(F.gPtr + e + 1); ++k) {
                 const double v = (l == 0) ? level0EntryT(S.K64, C.n, __ldg(F.gSrc + k))
@@ -490,13 +591,14 @@ template <typename T> __device__ __noinline__ void amgRefreshT(Shared &S, const 
             }
             cv[e] = T(s);
         }
-        __syncthreads();
+        SYNC();
     }
     for (int l = 1; l + 1 < L; ++l) {
         const DevAmgLevel &Lv = C.lev[l];
         const T *val = K.amgVal + Lv.valOff;
-        T *rdl = K.amgVec + Lv.vecOff + 4 * Lv.n;
-        for (int i = threadIdx.x; i < Lv.n; i += blockDim.x)
+        T *rdl = levelVec(S, K, l) + 4 * Lv.n;
+        const int ts = levelThreads(S, l);
+        for (int i = levelTid(S, l); i < Lv.n; i += ts)
             rdl[i] = T(1) / val[__ldg(Lv.diagPos + i)];
     }
     const DevAmgLevel &Q = C.lev[L - 1];
@@ -521,9 +623,9 @@ template <typename T> __device__ __noinline__ void amgRefreshT(Shared &S, const 
         } else {
             for (int r = threadIdx.x; r < m; r += blockDim.x)
                 for (int k = 0; k < Q.width; ++k) {
-                    const int c = __ldg(Q.ecol + k * m + r);
+                    const int e = ellRow(r, Q.width) + 32 * k, c = __ldg(Q.ecol + e);
                     if (c >= 0)
-                        a[r * m + c] = double(qv[k * m + r]);
+                        a[r * m + c] = double(qv[e]);
                 }
         }
         __syncthreads();
@@ -549,7 +651,11 @@ template <typename T> __device__ __noinline__ void amgRefreshT(Shared &S, const 
                 __syncwarp();
             }
         }
-        __syncthreads();
+        SYNC();
+        return;
+    }
+    if (ctaRank() != 0) { // the inverse is the work of one CTA
+        SYNC();
         return;
     }
     // m x 2m [A | I], row-major; the inverse ends in the right half of dense0
@@ -572,9 +678,9 @@ template <typename T> __device__ __noinline__ void amgRefreshT(Shared &S, const 
     } else {
         for (int r = threadIdx.x; r < m; r += blockDim.x)
             for (int k = 0; k < Q.width; ++k) {
-                const int c = __ldg(Q.ecol + k * m + r);
+                const int e = ellRow(r, Q.width) + 32 * k, c = __ldg(Q.ecol + e);
                 if (c >= 0)
-                    A0[r * m2 + c] = double(qv[k * m + r]);
+                    A0[r * m2 + c] = double(qv[e]);
             }
     }
     __syncthreads();
@@ -602,8 +708,8 @@ template <typename T> __device__ __noinline__ void amgRefreshT(Shared &S, const 
     if (A0 != W.dense0) { // keep the inverse in dense0
         for (int e = threadIdx.x; e < m * m2; e += blockDim.x)
             W.dense0[e] = A0[e];
-        __syncthreads();
     }
+    SYNC();
 }
 
 // Sum over the slots k = first, first + step, ... (< width) of one ELL row of
@@ -612,7 +718,9 @@ template <typename T> __device__ __noinline__ void amgRefreshT(Shared &S, const 
 // nothing), so a wide row costs a few load latencies, not one per slot.
 template <typename T, typename C, typename V>
 __device__ __forceinline__ T ellDot(const int32_t *cols, const C *coef, const V *vec, int width,
-                                    int stride, int row, int first = 0, int step = 1) {
+                                    int row, int first = 0, int step = 1) {
+    cols += ellRow(row, width);
+    coef += ellRow(row, width);
     T s = T(0);
     int k = first;
     for (; k + 3 * step < width; k += 4 * step) {
@@ -620,10 +728,10 @@ __device__ __forceinline__ T ellDot(const int32_t *cols, const C *coef, const V 
         T v[4], x[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-            c[u] = __ldg(cols + (k + u * step) * stride + row);
+            c[u] = __ldg(cols + (k + u * step) * 32);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            v[u] = T(coef[(k + u * step) * stride + row]);
+            v[u] = T(coef[(k + u * step) * 32]);
             x[u] = T(vec[c[u] < 0 ? 0 : c[u]]);
         }
 #pragma unroll
@@ -632,8 +740,8 @@ __device__ __forceinline__ T ellDot(const int32_t *cols, const C *coef, const V 
                 s += v[u] * x[u];
     }
     if (k + step < width) {
-        const int c0 = __ldg(cols + k * stride + row), c1 = __ldg(cols + (k + step) * stride + row);
-        const T v0 = T(coef[k * stride + row]), v1 = T(coef[(k + step) * stride + row]);
+        const int c0 = __ldg(cols + k * 32), c1 = __ldg(cols + (k + step) * 32);
+        const T v0 = T(coef[k * 32]), v1 = T(coef[(k + step) * 32]);
         const T x0 = T(vec[c0 < 0 ? 0 : c0]), x1 = T(vec[c1 < 0 ? 0 : c1]);
         if (c0 >= 0)
             s += v0 * x0;
@@ -642,19 +750,19 @@ __device__ __forceinline__ T ellDot(const int32_t *cols, const C *coef, const V 
         k += 2 * step;
     }
     if (k < width) {
-        const int c = __ldg(cols + k * stride + row);
+        const int c = __ldg(cols + k * 32);
         if (c >= 0)
-            s += T(coef[k * stride + row]) * T(vec[c]);
+            s += T(coef[k * 32]) * T(vec[c]);
     }
     return s;
 }
 
-// Threads per row of a pass over n rows: the largest power of two up to 32 for which
-// one pass of the CTA still covers every row (1 when there are more rows than half
-// the CTA's threads).
-__device__ __forceinline__ int segOf(int n) {
+// Threads per row of a pass of nt threads over n rows: the largest power of two up to 32
+// for which one pass still covers every row (1 when there are more rows than half the
+// threads).
+__device__ __forceinline__ int segOf(int n, int nt) {
     int seg = 1;
-    while (seg < 32 && 2 * seg * n <= static_cast<int>(blockDim.x))
+    while (seg < 32 && 2 * seg * n <= nt)
         seg *= 2;
     return seg;
 }
@@ -662,13 +770,13 @@ __device__ __forceinline__ int segOf(int n) {
 // A pass over the rows of a small level with several threads per row: lane j of a
 // row's segment computes part(i, j, seg), the partial sum of the row's terms j,
 // j + seg, ...; the partials are added by shuffles within the segment (a tree) and
-// the segment's first lane calls use(i, total). Every thread of the CTA takes part
-// (the shuffles need whole warps), so calls must be uniform across the CTA. With one
+// the segment's first lane calls use(i, total). Every one of the nt threads takes part, t
+// its index (the shuffles need whole warps), so calls must be uniform across them. With one
 // thread per row this is the plain row loop.
 template <typename T, typename Part, typename Use>
-__device__ __forceinline__ void segPass(int n, Part part, Use use) {
-    const int seg = segOf(n), per = static_cast<int>(blockDim.x) / seg;
-    const int r = threadIdx.x / seg, j = threadIdx.x - r * seg;
+__device__ __forceinline__ void segPass(int n, int t, int nt, Part part, Use use) {
+    const int seg = segOf(n, nt), per = nt / seg;
+    const int r = t / seg, j = t - r * seg;
     for (int base = 0; base < n; base += per) {
         const int i = base + r;
         T s = i < n ? part(i, j, seg) : T(0);
@@ -682,8 +790,10 @@ __device__ __forceinline__ void segPass(int n, Part part, Use use) {
 // row i of an ELL level times x, entries in column order
 template <typename T>
 __device__ __forceinline__ T csrRowT(const DevAmgLevel &L, const T *val, const T *x, int i) {
-    return ellDot<T>(L.ecol, val, x, L.width, L.n, i);
+    return ellDot<T>(L.ecol, val, x, L.width, i);
 }
+
+#include "rq_resident.cuh"
 
 // z = M^-1 b at level 0 (b = K.r, z -> K.z): on every level above the coarsest,
 // C.amgSweeps damped-Jacobi sweeps from zero, the residual, restriction by P^T (fused
@@ -702,91 +812,90 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
     const T om = T(C.amgW), al = T(C.amgAlpha);
     const Mat<T> M = matOf(K);
     T *const Krd = K.rd, *const Kr = K.r, *const Kz = K.z, *const Kxa = K.xa, *const Kxb = K.xb,
-             *const Krr = K.rr, *const amgVec = K.amgVec, *const amgVal = K.amgVal;
-    auto vb = [&](int l) { return amgVec + C.lev[l].vecOff; }; // b, xa, xb, r, 1/diag
-    auto sync = [] { __syncthreads(); };
-    const int t0 = threadIdx.x, ts = blockDim.x;
+             *const Krr = K.rr, *const amgVal = K.amgVal;
+    auto vb = [&](int l) { return levelVec(S, K, l); }; // b, xa, xb, r, 1/diag
+    auto sync = [&](int l) { levelSync(S, l); };
     // residual of level l-1 restricted to row I of level l: sum_k R_Ik r_k (lane j of
     // the row's segment: the terms j, j + seg, ...)
     auto restrictPart = [&](int l, int I, int j, int seg) {
         const DevAmgLevel &F = C.lev[l - 1];
         const T *fr = (l == 1) ? Krr : vb(l - 1) + 3 * F.n;
-        return ellDot<T>(F.rcol, F.rval, fr, F.rw, C.lev[l].n, I, j, seg);
+        return ellDot<T>(F.rcol, F.rval, fr, F.rw, I, j, seg);
     };
     // the prolongated coarse correction at row i of level l: sum_k P_ik x_c
     auto prolong = [&](int l, int i) {
         const DevAmgLevel &Lv = C.lev[l];
         const T *xc = vb(l + 1) + 2 * C.lev[l + 1].n;
-        return ellDot<T>(Lv.pcol, Lv.pval, xc, Lv.pw, Lv.n, i);
+        return ellDot<T>(Lv.pcol, Lv.pval, xc, Lv.pw, i);
     };
     // one level of the down sweep; the pre-smoothed iterate ends in xa (one sweep) or
     // xb (two sweeps), the residual in rr. Coarse levels run several threads per row.
     auto down = [&](int l) {
         const DevAmgLevel &Lv = C.lev[l];
-        const int n = Lv.n;
+        const int n = Lv.n, t0 = levelTid(S, l), ts = levelThreads(S, l);
         if (l == 0) {
             FOR_OWN(i, n)
                 Kxa[i] = om * Kr[i] * Krd[i];
-            sync();
+            sync(l);
             const T *xs = Kxa;
             if (two) {
                 FOR_OWN(i, n) {
                     const T ax = rowDotT(cellOf(C, i), M, Kxa, nx);
                     Kxb[i] = Kxa[i] + om * (Kr[i] - ax) * Krd[i];
                 }
-                sync();
+                sync(l);
                 xs = Kxb;
             }
             FOR_OWN(i, n)
                 Krr[i] = Kr[i] - rowDotT(cellOf(C, i), M, xs, nx);
-            sync();
+            sync(l);
             return;
         }
         T *b = vb(l), *xa = b + n, *xb = b + 2 * n, *rr = b + 3 * n;
         const T *rd = b + 4 * n;
         const T *val = amgVal + Lv.valOff;
-        segPass<T>(n, [&](int i, int j, int seg) { return restrictPart(l, i, j, seg); },
+        segPass<T>(n, t0, ts, [&](int i, int j, int seg) { return restrictPart(l, i, j, seg); },
                    [&](int i, T bi) {
                        b[i] = bi;
                        xa[i] = om * bi * rd[i];
                    });
-        sync();
+        sync(l);
         const T *xs = xa;
         if (two) {
-            segPass<T>(n,
+            segPass<T>(n, t0, ts,
                        [&](int i, int j, int seg) {
-                           return ellDot<T>(Lv.ecol, val, xa, Lv.width, n, i, j, seg);
+                           return ellDot<T>(Lv.ecol, val, xa, Lv.width, i, j, seg);
                        },
                        [&](int i, T ax) { xb[i] = xa[i] + om * (b[i] - ax) * rd[i]; });
-            sync();
+            sync(l);
             xs = xb;
         }
-        segPass<T>(n,
+        segPass<T>(n, t0, ts,
                    [&](int i, int j, int seg) {
-                       return ellDot<T>(Lv.ecol, val, xs, Lv.width, n, i, j, seg);
+                       return ellDot<T>(Lv.ecol, val, xs, Lv.width, i, j, seg);
                    },
                    [&](int i, T ax) { rr[i] = b[i] - ax; });
-        sync();
+        sync(l);
     };
     // the coarsest level: restriction of the level above, then the dense inverse
     auto coarsest = [&]() {
-        const int l = L - 1;
+        const int l = L - 1, t0 = levelTid(S, l), ts = levelThreads(S, l);
         const int m = C.lev[l].n, m2 = 2 * m;
         T *b = vb(l), *xb = b + 2 * m;
         if (L == 1) {
             FOR_OWN(i, m)
                 b[i] = Kr[i];
         } else {
-            segPass<T>(m, [&](int i, int j, int seg) { return restrictPart(l, i, j, seg); },
+            segPass<T>(m, t0, ts, [&](int i, int j, int seg) { return restrictPart(l, i, j, seg); },
                        [&](int i, T bi) { b[i] = bi; });
         }
-        sync();
+        sync(l);
         // the coarsest solve stays FP64 in both forms: the coarsest level of the
         // pinned all-Neumann pressure system is nearly singular, and an FP32
         // copy of its inverse loses the coarse correction
         const double *inv = (m <= 32) ? S.coarse : W.dense0 + m;
         const int ld = (m <= 32) ? m : m2;
-        segPass<double>(m,
+        segPass<double>(m, t0, ts,
                         [&](int i, int j, int seg) {
                             const double *row = inv + i * ld;
                             double s = 0.0;
@@ -795,7 +904,7 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
                             return s;
                         },
                         [&](int i, double s) { xb[i] = T(s); });
-        sync();
+        sync(l);
     };
     // one level of the up sweep (levels >= 1; level 0 ends in the reduction below):
     // x = x_pre + alpha P x_c, then the post sweeps; the result ends in xb. With a
@@ -805,7 +914,7 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
     // each neighbour's x once instead of re-forming it from P.
     auto up = [&](int l) {
         const DevAmgLevel &Lv = C.lev[l];
-        const int n = Lv.n;
+        const int n = Lv.n, t0 = levelTid(S, l), ts = levelThreads(S, l);
         T *b = vb(l), *xa = b + n, *xb = b + 2 * n, *xi = b + 3 * n;
         const T *rd = b + 4 * n;
         const T *xpre = two ? xb : xa;
@@ -814,10 +923,10 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
         if (Lv.pw > 1) {
             for (int i = t0; i < n; i += ts)
                 xi[i] = xpre[i] + al * prolong(l, i);
-            sync();
-            segPass<T>(n,
+            sync(l);
+            segPass<T>(n, t0, ts,
                        [&](int i, int j, int seg) {
-                           return ellDot<T>(Lv.ecol, val, xi, Lv.width, n, i, j, seg);
+                           return ellDot<T>(Lv.ecol, val, xi, Lv.width, i, j, seg);
                        },
                        [&](int i, T ax) { out[i] = xi[i] + om * (b[i] - ax) * rd[i]; });
         } else {
@@ -825,39 +934,57 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
                 const T x0 = xpre[i] + al * prolong(l, i);
                 T ax = T(0);
                 for (int k = 0; k < Lv.width; ++k) {
-                    const int jj = __ldg(Lv.ecol + k * n + i);
+                    const int e = ellRow(i, Lv.width) + 32 * k, jj = __ldg(Lv.ecol + e);
                     if (jj >= 0)
-                        ax += val[k * n + i] * (xpre[jj] + al * prolong(l, jj));
+                        ax += val[e] * (xpre[jj] + al * prolong(l, jj));
                 }
                 out[i] = x0 + om * (b[i] - ax) * rd[i];
             }
         }
-        sync();
+        sync(l);
         if (two) {
-            segPass<T>(n,
+            segPass<T>(n, t0, ts,
                        [&](int i, int j, int seg) {
-                           return ellDot<T>(Lv.ecol, val, xa, Lv.width, n, i, j, seg);
+                           return ellDot<T>(Lv.ecol, val, xa, Lv.width, i, j, seg);
                        },
                        [&](int i, T ax) { xb[i] = xa[i] + om * (b[i] - ax) * rd[i]; });
-            sync();
+            sync(l);
         }
     };
-    for (int l = 0; l + 1 < L; ++l)
-        down(l);
-    coarsest();
-    for (int l = L - 2; l >= 1; --l)
-        up(l);
-    const int tid = t0, nt = ts;
+    bool lean = false;
+    if constexpr (std::is_same_v<T, double>)
+        lean = S.lean;
+    if (L > 1)
+        down(0);
+    if (lean) {
+        if constexpr (std::is_same_v<T, double>)
+            coarseRes<false>(S, L > 1 ? Krr : Kr);
+    } else {
+        for (int l = 1; l + 1 < L; ++l)
+            down(l);
+        coarsest();
+        for (int l = L - 2; l >= 1; --l)
+            up(l);
+    }
     double rz = 0.0;
-    if (L > 1 && C.lev[0].pw > 1) { // level 0, smoothed P: x = x_pre + alpha P x_c in a
+    if (L > 1 && (lean || C.lev[0].pw > 1)) { // level 0, smoothed P: x = x_pre + alpha P x_c in a
         // sweep of its own (into rr, free since the restriction to level 1), then the
         // post sweep(s) read it (each x once, not re-formed at every neighbour)
         const int n = C.lev[0].n;
         const T *xprev = two ? Kxb : Kxa;
         T *out = two ? Kxa : Kz;
-        FOR_OWN(i, n)
-            Krr[i] = xprev[i] + al * prolong(0, i);
-        __syncthreads();
+        if (lean) {
+            if constexpr (std::is_same_v<T, double>) {
+                const ResLevel &R = S.RL[0];
+                const double *xc = S.RL[1].x;
+                FOR_OWN(i, n)
+                    Krr[i] = xprev[i] + al * rowRes(R.pc, R.pv, xc, R.pw, i);
+            }
+        } else {
+            FOR_OWN(i, n)
+                Krr[i] = xprev[i] + al * prolong(0, i);
+        }
+        SYNC();
         double part = 0.0;
         FOR_OWN(i, n) {
             const T ax = rowDotT(cellOf(C, i), M, Krr, nx);
@@ -867,7 +994,7 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
                 part += double(Kr[i]) * double(zi);
         }
         if (two) {
-            __syncthreads();
+            SYNC();
             FOR_OWN(i, n) {
                 const T ax = rowDotT(cellOf(C, i), M, Kxa, nx);
                 const T zi = Kxa[i] + om * (Kr[i] - ax) * Krd[i];
@@ -901,7 +1028,7 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
                 part += double(Kr[i]) * double(zi);
         }
         if (two) {
-            __syncthreads();
+            SYNC();
             FOR_OWN(i, n) {
                 const T ax = rowDotT(cellOf(C, i), M, Kxa, nx);
                 const T zi = Kxa[i] + om * (Kr[i] - ax) * Krd[i];
@@ -925,8 +1052,6 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
     }
     return rz;
 }
-
-#include "rq_resident.cuh"
 
 // The sweeps of one PCG iteration as functions of their own, so that the PCG loop
 // itself keeps only a few scalars live across the V-cycle call (every value live
@@ -986,7 +1111,7 @@ template <typename T> __device__ __noinline__ void pcgDirection(Shared &S, const
     } else {
         FOR_CELLS(c) p[c] = z[c] + T(beta) * p[c];
     }
-    __syncthreads();
+    SYNC();
 }
 // x += alpha p, r -= alpha Ap; returns (r, r) and the sum of r (the mixed form's
 // deflation of the constant vector needs it)
@@ -1086,7 +1211,7 @@ __device__ __noinline__ LinRes pcgT(Shared &S, int &rp, const KW<T> &K, T *x, do
                     F.aN[c] = float(M.aN[c]);
                     F.rd[c] = (fabs(double(F.d[c])) > 1e-30) ? 1.0f / F.d[c] : 1.0f;
                 }
-                __syncthreads();
+                SYNC();
             }
         }
     }
@@ -1094,11 +1219,14 @@ __device__ __noinline__ LinRes pcgT(Shared &S, int &rp, const KW<T> &K, T *x, do
         mark(S, 4);
         if constexpr (F32Precond)
             amgRefreshT<float>(S, S.K32);
-        else
+        else {
             amgRefreshT(S, K); // begins with a barrier-separated phase
+            if (S.lean)
+                denseOrder(S);
+        }
         mark(S, 5);
     } else {
-        __syncthreads();
+        SYNC();
     }
     // the mixed form deflates the constant vector (pcgPrecondF32): the row sum of the
     // pinned row and the running sum of r
@@ -1185,7 +1313,7 @@ __device__ __noinline__ LinRes mixedSolve(Shared &S, int &rp, double *x64, doubl
         K.aN[c] = float(W.aN[c]);
         K.r[c] = float(W.r[c]);
     }
-    __syncthreads();
+    SYNC();
     double rn = r0n;
     bool refreshNow = refresh;
     for (int round = 0; round < 8 && out.iterations < maxIter; ++round) {
@@ -1197,12 +1325,12 @@ __device__ __noinline__ LinRes mixedSolve(Shared &S, int &rp, double *x64, doubl
         const double r32n = sqrt(an[0]);
         LinRes in;
         FOR_CELLS(c) K.x[c] = 0.0f;
-        __syncthreads();
+        SYNC();
         in = bicgstabT<float>(S, rp, K, K.x, r32n, maxIter - out.iterations, innerTol);
         (void)refreshNow;
         out.iterations += in.iterations;
         FOR_CELLS(c) x64[c] += double(K.x[c]);
-        __syncthreads();
+        SYNC();
         double a[1] = {0.0};
         FOR_CELLS(c) {
             const Cell q = cellOf(C, c);
@@ -1268,7 +1396,7 @@ __device__ __forceinline__ LinRes solvePressure(Shared &S, int &rp, double *x, d
             pcgRes<false>(x, r0n, maxIter, tol, &S.L.resP);
         else if (static_cast<int>(threadIdx.x) < 32 * S.resWarps)
             bicgstabRes(x, r0n, maxIter, tol, &S.L.resP);
-        __syncthreads();
+        SYNC();
         res = S.L.resP;
     } else if (kind == kPBicgstab)
         res = mixed ? mixedSolve(S, rp, x, r0n, maxIter, tol, kind, refresh)
@@ -1329,12 +1457,12 @@ __device__ __forceinline__ Est estimate(const Shared &S, int e, int window, doub
 }
 
 __device__ __forceinline__ void pushSample(Shared &S, int e, double v) {
-    __syncthreads(); // everyone finished reading the ring
+    SYNC(); // everyone finished reading the ring
     if (threadIdx.x == 0) {
         S.ring[e][S.cnt[e] % kWindowCap] = v;
         S.cnt[e] += 1;
     }
-    __syncthreads();
+    SYNC();
 }
 
 // ---------------------------------------------------------------- the solve
@@ -1349,7 +1477,11 @@ __device__ void carve(Shared &S, double *ws, double *arena, long arenaDoubles) {
     long used = 0;
     // the resident solvers where a thread can hold its cells in registers
     S.resWarps = 0;
-    if (C.st.precision == kFP64 && static_cast<int>(blockDim.x) <= kResMaxThreads &&
+    S.locVec = arena;
+    const long arenaAll = arenaDoubles;
+    if constexpr (kCluster) // the CTAs share every array; the arena holds the local levels
+        arenaDoubles = 0;
+    if (!kCluster && C.st.precision == kFP64 && static_cast<int>(blockDim.x) <= kResMaxThreads &&
         n <= static_cast<long>(kResCells) * blockDim.x && resExchange(n) <= arenaDoubles) {
         used = resExchange(n); // the exchange vectors start the arena
         S.resWarps = resThreads(n) / 32;
@@ -1357,6 +1489,7 @@ __device__ void carve(Shared &S, double *ws, double *arena, long arenaDoubles) {
     // and their V-cycle, whose level vectors come next
     const long vecs = (C.amgVecs + 31) / 32 * 32;
     S.resAmg = S.resWarps && C.resAmg && used + vecs <= arenaDoubles;
+    S.lean = C.resAmg && C.st.precision == kFP64 && C.st.pSolver == kPAmg;
     auto take = [&](long cnt) {
         const long sz = (cnt + 31) / 32 * 32;
         double *gp = g;
@@ -1437,10 +1570,12 @@ __device__ void carve(Shared &S, double *ws, double *arena, long arenaDoubles) {
         // tier 2: AMG (vectors first: touched more often)
         W.amgVec = S.resAmg ? resVec : take(C.amgVecs);
         W.amgVal = take(C.amgVals);
-        if (S.resAmg)
+        if (S.lean)
             resPlace(S, [&](long cnt) {
                 const long sz = (cnt + 31) / 32 * 32;
-                if (used + sz > arenaDoubles)
+                if (kCluster && used == 0)
+                    used = C.locDoubles;
+                if (used + sz > arenaAll)
                     return static_cast<double *>(nullptr);
                 double *sp = arena + used;
                 used += sz;
@@ -1485,7 +1620,7 @@ __device__ void carve(Shared &S, double *ws, double *arena, long arenaDoubles) {
     W.wOld = take(n);
     W.dense0 = take(2L * m * m); // [A | I] ping-pong of a coarsest level above 32 rows
     W.dense1 = take(2L * m * m);
-    if (S.resAmg && !S.resInv)
+    if (S.lean && !S.resInv)
         S.resInv = W.dense1;
     if (mixed) {
         W.ph = W.s = W.sh = W.t = W.rh = nullptr;
@@ -1575,7 +1710,7 @@ __device__ __noinline__ void phInitWarm(Shared &S, const double *wf) {
 
 __device__ __noinline__ void phInitFlux(Shared &S) {
     RQ_PRELUDE
-    for (int f = threadIdx.x; f < n + nfy; f += blockDim.x) {
+    FOR_OWN(f, n + nfy) {
         double v = 0.0;
         if (f < n) {
             const int q = eastOf(C, f);
@@ -1599,7 +1734,7 @@ __device__ __noinline__ void phInitFlux(Shared &S) {
 
 __device__ __noinline__ void phStart(Shared &S, bool turbUpdate) {
     RQ_PRELUDE
-        for (int f = threadIdx.x; f < n + nfy; f += blockDim.x) {
+        FOR_OWN(f, n + nfy) {
             double v = 0.0;
             if (f < n) {
                 const int q = eastOf(C, f);
@@ -1704,7 +1839,7 @@ __device__ __noinline__ void phMomentumFaces(Shared &S, int comp) {
             const double *gUc_y = comp == 0 ? W.gUxy : W.gUyy;
             const double *colX = comp == 0 ? W.gUxx : W.gUxy;  // dUx/dx_comp
             const double *colY = comp == 0 ? W.gUyx : W.gUyy;  // dUy/dx_comp
-            for (int f = threadIdx.x; f < n + nfy; f += blockDim.x) {
+            FOR_OWN(f, n + nfy) {
                 int fi, o, qn;
                 const double *A, *NX, *NY, *WT, *DL;
                 double sh = 0.0;
@@ -1903,7 +2038,7 @@ __device__ __noinline__ void phMomentum(Shared &S, int comp, double (&acc)[3]) {
 __device__ __noinline__ void phPressureFaces(Shared &S, double (&fs)[1]) {
     RQ_PRELUDE
         const double relaxCorr = 1.0 - st.aU;
-        for (int f = threadIdx.x; f < n + nfy; f += blockDim.x) {
+        FOR_OWN(f, n + nfy) {
             int o, q;
             const double *A, *NX, *NY, *WT, *DL, *DX, *DY;
             int fi;
@@ -2019,7 +2154,7 @@ __device__ __noinline__ void phCorrect(Shared &S, bool turbUpdate) {
                 W.wOld[c] = W.w[c];
             }
         }
-        for (int f = threadIdx.x; f < n + nfy; f += blockDim.x) {
+        FOR_OWN(f, n + nfy) {
             double v;
             if (f < n) {
                 const int q = eastOf(C, f);
@@ -2060,7 +2195,7 @@ __device__ __noinline__ void phTurbFaces(Shared &S, int eq) {
     RQ_PRELUDE
     const double *X = eq == 0 ? W.k : W.w;
     const double *gX = eq == 0 ? W.gKx : W.gWx, *gY = eq == 0 ? W.gKy : W.gWy;
-            for (int f = threadIdx.x; f < n + nfy; f += blockDim.x) {
+            FOR_OWN(f, n + nfy) {
                 int fi, o, qn;
                 const double *A, *WT, *DL;
                 double sh = 0.0;
@@ -2351,10 +2486,10 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
             S.stage[t] = 0;
         S.tmark = clock64();
     }
-    __syncthreads();
+    SYNC();
     // phi = interpolated fluxes of the initial state (wall faces carry U_b = 0)
     phInitFlux(S);
-    __syncthreads();
+    SYNC();
 
     // the loop state lives in shared memory (LoopState); every thread writes the same
     // values, and reads after its own writes
@@ -2384,7 +2519,7 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
         const bool turbUpdate = turbActive && ((iter - st.turbStart) % st.turbInterval == 0);
         // ---- phase: save U, interpolated old flux, gradients of U and p
         phStart(S, turbUpdate);
-        __syncthreads();
+        SYNC();
 
         mark(S, 7);
         // ---- SST closure (SSTModel.cpp:157-241) and the startup nuT floor (:1322-1337)
@@ -2393,7 +2528,7 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
                 established = true;
             const double floorV = established ? 0.0 : 0.1 * nu;
             phClosure(S, floorV);
-            __syncthreads();
+            SYNC();
         }
 
         mark(S, 1);
@@ -2403,12 +2538,12 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
         for (int comp = 0; comp < 2; ++comp) {
             if (comp == 1) { // gradients of the updated Ux for the y assembly
                 phGradU(S);
-                __syncthreads();
+                SYNC();
             }
             double *U = comp == 0 ? W.Ux : W.Uy;
             double acc[3] = {0.0, 0.0, 0.0};
             phMomentumFaces(S, comp);
-            __syncthreads();
+            SYNC();
             phMomentum(S, comp, acc);
             blockSum<3>(acc, S, rp);
             momRes = comp == 0 ? acc[0] : dmax(momRes, acc[0]);
@@ -2417,14 +2552,14 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
             solveBicg(S, rp, U, sqrt(acc[1]), st.innerIter, st.innerTol, &resU[comp]);
             if (threadIdx.x == 0)
                 S.innerKrylov += resU[comp].iterations;
-            __syncthreads();
+            SYNC();
         }
 
         mark(S, 2);
         // ---- predicted flux (stored Rhie-Chow, :1401-1419) and p' assembly (:717-830)
         double fs[1] = {0.0};
         phPressureFaces(S, fs);
-        __syncthreads();
+        SYNC();
         double pacc[3] = {0.0, 0.0, fs[0]};
         phPressureCells(S, pacc);
         blockSum<3>(pacc, S, rp);
@@ -2436,12 +2571,12 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
                              amgNeed, amgAfter);
         if (threadIdx.x == 0)
             S.innerPressure += resP.iterations;
-        __syncthreads();
+        SYNC();
 
         mark(S, 4);
         // ---- corrections (:916-940, :1443-1467)
         phCorrect(S, turbUpdate);
-        __syncthreads();
+        SYNC();
 
         // ---- turbulence (:1476-1538)
         LinRes &resK = Ls.resK, &resW = Ls.resW;
@@ -2454,9 +2589,9 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
                 double *X = eq == 0 ? W.k : W.w;
                 double acc[1] = {0.0};
                 phTurbFaces(S, eq);
-                __syncthreads();
+                SYNC();
                 phTurbAssemble(S, eq);
-                __syncthreads();
+                SYNC();
                 // initial residual with the (constrained) initial guess: wall cells of
                 // omega start from their wall value (read through x0, never from X,
                 // so the in-place update below cannot race with a neighbour's read)
@@ -2466,7 +2601,7 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
                 solveBicg(S, rp, X, sqrt(acc[0]), st.innerIter, st.innerTol, &rr);
                 if (threadIdx.x == 0)
                     S.innerKrylov += rr.iterations;
-                __syncthreads();
+                SYNC();
             }
         }
 
@@ -2481,7 +2616,7 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
         }
         Ls.uChange = mx[5] / mx[4];
         // one barrier pair for every sample of this iteration (U, k, omega, monitor)
-        __syncthreads();
+        SYNC();
         if (threadIdx.x == 0) {
             S.ring[0][S.cnt[0] % kWindowCap] = Ls.uChange;
             S.cnt[0] += 1;
@@ -2492,11 +2627,11 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
                 S.cnt[2] += 1;
             }
         }
-        __syncthreads();
+        SYNC();
         const bool haveMonitor = C.nobs > 0;
         if (haveMonitor && iter % (st.monitorInterval > 1 ? st.monitorInterval : 1) == 0) {
             phProbes(S);
-            __syncthreads();
+            SYNC();
             bool finite = true;
             for (int t = 0; t < C.nobs; ++t)
                 finite = finite && isfinite(S.q[t]);
@@ -2515,12 +2650,12 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
                 }
                 pushSample(S, 3, dq);
             }
-            __syncthreads();
+            SYNC();
             if (threadIdx.x < C.nobs)
                 S.qPrev[threadIdx.x] = S.q[threadIdx.x];
             if (threadIdx.x == 0)
                 S.haveQPrev = 1;
-            __syncthreads();
+            SYNC();
         }
         // the history entry of this iteration (ResidualEntry order); no phase call follows
         const double tol = st.tol, negligible = 0.01 * tol;
@@ -2615,13 +2750,13 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
             break;
         }
     }
-    __syncthreads();
+    SYNC();
     const bool stalled = !converged && !diverged && status == 1 && isfinite(rateU) && rateU >= 1.0;
 
     // ---- outputs: verdict, probe predictions, log-likelihood (ObservationOperator.hpp:592-609)
     if (status == 0 || status == 1) {
         phProbes(S);
-        __syncthreads();
+        SYNC();
     }
     if (threadIdx.x == 0) {
         RowOut o;
@@ -2659,18 +2794,18 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
         for (int b = 0; b < 11; ++b)
             FOR_CELLS(c) job.fields[(long)b * n + c] = src[b] ? src[b][c] : 0.0;
     } else if (job.fields) { // a diverged solve leaves no valid state (ForwardModel.cpp:88-96)
-        for (long e = threadIdx.x; e < 11L * n; e += blockDim.x)
+        for (long e = gTid(); e < 11L * n; e += gThreads())
             job.fields[e] = __longlong_as_double(0x7ff8000000000000LL);
     }
     if (job.snap && status != 2) {
-        for (int f = threadIdx.x; f < n + nfy; f += blockDim.x)
+        FOR_OWN(f, n + nfy)
             job.snap[f] = W.phi[f];
         if (threadIdx.x == 0) {
             job.snap[n + nfy] = S.wallBeta;
             job.snap[n + nfy + 1] = established ? 1.0 : 0.0;
         }
     }
-    __syncthreads();
+    SYNC();
 }
 
 } // namespace
@@ -2706,7 +2841,7 @@ __device__ void runJob(Shared &S, const DevJob &job, double *ws, double *arena, 
             carve(S, ws, arena, arenaDoubles);
     }
     __syncthreads();
-    if (S.admitted && S.resAmg)
+    if (S.admitted && S.lean)
         resTables(S);
     if (S.admitted) {
         runSolve(S, job);
@@ -2719,11 +2854,11 @@ __device__ void runJob(Shared &S, const DevJob &job, double *ws, double *arena, 
         for (int t = threadIdx.x; t < S.C.nobs; t += blockDim.x)
             job.pred[t] = __longlong_as_double(0x7ff8000000000000LL);
         if (job.fields)
-            for (long e = threadIdx.x; e < 11L * S.C.n; e += blockDim.x)
+            for (long e = gTid(); e < 11L * S.C.n; e += gThreads())
                 job.fields[e] = __longlong_as_double(0x7ff8000000000000LL);
     }
     __syncthreads();
-    if (threadIdx.x == 0 && job.clock) {
+    if (gTid() == 0 && job.clock) {
         long long t1;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
         job.clock[0] = t0;
@@ -2741,18 +2876,33 @@ __device__ __forceinline__ long long globalNs() {
     return t;
 }
 
+// Resident CTAs that the register budget of a CTA size is set for (128 registers at 512
+// threads and 256, 168 below, 80 at 768, 64 at 1024). Said explicitly because ptxas may
+// otherwise halve the budget of the 512-thread kernels to fit two on an SM, which costs a
+// 384-cell solve 45 % (spills in every phase).
+constexpr int ctasPerSM(int nt) { return nt >= 512 ? 1 : nt == 256 ? 2 : nt == 128 ? 3 : 6; }
+
 // One kernel body, instantiated per CTA size so each gets its full register budget.
-template <int NT>
-__global__ void __launch_bounds__(NT) solveKernel(const DevJob *jobs, int njobs, int *nextJob,
+template <int NT, bool Cluster>
+__global__ void __launch_bounds__(NT, ctasPerSM(NT)) solveKernel(const DevJob *jobs, int njobs, int *nextJob,
                                                   double *wsBase, long wsStride, int arenaDoubles) {
     extern __shared__ __align__(16) unsigned char smemRaw[];
     Shared &S = *reinterpret_cast<Shared *>(smemRaw);
     double *arena = reinterpret_cast<double *>(smemRaw + kSharedBytes);
-    double *ws = wsBase + wsStride * blockIdx.x;
+    double *ws = wsBase + wsStride * (blockIdx.x / ctaCount());
+    if constexpr (kCluster)
+        SYNC(); // every CTA of the cluster has started: its shared memory can be written
     for (;;) {
-        if (threadIdx.x == 0)
+        if constexpr (kCluster) {
+            if (gTid() == 0) {
+                const int j = atomicAdd(nextJob, 1);
+                for (int r = 0; r < ctaCount(); ++r)
+                    putRemote(&S.job, j, r);
+            }
+        } else if (threadIdx.x == 0) {
             S.job = atomicAdd(nextJob, 1);
-        __syncthreads();
+        }
+        SYNC();
         const int j = S.job;
         if (j >= njobs)
             break;
@@ -2770,8 +2920,8 @@ __global__ void __launch_bounds__(NT) solveKernel(const DevJob *jobs, int njobs,
 // solves in its own pool region when it carries one (DevJob::ws), else in the CTA's
 // slot workspace. Results go straight to host-mapped rows; the request's done flag
 // is raised after a system-scope fence; every CTA counts its exit.
-template <int NT>
-__global__ void __launch_bounds__(NT) serveKernel(ServeQueue q, double *wsBase, long wsStride,
+template <int NT, bool Cluster>
+__global__ void __launch_bounds__(NT, ctasPerSM(NT)) serveKernel(ServeQueue q, double *wsBase, long wsStride,
                                                   int arenaDoubles) {
     extern __shared__ __align__(16) unsigned char smemRaw[];
     Shared &S = *reinterpret_cast<Shared *>(smemRaw);
@@ -2824,8 +2974,8 @@ __global__ void __launch_bounds__(NT) serveKernel(ServeQueue q, double *wsBase, 
 // ---------------------------------------------------------------- allocation-free single solve
 // One job passed by value (no job array, no queue counter), solved by one CTA in
 // the scratch array.
-template <int NT>
-__global__ void __launch_bounds__(NT) solveOneKernel(DevJob job, double *ws, int arenaDoubles) {
+template <int NT, bool Cluster>
+__global__ void __launch_bounds__(NT, ctasPerSM(NT)) solveOneKernel(DevJob job, double *ws, int arenaDoubles) {
     extern __shared__ __align__(16) unsigned char smemRaw[];
     Shared &S = *reinterpret_cast<Shared *>(smemRaw);
     double *arena = reinterpret_cast<double *>(smemRaw + kSharedBytes);
@@ -2839,27 +2989,30 @@ __global__ void __launch_bounds__(NT) solveOneKernel(DevJob job, double *ws, int
 // (the phases are separate functions that ptxas allocates for each kernel's register
 // budget, so one object for all sizes would compile serially), and once without for the
 // host entry points.
-enum SolveEntry { kEntrySolve = 0, kEntryServe = 1, kEntryOne = 2 };
-template <int NT> void *solveEntry(int kind);
+enum SolveEntry { kEntrySolve = 0, kEntryServe = 1, kEntryOne = 2, kEntryBytes = 3 };
+constexpr int kClusterThreads = 768; // CTA size of the cluster kernels
+template <int NT, bool Cluster> void *solveEntry(int kind);
 
 #ifdef RQ_CTA
-template <> void *solveEntry<RQ_CTA>(int kind) {
+template <> void *solveEntry<RQ_CTA, kCluster>(int kind) {
     switch (kind) {
-    case kEntrySolve: return reinterpret_cast<void *>(&solveKernel<RQ_CTA>);
-#if RQ_CTA >= 256
-    case kEntryServe: return reinterpret_cast<void *>(&serveKernel<RQ_CTA>);
+    case kEntrySolve: return reinterpret_cast<void *>(&solveKernel<RQ_CTA, kCluster>);
+#if RQ_CTA >= 256 && !defined(RQ_CLUSTER)
+    case kEntryServe: return reinterpret_cast<void *>(&serveKernel<RQ_CTA, kCluster>);
 #endif
-    case kEntryOne: return reinterpret_cast<void *>(&solveOneKernel<RQ_CTA>);
+    case kEntryOne: return reinterpret_cast<void *>(&solveOneKernel<RQ_CTA, kCluster>);
+    case kEntryBytes: return reinterpret_cast<void *>(kSharedBytes);
     default: return nullptr;
     }
 }
 #else
-template <> void *solveEntry<64>(int);
-template <> void *solveEntry<128>(int);
-template <> void *solveEntry<256>(int);
-template <> void *solveEntry<512>(int);
-template <> void *solveEntry<768>(int);
-template <> void *solveEntry<1024>(int);
+template <> void *solveEntry<64, false>(int);
+template <> void *solveEntry<128, false>(int);
+template <> void *solveEntry<256, false>(int);
+template <> void *solveEntry<512, false>(int);
+template <> void *solveEntry<768, false>(int);
+template <> void *solveEntry<1024, false>(int);
+template <> void *solveEntry<kClusterThreads, true>(int);
 
 // Workspace of rq_evaluate_noalloc: one solve's scratch in a fixed device array
 // that the module owns, so that the call itself needs no device allocation. It
@@ -2868,6 +3021,9 @@ constexpr long kNoAllocScratchDoubles = 1L << 20; // 8 MiB
 static __device__ __align__(256) double g_noallocScratch[kNoAllocScratchDoubles];
 
 size_t solveSharedBytes() { return kSharedBytes; }
+size_t clusterSharedBytes() {
+    return reinterpret_cast<size_t>(solveEntry<kClusterThreads, true>(kEntryBytes));
+}
 long residentDoubles(const DevClass &C) {
     if (C.n > kResCells * kResMaxThreads)
         return 0;
@@ -2877,17 +3033,49 @@ long residentDoubles(const DevClass &C) {
 namespace {
 void *entryOf(int kind, int block) {
     switch (block) {
-    case 64: return solveEntry<64>(kind);
-    case 128: return solveEntry<128>(kind);
-    case 256: return solveEntry<256>(kind);
-    case 512: return solveEntry<512>(kind);
-    case 768: return solveEntry<768>(kind);
-    case 1024: return solveEntry<1024>(kind);
+    case 64: return solveEntry<64, false>(kind);
+    case 128: return solveEntry<128, false>(kind);
+    case 256: return solveEntry<256, false>(kind);
+    case 512: return solveEntry<512, false>(kind);
+    case 768: return solveEntry<768, false>(kind);
+    case 1024: return solveEntry<1024, false>(kind);
     default: return nullptr;
     }
 }
 void *pick(int block) { return entryOf(kEntrySolve, block); }
 void *pickServe(int block) { return entryOf(kEntryServe, block); }
+// the function of a launch shape, and its dynamic shared memory
+void *shapeEntry(int kind, const LaunchShape &sh) {
+    if (sh.cluster > 1)
+        return sh.block == kClusterThreads ? solveEntry<kClusterThreads, true>(kind) : nullptr;
+    return entryOf(kind, sh.block);
+}
+size_t shapeBytes(const LaunchShape &sh) {
+    return (sh.cluster > 1 ? clusterSharedBytes() : solveSharedBytes()) + sizeof(double) * static_cast<size_t>(sh.arenaDoubles);
+}
+cudaError_t setAttributes(void *fn, const LaunchShape &sh) {
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(shapeBytes(sh)));
+    if (e == cudaSuccess && sh.cluster > 8)
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+cudaLaunchConfig_t configOf(const LaunchShape &sh, int solves, cudaStream_t stream,
+                            cudaLaunchAttribute *attr) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(solves * sh.cluster);
+    cfg.blockDim = dim3(sh.block);
+    cfg.dynamicSmemBytes = shapeBytes(sh);
+    cfg.stream = stream;
+    if (sh.cluster > 1) {
+        attr->id = cudaLaunchAttributeClusterDimension;
+        attr->val.clusterDim.x = sh.cluster;
+        attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    return cfg;
+}
 } // namespace
 
 bool launchVariantExists(int block) { return pick(block) != nullptr; }
@@ -2898,34 +3086,45 @@ int normalizeBlock(int block) {
 }
 
 cudaError_t launchSolve(const DevJob *jobs, int njobs, int *nextJob, double *ws, long wsStride,
-                        int grid, int block, int arenaDoubles, cudaStream_t stream) {
-    const size_t smem = solveSharedBytes() + sizeof(double) * static_cast<size_t>(arenaDoubles);
-    void *fn = pick(block);
+                        int solves, const LaunchShape &sh, cudaStream_t stream) {
+    void *fn = shapeEntry(kEntrySolve, sh);
     if (!fn)
         return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    cudaError_t e = setAttributes(fn, sh);
     if (e != cudaSuccess)
         return e;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = configOf(sh, solves, stream, &attr);
+    int arenaDoubles = sh.arenaDoubles;
     void *args[] = {&jobs, &njobs, &nextJob, &ws, &wsStride, &arenaDoubles};
-    e = cudaLaunchKernel(fn, dim3(grid), dim3(block), args, smem, stream);
+    e = cudaLaunchKernelExC(&cfg, fn, args);
     if (e != cudaSuccess)
         return e;
     return cudaGetLastError();
 }
 
-int solveBlocksPerSM(int block, int arenaDoubles) {
-    const size_t smem = solveSharedBytes() + sizeof(double) * static_cast<size_t>(arenaDoubles);
-    void *fn = pick(block);
-    if (!fn)
+int concurrentSolves(const LaunchShape &sh, int sms) {
+    void *fn = shapeEntry(kEntrySolve, sh);
+    if (!fn || setAttributes(fn, sh) != cudaSuccess) {
+        cudaGetLastError();
         return 0;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-        cudaSuccess)
+    }
+    int count = 0;
+    if (sh.cluster > 1) {
+        cudaLaunchAttribute attr;
+        const cudaLaunchConfig_t cfg = configOf(sh, sms, nullptr, &attr);
+        if (cudaOccupancyMaxActiveClusters(&count, fn, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return count;
+    }
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&count, fn, sh.block, shapeBytes(sh)) !=
+        cudaSuccess) {
+        cudaGetLastError();
         return 0;
-    int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, block, smem) != cudaSuccess)
-        return 0;
-    return blocks;
+    }
+    return count * sms;
 }
 
 cudaError_t launchServe(const ServeQueue &q, double *ws, long wsStride, int grid, int block,
@@ -2976,22 +3175,23 @@ cudaError_t noAllocScratch(double **out) {
     return cudaSuccess;
 }
 
-cudaError_t launchSolveNoAlloc(const DevJob &job, double *scratch, int block, int arenaDoubles,
+cudaError_t launchSolveNoAlloc(const DevJob &job, double *scratch, const LaunchShape &sh,
                                cudaStream_t stream) {
     if (!scratch)
         return cudaErrorInvalidDevicePointer;
     double *ws = scratch;
-    void *fn = entryOf(kEntryOne, block);
+    void *fn = shapeEntry(kEntryOne, sh);
     if (!fn)
         return cudaErrorInvalidConfiguration;
-    const size_t smem = solveSharedBytes() + sizeof(double) * static_cast<size_t>(arenaDoubles);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    cudaError_t e = setAttributes(fn, sh);
     if (e != cudaSuccess)
         return e;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = configOf(sh, 1, stream, &attr);
     DevJob j = job;
+    int arenaDoubles = sh.arenaDoubles;
     void *args[] = {&j, &ws, &arenaDoubles};
-    e = cudaLaunchKernel(fn, dim3(1), dim3(block), args, smem, stream);
+    e = cudaLaunchKernelExC(&cfg, fn, args);
     if (e != cudaSuccess)
         return e;
     return cudaGetLastError();
