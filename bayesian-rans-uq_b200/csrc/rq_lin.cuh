@@ -9,7 +9,9 @@
 namespace rq {
 
 constexpr int kLinMaxLevels = 16;
-constexpr int kLinThreads = 512;
+constexpr int kLinThreads = 1024;
+constexpr int kLinMaxCluster = 16;
+constexpr int kLinLocalRows = 2048; // rows of a level that every CTA of a cluster runs whole
 enum LinKind : int32_t { kLinAmg = 0, kLinPcg = 1, kLinBicgstab = 2 };
 
 // SolverResult (core/include/LinearSolver.hpp:137-143); the layout of rq_solver_result
@@ -20,8 +22,14 @@ struct LinOut {
 
 struct DevLinLevel {
     int32_t n, nc;                   // rows; rows of the next level (0 on the coarsest)
-    int64_t vecOff;                  // b, x, r of this level in the level-vector area (levels >= 1)
-    const int32_t *ptr, *col;        // CSR (level 0: diagonal, then faces in face order)
+    int64_t vecOff;                  // b, x, r of this level in the level-vector area (levels
+                                     // 1 .. loc - 1) or in a CTA's shared memory (loc and above)
+    // Rows (level 0: diagonal, then faces in face order; above: column order) in slices of
+    // 1 << sh rows, 32 of them (a warp's loads of entry k are consecutive) or, where equal
+    // widths would more than double the entries, one (plain CSR): entry k of row i is at
+    // ptr[i >> sh] + (k << sh) + (i & ((1 << sh) - 1)); padding has column -1.
+    int32_t sh, pad;
+    const int32_t *ptr, *col;
     const double *val, *rdg;         // values, 1/diag
     const float *val32, *rdg32;      // FP32 copies (mixed form)
     const int32_t *agg;              // row -> next-level row
@@ -30,6 +38,7 @@ struct DevLinLevel {
 
 struct DevLinSys {
     int32_t n, nlev, kind, precision, maxIter, m; // m: rows of the coarsest level
+    int32_t loc, pad; // first level (>= 1) of at most kLinLocalRows rows
     double tol;
     int64_t lvOff;    // doubles: FP64 level vectors (after 8n FP64 Krylov vectors)
     int64_t f32Off;   // doubles: start of the FP32 area (mixed form)
@@ -42,10 +51,12 @@ struct DevLinSys {
     DevLinLevel lev[kLinMaxLevels];
 };
 
-// Persistent CTAs of kLinThreads threads; *next zeroed by the caller; ws: grid
-// slots of wsStride doubles.
+// Persistent clusters of `cluster` CTAs of kLinThreads threads, one system at a time each;
+// *next zeroed by the caller; ws: `slots` workspaces of wsStride doubles, one per cluster;
+// localBytes: shared memory of the local levels' vectors.
 cudaError_t launchLinear(const DevLinSys *systems, int nsys, int *next, double *ws, long wsStride,
-                         int grid, cudaStream_t stream);
-int linBlocksPerSM();
+                         int slots, int cluster, size_t localBytes, cudaStream_t stream);
+// Clusters that run at once (0: the shape does not fit).
+int linConcurrent(int cluster, size_t localBytes);
 
 } // namespace rq

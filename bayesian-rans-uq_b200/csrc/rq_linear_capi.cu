@@ -7,12 +7,32 @@ using namespace rqc;
 
 // Standalone LDU systems resident on the device (rq_linsys_*).
 struct rq_linsys {
-    int nsys = 0, kind = 0, precision = 0, maxLevels = 0, grid = 1;
-    long wsStride = 0;
+    int nsys = 0, kind = 0, precision = 0, maxLevels = 0;
+    // systems of one cluster size: a range of `sys`, the clusters launched for it with a
+    // workspace each, and a stream beside the caller's (all but the first group)
+    struct Group {
+        int first = 0, count = 0, cluster = 1, slots = 1;
+        long wsStride = 0, wsOff = 0;
+        size_t localBytes = 0;
+        cudaStream_t stream = nullptr;
+        cudaEvent_t done = nullptr;
+    };
+    std::vector<Group> groups;
+    cudaEvent_t fork = nullptr;
+    ~rq_linsys() {
+        for (Group &g : groups) {
+            if (g.done)
+                cudaEventDestroy(g.done);
+            if (g.stream)
+                cudaStreamDestroy(g.stream);
+        }
+        if (fork)
+            cudaEventDestroy(fork);
+    }
     int64_t totalRows = 0, totalNnz = 0;
     std::vector<int> rows;
     std::vector<int64_t> xOff;
-    std::vector<rq::DevLinSys> sys; // queue order (largest first), device pointers
+    std::vector<rq::DevLinSys> sys; // queue order (groups, each largest first), device pointers
     DevBuf dI, dD, dF, dB, dX, dSys, dOut, dWs, dNext;
     std::mutex mu;
 };
@@ -23,6 +43,18 @@ void checkSolveArgs(int maxIter, double tol) {
     if (maxIter < 0 || !std::isfinite(tol) || tol <= 0.)
         throw std::invalid_argument("linear solve requires matching x, nonnegative iteration "
                                     "cap and positive finite tolerance");
+}
+
+// CTAs per system, by its rows alone (so that its result does not depend on the batch): the
+// smallest power of two that leaves a thread no more than two to four rows, at most 16.
+// Measured on a B200, ms per FP64 AMG solve to 1e-10 of one n x n system with 8 / 4 / 2 rows
+// per thread as the bound: n = 64 1.70 / 1.63 / 1.46, n = 128 3.16 / 2.53 / 2.30, n = 256
+// (16 CTAs in all three) 4.06, n = 512 11.4 (about 260 with one CTA).
+int linCluster(int rows) {
+    int c = 1;
+    while (c < rq::kLinMaxCluster && 2L * c * rq::kLinThreads <= rows)
+        c *= 2;
+    return c;
 }
 
 void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int precision) {
@@ -75,26 +107,34 @@ void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int preci
         int s, l, what;
         size_t off;
         const void *src; // std::vector<int> or std::vector<double> of the host set-up
+        const rq::LinLevelHost *lv; // P_COL, P_VAL, P_VAL32: the level, laid out in slices
+        size_t count;
     };
     std::vector<Piece> pieces;
     size_t nI = 0, nD = 0, nF = 0;
     auto addI = [&](int s, int l, int what, const std::vector<int> &v) {
-        pieces.push_back({s, l, what, nI, &v});
+        pieces.push_back({s, l, what, nI, &v, nullptr, v.size()});
         nI += (v.size() + 7) / 8 * 8;
     };
     auto addD = [&](int s, int l, int what, const std::vector<double> &v) {
-        pieces.push_back({s, l, what, nD, &v});
+        pieces.push_back({s, l, what, nD, &v, nullptr, v.size()});
         nD += (v.size() + 3) / 4 * 4;
     };
     auto addF = [&](int s, int l, int what, const std::vector<double> &v) {
-        pieces.push_back({s, l, what, nF, &v});
+        pieces.push_back({s, l, what, nF, &v, nullptr, v.size()});
         nF += (v.size() + 7) / 8 * 8;
+    };
+    auto addRows = [&](int s, int l, int what, const rq::LinLevelHost &lv, size_t &total) {
+        const size_t cnt = lv.slice.back();
+        pieces.push_back({s, l, what, total, nullptr, &lv, cnt});
+        total += (cnt + 7) / 8 * 8;
     };
     const bool mixed = precision == RQ_PREC_MIXED;
     L.rows.resize(n);
     L.xOff.resize(n);
     std::vector<rq::DevLinSys> byIndex(n);
-    long wsMax = 0;
+    std::vector<long> wsOf(n);
+    std::vector<size_t> localOf(n);
     for (int s = 0; s < n; ++s) {
         const rq::LinSysHost &h = H[s];
         rq::DevLinSys &d = byIndex[s];
@@ -107,21 +147,26 @@ void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int preci
         d.kind = kind;
         d.precision = mixed && kind != rq::kLinBicgstab ? 1 : 0;
         d.m = h.m;
-        long lvecs = 0;
+        d.loc = nl;
+        while (d.loc > 1 && h.lev[d.loc - 1].n <= rq::kLinLocalRows)
+            --d.loc;
+        long lvecs = 0, local = 0;
         for (int l = 0; l < nl; ++l) {
             const rq::LinLevelHost &lv = h.lev[l];
             rq::DevLinLevel &dl = d.lev[l];
             dl.n = lv.n;
             dl.nc = lv.nc;
-            dl.vecOff = l > 0 ? lvecs : 0;
+            dl.sh = lv.sh;
+            long &vecs = l >= d.loc ? local : lvecs;
+            dl.vecOff = l > 0 ? vecs : 0;
             if (l > 0)
-                lvecs += 3L * lv.n;
-            addI(s, l, P_PTR, lv.ptr);
-            addI(s, l, P_COL, lv.col);
-            addD(s, l, P_VAL, lv.val);
+                vecs += 3L * lv.n;
+            addI(s, l, P_PTR, lv.slice);
+            addRows(s, l, P_COL, lv, nI);
+            addRows(s, l, P_VAL, lv, nD);
             addD(s, l, P_RDG, lv.rdg);
             if (d.precision) {
-                addF(s, l, P_VAL32, lv.val);
+                addRows(s, l, P_VAL32, lv, nF);
                 addF(s, l, P_RDG32, lv.rdg);
             }
             if (l + 1 < nl) {
@@ -141,7 +186,8 @@ void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int preci
         d.f32Off = d.lvOff + pad32(lvecs);
         d.lvOff32 = 2 * pad32((6 * nn + 1) / 2);
         const long ws = d.f32Off + (d.precision ? (d.lvOff32 / 2 + pad32((lvecs + 1) / 2)) : 0);
-        wsMax = std::max(wsMax, ws);
+        wsOf[s] = ws;
+        localOf[s] = static_cast<size_t>(local) * (d.precision ? sizeof(float) : sizeof(double));
         L.rows[s] = h.n;
         L.xOff[s] = L.totalRows;
         L.totalRows += h.n;
@@ -156,17 +202,38 @@ void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int preci
                                                  static_cast<int>(std::thread::hardware_concurrency())));
         std::atomic<size_t> next{0};
         std::atomic<int> nextRhs{0};
+        // the entries of a level in slices: put(position, CSR entry or -1 for padding)
+        auto spread = [](const rq::LinLevelHost &lv, auto put) {
+            const int c = 1 << lv.sh;
+            for (int i = 0; i < (lv.n + c - 1) / c * c; ++i) {
+                const int at = lv.slice[i >> lv.sh], w = (lv.slice[(i >> lv.sh) + 1] - at) >> lv.sh;
+                const int k0 = i < lv.n ? lv.ptr[i] : 0, len = i < lv.n ? lv.ptr[i + 1] - k0 : 0;
+                for (int k = 0; k < w; ++k)
+                    put(at + (k << lv.sh) + (i & (c - 1)), k < len ? k0 + k : -1);
+            }
+        };
         auto work = [&] {
             for (size_t k = next++; k < pieces.size(); k = next++) {
                 const Piece &p = pieces[k];
                 switch (p.what) {
-                case P_PTR: case P_COL: case P_AGG: case P_CPTR: case P_CIDX: {
+                case P_COL:
+                    spread(*p.lv, [&](int at, int e) { I[p.off + at] = e < 0 ? -1 : p.lv->col[e]; });
+                    break;
+                case P_VAL:
+                    spread(*p.lv, [&](int at, int e) { D[p.off + at] = e < 0 ? 0.0 : p.lv->val[e]; });
+                    break;
+                case P_VAL32:
+                    spread(*p.lv, [&](int at, int e) {
+                        F[p.off + at] = e < 0 ? 0.0f : static_cast<float>(p.lv->val[e]);
+                    });
+                    break;
+                case P_PTR: case P_AGG: case P_CPTR: case P_CIDX: {
                     const auto &v = *static_cast<const std::vector<int> *>(p.src);
                     std::copy(v.begin(), v.end(), I.get() + p.off);
                     std::fill(I.get() + p.off + v.size(), I.get() + p.off + (v.size() + 7) / 8 * 8, 0);
                     break;
                 }
-                case P_VAL: case P_RDG: case P_INV: {
+                case P_RDG: case P_INV: {
                     const auto &v = *static_cast<const std::vector<double> *>(p.src);
                     std::copy(v.begin(), v.end(), D.get() + p.off);
                     std::fill(D.get() + p.off + v.size(), D.get() + p.off + (v.size() + 3) / 4 * 4, 0.0);
@@ -227,24 +294,47 @@ void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int preci
         byIndex[s].x = L.dX.as<double>() + L.xOff[s];
         byIndex[s].out = L.dOut.as<rq::LinOut>() + s;
     }
-    // queue order: largest systems first (longest-processing-time)
+    // queue order: by cluster size, largest systems first (longest-processing-time)
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return L.rows[a] > L.rows[b]; });
     L.sys.clear();
-    for (int s : order)
+    long wsTotal = 0;
+    for (int s : order) {
+        const int cluster = linCluster(L.rows[s]);
+        if (L.groups.empty() || L.groups.back().cluster != cluster) {
+            L.groups.emplace_back();
+            L.groups.back().first = static_cast<int>(L.sys.size());
+            L.groups.back().cluster = cluster;
+        }
+        rq_linsys::Group &g = L.groups.back();
+        ++g.count;
+        g.wsStride = std::max(g.wsStride, wsOf[s]);
+        g.localBytes = std::max(g.localBytes, localOf[s]);
         L.sys.push_back(byIndex[s]);
-    int dev = 0, sms = 1;
-    check(cudaGetDevice(&dev), "cudaGetDevice");
-    check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attribute");
-    const int perSM = std::max(1, rq::linBlocksPerSM());
-    L.grid = std::max(1, std::min(n, sms * perSM));
-    L.wsStride = wsMax;
-    L.dWs.ensure(sizeof(double) * wsMax * L.grid);
+    }
+    for (size_t k = 0; k < L.groups.size(); ++k) {
+        rq_linsys::Group &g = L.groups[k];
+        const int atOnce = rq::linConcurrent(g.cluster, g.localBytes);
+        if (atOnce < 1)
+            throw RqError(RQ_E_CUDA, "linear solve kernel does not fit on an SM");
+        g.slots = std::min(g.count, atOnce);
+        g.wsOff = wsTotal;
+        wsTotal += g.wsStride * g.slots;
+        if (k > 0) {
+            check(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking), "stream");
+            check(cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming), "event");
+        }
+    }
+    if (L.groups.size() > 1)
+        check(cudaEventCreateWithFlags(&L.fork, cudaEventDisableTiming), "event");
+    L.dWs.ensure(sizeof(double) * wsTotal);
     L.dSys.ensure(sizeof(rq::DevLinSys) * n);
-    L.dNext.ensure(sizeof(int));
+    L.dNext.ensure(sizeof(int) * L.groups.size());
 }
 
+// One launch per cluster size, side by side: the first on the caller's stream, the others
+// on streams of the handle that fork from it and join it.
 void launchLinsys(rq_linsys &L, int maxIter, double tol, cudaStream_t stream) {
     for (auto &d : L.sys) {
         d.maxIter = maxIter;
@@ -252,9 +342,22 @@ void launchLinsys(rq_linsys &L, int maxIter, double tol, cudaStream_t stream) {
     }
     check(cudaMemcpyAsync(L.dSys.p, L.sys.data(), sizeof(rq::DevLinSys) * L.nsys,
                           cudaMemcpyHostToDevice, stream), "systems");
-    check(cudaMemsetAsync(L.dNext.p, 0, sizeof(int), stream), "counter");
-    check(rq::launchLinear(L.dSys.as<rq::DevLinSys>(), L.nsys, L.dNext.as<int>(),
-                           L.dWs.as<double>(), L.wsStride, L.grid, stream), "linear solve launch");
+    check(cudaMemsetAsync(L.dNext.p, 0, sizeof(int) * L.groups.size(), stream), "counter");
+    if (L.fork)
+        check(cudaEventRecord(L.fork, stream), "event record");
+    for (size_t k = 0; k < L.groups.size(); ++k) {
+        const rq_linsys::Group &g = L.groups[k];
+        const cudaStream_t st = k ? g.stream : stream;
+        if (k)
+            check(cudaStreamWaitEvent(st, L.fork, 0), "stream wait");
+        check(rq::launchLinear(L.dSys.as<rq::DevLinSys>() + g.first, g.count,
+                               L.dNext.as<int>() + k, L.dWs.as<double>() + g.wsOff, g.wsStride,
+                               g.slots, g.cluster, g.localBytes, st), "linear solve launch");
+        if (k) {
+            check(cudaEventRecord(g.done, st), "event record");
+            check(cudaStreamWaitEvent(stream, g.done, 0), "stream wait");
+        }
+    }
 }
 
 void fetchLinsys(rq_linsys &L, double *const *x, rq_solver_result *results) {
@@ -262,12 +365,10 @@ void fetchLinsys(rq_linsys &L, double *const *x, rq_solver_result *results) {
     if (results)
         check(cudaMemcpy(results, L.dOut.p, sizeof(rq::LinOut) * L.nsys, cudaMemcpyDeviceToHost),
               "results");
-    if (x) {
-        std::vector<double> hx(L.totalRows);
-        check(cudaMemcpy(hx.data(), L.dX.p, sizeof(double) * hx.size(), cudaMemcpyDeviceToHost), "x");
+    if (x) // straight into the caller's arrays
         for (int s = 0; s < L.nsys; ++s)
-            std::memcpy(x[s], hx.data() + L.xOff[s], sizeof(double) * L.rows[s]);
-    }
+            check(cudaMemcpy(x[s], L.dX.as<double>() + L.xOff[s], sizeof(double) * L.rows[s],
+                             cudaMemcpyDeviceToHost), "x");
 }
 
 } // namespace

@@ -1,6 +1,6 @@
-// Standalone batched linear solves on the device: one CTA per LDU system,
-// persistent CTAs pulling systems from a queue (largest first, as the host
-// orders them). The solvers restate core/include/LinearSolver.hpp on CSR:
+// Standalone batched linear solves on the device: one thread-block cluster per LDU system
+// (1 to 16 CTAs by its rows), persistent clusters pulling systems from a queue (largest
+// first, as the host orders them). The solvers restate core/include/LinearSolver.hpp:
 //   PCG (:184-246) with the Jacobi preconditioner or the AMG V-cycle of this
 //   project (damped-Jacobi smoothing, aggregate-sum restriction, aggregate
 //   broadcast prolongation scaled by an over-correction factor, dense coarsest
@@ -8,9 +8,15 @@
 //   (:251-345), and a mixed form: FP32 PCG corrections inside an FP64
 //   residual-refinement loop.
 // Level 0 keeps the reference's matvec order per row (diagonal, then faces in
-// increasing index); coarse levels are column-sorted CSR. Every dot product
+// increasing index); coarse levels are column-sorted. Every dot product
 // and norm is an FP64 block reduction whose result all threads share, so
-// control flow is uniform and results do not depend on the launch shape.
+// control flow is uniform.
+//
+// What bounds it: a large system streams its rows and vectors from HBM or L2, a small one
+// is a chain of phases of a microsecond each. Rows are stored in slices of 32, so that a
+// warp's loads of entry k are consecutive; a damped-Jacobi sweep is one pass from one
+// vector to another; the levels of up to 2048 rows run whole in every CTA of the cluster,
+// on vectors in its shared memory and with its own barrier (about 80 cycles against 500).
 #include "rq_lin.cuh"
 
 #include <cuda_runtime.h>
@@ -28,16 +34,39 @@ constexpr int kSweeps = 2;     // pre- and post-smoothing sweeps
 constexpr int kMixedRounds = 12;
 constexpr double kMixedInnerTol = 1e-4; // relative drop asked of each FP32 correction
 
-template <int NT> struct LinShared {
-    DevLinSys sys;
-    double red[4][NT / 32];
-    int job;
-};
+constexpr int NT = kLinThreads;
 
-// Sum of K per-thread values over the CTA. Each warp reduces by shuffles, lane 0
-// parks the partial, and every warp re-reduces all partials in the same order,
-// so every thread returns the same bits.
-template <int NT, int K> __device__ __forceinline__ void blockSum(double (&v)[K], LinShared<NT> &S) {
+struct LinShared {
+    DevLinSys sys;
+    double red[2][NT / 32];
+    double cred[2][2][kLinMaxCluster]; // the CTAs' sums, in alternating buffers
+    int job;
+    int rank, ctas;
+};
+extern __shared__ __align__(16) unsigned char linSmem[]; // vectors of the local levels
+
+// thread index in the cluster and its threads; the cluster's barrier
+__device__ __forceinline__ int gTid(const LinShared &S) { return S.rank * NT + threadIdx.x; }
+__device__ __forceinline__ int gThreads(const LinShared &S) { return S.ctas * NT; }
+__device__ __forceinline__ void gSync(const LinShared &S) {
+    if (S.ctas > 1)
+        asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    else
+        __syncthreads();
+}
+template <typename V> __device__ __forceinline__ void putRemote(V *p, V v, int rank) {
+    unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(p)), r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    if constexpr (sizeof(V) == 8)
+        asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(r), "l"(__double_as_longlong(v)) : "memory");
+    else
+        asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(r), "r"(static_cast<int>(v)) : "memory");
+}
+
+// Sum of K per-thread values over the cluster. Each warp reduces by shuffles, lane 0
+// parks the partial, every warp re-reduces all partials in the same order, and the CTAs'
+// sums are exchanged and added in rank order, so every thread returns the same bits.
+template <int K> __device__ __forceinline__ void blockSum(double (&v)[K], LinShared &S, int &rp) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -51,134 +80,206 @@ template <int NT, int K> __device__ __forceinline__ void blockSum(double (&v)[K]
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        double s = lane < NT / 32 ? S.red[k][lane] : 0.0;
+        double s = S.red[k][lane];
         for (int o = 16; o > 0; o >>= 1)
             s += __shfl_xor_sync(FULL, s, o);
-        v[k] = __shfl_sync(FULL, s, 0);
+        v[k] = s;
+    }
+    if (S.ctas > 1) {
+        if (static_cast<int>(threadIdx.x) < S.ctas)
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                putRemote(&S.cred[rp][k][S.rank], v[k], threadIdx.x);
+        gSync(S);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            v[k] = S.cred[rp][k][0];
+            for (int c = 1; c < S.ctas; ++c)
+                v[k] += S.cred[rp][k][c];
+        }
+        rp ^= 1;
     }
 }
+static_assert(NT / 32 == 32, "blockSum reads one partial per lane");
 
 // one level of the hierarchy in value type T (FP64, or the FP32 copies)
 template <typename T> struct Lv {
-    int n, nc;
+    int n, nc, sh;
     const int *ptr, *col;
     const T *val, *rdg;
     const int *agg, *childPtr, *childIdx;
     T *b, *x, *r; // workspace vectors (levels >= 1; level 0 uses the caller's)
 };
 
+// Row i times x, entries in order. Five columns and values (a grid system's row) are
+// loaded before the first is used.
 template <typename T> __device__ __forceinline__ T rowTimes(const Lv<T> &A, int i, const T *x) {
-    const int k0 = __ldg(A.ptr + i), k1 = __ldg(A.ptr + i + 1);
+    const int k0 = __ldg(A.ptr + (i >> A.sh)), k1 = __ldg(A.ptr + (i >> A.sh) + 1);
+    const int step = 1 << A.sh;
     T s = T(0);
-    for (int k = k0; k < k1; ++k)
-        s += __ldg(A.val + k) * x[__ldg(A.col + k)];
+    for (int e = k0 + (i & (step - 1)); e < k1; e += 5 * step) {
+        int c[5];
+        T v[5], xc[5];
+#pragma unroll
+        for (int u = 0; u < 5; ++u) {
+            const bool in = e + u * step < k1;
+            c[u] = in ? __ldg(A.col + e + u * step) : -1;
+            v[u] = in ? __ldg(A.val + e + u * step) : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < 5; ++u)
+            xc[u] = c[u] >= 0 ? x[c[u]] : T(0);
+#pragma unroll
+        for (int u = 0; u < 5; ++u)
+            if (c[u] >= 0)
+                s += v[u] * xc[u];
+    }
     return s;
 }
 
-template <typename T> __device__ __forceinline__ Lv<T> levelOf(const DevLinSys &S, int l, void *ws);
-
-template <> __device__ __forceinline__ Lv<double> levelOf<double>(const DevLinSys &S, int l, void *ws) {
+template <typename T>
+__device__ __forceinline__ Lv<T> levelOf(const DevLinSys &S, int l, void *ws) {
     const DevLinLevel &d = S.lev[l];
-    double *w = static_cast<double *>(ws);
-    return Lv<double>{d.n, d.nc, d.ptr, d.col, d.val, d.rdg, d.agg, d.childPtr, d.childIdx,
-                      w + d.vecOff, w + d.vecOff + d.n, w + d.vecOff + 2L * d.n};
-}
-template <> __device__ __forceinline__ Lv<float> levelOf<float>(const DevLinSys &S, int l, void *ws) {
-    const DevLinLevel &d = S.lev[l];
-    float *w = static_cast<float *>(ws);
-    return Lv<float>{d.n, d.nc, d.ptr, d.col, d.val32, d.rdg32, d.agg, d.childPtr, d.childIdx,
-                     w + d.vecOff, w + d.vecOff + d.n, w + d.vecOff + 2L * d.n};
+    T *w = static_cast<T *>(l >= S.loc ? static_cast<void *>(linSmem) : ws) + d.vecOff;
+    Lv<T> A{d.n, d.nc, d.sh, d.ptr, d.col, nullptr, nullptr, d.agg, d.childPtr, d.childIdx,
+            w, w + d.n, w + 2L * d.n};
+    if constexpr (sizeof(T) == 8) {
+        A.val = d.val;
+        A.rdg = d.rdg;
+    } else {
+        A.val = d.val32;
+        A.rdg = d.rdg32;
+    }
+    return A;
 }
 
 // z = M^-1 r by one V-cycle: damped Jacobi from zero, residual restricted by
 // aggregate sums, the coarsest level by its dense inverse, the correction
 // broadcast back and the same sweeps after it (a symmetric preconditioner).
-// lvws: the level vectors of levels >= 1; t: a level-0 scratch vector.
-template <int NT, typename T>
-__device__ void vcycle(LinShared<NT> &S, const T *r, T *z, T *t, void *lvws, const T *inv) {
+// lvws: the level vectors of levels 1 .. loc - 1; t: a level-0 scratch vector. A level's
+// iterate alternates between x and r; its solution ends in r (the coarsest's in x).
+// Returns this thread's part of (r, z).
+template <typename T>
+__device__ double vcycle(LinShared &S, const T *r, T *z, T *t, void *lvws, const T *inv) {
+    static_assert(kSweeps == 2, "the buffers alternate for two sweeps");
     const DevLinSys &sys = S.sys;
     const int L = sys.nlev;
     const T w = T(kOmega);
+    double rz = 0.0;
     if (L == 1) { // the whole system is the coarsest level
         const int m = sys.m;
-        for (int i = threadIdx.x; i < m; i += NT) {
+        for (int i = gTid(S); i < m; i += gThreads(S)) {
             T s = T(0);
             for (int j = 0; j < m; ++j)
                 s += inv[i * m + j] * r[j];
             z[i] = s;
+            rz += double(r[i]) * double(s);
         }
-        __syncthreads();
-        return;
+        return rz;
     }
+    auto tid = [&](int l) { return l >= sys.loc ? static_cast<int>(threadIdx.x) : gTid(S); };
+    auto threads = [&](int l) { return l >= sys.loc ? NT : gThreads(S); };
+    auto sync = [&](int l) {
+        if (l >= sys.loc)
+            __syncthreads();
+        else
+            gSync(S);
+    };
+    const T *fr = nullptr; // residual of the level above
     for (int l = 0; l + 1 < L; ++l) {
         Lv<T> A = levelOf<T>(sys, l, lvws);
+        const int t0 = tid(l), nt = threads(l);
         const T *b = l == 0 ? r : A.b;
-        T *x = l == 0 ? z : A.x;
-        T *res = l == 0 ? t : A.r;
-        for (int i = threadIdx.x; i < A.n; i += NT)
-            x[i] = w * b[i] * __ldg(A.rdg + i);
-        __syncthreads();
-        for (int s = 1; s < kSweeps; ++s) {
-            for (int i = threadIdx.x; i < A.n; i += NT)
-                res[i] = b[i] - rowTimes(A, i, x);
-            __syncthreads();
-            for (int i = threadIdx.x; i < A.n; i += NT)
-                x[i] += w * res[i] * __ldg(A.rdg + i);
-            __syncthreads();
+        T *x = l == 0 ? t : A.x, *y = l == 0 ? z : A.r;
+        if (l == 0) {
+            for (int i = t0; i < A.n; i += nt)
+                x[i] = w * b[i] * __ldg(A.rdg + i);
+        } else { // restricted right-hand side
+            const Lv<T> F = levelOf<T>(sys, l - 1, lvws);
+            for (int i = t0; i < A.n; i += nt) {
+                T s = T(0);
+                for (int k = __ldg(F.childPtr + i); k < __ldg(F.childPtr + i + 1); ++k)
+                    s += fr[__ldg(F.childIdx + k)];
+                A.b[i] = s;
+                x[i] = w * s * __ldg(A.rdg + i);
+            }
         }
-        for (int i = threadIdx.x; i < A.n; i += NT)
-            res[i] = b[i] - rowTimes(A, i, x);
-        __syncthreads();
-        Lv<T> Cn = levelOf<T>(sys, l + 1, lvws);
-        for (int I = threadIdx.x; I < A.nc; I += NT) {
-            T s = T(0);
-            for (int k = __ldg(A.childPtr + I); k < __ldg(A.childPtr + I + 1); ++k)
-                s += res[__ldg(A.childIdx + k)];
-            Cn.b[I] = s;
+        sync(l);
+        for (int i = t0; i < A.n; i += nt) {
+            const T res = b[i] - rowTimes(A, i, x);
+            y[i] = x[i] + w * res * __ldg(A.rdg + i);
         }
-        __syncthreads();
+        sync(l);
+        for (int i = t0; i < A.n; i += nt)
+            x[i] = b[i] - rowTimes(A, i, y);
+        sync(l);
+        fr = x;
     }
+    const T *xc;
     {
-        Lv<T> Cl = levelOf<T>(sys, L - 1, lvws);
-        const int m = Cl.n;
-        for (int i = threadIdx.x; i < m; i += NT) {
+        const int l = L - 1, t0 = tid(l), nt = threads(l);
+        Lv<T> A = levelOf<T>(sys, l, lvws);
+        const Lv<T> F = levelOf<T>(sys, l - 1, lvws);
+        const int m = A.n;
+        for (int i = t0; i < m; i += nt) {
+            T s = T(0);
+            for (int k = __ldg(F.childPtr + i); k < __ldg(F.childPtr + i + 1); ++k)
+                s += fr[__ldg(F.childIdx + k)];
+            A.b[i] = s;
+        }
+        sync(l);
+        for (int i = t0; i < m; i += nt) {
             T s = T(0);
             for (int j = 0; j < m; ++j)
-                s += inv[i * m + j] * Cl.b[j];
-            Cl.x[i] = s;
+                s += inv[i * m + j] * A.b[j];
+            A.x[i] = s;
         }
-        __syncthreads();
+        sync(l);
+        xc = A.x;
     }
     for (int l = L - 2; l >= 0; --l) {
         Lv<T> A = levelOf<T>(sys, l, lvws);
-        const Lv<T> Cn = levelOf<T>(sys, l + 1, lvws);
+        const int t0 = tid(l), nt = threads(l);
         const T *b = l == 0 ? r : A.b;
-        T *x = l == 0 ? z : A.x;
-        T *res = l == 0 ? t : A.r;
-        for (int i = threadIdx.x; i < A.n; i += NT)
-            x[i] += T(kAlpha) * Cn.x[__ldg(A.agg + i)];
-        __syncthreads();
-        for (int s = 0; s < kSweeps; ++s) {
-            for (int i = threadIdx.x; i < A.n; i += NT)
-                res[i] = b[i] - rowTimes(A, i, x);
-            __syncthreads();
-            for (int i = threadIdx.x; i < A.n; i += NT)
-                x[i] += w * res[i] * __ldg(A.rdg + i);
-            __syncthreads();
+        T *x = l == 0 ? t : A.x, *y = l == 0 ? z : A.r;
+        for (int i = t0; i < A.n; i += nt)
+            y[i] += T(kAlpha) * xc[__ldg(A.agg + i)];
+        sync(l);
+        for (int i = t0; i < A.n; i += nt) {
+            const T res = b[i] - rowTimes(A, i, y);
+            x[i] = y[i] + w * res * __ldg(A.rdg + i);
         }
+        sync(l);
+        for (int i = t0; i < A.n; i += nt) {
+            const T res = b[i] - rowTimes(A, i, x);
+            const T zi = x[i] + w * res * __ldg(A.rdg + i);
+            y[i] = zi;
+            if (l == 0)
+                rz += double(r[i]) * double(zi);
+        }
+        if (l > 0) // level 0: the caller's block sum
+            sync(l);
+        xc = y;
     }
+    return rz;
 }
 
-template <int NT, typename T>
-__device__ __forceinline__ void precondition(LinShared<NT> &S, bool amg, const T *r, T *z, T *t,
-                                             void *lvws, const T *inv, const T *rdg0) {
+// z = M^-1 r; returns (r, z)
+template <typename T>
+__device__ __forceinline__ double precondition(LinShared &S, int &rp, bool amg, const T *r, T *z,
+                                               T *t, void *lvws, const T *inv, const T *rdg0) {
+    double a[1] = {0.0};
     if (amg) {
-        vcycle<NT, T>(S, r, z, t, lvws, inv);
+        a[0] = vcycle<T>(S, r, z, t, lvws, inv);
     } else {
-        for (int i = threadIdx.x; i < S.sys.n; i += NT)
-            z[i] = r[i] * __ldg(rdg0 + i);
-        __syncthreads();
+        for (int i = gTid(S); i < S.sys.n; i += gThreads(S)) {
+            const T zi = r[i] * __ldg(rdg0 + i);
+            z[i] = zi;
+            a[0] += double(r[i]) * double(zi);
+        }
     }
+    blockSum<1>(a, S, rp);
+    return a[0];
 }
 
 struct PcgOut {
@@ -189,132 +290,123 @@ struct PcgOut {
 
 // PCG from x (in T) with r = b - A x already in r and r0n = ||r||; the
 // reference's loop (LinearSolver.hpp:206-245). Vectors r, z, p, q, t: n each.
-template <int NT, typename T>
-__device__ PcgOut pcg(LinShared<NT> &S, const Lv<T> &A0, T *x, T *r, T *z, T *p, T *q, T *t,
+template <typename T>
+__device__ PcgOut pcg(LinShared &S, int &rp, const Lv<T> &A0, T *x, T *r, T *z, T *p, T *q, T *t,
                       void *lvws, const T *inv, double r0n, int maxIter, double tol, bool amg) {
     const int n = A0.n;
     PcgOut o{0, false, 0.0};
-    precondition<NT, T>(S, amg, r, z, t, lvws, inv, A0.rdg);
-    double a[1] = {0.0};
-    for (int i = threadIdx.x; i < n; i += NT) {
+    double rz = precondition<T>(S, rp, amg, r, z, t, lvws, inv, A0.rdg);
+    for (int i = gTid(S); i < n; i += gThreads(S))
         p[i] = z[i];
-        a[0] += double(r[i]) * double(z[i]);
-    }
-    blockSum<NT, 1>(a, S);
-    double rz = a[0];
+    gSync(S);
     for (int it = 0; it < maxIter; ++it) {
         double b1[1] = {0.0};
-        for (int i = threadIdx.x; i < n; i += NT) {
+        for (int i = gTid(S); i < n; i += gThreads(S)) {
             const T v = rowTimes(A0, i, p);
             q[i] = v;
             b1[0] += double(p[i]) * double(v);
         }
-        blockSum<NT, 1>(b1, S);
+        blockSum<1>(b1, S, rp);
         const double pAp = b1[0];
         if (fabs(pAp) < 1e-30)
             break;
         const double alpha = rz / pAp;
         double b2[1] = {0.0};
-        for (int i = threadIdx.x; i < n; i += NT) {
+        for (int i = gTid(S); i < n; i += gThreads(S)) {
             x[i] += T(alpha) * p[i];
             const T ri = r[i] - T(alpha) * q[i];
             r[i] = ri;
             b2[0] += double(ri) * double(ri);
         }
-        blockSum<NT, 1>(b2, S);
+        blockSum<1>(b2, S, rp);
         o.iterations = it + 1;
         o.finalRes = sqrt(b2[0]) / r0n;
         if (o.finalRes < tol) {
             o.converged = true;
             return o;
         }
-        precondition<NT, T>(S, amg, r, z, t, lvws, inv, A0.rdg);
-        double b3[1] = {0.0};
-        for (int i = threadIdx.x; i < n; i += NT)
-            b3[0] += double(r[i]) * double(z[i]);
-        blockSum<NT, 1>(b3, S);
-        const double beta = b3[0] / (rz + 1e-30);
-        for (int i = threadIdx.x; i < n; i += NT)
+        const double rzNew = precondition<T>(S, rp, amg, r, z, t, lvws, inv, A0.rdg);
+        const double beta = rzNew / (rz + 1e-30);
+        for (int i = gTid(S); i < n; i += gThreads(S))
             p[i] = z[i] + T(beta) * p[i];
-        __syncthreads();
-        rz = b3[0];
+        gSync(S);
+        rz = rzNew;
     }
     return o;
 }
 
 // Right-Jacobi BiCGSTAB (LinearSolver.hpp:251-345) in FP64; r holds b - A x.
-template <int NT>
-__device__ PcgOut bicgstab(LinShared<NT> &S, const Lv<double> &A0, double *x, double *ws,
+__device__ PcgOut bicgstab(LinShared &S, int &rp, const Lv<double> &A0, double *x, double *ws,
                            double r0n, int maxIter, double tol) {
     const int n = A0.n;
     double *r = ws, *rh = ws + n, *p = ws + 2L * n, *v = ws + 3L * n, *s = ws + 4L * n,
            *t = ws + 5L * n, *ph = ws + 6L * n, *sh = ws + 7L * n;
     PcgOut o{0, false, 0.0};
     double a[1] = {0.0};
-    for (int i = threadIdx.x; i < n; i += NT) {
+    for (int i = gTid(S); i < n; i += gThreads(S)) {
         rh[i] = r[i];
         p[i] = 0.0;
         v[i] = 0.0;
         a[0] += r[i] * r[i];
     }
-    blockSum<NT, 1>(a, S);
+    blockSum<1>(a, S, rp);
     double rhoN = a[0], rho = 1, alpha = 1, omega = 1;
     for (int it = 0; it < maxIter; ++it) {
         if (fabs(rhoN) < 1e-30)
             break;
         const double beta = (rhoN / (rho + 1e-30)) * (alpha / (omega + 1e-30));
-        for (int i = threadIdx.x; i < n; i += NT) {
+        for (int i = gTid(S); i < n; i += gThreads(S)) {
             const double pi = r[i] + beta * (p[i] - omega * v[i]);
             p[i] = pi;
             ph[i] = pi * __ldg(A0.rdg + i);
         }
-        __syncthreads();
+        gSync(S);
         double a1[1] = {0.0};
-        for (int i = threadIdx.x; i < n; i += NT) {
+        for (int i = gTid(S); i < n; i += gThreads(S)) {
             const double vi = rowTimes(A0, i, ph);
             v[i] = vi;
             a1[0] += rh[i] * vi;
         }
-        blockSum<NT, 1>(a1, S);
+        blockSum<1>(a1, S, rp);
         if (fabs(a1[0]) < 1e-30)
             break;
         alpha = rhoN / a1[0];
         double a2[1] = {0.0};
-        for (int i = threadIdx.x; i < n; i += NT) {
+        for (int i = gTid(S); i < n; i += gThreads(S)) {
             const double si = r[i] - alpha * v[i];
             s[i] = si;
             sh[i] = si * __ldg(A0.rdg + i);
             a2[0] += si * si;
         }
-        blockSum<NT, 1>(a2, S);
+        blockSum<1>(a2, S, rp);
         const double sn = sqrt(a2[0]);
         if (sn / r0n < tol) {
-            for (int i = threadIdx.x; i < n; i += NT)
+            for (int i = gTid(S); i < n; i += gThreads(S))
                 x[i] += alpha * ph[i];
-            __syncthreads();
+            gSync(S);
             o.iterations = it + 1;
             o.finalRes = sn / r0n;
             o.converged = true;
             return o;
         }
         double a3[2] = {0.0, 0.0};
-        for (int i = threadIdx.x; i < n; i += NT) {
+        for (int i = gTid(S); i < n; i += gThreads(S)) {
             const double ti = rowTimes(A0, i, sh);
             t[i] = ti;
             a3[0] += ti * ti;
             a3[1] += ti * s[i];
         }
-        blockSum<NT, 2>(a3, S);
+        blockSum<2>(a3, S, rp);
         omega = a3[0] > 1e-30 ? a3[1] / a3[0] : 0.0;
         double a4[2] = {0.0, 0.0};
-        for (int i = threadIdx.x; i < n; i += NT) {
+        for (int i = gTid(S); i < n; i += gThreads(S)) {
             x[i] += alpha * ph[i] + omega * sh[i];
             const double ri = s[i] - omega * t[i];
             r[i] = ri;
             a4[0] += ri * ri;
             a4[1] += rh[i] * ri;
         }
-        blockSum<NT, 2>(a4, S);
+        blockSum<2>(a4, S, rp);
         o.iterations = it + 1;
         o.finalRes = sqrt(a4[0]) / r0n;
         if (o.finalRes < tol) {
@@ -326,42 +418,41 @@ __device__ PcgOut bicgstab(LinShared<NT> &S, const Lv<double> &A0, double *x, do
         rho = rhoN;
         rhoN = a4[1];
     }
-    __syncthreads();
+    gSync(S);
     return o;
 }
 
 // r = b - A x in FP64; returns ||r||
-template <int NT>
-__device__ double residual(LinShared<NT> &S, const Lv<double> &A0, const double *b,
+__device__ double residual(LinShared &S, int &rp, const Lv<double> &A0, const double *b,
                            const double *x, double *r) {
     double a[1] = {0.0};
-    for (int i = threadIdx.x; i < A0.n; i += NT) {
+    for (int i = gTid(S); i < A0.n; i += gThreads(S)) {
         const double ri = b[i] - rowTimes(A0, i, x);
         r[i] = ri;
         a[0] += ri * ri;
     }
-    blockSum<NT, 1>(a, S);
+    blockSum<1>(a, S, rp);
     return sqrt(a[0]);
 }
 
-template <int NT> __device__ void solveOne(LinShared<NT> &S, double *ws) {
+__device__ void solveOne(LinShared &S, int &rp, double *ws) {
     const DevLinSys &sys = S.sys;
     const int n = sys.n;
     const bool amg = sys.kind == kLinAmg;
     const Lv<double> A0 = levelOf<double>(sys, 0, ws + sys.lvOff);
     double *x = sys.x;
     double *r = ws;
-    const double r0n = residual<NT>(S, A0, sys.b, x, r);
+    const double r0n = residual(S, rp, A0, sys.b, x, r);
     LinOut out{0, 0, 0.0, r0n};
     if (r0n < 1e-30) {
         out.converged = 1;
     } else if (sys.kind == kLinBicgstab) {
-        const PcgOut o = bicgstab<NT>(S, A0, x, ws, r0n, sys.maxIter, sys.tol);
+        const PcgOut o = bicgstab(S, rp, A0, x, ws, r0n, sys.maxIter, sys.tol);
         out.iterations = o.iterations;
         out.converged = o.converged;
         out.finalRes = o.finalRes;
     } else if (sys.precision == 0) {
-        const PcgOut o = pcg<NT, double>(S, A0, x, r, ws + n, ws + 2L * n, ws + 3L * n,
+        const PcgOut o = pcg<double>(S, rp, A0, x, r, ws + n, ws + 2L * n, ws + 3L * n,
                                          ws + 4L * n, ws + sys.lvOff, sys.inv, r0n, sys.maxIter,
                                          sys.tol, amg);
         out.iterations = o.iterations;
@@ -376,19 +467,19 @@ template <int NT> __device__ void solveOne(LinShared<NT> &S, double *ws) {
         double rn = r0n;
         int total = 0;
         for (int round = 0; round < kMixedRounds && total < sys.maxIter; ++round) {
-            for (int i = threadIdx.x; i < n; i += NT) {
+            for (int i = gTid(S); i < n; i += gThreads(S)) {
                 fr[i] = float(r[i]);
                 fd[i] = 0.0f;
             }
-            __syncthreads();
+            gSync(S);
             const double innerTol = fmax(kMixedInnerTol, 0.5 * sys.tol * r0n / rn);
-            const PcgOut o = pcg<NT, float>(S, F0, fd, fr, fz, fp, fq, ft, f + sys.lvOff32,
+            const PcgOut o = pcg<float>(S, rp, F0, fd, fr, fz, fp, fq, ft, f + sys.lvOff32,
                                             sys.inv32, rn, sys.maxIter - total, innerTol, amg);
             total += o.iterations;
-            for (int i = threadIdx.x; i < n; i += NT)
+            for (int i = gTid(S); i < n; i += gThreads(S))
                 x[i] += double(fd[i]);
-            __syncthreads();
-            rn = residual<NT>(S, A0, sys.b, x, r);
+            gSync(S);
+            rn = residual(S, rp, A0, sys.b, x, r);
             out.finalRes = rn / r0n;
             if (out.finalRes < sys.tol) {
                 out.converged = 1;
@@ -399,20 +490,32 @@ template <int NT> __device__ void solveOne(LinShared<NT> &S, double *ws) {
         }
         out.iterations = total;
     }
-    __syncthreads();
-    if (threadIdx.x == 0)
+    gSync(S);
+    if (gTid(S) == 0)
         *sys.out = out;
 }
 
-template <int NT>
 __global__ void __launch_bounds__(NT, 1) linKernel(const DevLinSys *systems, int nsys, int *next,
-                                                double *wsBase, long wsStride) {
-    __shared__ LinShared<NT> S;
-    double *ws = wsBase + wsStride * blockIdx.x;
+                                                   double *wsBase, long wsStride) {
+    __shared__ LinShared S;
+    if (threadIdx.x == 0) {
+        unsigned rank, ctas;
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(ctas));
+        S.rank = static_cast<int>(rank);
+        S.ctas = static_cast<int>(ctas);
+    }
+    __syncthreads();
+    gSync(S); // every CTA of the cluster has started: its shared memory can be written
+    double *ws = wsBase + wsStride * (blockIdx.x / S.ctas);
+    int rp = 0;
     for (;;) {
-        if (threadIdx.x == 0)
-            S.job = atomicAdd(next, 1);
-        __syncthreads();
+        if (gTid(S) == 0) {
+            const int j = atomicAdd(next, 1);
+            for (int r = 0; r < S.ctas; ++r)
+                putRemote(&S.job, j, r);
+        }
+        gSync(S);
         const int j = S.job;
         if (j >= nsys)
             break;
@@ -424,25 +527,54 @@ __global__ void __launch_bounds__(NT, 1) linKernel(const DevLinSys *systems, int
                 dst[t] = src[t];
         }
         __syncthreads();
-        solveOne<NT>(S, ws);
-        __syncthreads();
+        solveOne(S, rp, ws);
+        gSync(S);
     }
 }
 
 } // namespace
 
+namespace {
+cudaError_t linConfig(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, int slots, int cluster,
+                      size_t localBytes, cudaStream_t stream) {
+    cudaError_t e = cudaFuncSetAttribute(linKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(localBytes));
+    if (e == cudaSuccess && cluster > 8)
+        e = cudaFuncSetAttribute(linKernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3(slots * cluster);
+    cfg.blockDim = dim3(kLinThreads);
+    cfg.dynamicSmemBytes = localBytes;
+    cfg.stream = stream;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = cluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return e;
+}
+} // namespace
+
 cudaError_t launchLinear(const DevLinSys *systems, int nsys, int *next, double *ws, long wsStride,
-                         int grid, cudaStream_t stream) {
-    linKernel<kLinThreads><<<grid, kLinThreads, 0, stream>>>(systems, nsys, next, ws, wsStride);
-    return cudaGetLastError();
+                         int slots, int cluster, size_t localBytes, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    cudaError_t e = linConfig(cfg, attr, slots, cluster, localBytes, stream);
+    if (e != cudaSuccess)
+        return e;
+    return cudaLaunchKernelEx(&cfg, linKernel, systems, nsys, next, ws, wsStride);
 }
 
-int linBlocksPerSM() {
-    int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, linKernel<kLinThreads>, kLinThreads,
-                                                      0) != cudaSuccess)
+int linConcurrent(int cluster, size_t localBytes) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    int count = 0;
+    if (linConfig(cfg, attr, 1, cluster, localBytes, nullptr) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&count, linKernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
         return 0;
-    return blocks;
+    }
+    return count;
 }
 
 } // namespace rq

@@ -159,6 +159,29 @@ bool gaussJordanInverse(int m, std::vector<double> a, std::vector<double> &inv) 
 
 } // namespace
 
+// Device layout of a level: slices of 32 rows of equal width, unless that takes more than
+// twice the entries (a few very long rows).
+static void setSlices(LinLevelHost &lv) {
+    const int ns = (lv.n + 31) / 32;
+    std::vector<int> first(ns + 1, 0);
+    int64_t at = 0;
+    for (int s = 0; s < ns; ++s) {
+        int w = 0;
+        for (int i = 32 * s; i < std::min(lv.n, 32 * s + 32); ++i)
+            w = std::max(w, lv.ptr[i + 1] - lv.ptr[i]);
+        at += 32LL * w;
+        first[s + 1] = static_cast<int>(std::min<int64_t>(at, INT32_MAX));
+    }
+    const int64_t nnz = static_cast<int64_t>(lv.col.size());
+    if (at <= 2 * nnz + 1024 && at < INT32_MAX) {
+        lv.sh = 5;
+        lv.slice = std::move(first);
+    } else {
+        lv.sh = 0;
+        lv.slice = lv.ptr;
+    }
+}
+
 LinSysHost buildLinSys(int n, int nf, const double *diag, const double *upper,
                        const double *lower, const int32_t *own, const int32_t *nbr, bool withAmg,
                        int minCoarse, int maxLevels, int maxCoarse) {
@@ -196,8 +219,10 @@ LinSysHost buildLinSys(int n, int nf, const double *diag, const double *upper,
         }
     }
     S.lev.push_back(std::move(L0));
-    if (!withAmg)
+    if (!withAmg) {
+        setSlices(S.lev[0]);
         return S;
+    }
 
     // the hierarchy walks column-sorted rows
     std::vector<int> ptr, col;
@@ -277,6 +302,8 @@ LinSysHost buildLinSys(int n, int nf, const double *diag, const double *upper,
             dense[static_cast<size_t>(i) * S.m + col[k]] = val[k];
     if (!gaussJordanInverse(S.m, std::move(dense), S.inv))
         throw LinUnsupported("zero pivot in the coarsest AMG level");
+    for (LinLevelHost &lv : S.lev)
+        setSlices(lv);
     return S;
 }
 

@@ -19,6 +19,8 @@ struct LinUnsupported : std::runtime_error {
 struct LinLevelHost {
     int n = 0, nc = 0;                 // rows; rows of the next level (0 on the coarsest)
     std::vector<int> ptr, col;         // CSR
+    int sh = 0;                        // device layout (DevLinLevel): slices of 1 << sh rows,
+    std::vector<int> slice;            // their first entries (last: the entry count)
     std::vector<double> val, rdg;      // values; 1/diag (1 where |diag| <= 1e-30)
     std::vector<int> agg;              // row -> next-level row
     std::vector<int> childPtr, childIdx; // next-level row -> rows, ascending
