@@ -214,30 +214,64 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
     st.kMin = s.k_min;
     st.kMax = s.k_max;
     st.wMin = s.omega_min;
-    addD(&C.cx, m.cx);
-    addD(&C.cy, m.cy);
-    addD(&C.vol, m.vol);
-    addD(&C.wd, m.wd);
-    addD(&C.xa, m.xa);
-    addD(&C.xnx, m.xnx);
-    addD(&C.xny, m.xny);
-    addD(&C.xw, m.xw);
-    addD(&C.xdl, m.xdl);
-    addD(&C.xdx, m.xdx);
-    addD(&C.xdy, m.xdy);
-    addD(&C.xsh, m.xsh);
-    addD(&C.ya, m.ya);
-    addD(&C.ynx, m.ynx);
-    addD(&C.yny, m.yny);
-    addD(&C.yw, m.yw);
-    addD(&C.ydl, m.ydl);
-    addD(&C.ydx, m.ydx);
-    addD(&C.ydy, m.ydy);
-    if (m.balance) {
-        addD(&C.sing, m.sing);
-        addD(&C.slap, m.slap);
-        addD(&C.sgx, m.sgx);
-        addD(&C.sgy, m.sgy);
+    for (int e = 0; e < 3; ++e) {
+        const double al = e == 0 ? s.alpha_u : e == 1 ? s.alpha_k : s.alpha_omega;
+        C.relax[2 * e] = (1.0 - al) / al;
+        C.relax[2 * e + 1] = 1.0 / al;
+    }
+    { // geometry in the form that the face and cell sweeps use
+        const int nf = m.n + m.nfy();
+        std::vector<double> ivol(m.n), fw(nf), sx(nf), sy(nf), ad(nf), ex(nf), ey(nf), dx(nf), dy(nf);
+        for (int c = 0; c < m.n; ++c)
+            ivol[c] = m.vol[c] > 1e-30 ? 1.0 / m.vol[c] : 1.0;
+        for (int f = 0; f < nf; ++f) {
+            const bool x = f < m.n;
+            const int g = x ? f : f - m.n;
+            const double a = x ? m.xa[g] : m.ya[g];
+            const double dl = std::max(x ? m.xdl[g] : m.ydl[g], 1e-20);
+            fw[f] = x ? m.xw[g] : m.yw[g];
+            sx[f] = (x ? m.xnx[g] : m.ynx[g]) * a;
+            sy[f] = (x ? m.xny[g] : m.yny[g]) * a;
+            ad[f] = a / dl;
+            dx[f] = x ? m.xdx[g] : m.ydx[g];
+            dy[f] = x ? m.xdy[g] : m.ydy[g];
+            ex[f] = a * (dx[f] / dl);
+            ey[f] = a * (dy[f] / dl);
+        }
+        std::vector<double> wf(2 * m.nx), ww(2 * m.nx);
+        for (int k = 0; k < 2 * m.nx; ++k) {
+            const double y = std::max(m.ydl[k < m.nx ? k : m.ny * m.nx + k - m.nx], 1e-20);
+            wf[k] = 60.0 * nu / (y * y);
+            ww[k] = (m.balance ? 6.0 : 60.0) * nu / (y * y);
+        }
+        addD(&C.vol, m.vol);
+        addD(&C.ivol, ivol);
+        addD(&C.wd, m.wd);
+        addD(&C.fw, fw);
+        addD(&C.fsx, sx);
+        addD(&C.fsy, sy);
+        addD(&C.fad, ad);
+        addD(&C.fex, ex);
+        addD(&C.fey, ey);
+        addD(&C.fdx, dx);
+        addD(&C.fdy, dy);
+        addD(&C.wallFw, wf);
+        addD(&C.wallW, ww);
+        if (m.balance) {
+            std::vector<double> g1(nf, 0.0), g2(nf, 0.0);
+            for (int f = 0; f < nf; ++f) {
+                const bool x = f < m.n;
+                const int g = x ? f : f - m.n;
+                const int o = x ? f : g - m.nx, q = x ? (f % m.nx == m.nx - 1 ? f - m.nx + 1 : f + 1) : g;
+                if (o < 0 || q >= m.n)
+                    continue;
+                g1[f] = (x ? m.xa[g] * m.sgx[g] : m.ya[g] * m.sgy[g]);
+                g2[f] = ad[f] * (m.sing[q] - m.sing[o]);
+            }
+            addD(&C.fb1, g1);
+            addD(&C.fb2, g2);
+            addD(&C.slap, m.slap);
+        }
     }
     // probes
     const int nobs = obs ? obs->n_obs : 0;

@@ -63,13 +63,18 @@ struct DevClass {
     double init[6];            // U xyz, p, k, omega
     DevSettings st;
     // cells
-    const double *cx, *cy, *vol, *wd;
-    // east faces (n)
-    const double *xa, *xnx, *xny, *xw, *xdl, *xdx, *xdy, *xsh;
-    // y faces (n + nx)
-    const double *ya, *ynx, *yny, *yw, *ydl, *ydx, *ydy;
-    // planar singular omega balance
-    const double *sing, *slap, *sgx, *sgy;
+    const double *vol, *ivol, *wd; // volume, 1 / volume (1 where it is below 1e-30), wall distance
+    // faces (x faces 0 .. n-1, then y faces): owner weight, area vector, A / delta, A times
+    // the unit vector along d, d = owner-to-neighbour vector
+    const double *fw, *fsx, *fsy, *fad, *fex, *fey, *fdx, *fdy;
+    // wall columns (bottom, then top): 60 nu / y^2 of the omega wall face value and
+    // (6 or 60) nu / y^2 of the wall cell value (resolvedWallOmega), both to be divided by beta1
+    const double *wallFw, *wallW;
+    // planar singular omega balance: A times the singular gradient and A times the
+    // difference quotient per face, the singular Laplacian per cell
+    const double *fb1, *fb2, *slap;
+    // (1 - alpha) / alpha and 1 / alpha of U, k and omega
+    double relax[6];
     // probes: 4 neighbour slots each
     const int32_t *pcell, *pnnb, *pnb;
     const double *pox, *poy, *paxx, *paxy, *payy, *pdet, *pdx, *pdy, *pwt;

@@ -30,14 +30,6 @@ __device__ __forceinline__ void groupSync(int threads) {
     asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
 
-// D = A B of one FP64 m8n8k4 product: a is this lane's A[lane / 4][lane % 4], b its
-// B[lane % 4][lane / 4]; d0, d1 receive D[lane / 4][2 (lane % 4) + 0, 1].
-__device__ __forceinline__ void mma884(double &d0, double &d1, double a, double b) {
-    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%4};"
-        : "=d"(d0), "=d"(d1)
-        : "d"(a), "d"(b), "d"(0.0));
-}
-
 // Sums of K values over the working group (nw warps), the same bits in every thread. A
 // warp adds its lanes with two FP64 matrix products: ones times the lanes' values gives
 // column sums of four lanes, of which each lane adds two and which a second product with
@@ -73,23 +65,6 @@ template <int K> __device__ __forceinline__ void sumRes(double (&v)[K], int &rp,
         for (int k = 0; k < K; ++k)
             mma884(v[k], w[k], v[k], 1.0);
     rp ^= 1;
-}
-
-// a / b by Newton-Raphson iteration from the hardware's approximate reciprocal, and one
-// correction of the quotient: within one unit in the last place for operands and quotients
-// of normal size (the solvers' guards keep |b| above 1e-30). Unlike the division operator
-// it has no branch, so its latency overlaps the block sum beside it (85 cycles each, four
-// per BiCGSTAB iteration).
-__device__ __forceinline__ double recip(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    y = fma(y, fma(-b, y, 1.0), y);
-    y = fma(y, fma(-b, y, 1.0), y);
-    return y;
-}
-__device__ __forceinline__ double quot(double a, double b) {
-    const double y = recip(b), q = a * y;
-    return fma(fma(-b, q, a), y, q);
 }
 
 // Whether the square sum q passes sqrt(q) / r0n < tol: decided by q against the squared

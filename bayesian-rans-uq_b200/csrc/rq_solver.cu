@@ -78,9 +78,9 @@ constexpr int kRedSlots = 8;             // values per block reduction
 struct Work {
     double *Ux, *Uy, *p, *k, *w, *nuT, *F1, *F2, *Pk, *CD, *S;
     double *gUxx, *gUxy, *gUyx, *gUyy, *gKx, *gKy, *gWx, *gWy, *gPx, *gPy;
-    double *phi, *phiOld, *phiPred, *pCoeff; // x faces [0,n) then y faces [n, n+nfy)
+    double *phi, *phiPred, *pCoeff; // x faces [0,n) then y faces [n, n+nfy)
     double *fScr;                            // face scratch of the transport assemblies
-    double *d, *aW, *aE, *aS, *aN, *b, *aP, *aPraw;
+    double *d, *aW, *aE, *aS, *aN, *b, *aP; // aP: V / a_P of the x momentum rows
     double *Uxp, *Uyp, *kOld, *wOld, *pp;
     double *r, *rh, *pv, *v, *s, *t, *ph, *sh;
     double *z, *xa, *xb, *rr;                // PCG / level-0 V-cycle
@@ -144,7 +144,7 @@ struct Shared {
     KW<double> K64;
     KW<float> K32;
     double coeff[11];
-    double red[2][kRedSlots][32];
+    alignas(16) double red[2][kRedSlots][32];
     double cred[2][kRedSlots][kCluster ? kMaxCluster : 1]; // the cluster's CTA sums
     double ring[4][kWindowCap];  // U, k, omega, Q change samples
     int cnt[4];
@@ -185,22 +185,48 @@ __device__ __forceinline__ void mark(Shared &S, int k) {
     }
 }
 
-// ---------------------------------------------------------------- reductions
-template <int K> struct Red {
-    double v[K];
-};
+// ---------------------------------------------------------------- arithmetic
+// a / b by Newton-Raphson iteration from the hardware's approximate reciprocal, and one
+// correction of the quotient: within one unit in the last place for operands and quotients
+// of normal size (the solvers' guards keep |b| above 1e-30). Unlike the division operator
+// it has no branch, so its latency overlaps the block sum beside it (85 cycles each, four
+// per BiCGSTAB iteration).
+__device__ __forceinline__ double recip(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = fma(y, fma(-b, y, 1.0), y);
+    y = fma(y, fma(-b, y, 1.0), y);
+    return y;
+}
+__device__ __forceinline__ double quot(double a, double b) {
+    const double y = recip(b), q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
 
-// Block reductions. Each warp tree-reduces its lanes (lane 0 holds the sum),
-// lane 0 parks it in shared memory, and after one barrier EVERY warp
-// tree-reduces the same partials in the same order and broadcasts lane 0's
-// result -- so all threads of the CTA hold bit-identical values and branch alike.
+// ---------------------------------------------------------------- reductions
+// D = A B of one FP64 m8n8k4 product: a is this lane's A[lane / 4][lane % 4], b its
+// B[lane % 4][lane / 4]; d0, d1 receive D[lane / 4][2 (lane % 4) + 0, 1].
+__device__ __forceinline__ void mma884(double &d0, double &d1, double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%4};"
+        : "=d"(d0), "=d"(d1)
+        : "d"(a), "d"(b), "d"(0.0));
+}
+
+// Block reductions. A warp adds its lanes with two FP64 matrix products (sumRes); lane 0
+// parks the sum in shared memory, and after one barrier every warp adds the same partials
+// in the same order (eight per lane, then a product) -- so all threads of the CTA hold
+// bit-identical values and branch alike. Partials of warps that the CTA lacks are zero
+// (runJob). 480 cycles with shuffles at 16 warps, 631 at 24.
 template <int K>
 __device__ __forceinline__ void blockSum(double (&v)[K], Shared &S, int &rp) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double u[K], w[K];
 #pragma unroll
     for (int k = 0; k < K; ++k)
-        for (int o = 16; o > 0; o >>= 1)
-            v[k] += __shfl_down_sync(FULL, v[k], o);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+        mma884(u[k], w[k], 1.0, v[k]);
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        mma884(v[k], w[k], u[k] + w[k], 1.0);
     if (lane == 0)
 #pragma unroll
         for (int k = 0; k < K; ++k)
@@ -208,11 +234,13 @@ __device__ __forceinline__ void blockSum(double (&v)[K], Shared &S, int &rp) {
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        double s = lane < nw ? S.red[rp][k][lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1)
-            s += __shfl_down_sync(FULL, s, o);
-        v[k] = __shfl_sync(FULL, s, 0);
+        const double2 *r = reinterpret_cast<const double2 *>(&S.red[rp][k][8 * (lane & 3)]);
+        const double2 a = r[0], b = r[1], c = r[2], d = r[3];
+        v[k] = ((a.x + b.x) + (c.x + d.x)) + ((a.y + b.y) + (c.y + d.y));
     }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        mma884(v[k], w[k], v[k], 1.0);
     if constexpr (kCluster) { // every CTA adds the CTA sums in the order of the ranks
         const int nc = ctaCount(), rank = ctaRank();
         if (static_cast<int>(threadIdx.x) < nc)
@@ -230,25 +258,31 @@ __device__ __forceinline__ void blockSum(double (&v)[K], Shared &S, int &rp) {
     rp ^= 1;
 }
 
+// Maximum over a warp of nonnegative values: their bit patterns are ordered as integers, so
+// the high words' maximum and then the low words' among its holders (two reductions in place
+// of ten shuffles).
+__device__ __forceinline__ double warpMax(double v) {
+    const unsigned hi = static_cast<unsigned>(__double2hiint(v));
+    const unsigned mh = __reduce_max_sync(FULL, hi);
+    const unsigned ml =
+        __reduce_max_sync(FULL, hi == mh ? static_cast<unsigned>(__double2loint(v)) : 0u);
+    return __hiloint2double(static_cast<int>(mh), static_cast<int>(ml));
+}
+// Maxima of K nonnegative values over the block.
 template <int K>
 __device__ __forceinline__ void blockMax(double (&v)[K], Shared &S, int &rp) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
 #pragma unroll
     for (int k = 0; k < K; ++k)
-        for (int o = 16; o > 0; o >>= 1)
-            v[k] = fmax(v[k], __shfl_xor_sync(FULL, v[k], o));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+        v[k] = warpMax(v[k]);
     if (lane == 0)
 #pragma unroll
         for (int k = 0; k < K; ++k)
             S.red[rp][k][warp] = v[k];
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        double s = lane < nw ? S.red[rp][k][lane] : S.red[rp][k][0];
-        for (int o = 16; o > 0; o >>= 1)
-            s = fmax(s, __shfl_xor_sync(FULL, s, o));
-        v[k] = s;
-    }
+    for (int k = 0; k < K; ++k)
+        v[k] = warpMax(lane < nw ? S.red[rp][k][lane] : 0.0);
     if constexpr (kCluster) {
         const int nc = ctaCount(), rank = ctaRank();
         if (static_cast<int>(threadIdx.x) < nc)
@@ -300,12 +334,6 @@ __device__ __forceinline__ Cell cellOf(const DevClass &C, int c) {
     return q;
 }
 
-// sum four face terms in the reference's face-index order
-__device__ __forceinline__ double order4(const Cell &q, double tW, double tE, double tS, double tN) {
-    const double x1 = q.xEfirst ? tE : tW, x2 = q.xEfirst ? tW : tE;
-    const double y1 = q.yNfirst ? tN : tS, y2 = q.yNfirst ? tS : tN;
-    return ((x1 + x2) + y1) + y2;
-}
 // accumulate onto a running value in face order
 __device__ __forceinline__ double accum4(const Cell &q, double acc, double tW, double tE, double tS,
                                          double tN) {
@@ -314,67 +342,80 @@ __device__ __forceinline__ double accum4(const Cell &q, double acc, double tW, d
     return (((acc + x1) + x2) + y1) + y2;
 }
 
-// the wall face of a wall cell; a cell touching both walls keeps the last (top) one
-__device__ __forceinline__ int wallFaceOf(const DevClass &C, int c) {
-    const int j = rowOf(C, c);
-    return (j == C.ny - 1 ? C.ny : 0) * C.nx + (c - j * C.nx);
-}
-__device__ __forceinline__ bool isWallCell(const DevClass &C, int c) {
-    return c < C.nx || c >= C.n - C.nx;
+// column of wall values of a wall cell: bottom 0 .. nx - 1, top nx .. 2 nx - 1 (a cell
+// touching both walls keeps the top one)
+__device__ __forceinline__ int wallSlot(const DevClass &C, const Cell &q) {
+    return q.i + (q.j == C.ny - 1 ? C.nx : 0);
 }
 
-__device__ __forceinline__ double wallOmega(const DevClass &C, double b1, double y) {
-    const double coefficient = C.balance ? 6.0 : 60.0; // resolvedWallOmega, SIMPLESolver.cpp:155-161
-    return coefficient * C.nu / (b1 * y * y);
-}
-// wall face value of omega (applyOmegaBC, BoundaryCondition.hpp:361-384)
-__device__ __forceinline__ double wallFaceOmega(const DevClass &C, double b1, int f) {
-    const double y1 = dmax(C.ydl[f], 1e-20);
-    return 60.0 * C.nu / (b1 * y1 * y1);
+// Geometry of a cell's Green-Gauss gradients (Field.hpp:178-212), shared by all fields:
+// the interpolation weights (owner side) and outward area vectors of its faces, 1 / volume.
+// At a wall face the weight picks the neighbour value, which grad() takes from the wall.
+struct GradGeo {
+    double wW, wE, wS, wN, xW, yW, xE, yE, xS, yS, xN, yN, iV;
+    __device__ __forceinline__ GradGeo(const DevClass &C, const Cell &q) {
+        const int c = q.c, fS = C.n + c, fN = fS + C.nx;
+        wW = __ldg(C.fw + q.W);
+        wE = __ldg(C.fw + c);
+        wS = q.south ? __ldg(C.fw + fS) : 1.0;
+        wN = q.north ? __ldg(C.fw + fN) : 0.0;
+        xW = __ldg(C.fsx + q.W);
+        yW = __ldg(C.fsy + q.W);
+        xE = __ldg(C.fsx + c);
+        yE = __ldg(C.fsy + c);
+        xS = __ldg(C.fsx + fS);
+        yS = __ldg(C.fsy + fS);
+        if (q.south) { // owner below: outward is the other way
+            xS = -xS;
+            yS = -yS;
+        }
+        xN = __ldg(C.fsx + fN);
+        yN = __ldg(C.fsy + fN);
+        iV = __ldg(C.ivol + c);
+    }
+    // gradient from the cell's value and its neighbours' (S, N: the wall value at a wall).
+    // The products of the x pair are rounded before they are added, so that they cancel
+    // exactly where the flow does not vary along x.
+    __device__ __forceinline__ void grad(double pc, double pW, double pE, double pS, double pN,
+                                         double &gx, double &gy) const {
+        const double fW = pW * wW + pc * (1.0 - wW), fE = pc * wE + pE * (1.0 - wE);
+        const double fS = pS * wS + pc * (1.0 - wS), fN = pc * wN + pN * (1.0 - wN);
+        const double tx = __dmul_rn(xE, fE) - __dmul_rn(xW, fW);
+        const double ty = __dmul_rn(yE, fE) - __dmul_rn(yW, fW);
+        gx = ((tx + __dmul_rn(xS, fS)) + __dmul_rn(xN, fN)) * iV;
+        gy = ((ty + __dmul_rn(yS, fS)) + __dmul_rn(yN, fN)) * iV;
+    }
+    // the same of a field with wall values bS, bN
+    __device__ __forceinline__ void of(const Cell &q, int nx, const double *phi, double bS, double bN,
+                                       double &gx, double &gy) const {
+        const int c = q.c;
+        grad(phi[c], phi[q.W], phi[q.E], q.south ? phi[c - nx] : bS, q.north ? phi[c + nx] : bN, gx,
+             gy);
+    }
+};
+
+// Owner and neighbour cell of face f (x faces, then y faces); false for a wall face.
+__device__ __forceinline__ bool faceCells(const DevClass &C, int f, int &o, int &q) {
+    if (f < C.n) {
+        o = f;
+        q = eastOf(C, f);
+        return true;
+    }
+    q = f - C.n;
+    o = q - C.nx;
+    return o >= 0 && q < C.n;
 }
 
-// Green-Gauss gradient of one cell (Field.hpp:178-212); bS / bN are the wall
-// face values used where the cell touches the bottom / top wall.
-__device__ __forceinline__ void ggCell(const DevClass &C, const Cell &q, const double *phi,
-                                       double bS, double bN, double &gx, double &gy) {
-    const int c = q.c;
-    const double pc = phi[c];
-    // east (owner c)
-    const double wE = __ldg(C.xw + (c));
-    const double fE = pc * wE + phi[q.E] * (1.0 - wE);
-    const double sxE = __ldg(C.xnx + (c)) * __ldg(C.xa + (c)), syE = __ldg(C.xny + (c)) * __ldg(C.xa + (c));
-    // west (owner W, neighbour c)
-    const double wWf = __ldg(C.xw + (q.W));
-    const double fW = phi[q.W] * wWf + pc * (1.0 - wWf);
-    const double sxW = __ldg(C.xnx + (q.W)) * __ldg(C.xa + (q.W)), syW = __ldg(C.xny + (q.W)) * __ldg(C.xa + (q.W));
-    // north: internal (owner c) or top wall (owner c)
-    const int fn = c + C.nx;
-    double fN;
-    if (q.north) {
-        const double w = __ldg(C.yw + (fn));
-        fN = pc * w + phi[c + C.nx] * (1.0 - w);
-    } else {
-        fN = bN;
-    }
-    const double sxN = __ldg(C.ynx + (fn)) * __ldg(C.ya + (fn)), syN = __ldg(C.yny + (fn)) * __ldg(C.ya + (fn));
-    // south: internal (owner c - nx, neighbour c) or bottom wall (owner c)
-    const int fs = c;
-    double fS;
-    if (q.south) {
-        const double w = __ldg(C.yw + (fs));
-        fS = phi[c - C.nx] * w + pc * (1.0 - w);
-    } else {
-        fS = bS;
-    }
-    const double sxS = __ldg(C.ynx + (fs)) * __ldg(C.ya + (fs)), syS = __ldg(C.yny + (fs)) * __ldg(C.ya + (fs));
-    const double sgnS = q.south ? -1.0 : 1.0;
-    gx = order4(q, -(sxW * fW), sxE * fE, sgnS * (sxS * fS), sxN * fN);
-    gy = order4(q, -(syW * fW), syE * fE, sgnS * (syS * fS), syN * fN);
-    const double V = __ldg(C.vol + (c));
-    if (V > 1e-30) {
-        gx = gx / V;
-        gy = gy / V;
-    }
+// Deferred correction F (phi_f - phi_up) of the limitedLinearUpwind face value (:495-552):
+// phi_up + 0.5 psi(r) (phi_dn - phi_up) with r = 2 (grad phi)_up . d / (phi_dn - phi_up) - 1.
+// dphi = phi_q - phi_o, d the vector from o to q: with q upwind both change sign in r.
+__device__ __forceinline__ double limitedCorr(double F, double dphi, double gx, double gy, double dx,
+                                              double dy) {
+    if (!(fabs(dphi) > 1e-300) || F == 0.0)
+        return 0.0;
+    const double r = quot(2.0 * (gx * dx + gy * dy), dphi) - 1.0;
+    const double psi = r > 0.0 ? quot(r * r + r, r * r + 1.0) : 0.0;
+    return 0.5 * psi * (fabs(F) * dphi);
 }
 
 // matrix row times x in the reference's matvec order (diagonal first, then faces)
@@ -1612,8 +1653,6 @@ __device__ void carve(Shared &S, double *ws, double *arena, long arenaDoubles) {
     W.Pk = take(n);
     W.CD = take(n);
     W.S = take(n);
-    W.phiOld = take(nf);
-    W.aPraw = take(n);
     W.Uxp = take(n);
     W.Uyp = take(n);
     W.kOld = take(n);
@@ -1661,10 +1700,9 @@ __device__ void carve(Shared &S, double *ws, double *arena, long arenaDoubles) {
     const double sk2 = S.coeff[4], sw2 = S.coeff[5], b2 = S.coeff[6], al2 = S.coeff[7];         \
     const double bs = S.coeff[8], a1 = S.coeff[9];                                              \
     auto blend = [](double p1, double p2, double F1) { return F1 * p1 + (1.0 - F1) * p2; };    \
-    auto bwOf = [&](int f) { return wallFaceOmega(C, S.wallBeta, f); };                        \
     (void)st; (void)n; (void)nx; (void)ny; (void)nfy; (void)nu; (void)sk1; (void)sw1;          \
     (void)b1; (void)al1; (void)sk2; (void)sw2; (void)b2; (void)al2; (void)bs; (void)a1;         \
-    (void)blend; (void)bwOf;
+    (void)blend;
 
 // ---------------------------------------------------------------- phases
 // Each phase is a barrier-free sweep over cells or faces; the caller places
@@ -1678,7 +1716,8 @@ __device__ __noinline__ void phInitCells(Shared &S) {
         W.Uy[c] = U1;
         W.p[c] = P0;
         W.k[c] = K0;
-        const double om = dmax(wallOmega(C, b1, dmax(C.wd[c], 1e-20)), W0);
+        const double y = dmax(C.wd[c], 1e-20);
+        const double om = dmax((C.balance ? 6.0 : 60.0) * C.nu / (b1 * y * y), W0);
         W.w[c] = om;
         W.F1[c] = 1.0;
         W.F2[c] = 1.0;
@@ -1708,76 +1747,55 @@ __device__ __noinline__ void phInitWarm(Shared &S, const double *wf) {
     }
 }
 
+// interpolated flux of the velocity (ux, uy given at owner o and neighbour q) through face f
+__device__ __forceinline__ double faceFlux(const DevClass &C, int f, int o, int q, const double *ux,
+                                           const double *uy) {
+    const double w = __ldg(C.fw + f);
+    const double x = ux[o] * w + ux[q] * (1.0 - w), y = uy[o] * w + uy[q] * (1.0 - w);
+    return x * __ldg(C.fsx + f) + y * __ldg(C.fsy + f);
+}
+
 __device__ __noinline__ void phInitFlux(Shared &S) {
     RQ_PRELUDE
     FOR_OWN(f, n + nfy) {
-        double v = 0.0;
-        if (f < n) {
-            const int q = eastOf(C, f);
-            const double w = C.xw[f];
-            const double ux = W.Ux[f] * w + W.Ux[q] * (1.0 - w), uy = W.Uy[f] * w + W.Uy[q] * (1.0 - w);
-            v = (ux * C.xnx[f] + uy * C.xny[f]) * C.xa[f];
-        } else {
-            const int g = f - n, jf = rowOf(C, g);
-            if (jf > 0 && jf < ny) {
-                const int o = g - nx;
-                const double w = C.yw[g];
-                const double ux = W.Ux[o] * w + W.Ux[g] * (1.0 - w), uy = W.Uy[o] * w + W.Uy[g] * (1.0 - w);
-                v = (ux * C.ynx[g] + uy * C.yny[g]) * C.ya[g];
-            } else {
-                v = (0.0 * C.ynx[g] + 0.0 * C.yny[g]) * C.ya[g];
-            }
-        }
-        W.phi[f] = v;
+        int o, q;
+        W.phi[f] = faceCells(C, f, o, q) ? faceFlux(C, f, o, q, W.Ux, W.Uy) : 0.0;
     }
 }
 
+// Iteration start: the velocity to compare against, and the gradients of U, p and (on a
+// turbulence update) k and omega from one load of the cell's geometry. One CTA of a 384-cell
+// class spends its time here on issuing instructions, not on data: with the geometry formed
+// per field and two divisions per gradient this phase took 10 800 cycles.
 __device__ __noinline__ void phStart(Shared &S, bool turbUpdate) {
     RQ_PRELUDE
-        FOR_OWN(f, n + nfy) {
-            double v = 0.0;
-            if (f < n) {
-                const int q = eastOf(C, f);
-                const double w = C.xw[f];
-                const double ux = W.Ux[f] * w + W.Ux[q] * (1.0 - w), uy = W.Uy[f] * w + W.Uy[q] * (1.0 - w);
-                v = (ux * C.xnx[f] + uy * C.xny[f]) * C.xa[f];
-            } else {
-                const int g = f - n, jf = rowOf(C, g);
-                if (jf > 0 && jf < ny) {
-                    const int o = g - nx;
-                    const double w = C.yw[g];
-                    const double ux = W.Ux[o] * w + W.Ux[g] * (1.0 - w), uy = W.Uy[o] * w + W.Uy[g] * (1.0 - w);
-                    v = (ux * C.ynx[g] + uy * C.yny[g]) * C.ya[g];
-                } else {
-                    v = (0.0 * C.ynx[g] + 0.0 * C.yny[g]) * C.ya[g];
-                }
-            }
-            W.phiOld[f] = v;
+    const double iBeta = 1.0 / S.wallBeta;
+    FOR_CELLS(c) {
+        const Cell q = cellOf(C, c);
+        const GradGeo G(C, q);
+        double gx, gy;
+        W.Uxp[c] = W.Ux[c];
+        W.Uyp[c] = W.Uy[c];
+        G.of(q, nx, W.Ux, 0.0, 0.0, gx, gy);
+        W.gUxx[c] = gx;
+        W.gUxy[c] = gy;
+        G.of(q, nx, W.Uy, 0.0, 0.0, gx, gy);
+        W.gUyx[c] = gx;
+        W.gUyy[c] = gy;
+        const double pc = W.p[c]; // pressure wall faces carry the owner value (Neumann)
+        G.of(q, nx, W.p, pc, pc, gx, gy);
+        W.gPx[c] = gx;
+        W.gPy[c] = gy;
+        if (turbUpdate) {
+            G.of(q, nx, W.k, 0.0, 0.0, gx, gy);
+            W.gKx[c] = gx;
+            W.gKy[c] = gy;
+            G.of(q, nx, W.w, q.south ? 0.0 : __ldg(C.wallFw + q.i) * iBeta,
+                 q.north ? 0.0 : __ldg(C.wallFw + nx + q.i) * iBeta, gx, gy);
+            W.gWx[c] = gx;
+            W.gWy[c] = gy;
         }
-        FOR_CELLS(c) {
-            const Cell q = cellOf(C, c);
-            W.Uxp[c] = W.Ux[c];
-            W.Uyp[c] = W.Uy[c];
-            double gx, gy;
-            ggCell(C, q, W.Ux, 0.0, 0.0, gx, gy);
-            W.gUxx[c] = gx;
-            W.gUxy[c] = gy;
-            ggCell(C, q, W.Uy, 0.0, 0.0, gx, gy);
-            W.gUyx[c] = gx;
-            W.gUyy[c] = gy;
-            // pressure faces carry the owner value (Neumann walls)
-            ggCell(C, q, W.p, W.p[c], W.p[c], gx, gy);
-            W.gPx[c] = gx;
-            W.gPy[c] = gy;
-            if (turbUpdate) {
-                ggCell(C, q, W.k, 0.0, 0.0, gx, gy);
-                W.gKx[c] = gx;
-                W.gKy[c] = gy;
-                ggCell(C, q, W.w, bwOf(q.i), bwOf(C.ny * nx + q.i), gx, gy);
-                W.gWx[c] = gx;
-                W.gWy[c] = gy;
-            }
-        }
+    }
 }
 
 __device__ __noinline__ void phClosure(Shared &S, double floorV) {
@@ -1789,23 +1807,23 @@ __device__ __noinline__ void phClosure(Shared &S, double floorV) {
                 W.S[c] = Sc;
                 const double kc = dmax(W.k[c], 0.0), wc = dmax(W.w[c], 1e-20);
                 const double y = dmax(C.wd[c], 1e-20);
-                const double cd = 2.0 * sw2 / dmax(wc, 1e-20) * (W.gKx[c] * W.gWx[c] + W.gKy[c] * W.gWy[c]);
+                const double cd = quot(2.0 * sw2, wc) * (W.gKx[c] * W.gWx[c] + W.gKy[c] * W.gWy[c]);
                 W.CD[c] = cd;
                 const double sqk = sqrt(dmax(kc, 0.0)), ws = dmax(wc, 1e-20);
                 const double ys = dmax(y, 1e-20), y2 = ys * ys;
-                const double t1 = sqk / (bs * ws * ys);
-                const double t2 = 500.0 * nu / (y2 * ws);
-                const double t3 = 4.0 * sw2 * dmax(kc, 0.0) / (dmax(cd, 1e-10) * y2);
+                const double t1 = quot(sqk, bs * ws * ys);
+                const double t2 = quot(500.0 * nu, y2 * ws);
+                const double t3 = quot(4.0 * sw2 * kc, dmax(cd, 1e-10) * y2);
                 const double arg1 = dmin(dmax(t1, t2), t3);
                 const double F1 = tanh(arg1 * arg1 * arg1 * arg1);
                 W.F1[c] = F1;
-                const double u1 = 2.0 * sqk / (bs * ws * ys);
+                const double u1 = 2.0 * t1;
                 const double arg2 = dmax(u1, t2);
                 const double F2 = tanh(arg2 * arg2);
                 W.F2[c] = F2;
                 double den = dmax(a1 * wc, Sc * F2);
                 den = dmax(den, 1e-20);
-                const double nut = a1 * dmax(kc, 0.0) / den;
+                const double nut = quot(a1 * kc, den);
                 const double raw = nut * Sc * Sc;
                 const double lim = 10.0 * bs * dmax(kc, 0.0) * dmax(wc, 1e-20);
                 W.Pk[c] = dmin(raw, lim);
@@ -1817,268 +1835,138 @@ __device__ __noinline__ void phClosure(Shared &S, double floorV) {
 // phStart, is unchanged until the y solve)
 __device__ __noinline__ void phGradU(Shared &S) {
     RQ_PRELUDE
-                FOR_CELLS(c) {
-                    const Cell q = cellOf(C, c);
-                    double gx, gy;
-                    ggCell(C, q, W.Ux, 0.0, 0.0, gx, gy);
-                    W.gUxx[c] = gx;
-                    W.gUxy[c] = gy;
-                }
+    FOR_CELLS(c) {
+        const Cell q = cellOf(C, c);
+        const GradGeo G(C, q);
+        double gx, gy;
+        G.of(q, nx, W.Ux, 0.0, 0.0, gx, gy);
+        W.gUxx[c] = gx;
+        W.gUxy[c] = gy;
+    }
 }
 
 // The internal faces of the momentum assembly, each once (assembleMomentum
 // :303-482): the diffusion coefficient D = nu_f A / delta (both components: stored
 // by the x pass in pCoeff, free until the p' assembly), the transpose-stress flux of
 // this component (phiPred, free likewise) and its limitedLinearUpwind deferred
-// correction F (phi_f - phi_up) (fScr, :495-532). Wall faces belong to one cell and
-// are formed by the cell sweep.
+// correction (fScr, :495-532). Wall faces belong to one cell and are formed by the cell
+// sweep.
 __device__ __noinline__ void phMomentumFaces(Shared &S, int comp) {
     RQ_PRELUDE
-            const double *U = comp == 0 ? W.Ux : W.Uy;
-            const double *gUc_x = comp == 0 ? W.gUxx : W.gUyx; // grad of this component
-            const double *gUc_y = comp == 0 ? W.gUxy : W.gUyy;
-            const double *colX = comp == 0 ? W.gUxx : W.gUxy;  // dUx/dx_comp
-            const double *colY = comp == 0 ? W.gUyx : W.gUyy;  // dUy/dx_comp
-            FOR_OWN(f, n + nfy) {
-                int fi, o, qn;
-                const double *A, *NX, *NY, *WT, *DL;
-                double sh = 0.0;
-                if (f < n) {
-                    fi = f;
-                    o = f;
-                    qn = eastOf(C, f);
-                    A = C.xa; NX = C.xnx; NY = C.xny; WT = C.xw; DL = C.xdl;
-                    sh = C.xsh[fi];
-                } else {
-                    fi = f - n;
-                    const int jf = rowOf(C, fi);
-                    if (jf == 0 || jf == ny)
-                        continue;
-                    o = fi - nx;
-                    qn = fi;
-                    A = C.ya; NX = C.ynx; NY = C.yny; WT = C.yw; DL = C.ydl;
-                }
-                const double delta = dmax(DL[fi], 1e-20);
-                const double F = W.phi[f];
-                const double w = WT[fi];
-                if (comp == 0) {
-                    const double nuO = nu + W.nuT[o], nuN = nu + W.nuT[qn];
-                    const double nuF = w * nuO + (1.0 - w) * nuN;
-                    W.pCoeff[f] = nuF * A[fi] / delta;
-                }
-                const double cf = w * W.nuT[o] + (1.0 - w) * W.nuT[qn];
-                const double gxf = colX[o] * w + colX[qn] * (1.0 - w);
-                const double gyf = colY[o] * w + colY[qn] * (1.0 - w);
-                W.phiPred[f] = cf * (gxf * NX[fi] + gyf * NY[fi]) * A[fi];
-                double corr = 0.0;
-                if (F != 0.0) {
-                    const bool ownerUp = F > 0.0;
-                    const int up = ownerUp ? o : qn, dn = ownerUp ? qn : o;
-                    const double xUx = C.cx[up], xUy = C.cy[up];
-                    const double xDx = ownerUp ? C.cx[qn] + sh : C.cx[o] - sh;
-                    const double xDy = ownerUp ? C.cy[qn] + 0.0 : C.cy[o] - 0.0;
-                    const double dphi = U[dn] - U[up];
-                    double psi = 0.0;
-                    if (fabs(dphi) > 1e-300) {
-                        const double rr = 2.0 * (gUc_x[up] * (xDx - xUx) + gUc_y[up] * (xDy - xUy)) / dphi - 1.0;
-                        psi = rr > 0.0 ? (rr * rr + rr) / (rr * rr + 1.0) : 0.0;
-                    }
-                    const double pf = U[up] + 0.5 * psi * dphi;
-                    corr = F * (pf - U[up]);
-                }
-                W.fScr[f] = corr;
-            }
+    const double *U = comp == 0 ? W.Ux : W.Uy;
+    const double *gUx = comp == 0 ? W.gUxx : W.gUyx; // grad of this component
+    const double *gUy = comp == 0 ? W.gUxy : W.gUyy;
+    const double *colX = comp == 0 ? W.gUxx : W.gUxy; // dUx/dx_comp
+    const double *colY = comp == 0 ? W.gUyx : W.gUyy; // dUy/dx_comp
+    const double *nuT = W.nuT, *phi = W.phi;
+    double *D = W.pCoeff, *ts = W.phiPred, *cc = W.fScr;
+    FOR_OWN(f, n + nfy) {
+        int o, q;
+        if (!faceCells(C, f, o, q))
+            continue;
+        const double w = __ldg(C.fw + f), v = 1.0 - w, F = phi[f];
+        const double cf = w * nuT[o] + v * nuT[q];
+        const double gxf = colX[o] * w + colX[q] * v, gyf = colY[o] * w + colY[q] * v;
+        const int up = F > 0.0 ? o : q;
+        const double corr = limitedCorr(F, U[q] - U[o], gUx[up], gUy[up], __ldg(C.fdx + f),
+                                        __ldg(C.fdy + f));
+        if (comp == 0)
+            D[f] = (nu + cf) * __ldg(C.fad + f);
+        ts[f] = cf * (gxf * __ldg(C.fsx + f) + gyf * __ldg(C.fsy + f));
+        cc[f] = corr;
+    }
 }
 
-// The momentum rows of one component from the face values of phMomentumFaces
-// (the wall faces here), summed in the reference's face order; the row's residual.
+// The momentum rows of one component from the face values of phMomentumFaces (a resolved
+// wall: molecular viscosity, U_b = 0, no flux), summed in the reference's order (x faces, y
+// faces, walls); the row's residual. The x pass leaves V / a_P in aP for the p' equation.
 __device__ __noinline__ void phMomentum(Shared &S, int comp, double (&acc)[3]) {
     RQ_PRELUDE
-            double *U = comp == 0 ? W.Ux : W.Uy;
-            const double *colX = comp == 0 ? W.gUxx : W.gUxy;  // dUx/dx_comp
-            const double *colY = comp == 0 ? W.gUyx : W.gUyy;  // dUy/dx_comp
-            const double fb = comp == 0 ? st.fx : st.fy;
-            FOR_CELLS(c) {
-                const Cell q = cellOf(C, c);
-                const int i = q.i, j = q.j;
-                // faces: 0 W 1 E 2 S 3 N
-                double dT[4], aT[4], tsT[4], ccT[4];
-                const bool isWall[4] = {false, false, !q.south, !q.north};
-                for (int k = 0; k < 4; ++k) {
-                    dT[k] = 0.0;
-                    aT[k] = 0.0;
-                    tsT[k] = 0.0;
-                    ccT[k] = 0.0;
-                }
-                for (int k = 0; k < 4; ++k) {
-                    bool own;
-                    int f, fi;
-                    const double *A, *DL;
-                    if (k < 2) {
-                        fi = (k == 0) ? q.W : c;
-                        own = (k == 1);
-                        A = C.xa; DL = C.xdl;
-                        f = fi;
-                    } else {
-                        fi = (k == 2) ? c : c + nx;
-                        own = (k == 3) || isWall[k];
-                        A = C.ya; DL = C.ydl;
-                        f = n + fi;
-                    }
-                    const double F = W.phi[f];
-                    if (isWall[k]) { // resolved wall: molecular viscosity, U_b = 0
-                        const double delta = dmax(DL[fi], 1e-20);
-                        const double Db = nu * A[fi] / delta;
-                        const double Ub = 0.0;
-                        if (F >= 0) {
-                            dT[k] = F + Db;
-                            tsT[k] = Db * Ub; // boundary source
-                        } else {
-                            dT[k] = Db;
-                            tsT[k] = (Db - F) * Ub;
-                        }
-                        continue;
-                    }
-                    const double D = W.pCoeff[f];
-                    const double cp = dmax(F, 0.0), cn = dmax(-F, 0.0);
-                    dT[k] = own ? D + cp : D + cn;
-                    aT[k] = own ? -(D + cn) : -(D + cp);
-                    // transpose stress flux through this face (StressOperators.hpp:31-81)
-                    const double fl = W.phiPred[f];
-                    tsT[k] = own ? fl : -fl;
-                    if (F != 0.0) {
-                        const double corr = W.fScr[f];
-                        ccT[k] = own ? -corr : corr;
-                    }
-                }
-                (void)i;
-                (void)j;
-                // internal faces first in face order, then the wall (boundary faces come last)
-                double dsum = 0.0, bsrc = 0.0, ts = 0.0, bcc;
-                {
-                    const double x1 = q.xEfirst ? dT[1] : dT[0], x2 = q.xEfirst ? dT[0] : dT[1];
-                    dsum = dsum + x1;
-                    dsum = dsum + x2;
-                    const int y1 = q.yNfirst ? 3 : 2, y2 = q.yNfirst ? 2 : 3;
-                    // walls come after internal faces: j == 0 puts S (wall) last via yNfirst
-                    if (!isWall[y1])
-                        dsum = dsum + dT[y1];
-                    if (!isWall[y2])
-                        dsum = dsum + dT[y2];
-                    if (isWall[y1]) {
-                        dsum = dsum + dT[y1];
-                        bsrc = bsrc + tsT[y1];
-                    }
-                    if (isWall[y2]) {
-                        dsum = dsum + dT[y2];
-                        bsrc = bsrc + tsT[y2];
-                    }
-                    // transpose stress: internal faces in order, then the zero-coefficient wall
-                    const double t1 = q.xEfirst ? tsT[1] : tsT[0], t2 = q.xEfirst ? tsT[0] : tsT[1];
-                    ts = ts + t1;
-                    ts = ts + t2;
-                    if (!isWall[y1])
-                        ts = ts + tsT[y1];
-                    if (!isWall[y2])
-                        ts = ts + tsT[y2];
-                    for (int k = 2; k < 4; ++k)
-                        if (isWall[k]) {
-                            const double gcx = colX[c], gcy = colY[c];
-                            const int fi = (k == 2) ? c : c + nx;
-                            ts = ts + 0.0 * (gcx * C.ynx[fi] + gcy * C.yny[fi]) * C.ya[fi];
-                        }
-                    // deferred correction in face order (internal faces only)
-                    bcc = 0.0;
-                    (void)bcc;
-                }
-                double bsum = bsrc;
-                bsum -= (comp == 0 ? W.gPx[c] : W.gPy[c]) * C.vol[c];
-                if (fb != 0.0)
-                    bsum += fb * C.vol[c];
-                bsum += ts;
-                {
-                    const double x1 = q.xEfirst ? ccT[1] : ccT[0], x2 = q.xEfirst ? ccT[0] : ccT[1];
-                    bsum += x1;
-                    bsum += x2;
-                    const int y1 = q.yNfirst ? 3 : 2, y2 = q.yNfirst ? 2 : 3;
-                    if (!isWall[y1])
-                        bsum += ccT[y1];
-                    if (!isWall[y2])
-                        bsum += ccT[y2];
-                }
-                const double aU = st.aU;
-                const double draw = dsum;
-                bsum += (1.0 - aU) / aU * draw * U[c];
-                const double dd = draw / aU;
-                W.aPraw[c] = draw;
-                if (comp == 0)
-                    W.aP[c] = dd;
-                W.d[c] = dd;
-                W.aW[c] = aT[0];
-                W.aE[c] = aT[1];
-                W.aS[c] = aT[2];
-                W.aN[c] = aT[3];
-                W.b[c] = bsum;
-                // residual b - A U of this row (relaxation cancels at U)
-                const double tW = aT[0] * U[q.W], tE = aT[1] * U[q.E];
-                const double tS = q.south ? aT[2] * U[c - nx] : 0.0;
-                const double tN = q.north ? aT[3] * U[c + nx] : 0.0;
-                const double rc = bsum - accum4(q, dd * U[c], tW, tE, tS, tN);
-                W.r[c] = rc;
-                acc[0] += fabs(rc);
-                acc[1] += rc * rc;
-                if (comp == 0) {
-                    const double un = sqrt(W.Ux[c] * W.Ux[c] + W.Uy[c] * W.Uy[c] + 0.0);
-                    const double contribution = draw * un;
-                    acc[2] += contribution;
-                }
-            }
+    const double *U = comp == 0 ? W.Ux : W.Uy, *gP = comp == 0 ? W.gPx : W.gPy;
+    const double *phi = W.phi, *D = W.pCoeff, *tsf = W.phiPred, *ccf = W.fScr;
+    const double fb = comp == 0 ? st.fx : st.fy;
+    FOR_CELLS(c) {
+        const Cell q = cellOf(C, c);
+        const int fW = q.W, fE = c, fS = n + c, fN = n + c + nx;
+        const double FW = phi[fW], FE = phi[fE], DW = D[fW], DE = D[fE];
+        double aS = 0.0, aN = 0.0, dS, dN, ts = tsf[fE] - tsf[fW], cc = ccf[fW] - ccf[fE];
+        if (q.south) {
+            const double F = phi[fS], d = D[fS];
+            dS = d + dmax(-F, 0.0);
+            aS = -(d + dmax(F, 0.0));
+            ts -= tsf[fS];
+            cc += ccf[fS];
+        } else {
+            dS = nu * __ldg(C.fad + fS);
+        }
+        if (q.north) {
+            const double F = phi[fN], d = D[fN];
+            dN = d + dmax(F, 0.0);
+            aN = -(d + dmax(-F, 0.0));
+            ts += tsf[fN];
+            cc -= ccf[fN];
+        } else {
+            dN = nu * __ldg(C.fad + fN);
+        }
+        const double aW = -(DW + dmax(FW, 0.0)), aE = -(DE + dmax(-FE, 0.0));
+        double dsum = (DW + dmax(-FW, 0.0)) + (DE + dmax(FE, 0.0));
+        dsum = q.south ? (dsum + dS) + dN : (dsum + dN) + dS; // the wall comes last
+        const double V = __ldg(C.vol + c), Uc = U[c];
+        double bsum = -(gP[c] * V);
+        if (fb != 0.0)
+            bsum += fb * V;
+        bsum += ts;
+        bsum += cc;
+        bsum += C.relax[0] * dsum * Uc; // (1 - alpha) / alpha
+        const double dd = dsum * C.relax[1];
+        if (comp == 0) {
+            W.aP[c] = fabs(dd) > 1e-30 ? quot(V, dd) : 0.0;
+            const double uy = W.Uy[c];
+            acc[2] += dsum * sqrt(Uc * Uc + uy * uy);
+        }
+        W.d[c] = dd;
+        W.aW[c] = aW;
+        W.aE[c] = aE;
+        W.aS[c] = aS;
+        W.aN[c] = aN;
+        W.b[c] = bsum;
+        // residual b - A U of this row (relaxation cancels at U)
+        const double tS = q.south ? aS * U[c - nx] : 0.0, tN = q.north ? aN * U[c + nx] : 0.0;
+        const double rc = bsum - accum4(q, dd * Uc, aW * U[q.W], aE * U[q.E], tS, tN);
+        W.r[c] = rc;
+        acc[0] += fabs(rc);
+        acc[1] += rc * rc;
+    }
 }
 
+// Predicted face flux (stored Rhie-Chow, :1401-1419) and the coefficient of p'. The flux of
+// the velocity at the iteration start is interpolated here, beside the new one, from the
+// same geometry (a sweep of its own in phStart cost a store and ten loads per face).
 __device__ __noinline__ void phPressureFaces(Shared &S, double (&fs)[1]) {
     RQ_PRELUDE
-        const double relaxCorr = 1.0 - st.aU;
-        FOR_OWN(f, n + nfy) {
-            int o, q;
-            const double *A, *NX, *NY, *WT, *DL, *DX, *DY;
-            int fi;
-            bool wall = false;
-            if (f < n) {
-                fi = f;
-                o = f;
-                q = eastOf(C, f);
-                A = C.xa; NX = C.xnx; NY = C.xny; WT = C.xw; DL = C.xdl; DX = C.xdx; DY = C.xdy;
-            } else {
-                fi = f - n;
-                const int jf = rowOf(C, fi);
-                wall = (jf == 0 || jf == ny);
-                o = fi - nx;
-                q = fi;
-                A = C.ya; NX = C.ynx; NY = C.yny; WT = C.yw; DL = C.ydl; DX = C.ydx; DY = C.ydy;
-            }
-            double ph, pc = 0.0;
-            if (wall) {
-                ph = (0.0 * NX[fi] + 0.0 * NY[fi]) * A[fi];
-            } else {
-                const double w = WT[fi];
-                const double ux = W.Ux[o] * w + W.Ux[q] * (1.0 - w), uy = W.Uy[o] * w + W.Uy[q] * (1.0 - w);
-                ph = (ux * NX[fi] + uy * NY[fi]) * A[fi];
-                const double delta = dmax(DL[fi], 1e-20);
-                const double dO = (fabs(W.aP[o]) > 1e-30) ? C.vol[o] / W.aP[o] : 0.0;
-                const double dN = (fabs(W.aP[q]) > 1e-30) ? C.vol[q] / W.aP[q] : 0.0;
-                const double dF = w * dO + (1.0 - w) * dN;
-                const double dl = dmax(DL[fi], 1e-30);
-                const double ex = DX[fi] / dl, ey = DY[fi] / dl;
-                const double gbx = W.gPx[o] * w + W.gPx[q] * (1.0 - w);
-                const double gby = W.gPy[o] * w + W.gPy[q] * (1.0 - w);
-                ph += -dF * A[fi] * ((W.p[q] - W.p[o]) / delta - (gbx * ex + gby * ey));
-                ph += relaxCorr * (W.phi[f] - W.phiOld[f]);
-                pc = dF * A[fi] / delta;
-            }
-            W.phiPred[f] = ph;
-            W.pCoeff[f] = pc;
-            fs[0] += fabs(ph);
+    const double relaxCorr = 1.0 - st.aU;
+    const double *Ux = W.Ux, *Uy = W.Uy, *Uxp = W.Uxp, *Uyp = W.Uyp, *dP = W.aP, *p = W.p;
+    const double *gPx = W.gPx, *gPy = W.gPy, *phi = W.phi;
+    double *pred = W.phiPred, *coeff = W.pCoeff;
+    FOR_OWN(f, n + nfy) {
+        int o, q;
+        double ph = 0.0, pc = 0.0;
+        if (faceCells(C, f, o, q)) {
+            const double w = __ldg(C.fw + f), v = 1.0 - w, sx = __ldg(C.fsx + f),
+                         sy = __ldg(C.fsy + f), ad = __ldg(C.fad + f);
+            const double x = Ux[o] * w + Ux[q] * v, y = Uy[o] * w + Uy[q] * v;
+            const double x0 = Uxp[o] * w + Uxp[q] * v, y0 = Uyp[o] * w + Uyp[q] * v;
+            const double dF = w * dP[o] + v * dP[q];
+            const double gbx = gPx[o] * w + gPx[q] * v, gby = gPy[o] * w + gPy[q] * v;
+            ph = x * sx + y * sy;
+            ph -= dF * ((p[q] - p[o]) * ad - (gbx * __ldg(C.fex + f) + gby * __ldg(C.fey + f)));
+            ph += relaxCorr * (phi[f] - (x0 * sx + y0 * sy));
+            pc = dF * ad;
         }
+        pred[f] = ph;
+        coeff[f] = pc;
+        fs[0] += fabs(ph);
+    }
 }
 
 __device__ __noinline__ void phPressureCells(Shared &S, double (&pacc)[3]) {
@@ -2141,33 +2029,27 @@ __device__ __noinline__ void phPressureCells(Shared &S, double (&pacc)[3]) {
 // k and omega do not change between the start of the iteration and their solves.
 __device__ __noinline__ void phCorrect(Shared &S, bool turbUpdate) {
     RQ_PRELUDE
-        FOR_CELLS(c) {
-            const Cell q = cellOf(C, c);
-            double gx, gy;
-            ggCell(C, q, W.pp, W.pp[c], W.pp[c], gx, gy);
-            const double rA = (fabs(W.aP[c]) > 1e-30) ? 1.0 / W.aP[c] : 0.0;
-            W.Ux[c] -= rA * gx * C.vol[c];
-            W.Uy[c] -= rA * gy * C.vol[c];
-            W.p[c] += st.aP * W.pp[c];
-            if (turbUpdate) {
-                W.kOld[c] = W.k[c];
-                W.wOld[c] = W.w[c];
-            }
+    const double *pp = W.pp;
+    FOR_CELLS(c) {
+        const Cell q = cellOf(C, c);
+        const GradGeo G(C, q);
+        double gx, gy;
+        const double pc = pp[c], dP = W.aP[c]; // V / a_P
+        G.of(q, nx, pp, pc, pc, gx, gy);
+        W.Ux[c] -= dP * gx;
+        W.Uy[c] -= dP * gy;
+        W.p[c] += st.aP * pc;
+        if (turbUpdate) {
+            W.kOld[c] = W.k[c];
+            W.wOld[c] = W.w[c];
         }
-        FOR_OWN(f, n + nfy) {
-            double v;
-            if (f < n) {
-                const int q = eastOf(C, f);
-                v = W.phiPred[f] - W.pCoeff[f] * (W.pp[q] - W.pp[f]);
-            } else {
-                const int g = f - n, jf = rowOf(C, g);
-                if (jf > 0 && jf < ny)
-                    v = W.phiPred[f] - W.pCoeff[f] * (W.pp[g] - W.pp[g - nx]);
-                else
-                    v = W.phiPred[f] + W.pCoeff[f] * W.pp[jf == 0 ? g : g - nx];
-            }
-            W.phi[f] = v;
-        }
+    }
+    const double *pred = W.phiPred, *coeff = W.pCoeff;
+    double *phi = W.phi;
+    FOR_OWN(f, n + nfy) {
+        int o, q;
+        phi[f] = faceCells(C, f, o, q) ? pred[f] - coeff[f] * (pp[q] - pp[o]) : 0.0;
+    }
 }
 
 // bounds of the solved k and omega (:1489, :1505-1513); a wall cell of omega takes its wall
@@ -2176,13 +2058,14 @@ __device__ __forceinline__ void clampK(const Shared &S, int c) {
     const DevSettings &st = S.C.st;
     S.W.k[c] = dmax(st.kMin, dmin(st.kMax, S.W.k[c]));
 }
-__device__ __forceinline__ void clampW(const Shared &S, int c) {
+__device__ __forceinline__ double clampW(const Shared &S, int c, double iB1) {
     const DevClass &C = S.C;
     const Cell q = cellOf(C, c);
     double v = dmax(C.st.wMin, dmin(1e15, S.W.w[c]));
     if (!q.south || !q.north)
-        v = wallOmega(C, S.coeff[2], dmax(C.ydl[wallFaceOf(C, c)], 1e-20));
+        v = __ldg(C.wallW + wallSlot(C, q)) * iB1;
     S.W.w[c] = v;
+    return v;
 }
 
 // The internal faces of the k or omega assembly, each once (assembleKEquation
@@ -2195,240 +2078,150 @@ __device__ __noinline__ void phTurbFaces(Shared &S, int eq) {
     RQ_PRELUDE
     const double *X = eq == 0 ? W.k : W.w;
     const double *gX = eq == 0 ? W.gKx : W.gWx, *gY = eq == 0 ? W.gKy : W.gWy;
-            FOR_OWN(f, n + nfy) {
-                int fi, o, qn;
-                const double *A, *WT, *DL;
-                double sh = 0.0;
-                const bool xFace = f < n;
-                if (xFace) {
-                    fi = f;
-                    o = f;
-                    qn = eastOf(C, f);
-                    A = C.xa; WT = C.xw; DL = C.xdl;
-                    sh = C.xsh[fi];
-                } else {
-                    fi = f - n;
-                    const int jf = rowOf(C, fi);
-                    if (jf == 0 || jf == ny)
-                        continue;
-                    o = fi - nx;
-                    qn = fi;
-                    A = C.ya; WT = C.yw; DL = C.ydl;
-                }
-                const double delta = dmax(DL[fi], 1e-20);
-                const double F = W.phi[f];
-                const double w = WT[fi];
-                const double F1f = w * W.F1[o] + (1.0 - w) * W.F1[qn];
-                const double sg = eq == 0 ? blend(sk1, sk2, F1f) : blend(sw1, sw2, F1f);
-                const double eO = nu + sg * W.nuT[o], eN = nu + sg * W.nuT[qn];
-                const double ef = w * eO + (1.0 - w) * eN;
-                W.pCoeff[f] = ef * A[fi] / delta;
-                if (eq == 1 && C.balance) { // singular near-wall balance (:1073-1087)
-                    const double amp = 6 * nu / b1;
-                    const double diff = (C.sing[qn] - C.sing[o]) / delta;
-                    const double sgd = xFace ? C.sgx[fi] : C.sgy[fi];
-                    W.phiPred[f] = amp * A[fi] * ((ef - nu) * sgd - ef * diff);
-                }
-                double corr = 0.0;
-                if (F != 0.0) {
-                    const bool ownerUp = F > 0.0;
-                    const int up = ownerUp ? o : qn, dn = ownerUp ? qn : o;
-                    const double xDx = ownerUp ? C.cx[qn] + sh : C.cx[o] - sh;
-                    const double xDy = ownerUp ? C.cy[qn] + 0.0 : C.cy[o] - 0.0;
-                    const double dphi = X[dn] - X[up];
-                    double psi = 0.0;
-                    if (fabs(dphi) > 1e-300) {
-                        const double rr = 2.0 * (gX[up] * (xDx - C.cx[up]) + gY[up] * (xDy - C.cy[up])) / dphi - 1.0;
-                        psi = rr > 0.0 ? (rr * rr + rr) / (rr * rr + 1.0) : 0.0;
-                    }
-                    const double pf = X[up] + 0.5 * psi * dphi;
-                    corr = F * (pf - X[up]);
-                }
-                W.fScr[f] = corr;
-            }
+    const double s1 = eq == 0 ? sk1 : sw1, s2 = eq == 0 ? sk2 : sw2;
+    const bool balance = eq == 1 && C.balance;
+    const double amp = balance ? 6 * nu / b1 : 0.0;
+    const double *nuT = W.nuT, *F1 = W.F1, *phi = W.phi;
+    double *D = W.pCoeff, *bal = W.phiPred, *cc = W.fScr;
+    FOR_OWN(f, n + nfy) {
+        int o, q;
+        if (!faceCells(C, f, o, q))
+            continue;
+        const double w = __ldg(C.fw + f), v = 1.0 - w, F = phi[f];
+        const double sg = blend(s1, s2, w * F1[o] + v * F1[q]);
+        const double et = sg * (w * nuT[o] + v * nuT[q]); // the turbulent part
+        const int up = F > 0.0 ? o : q;
+        const double corr =
+            limitedCorr(F, X[q] - X[o], gX[up], gY[up], __ldg(C.fdx + f), __ldg(C.fdy + f));
+        D[f] = (nu + et) * __ldg(C.fad + f);
+        if (balance) // singular near-wall balance (:1073-1087)
+            bal[f] = amp * (et * __ldg(C.fb1 + f) - (nu + et) * __ldg(C.fb2 + f));
+        cc[f] = corr;
+    }
 }
 
 // The k or omega rows from the face values of phTurbFaces (the wall faces here),
-// sources, relaxation and the omega wall constraint, summed in face order.
-__device__ __noinline__ void phTurbAssemble(Shared &S, int eq) {
+// sources, relaxation and the omega wall constraint (constrainOmega :687-704), summed in
+// face order, and the residual of the constrained initial guess: a wall cell of omega holds
+// its wall value, its row is decoupled and its neighbours take the value to their right-hand
+// side, so no row reads a wall cell's unknown and it is set here. (The residual as a sweep
+// of its own re-read the five coefficients: 3300 cycles at 384 cells, 8700 at 1536.)
+__device__ __noinline__ void phTurbAssemble(Shared &S, int eq, double (&acc)[1]) {
     RQ_PRELUDE
     double *X = eq == 0 ? W.k : W.w;
-                FOR_CELLS(c) {
-                    if (eq == 1) // the bounds of the k just solved (read below at this cell only)
-                        clampK(S, c);
-                    const Cell q = cellOf(C, c);
-                    const bool isWall[4] = {false, false, !q.south, !q.north};
-                    double dT[4] = {0, 0, 0, 0}, aT[4] = {0, 0, 0, 0}, ccT[4] = {0, 0, 0, 0};
-                    double bT[4] = {0, 0, 0, 0}, balT[4] = {0, 0, 0, 0};
-                    for (int k = 0; k < 4; ++k) {
-                        bool own;
-                        int fi, f;
-                        const double *A, *DL;
-                        if (k < 2) {
-                            fi = (k == 0) ? q.W : c;
-                            own = (k == 1);
-                            A = C.xa; DL = C.xdl;
-                            f = fi;
-                        } else {
-                            fi = (k == 2) ? c : c + nx;
-                            own = (k == 3) || isWall[k];
-                            A = C.ya; DL = C.ydl;
-                            f = n + fi;
-                        }
-                        const double F = W.phi[f];
-                        if (isWall[k]) {
-                            const double delta = dmax(DL[fi], 1e-20);
-                            const double sg = eq == 0 ? blend(sk1, sk2, W.F1[c]) : blend(sw1, sw2, W.F1[c]);
-                            const double Db = (nu + sg * W.nuT[c]) * A[fi] / delta;
-                            const double xb = eq == 0 ? 0.0 : bwOf(fi);
-                            if (F >= 0) {
-                                dT[k] = F + Db;
-                                bT[k] = Db * xb;
-                            } else {
-                                dT[k] = Db;
-                                bT[k] = (Db - F) * xb;
-                            }
-                            continue;
-                        }
-                        const double D = W.pCoeff[f];
-                        const double cp = dmax(F, 0.0), cn = dmax(-F, 0.0);
-                        dT[k] = own ? D + cp : D + cn;
-                        aT[k] = own ? -(D + cn) : -(D + cp);
-                        if (eq == 1 && C.balance) {
-                            const double corr = W.phiPred[f];
-                            balT[k] = own ? corr : -corr;
-                        }
-                        if (F != 0.0) {
-                            const double corr = W.fScr[f];
-                            ccT[k] = own ? -corr : corr;
-                        }
-                    }
-                    // face-order sums: internal faces, then the wall face
-                    const int y1 = q.yNfirst ? 3 : 2, y2 = q.yNfirst ? 2 : 3;
-                    const int x1 = q.xEfirst ? 1 : 0, x2 = q.xEfirst ? 0 : 1;
-                    const int ord[4] = {x1, x2, y1, y2};
-                    double dsum = 0.0, bsum = 0.0, bal = 0.0;
-                    for (int t = 0; t < 4; ++t)
-                        if (!isWall[ord[t]]) {
-                            dsum = dsum + dT[ord[t]];
-                            bal = bal + balT[ord[t]];
-                        }
-                    for (int t = 0; t < 4; ++t)
-                        if (isWall[ord[t]]) {
-                            dsum = dsum + dT[ord[t]];
-                            bsum = bsum + bT[ord[t]];
-                        }
-                    const double V = C.vol[c], F1 = W.F1[c];
-                    if (eq == 0) {
-                        bsum += W.Pk[c] * V;
-                        dsum += bs * dmax(W.w[c], 1e-20) * V;
-                    } else {
-                        const double wc = dmax(W.w[c], 1e-20);
-                        const double Sv = W.S[c];
-                        const double S2 = Sv * Sv;
-                        const double lim = 10.0 * bs * dmax(W.k[c], 0.0) * dmax(W.w[c], 1e-20) / dmax(W.nuT[c], 1e-30);
-                        const double prod = dmin(S2, lim);
-                        bsum += blend(al1, al2, F1) * prod * V;
-                        dsum += blend(b1, b2, F1) * wc * V;
-                        bsum += (1.0 - F1) * W.CD[c] * V;
-                        if (C.balance) {
-                            const double corr = bal + nu * (6 * nu / b1) * C.slap[c] * V;
-                            if (corr < 0)
-                                dsum -= corr / wc;
-                            else
-                                bsum += corr;
-                        }
-                    }
-                    for (int t = 0; t < 4; ++t)
-                        if (!isWall[ord[t]])
-                            bsum += ccT[ord[t]];
-                    const double al = eq == 0 ? st.aK : st.aW;
-                    bsum += (1.0 - al) / al * dsum * X[c];
-                    dsum /= al;
-                    // omega: eliminate constrained wall cells (constrainOmega :687-704)
-                    double x0 = X[c];
-                    if (eq == 1) {
-                        const int nbc[4] = {q.W, q.E, c - nx, c + nx};
-                        const bool selfW = !q.south || !q.north;
-                        for (int t = 0; t < 4; ++t) {
-                            const int k = ord[t];
-                            if (isWall[k])
-                                continue;
-                            const int qq = nbc[k];
-                            const bool nbW = qq < nx || qq >= n - nx; // first or last row
-                            const bool own = (k == 1 || k == 3);
-                            if (own) {
-                                if (selfW) {
-                                    aT[k] = 0.0;
-                                } else if (nbW) {
-                                    bsum -= aT[k] * wallOmega(C, b1, dmax(C.ydl[wallFaceOf(C, qq)], 1e-20));
-                                    aT[k] = 0.0;
-                                }
-                            } else {
-                                if (nbW) {
-                                    bsum -= aT[k] * wallOmega(C, b1, dmax(C.ydl[wallFaceOf(C, qq)], 1e-20));
-                                    aT[k] = 0.0;
-                                } else if (selfW) {
-                                    aT[k] = 0.0;
-                                }
-                            }
-                        }
-                        if (selfW) {
-                            const double val = wallOmega(C, b1, dmax(C.ydl[wallFaceOf(C, c)], 1e-20));
-                            bsum = dsum * val;
-                            x0 = val;
-                        }
-                    }
-                    W.d[c] = dsum;
-                    W.aW[c] = aT[0];
-                    W.aE[c] = aT[1];
-                    W.aS[c] = aT[2];
-                    W.aN[c] = aT[3];
-                    W.b[c] = bsum;
-                    (void)x0;
-                }
+    const double *phi = W.phi, *D = W.pCoeff, *bal = W.phiPred, *ccf = W.fScr;
+    const double s1 = eq == 0 ? sk1 : sw1, s2 = eq == 0 ? sk2 : sw2;
+    const bool balance = eq == 1 && C.balance;
+    const double iB1 = 1.0 / b1, iBeta = 1.0 / S.wallBeta;
+    FOR_CELLS(c) {
+        if (eq == 1) // the bounds of the k just solved (read below at this cell only)
+            clampK(S, c);
+        const Cell q = cellOf(C, c);
+        const int fW = q.W, fE = c, fS = n + c, fN = n + c + nx;
+        const double F1 = W.F1[c], nuT = W.nuT[c];
+        const double FW = phi[fW], FE = phi[fE], DW = D[fW], DE = D[fE];
+        const double wall = nu + blend(s1, s2, F1) * nuT; // viscosity at a wall face
+        double aW = -(DW + dmax(FW, 0.0)), aE = -(DE + dmax(-FE, 0.0)), aS = 0.0, aN = 0.0;
+        double dS, dN, bsum = 0.0, bl = 0.0, cc = ccf[fW] - ccf[fE];
+        if (balance)
+            bl = bal[fE] - bal[fW];
+        if (q.south) {
+            const double F = phi[fS], d = D[fS];
+            dS = d + dmax(-F, 0.0);
+            aS = -(d + dmax(F, 0.0));
+            cc += ccf[fS];
+            if (balance)
+                bl -= bal[fS];
+        } else {
+            dS = wall * __ldg(C.fad + fS);
+            if (eq == 1)
+                bsum += dS * (__ldg(C.wallFw + q.i) * iBeta);
+        }
+        if (q.north) {
+            const double F = phi[fN], d = D[fN];
+            dN = d + dmax(F, 0.0);
+            aN = -(d + dmax(-F, 0.0));
+            cc -= ccf[fN];
+            if (balance)
+                bl += bal[fN];
+        } else {
+            dN = wall * __ldg(C.fad + fN);
+            if (eq == 1)
+                bsum += dN * (__ldg(C.wallFw + nx + q.i) * iBeta);
+        }
+        double dsum = (DW + dmax(-FW, 0.0)) + (DE + dmax(FE, 0.0));
+        dsum = q.south ? (dsum + dS) + dN : (dsum + dN) + dS; // the wall comes last
+        const double V = __ldg(C.vol + c), wc = dmax(W.w[c], 1e-20);
+        if (eq == 0) {
+            bsum += W.Pk[c] * V;
+            dsum += bs * wc * V;
+        } else {
+            const double Sv = W.S[c];
+            const double lim = quot(10.0 * bs * dmax(W.k[c], 0.0) * wc, dmax(nuT, 1e-30));
+            bsum += blend(al1, al2, F1) * dmin(Sv * Sv, lim) * V;
+            dsum += blend(b1, b2, F1) * wc * V;
+            bsum += (1.0 - F1) * W.CD[c] * V;
+            if (balance) {
+                const double corr = bl + nu * (6 * nu * iB1) * __ldg(C.slap + c) * V;
+                if (corr < 0)
+                    dsum -= quot(corr, wc);
+                else
+                    bsum += corr;
+            }
+        }
+        bsum += cc;
+        const double xo = X[c];
+        bsum += C.relax[2 + 2 * eq] * dsum * xo; // (1 - alpha) / alpha
+        dsum *= C.relax[3 + 2 * eq];
+        double rc;
+        if (eq == 1 && (!q.south || !q.north)) {
+            const double val = __ldg(C.wallW + wallSlot(C, q)) * iB1;
+            aW = aE = aS = aN = 0.0;
+            bsum = dsum * val;
+            X[c] = val;
+            rc = 0.0;
+        } else {
+            if (eq == 1 && q.j == 1) {
+                bsum -= aS * (__ldg(C.wallW + q.i) * iB1);
+                aS = 0.0;
+            }
+            if (eq == 1 && q.j == ny - 2) {
+                bsum -= aN * (__ldg(C.wallW + nx + q.i) * iB1);
+                aN = 0.0;
+            }
+            const double tS = q.south && !(eq == 1 && q.j == 1) ? aS * X[c - nx] : 0.0;
+            const double tN = q.north && !(eq == 1 && q.j == ny - 2) ? aN * X[c + nx] : 0.0;
+            rc = bsum - accum4(q, dsum * xo, aW * X[q.W], aE * X[q.E], tS, tN);
+        }
+        W.d[c] = dsum;
+        W.aW[c] = aW;
+        W.aE[c] = aE;
+        W.aS[c] = aS;
+        W.aN[c] = aN;
+        W.b[c] = bsum;
+        W.r[c] = rc;
+        acc[0] += rc * rc;
+    }
 }
 
-__device__ __noinline__ void phTurbResidual(Shared &S, int eq, double (&acc)[1]) {
-    RQ_PRELUDE
-    double *X = eq == 0 ? W.k : W.w;
-    const double *gX = eq == 0 ? W.gKx : W.gWx, *gY = eq == 0 ? W.gKy : W.gWy;
-    (void)gX; (void)gY;
-                FOR_CELLS(c) {
-                    const Cell q = cellOf(C, c);
-                    auto x0 = [&](int cc) {
-                        return (eq == 1 && isWallCell(C, cc))
-                                   ? wallOmega(C, b1, dmax(C.ydl[wallFaceOf(C, cc)], 1e-20))
-                                   : X[cc];
-                    };
-                    const double tW = W.aW[c] * x0(q.W), tE = W.aE[c] * x0(q.E);
-                    const double tS = q.south ? W.aS[c] * x0(c - nx) : 0.0;
-                    const double tN = q.north ? W.aN[c] * x0(c + nx) : 0.0;
-                    const double xc = x0(c);
-                    const double rc = W.b[c] - accum4(q, W.d[c] * xc, tW, tE, tS, tN);
-                    W.r[c] = rc;
-                    acc[0] += rc * rc;
-                    if (eq == 1)
-                        X[c] = xc;
-                }
-}
-
+// Change norms; mx[4], mx[5]: squares of the largest |U| and |dU|.
 __device__ __noinline__ void phNorms(Shared &S, bool turbUpdate, double (&mx)[6]) {
     RQ_PRELUDE
-        if (turbUpdate && threadIdx.x == 0)
-            S.wallBeta = b1;
-        FOR_CELLS(c) {
-            if (turbUpdate) {
-                clampW(S, c);
-                mx[0] = dmax(mx[0], fabs(W.k[c]));
-                mx[1] = dmax(mx[1], fabs(W.w[c]));
-                mx[2] = dmax(mx[2], fabs(W.k[c] - W.kOld[c]));
-                mx[3] = dmax(mx[3], fabs(W.w[c] - W.wOld[c]));
-            }
-            mx[4] = dmax(mx[4], sqrt(W.Ux[c] * W.Ux[c] + W.Uy[c] * W.Uy[c] + 0.0));
-            const double ax = W.Ux[c] - W.Uxp[c], ay = W.Uy[c] - W.Uyp[c];
-            mx[5] = dmax(mx[5], sqrt(ax * ax + ay * ay + 0.0));
+    if (turbUpdate && threadIdx.x == 0)
+        S.wallBeta = b1;
+    const double iB1 = 1.0 / b1;
+    FOR_CELLS(c) {
+        if (turbUpdate) {
+            const double w = clampW(S, c, iB1), k = W.k[c];
+            mx[0] = dmax(mx[0], fabs(k));
+            mx[1] = dmax(mx[1], fabs(w));
+            mx[2] = dmax(mx[2], fabs(k - W.kOld[c]));
+            mx[3] = dmax(mx[3], fabs(w - W.wOld[c]));
         }
+        const double x = W.Ux[c], y = W.Uy[c], ax = x - W.Uxp[c], ay = y - W.Uyp[c];
+        mx[4] = dmax(mx[4], x * x + y * y);
+        mx[5] = dmax(mx[5], ax * ax + ay * ay);
+    }
 }
 
 __device__ __noinline__ void phProbes(Shared &S) {
@@ -2590,12 +2383,7 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
                 double acc[1] = {0.0};
                 phTurbFaces(S, eq);
                 SYNC();
-                phTurbAssemble(S, eq);
-                SYNC();
-                // initial residual with the (constrained) initial guess: wall cells of
-                // omega start from their wall value (read through x0, never from X,
-                // so the in-place update below cannot race with a neighbour's read)
-                phTurbResidual(S, eq, acc);
+                phTurbAssemble(S, eq, acc);
                 blockSum<1>(acc, S, rp);
                 LinRes &rr = eq == 0 ? resK : resW;
                 solveBicg(S, rp, X, sqrt(acc[0]), st.innerIter, st.innerTol, &rr);
@@ -2607,14 +2395,14 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
 
         mark(S, 6);
         // ---- change norms and bookkeeping (:1520-1715)
-        double mx[6] = {1e-30, 1e-30, 0.0, 0.0, 1e-300, 0.0};
+        double mx[6] = {1e-30, 1e-30, 0.0, 0.0, 0.0, 0.0};
         phNorms(S, turbUpdate, mx);
         blockMax<6>(mx, S, rp);
         if (turbUpdate) {
             lastK = mx[2] / mx[0];
             lastW = mx[3] / mx[1];
         }
-        Ls.uChange = mx[5] / mx[4];
+        Ls.uChange = sqrt(mx[5]) / dmax(sqrt(mx[4]), 1e-300);
         // one barrier pair for every sample of this iteration (U, k, omega, monitor)
         SYNC();
         if (threadIdx.x == 0) {
@@ -2823,6 +2611,8 @@ __device__ void runJob(Shared &S, const DevJob &job, double *ws, double *arena, 
         int *dst = reinterpret_cast<int *>(&S.C);
         for (int t = threadIdx.x; t < words; t += blockDim.x)
             dst[t] = src[t];
+        for (int t = threadIdx.x; t < 2 * kRedSlots * 32; t += blockDim.x)
+            (&S.red[0][0][0])[t] = 0.0;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
