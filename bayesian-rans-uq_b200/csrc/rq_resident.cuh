@@ -534,7 +534,7 @@ __device__ __forceinline__ void coarseRes(Shared &S, const double *rr0) {
     }
 }
 
-// PCG (LinearSolver.hpp:184-246 / :908-982) from x = 0, with the V-cycle or the Jacobi
+// PCG (LinearSolver.hpp:184-246 / :908-982) from x = 0 (set by the assembly), with the V-cycle or the Jacobi
 // preconditioner; K64.r holds b and r0n its norm. The working group
 // holds the finest level in registers; all threads of the CTA run the coarse levels. The
 // caller's next CTA barrier makes x and *out visible.
@@ -561,7 +561,7 @@ __device__ __noinline__ void pcgRes(double *x, double r0n, int maxIter, double t
     const double om = C.amgW, al = C.amgAlpha;
     const double bound2 = (tol * r0n) * (tol * r0n);
     ResRows A;
-    double r[kResCells], p[kResCells], xv[kResCells];
+    double r[kResCells], p[kResCells];
     int rp = 0;
     double rz = 0.0;
     if (mine) {
@@ -570,38 +570,30 @@ __device__ __noinline__ void pcgRes(double *x, double r0n, int maxIter, double t
         for (int k = 0; k < kResCells; ++k) {
             const int c = threadIdx.x + k * T;
             r[k] = c < n ? S.K64.r[c] : 0.0;
-            p[k] = xv[k] = 0.0;
+            p[k] = 0.0;
         }
         resClear(S, e0, e1, T);
     }
     for (int it = 0;; ++it) {
         double z[kResCells], q[1] = {0.0};
         if constexpr (AMG) {
-            if (mine && L > 1) { // pre-smoothed iterate in z, the residual in e1
+            if (mine && L > 1) { // pre-smoothed iterate in e0, the residual in e1
+                double *first = two ? e1 : e0;
 #pragma unroll
-                for (int k = 0; k < kResCells; ++k) {
-                    z[k] = om * r[k] * A.rd[k];
-                    e0[threadIdx.x + k * T] = z[k];
-                }
+                for (int k = 0; k < kResCells; ++k)
+                    first[threadIdx.x + k * T] = om * r[k] * A.rd[k];
                 groupSync(T);
                 if (two) {
 #pragma unroll
                     for (int k = 0; k < kResCells; ++k) {
-                        z[k] += om * (r[k] - A.times(k, z[k], e0)) * A.rd[k];
-                        e1[threadIdx.x + k * T] = z[k];
+                        const double z0 = om * r[k] * A.rd[k];
+                        e0[threadIdx.x + k * T] = z0 + om * (r[k] - A.times(k, z0, e1)) * A.rd[k];
                     }
                     groupSync(T);
                 }
-                const double *e = two ? e1 : e0;
-                double rr[kResCells];
 #pragma unroll
                 for (int k = 0; k < kResCells; ++k)
-                    rr[k] = r[k] - A.times(k, z[k], e);
-                if (two)
-                    groupSync(T); // e1 is read until here
-#pragma unroll
-                for (int k = 0; k < kResCells; ++k)
-                    e1[threadIdx.x + k * T] = rr[k];
+                    e1[threadIdx.x + k * T] = r[k] - A.times(k, e0[threadIdx.x + k * T], e0);
             } else if (mine) {
 #pragma unroll
                 for (int k = 0; k < kResCells; ++k)
@@ -622,17 +614,14 @@ __device__ __noinline__ void pcgRes(double *x, double r0n, int maxIter, double t
                 }
 #pragma unroll
                 for (int k = 0; k < kResCells; ++k) {
-                    z[k] += al * pz[k];
+                    z[k] = e0[threadIdx.x + k * T] + al * pz[k];
                     e0[threadIdx.x + k * T] = z[k];
                 }
                 groupSync(T);
                 if (two) {
 #pragma unroll
-                    for (int k = 0; k < kResCells; ++k)
-                        pz[k] = z[k] + om * (r[k] - A.times(k, z[k], e0)) * A.rd[k];
-#pragma unroll
                     for (int k = 0; k < kResCells; ++k) {
-                        z[k] = pz[k];
+                        z[k] += om * (r[k] - A.times(k, z[k], e0)) * A.rd[k];
                         e1[threadIdx.x + k * T] = z[k];
                     }
                     groupSync(T);
@@ -677,9 +666,11 @@ __device__ __noinline__ void pcgRes(double *x, double r0n, int maxIter, double t
                 q[0] = 0.0;
 #pragma unroll
                 for (int k = 0; k < kResCells; ++k) {
-                    xv[k] += alpha * p[k];
+                    const int c = threadIdx.x + k * T;
                     r[k] -= alpha * Ap[k];
                     q[0] += r[k] * r[k];
+                    if (c < n)
+                        x[c] += alpha * p[k];
                 }
                 sumRes<1>(q, rp, nw);
                 res.iterations = it + 1;
@@ -699,14 +690,6 @@ __device__ __noinline__ void pcgRes(double *x, double r0n, int maxIter, double t
         } else if (!mine) {
             break;
         }
-    }
-    if (!mine)
-        return;
-#pragma unroll
-    for (int k = 0; k < kResCells; ++k) {
-        const int c = threadIdx.x + k * T;
-        if (c < n)
-            x[c] = xv[k];
     }
     if (threadIdx.x == 0) {
         res.finalRes = sqrt(res.finalRes) / r0n;
