@@ -26,10 +26,6 @@ __host__ __device__ inline long resExchange(long n) {
 
 extern __shared__ __align__(16) unsigned char rqSmem[];
 
-__device__ __forceinline__ void groupSync(int threads) {
-    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
-}
-
 // Sums of K values over the working group (nw warps), the same bits in every thread. A
 // warp adds its lanes with two FP64 matrix products: ones times the lanes' values gives
 // column sums of four lanes, of which each lane adds two and which a second product with

@@ -185,6 +185,11 @@ __device__ __forceinline__ void mark(Shared &S, int k) {
     }
 }
 
+// barrier of the CTA's first `threads` threads (a multiple of 32)
+__device__ __forceinline__ void groupSync(int threads) {
+    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
+
 // ---------------------------------------------------------------- arithmetic
 // a / b by Newton-Raphson iteration from the hardware's approximate reciprocal, and one
 // correction of the quotient: within one unit in the last place for operands and quotients
@@ -604,11 +609,79 @@ __device__ __forceinline__ T *levelVec(const Shared &S, const KW<T> &K, int l) {
     return K.amgVec + off;
 }
 
+// In-place inverse of the m x m matrix A (row-major, m <= kMaxCoarse; Gauss-Jordan, SPD: no
+// pivoting) by the CTA's first 512 threads: each holds a tile of 8 x 4 entries, 16 rows and 32
+// columns apart, and a pivot's row and column pass through shared memory (alternating
+// buffers, one barrier per pivot). The inverse goes to out with leading dimension ld.
+// Bound by issue and the barrier: a sweep over [A | I] in global memory moved 2 m^2 doubles in
+// and out per pivot, 375 us for 96 rows.
+constexpr int kInvThreads = 512;
+__device__ __noinline__ void invertTiled(Shared &S, const double *A, int m, double *out, int ld) {
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    double a[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = ty + 16 * i, c = tx + 32 * j;
+            a[i][j] = r < m && c < m ? A[r * m + c] : 0.0;
+        }
+    // rows and columns of the pivot, alternating: 4 x kMaxCoarse doubles
+    double *buf = S.coarse;
+    auto publish = [&](int p) {
+        double *row = buf + (p & 1) * 2 * kMaxCoarse, *col = row + kMaxCoarse;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (ty + 16 * i == p)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    row[tx + 32 * j] = a[i][j];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (tx + 32 * j == p)
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    col[ty + 16 * i] = a[i][j];
+        groupSync(kInvThreads);
+    };
+    publish(0);
+    for (int p = 0; p < m; ++p) {
+        const double *row = buf + (p & 1) * 2 * kMaxCoarse, *col = row + kMaxCoarse;
+        const double inv = 1.0 / row[p];
+        double pr[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            pr[j] = row[tx + 32 * j] * inv;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (16 * i >= m)
+                break;
+            const double f = col[ty + 16 * i];
+            const bool own = ty + 16 * i == p;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const double v = tx + 32 * j == p ? -f * inv : a[i][j] - f * pr[j];
+                a[i][j] = own ? (tx + 32 * j == p ? inv : pr[j]) : v;
+            }
+        }
+        if (p + 1 < m)
+            publish(p + 1);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = ty + 16 * i, c = tx + 32 * j;
+            if (r < m && c < m)
+                out[r * ld + c] = a[i][j];
+        }
+}
+
 // Galerkin values of every coarse level from the current pressure system, the
 // reciprocal diagonals of the smoothed levels, then the inverse of the coarsest
 // level (Gauss-Jordan, SPD: no pivoting): in place by one warp, one row per lane,
-// when it has at most 32 rows; above that (up to 128) by the whole CTA, one
-// barrier per pivot, ping-ponging [A | I] between two workspace buffers. (One warp
+// when it has at most 32 rows; above that (up to 128) in register tiles (invertTiled), in
+// CTAs of fewer than 512 threads by sweeps over [A | I] between two workspace buffers. (One warp
 // with two rows per lane was measured 17 % slower per outer iteration at 1536
 // cells: 128 dependent updates per lane and pivot against 16 per thread.) The
 // inverse is FP64 in both forms.
@@ -699,11 +772,13 @@ template <typename T> __device__ __noinline__ void amgRefreshT(Shared &S, const 
         SYNC();
         return;
     }
-    // m x 2m [A | I], row-major; the inverse ends in the right half of dense0
-    const int m2 = 2 * m;
-    double *A0 = W.dense0, *A1 = W.dense1;
+    // m x 2m [A | I], row-major; the inverse ends in the right half of dense0 (the tiled
+    // inversion takes A alone, in dense1)
+    const bool tiled = static_cast<int>(blockDim.x) >= kInvThreads;
+    const int m2 = tiled ? m : 2 * m;
+    double *A0 = tiled ? W.dense1 : W.dense0, *A1 = W.dense1;
     for (int e = threadIdx.x; e < m * m2; e += blockDim.x)
-        A0[e] = ((e % m2) == m + e / m2) ? 1.0 : 0.0;
+        A0[e] = !tiled && ((e % m2) == m + e / m2) ? 1.0 : 0.0;
     __syncthreads();
     if (L == 1) {
         for (int r = threadIdx.x; r < m; r += blockDim.x) {
@@ -725,6 +800,12 @@ template <typename T> __device__ __noinline__ void amgRefreshT(Shared &S, const 
             }
     }
     __syncthreads();
+    if (tiled) {
+        if (threadIdx.x < kInvThreads)
+            invertTiled(S, A0, m, W.dense0 + m, 2 * m);
+        SYNC();
+        return;
+    }
     // the (row, column) of a thread's entries advance by the CTA width without a division
     const int dq = static_cast<int>(blockDim.x) / m2, dr = static_cast<int>(blockDim.x) - dq * m2;
     const int r0 = static_cast<int>(threadIdx.x) / m2, c0 = static_cast<int>(threadIdx.x) - r0 * m2;
