@@ -942,6 +942,10 @@ int rq_evaluate_batch(rq_problem *p, const double *theta, int64_t n, rq_row_out 
         launchRows(*p, probOfRow, p->dTheta.as<double>(), na, p->dRows.as<rq::RowOut>(),
                    p->dPred.as<double>(), no, fields ? p->dFields.as<double>() : nullptr, 11L * nc,
                    wantHist ? p->dHist.as<double>() : nullptr, hist_cap, nullptr, nullptr);
+        if (fields)
+            prefault(fields, sizeof(double) * n * 11L * nc);
+        if (wantHist)
+            prefault(history, sizeof(double) * n * 11L * hist_cap);
         std::vector<rq::RowOut> hr(n);
         std::vector<double> hp(static_cast<size_t>(n) * no);
         check(cudaMemcpy(hr.data(), p->dRows.p, sizeof(rq::RowOut) * n, cudaMemcpyDeviceToHost), "rows");

@@ -133,11 +133,16 @@ class LinearBatch:
     def solve(self, max_iter: int = 500, tol: float = 1e-6, xs=None):
         """From xs (or zero); returns (results, solutions)."""
         out = (N.SolverResult * len(self.systems))()
-        sol = [np.zeros(s.n_cells) for s in self.systems] if xs is None else xs
-        N.call("rq_linsys_solve", self.handle, C.c_int32(max_iter), C.c_double(tol),
-               _x_pointers(sol) if xs is not None else None, out)
         if xs is None:
-            N.call("rq_linsys_results", self.handle, None, _x_pointers(sol))
+            # the solutions' pages are touched while the device solves
+            N.call("rq_linsys_solve_device", self.handle, C.c_int32(max_iter), C.c_double(tol),
+                   C.c_void_p(0))
+            sol = [np.full(s.n_cells, 0.0) for s in self.systems]
+            N.call("rq_linsys_results", self.handle, out, _x_pointers(sol))
+        else:
+            sol = xs
+            N.call("rq_linsys_solve", self.handle, C.c_int32(max_iter), C.c_double(tol),
+                   _x_pointers(sol), out)
         return [_result(r) for r in out], sol
 
     def solve_device(self, max_iter: int, tol: float, stream: int = 0) -> None:
