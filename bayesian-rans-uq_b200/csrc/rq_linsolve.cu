@@ -80,7 +80,7 @@ template <int K> __device__ __forceinline__ void blockSum(double (&v)[K], LinSha
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        double s = S.red[k][lane];
+        double s = lane < NT / 32 ? S.red[k][lane] : 0.0;
         for (int o = 16; o > 0; o >>= 1)
             s += __shfl_xor_sync(FULL, s, o);
         v[k] = s;
@@ -100,7 +100,7 @@ template <int K> __device__ __forceinline__ void blockSum(double (&v)[K], LinSha
         rp ^= 1;
     }
 }
-static_assert(NT / 32 == 32, "blockSum reads one partial per lane");
+static_assert(NT / 32 <= 32, "blockSum reads one partial per lane");
 
 // one level of the hierarchy in value type T (FP64, or the FP32 copies)
 template <typename T> struct Lv {
@@ -111,30 +111,36 @@ template <typename T> struct Lv {
     T *b, *x, *r; // workspace vectors (levels >= 1; level 0 uses the caller's)
 };
 
-// Row i times x, entries in order. Five columns and values (a grid system's row) are
-// loaded before the first is used.
-template <typename T> __device__ __forceinline__ T rowTimes(const Lv<T> &A, int i, const T *x) {
-    const int k0 = __ldg(A.ptr + (i >> A.sh)), k1 = __ldg(A.ptr + (i >> A.sh) + 1);
+// use(i, row i times x) for the rows t0, t0 + nt, ...; entries in order. The first five columns
+// and values (a grid system's row) are loaded before the first is used. (Two rows at a time
+// with 1024 threads, two or four with 512: 2 to 18 % slower at every size but 512 x 512 with
+// 1024 threads, 1 % slower there; the registers spill or the warps are too few.)
+template <typename T, typename Use>
+__device__ __forceinline__ void passRows(const Lv<T> &A, const T *x, int t0, int nt, Use use) {
+    constexpr int B = 5;
     const int step = 1 << A.sh;
-    T s = T(0);
-    for (int e = k0 + (i & (step - 1)); e < k1; e += 5 * step) {
-        int c[5];
-        T v[5], xc[5];
+    for (int i = t0; i < A.n; i += nt) {
+        const int k1 = __ldg(A.ptr + (i >> A.sh) + 1);
+        T s = T(0);
+        for (int e = __ldg(A.ptr + (i >> A.sh)) + (i & (step - 1)); e < k1; e += B * step) {
+            int c[B];
+            T v[B], xc[B];
 #pragma unroll
-        for (int u = 0; u < 5; ++u) {
-            const bool in = e + u * step < k1;
-            c[u] = in ? __ldg(A.col + e + u * step) : -1;
-            v[u] = in ? __ldg(A.val + e + u * step) : T(0);
+            for (int u = 0; u < B; ++u) {
+                const bool in = e + u * step < k1;
+                c[u] = in ? __ldg(A.col + e + u * step) : -1;
+                v[u] = in ? __ldg(A.val + e + u * step) : T(0);
+            }
+#pragma unroll
+            for (int u = 0; u < B; ++u)
+                xc[u] = c[u] >= 0 ? x[c[u]] : T(0);
+#pragma unroll
+            for (int u = 0; u < B; ++u)
+                if (c[u] >= 0)
+                    s += v[u] * xc[u];
         }
-#pragma unroll
-        for (int u = 0; u < 5; ++u)
-            xc[u] = c[u] >= 0 ? x[c[u]] : T(0);
-#pragma unroll
-        for (int u = 0; u < 5; ++u)
-            if (c[u] >= 0)
-                s += v[u] * xc[u];
+        use(i, s);
     }
-    return s;
 }
 
 template <typename T>
@@ -205,13 +211,12 @@ __device__ double vcycle(LinShared &S, const T *r, T *z, T *t, void *lvws, const
             }
         }
         sync(l);
-        for (int i = t0; i < A.n; i += nt) {
-            const T res = b[i] - rowTimes(A, i, x);
+        passRows<T>(A, x, t0, nt, [&](int i, T ax) {
+            const T res = b[i] - ax;
             y[i] = x[i] + w * res * __ldg(A.rdg + i);
-        }
+        });
         sync(l);
-        for (int i = t0; i < A.n; i += nt)
-            x[i] = b[i] - rowTimes(A, i, y);
+        passRows<T>(A, y, t0, nt, [&](int i, T ax) { x[i] = b[i] - ax; });
         sync(l);
         fr = x;
     }
@@ -245,18 +250,18 @@ __device__ double vcycle(LinShared &S, const T *r, T *z, T *t, void *lvws, const
         for (int i = t0; i < A.n; i += nt)
             y[i] += T(kAlpha) * xc[__ldg(A.agg + i)];
         sync(l);
-        for (int i = t0; i < A.n; i += nt) {
-            const T res = b[i] - rowTimes(A, i, y);
+        passRows<T>(A, y, t0, nt, [&](int i, T ax) {
+            const T res = b[i] - ax;
             x[i] = y[i] + w * res * __ldg(A.rdg + i);
-        }
+        });
         sync(l);
-        for (int i = t0; i < A.n; i += nt) {
-            const T res = b[i] - rowTimes(A, i, x);
+        passRows<T>(A, x, t0, nt, [&](int i, T ax) {
+            const T res = b[i] - ax;
             const T zi = x[i] + w * res * __ldg(A.rdg + i);
             y[i] = zi;
             if (l == 0)
                 rz += double(r[i]) * double(zi);
-        }
+        });
         if (l > 0) // level 0: the caller's block sum
             sync(l);
         xc = y;
@@ -301,11 +306,10 @@ __device__ PcgOut pcg(LinShared &S, int &rp, const Lv<T> &A0, T *x, T *r, T *z, 
     gSync(S);
     for (int it = 0; it < maxIter; ++it) {
         double b1[1] = {0.0};
-        for (int i = gTid(S); i < n; i += gThreads(S)) {
-            const T v = rowTimes(A0, i, p);
+        passRows<T>(A0, p, gTid(S), gThreads(S), [&](int i, T v) {
             q[i] = v;
             b1[0] += double(p[i]) * double(v);
-        }
+        });
         blockSum<1>(b1, S, rp);
         const double pAp = b1[0];
         if (fabs(pAp) < 1e-30)
@@ -362,11 +366,10 @@ __device__ PcgOut bicgstab(LinShared &S, int &rp, const Lv<double> &A0, double *
         }
         gSync(S);
         double a1[1] = {0.0};
-        for (int i = gTid(S); i < n; i += gThreads(S)) {
-            const double vi = rowTimes(A0, i, ph);
+        passRows<double>(A0, ph, gTid(S), gThreads(S), [&](int i, double vi) {
             v[i] = vi;
             a1[0] += rh[i] * vi;
-        }
+        });
         blockSum<1>(a1, S, rp);
         if (fabs(a1[0]) < 1e-30)
             break;
@@ -390,12 +393,11 @@ __device__ PcgOut bicgstab(LinShared &S, int &rp, const Lv<double> &A0, double *
             return o;
         }
         double a3[2] = {0.0, 0.0};
-        for (int i = gTid(S); i < n; i += gThreads(S)) {
-            const double ti = rowTimes(A0, i, sh);
+        passRows<double>(A0, sh, gTid(S), gThreads(S), [&](int i, double ti) {
             t[i] = ti;
             a3[0] += ti * ti;
             a3[1] += ti * s[i];
-        }
+        });
         blockSum<2>(a3, S, rp);
         omega = a3[0] > 1e-30 ? a3[1] / a3[0] : 0.0;
         double a4[2] = {0.0, 0.0};
@@ -426,11 +428,11 @@ __device__ PcgOut bicgstab(LinShared &S, int &rp, const Lv<double> &A0, double *
 __device__ double residual(LinShared &S, int &rp, const Lv<double> &A0, const double *b,
                            const double *x, double *r) {
     double a[1] = {0.0};
-    for (int i = gTid(S); i < A0.n; i += gThreads(S)) {
-        const double ri = b[i] - rowTimes(A0, i, x);
+    passRows<double>(A0, x, gTid(S), gThreads(S), [&](int i, double ax) {
+        const double ri = b[i] - ax;
         r[i] = ri;
         a[0] += ri * ri;
-    }
+    });
     blockSum<1>(a, S, rp);
     return sqrt(a[0]);
 }
