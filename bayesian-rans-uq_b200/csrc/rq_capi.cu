@@ -477,7 +477,10 @@ void upload(rq_problem &P, const rq_obs_desc *obs, double nu, const rq_settings 
 // (1536 cells over the first 400 iterations: 332 us; 397 us with 768 threads, whose 80
 // registers leave only the general solvers), 768 threads above (200 x 100 bump, general
 // solvers: 12.4 ms against 17.0 ms with 512).
-int defaultBlock(int nCells) { return nCells > 1536 ? 768 : 512; }
+// (The mixed form has no resident solvers: 768 threads above 1024 cells.)
+int defaultBlock(int nCells, int precision) {
+    return nCells > (precision == RQ_PREC_MIXED ? 1024 : 1536) ? 768 : 512;
+}
 
 
 
@@ -678,7 +681,7 @@ int rq_problem_create(const rq_mesh_desc *mesh, const rq_bc_desc *bc, double nu,
         std::memcpy(P->base, base, sizeof(P->base));
         P->nObs = obs ? obs->n_obs : 0;
         P->block = settings->block_threads ? rq::normalizeBlock(settings->block_threads)
-                                           : defaultBlock(P->mesh.n);
+                                           : defaultBlock(P->mesh.n, settings->precision);
         upload(*P, obs, nu, *settings, init);
         // the device address of rq_evaluate_noalloc's fixed scratch array, resolved here
         // (this call allocates anyway) so that the allocation-free call itself only launches

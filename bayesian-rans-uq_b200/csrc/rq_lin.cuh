@@ -11,6 +11,7 @@ namespace rq {
 constexpr int kLinMaxLevels = 16;
 constexpr int kLinThreads = 1024;
 constexpr int kLinMaxCluster = 16;
+constexpr int kLinMaxLocalBytes = 220 * 1024; // shared memory of the local levels' vectors
 constexpr int kLinLocalRows = 2048; // rows of a level that every CTA of a cluster runs whole
 enum LinKind : int32_t { kLinAmg = 0, kLinPcg = 1, kLinBicgstab = 2 };
 

@@ -148,8 +148,10 @@ void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int preci
         d.precision = mixed && kind != rq::kLinBicgstab ? 1 : 0;
         d.m = h.m;
         d.loc = nl;
-        while (d.loc > 1 && h.lev[d.loc - 1].n <= rq::kLinLocalRows)
-            --d.loc;
+        long localRows = 0; // b, x and r of the local levels fit in shared memory
+        while (d.loc > 1 && h.lev[d.loc - 1].n <= rq::kLinLocalRows &&
+               24 * (localRows + h.lev[d.loc - 1].n) <= rq::kLinMaxLocalBytes)
+            localRows += h.lev[--d.loc].n;
         long lvecs = 0, local = 0;
         for (int l = 0; l < nl; ++l) {
             const rq::LinLevelHost &lv = h.lev[l];

@@ -539,9 +539,11 @@ __global__ void __launch_bounds__(NT, 1) linKernel(const DevLinSys *systems, int
 namespace {
 cudaError_t linConfig(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, int slots, int cluster,
                       size_t localBytes, cudaStream_t stream) {
+    // the limit of the largest local levels, not of this launch: it belongs to the function, and
+    // another thread may be launching it for other systems
     cudaError_t e = cudaFuncSetAttribute(linKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(localBytes));
-    if (e == cudaSuccess && cluster > 8)
+                                         kLinMaxLocalBytes);
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute(linKernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cfg = cudaLaunchConfig_t{};
     cfg.gridDim = dim3(slots * cluster);

@@ -2924,9 +2924,15 @@ void *shapeEntry(int kind, const LaunchShape &sh) {
 size_t shapeBytes(const LaunchShape &sh) {
     return (sh.cluster > 1 ? clusterSharedBytes() : solveSharedBytes()) + sizeof(double) * static_cast<size_t>(sh.arenaDoubles);
 }
+// The limits are set to the device's own, not to the launch's: they belong to the function, and
+// another thread may be launching it with another arena.
 cudaError_t setAttributes(void *fn, const LaunchShape &sh) {
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(shapeBytes(sh)));
+    int dev = 0, optin = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e == cudaSuccess && sh.cluster > 8)
         e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
@@ -3004,8 +3010,7 @@ cudaError_t launchServe(const ServeQueue &q, double *ws, long wsStride, int grid
     void *fn = pickServe(block);
     if (!fn)
         return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    cudaError_t e = setAttributes(fn, {block, arenaDoubles, 1});
     if (e != cudaSuccess)
         return e;
     ServeQueue qq = q;
@@ -3019,10 +3024,7 @@ cudaError_t launchServe(const ServeQueue &q, double *ws, long wsStride, int grid
 int serveBlocksPerSM(int block, int arenaDoubles) {
     const size_t smem = solveSharedBytes() + sizeof(double) * static_cast<size_t>(arenaDoubles);
     void *fn = pickServe(block);
-    if (!fn)
-        return 0;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-        cudaSuccess)
+    if (!fn || setAttributes(fn, {block, arenaDoubles, 1}) != cudaSuccess)
         return 0;
     int blocks = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, block, smem) != cudaSuccess)
