@@ -53,8 +53,11 @@ void runOneJob(rq_problem &p, const rq::DevJob &job) {
 }
 
 // Shared-memory arena of a cluster's CTA, in doubles: the vectors of the levels that it runs
-// whole, their tables and operator values, and the coarsest inverse (resPlace), as far as
-// they fit.
+// whole, and of their tables and operator values and the coarsest inverse (resPlace) what fits
+// in 112 KB; the rest of the SM's storage serves the assemblies and the upper levels as L1
+// (us per outer iteration with 70 / 110 / 150 / 208 KB: 100 x 50 cells 1039 / 1049 / 1045 / 1050,
+// 200 x 100 2437 / 2441 / 2451 / 2502, 400 x 200 7877 / 8002 / 8207 / 8670).
+constexpr long kClusterArenaKb = 112;
 long clusterArena(const rq::DevClass &C) {
     long need = pad32(C.locDoubles);
     auto table = [&](int width, int rows) {
@@ -70,7 +73,7 @@ long clusterArena(const rq::DevClass &C) {
     }
     const long m = C.lev[C.nlev - 1].n;
     need += pad32(2 * m * m);
-    return std::min(need, (maxSmemOptin() - static_cast<long>(rq::clusterSharedBytes())) / 256 * 32);
+    return std::max<long>(pad32(C.locDoubles), std::min<long>(need, kClusterArenaKb * 1024 / 8));
 }
 
 // CTAs per solve, by the class's size alone, so that a row's result does not depend on the
@@ -80,7 +83,8 @@ long clusterArena(const rq::DevClass &C) {
 // 38 / 28, but 32 draws of 200 x 100 51 / 85: 36 clusters of 4 fit the GPU at once, only 14
 // of 8. 400 x 200 cells: 14.5 / 8.8 ms per outer iteration.
 int clusterOf(const rq_problem &p, int block, int arenaKb) {
-    if (p.mesh.n <= 1536 || block != 768 || arenaKb >= 0 || p.cls.locDoubles > clusterArena(p.cls))
+    if (p.mesh.n <= 1536 || block != 768 || arenaKb >= 0 ||
+        8 * clusterArena(p.cls) > maxSmemOptin() - static_cast<long>(rq::clusterSharedBytes()))
         return 1;
     return p.mesh.n < 32768 ? 4 : 8;
 }
