@@ -19,13 +19,12 @@ int maxSmemOptin() {
     return v;
 }
 
-// Shared-memory arena of a launch, in doubles. Classes of up to 768 cells run two
-// CTAs per SM and place their whole hot set in half the SM's shared memory each.
-// Larger classes run one CTA per SM and take no arena: their hot set does not fit
-// (14 level-0 Krylov arrays plus the AMG coarse levels), and leaving the unified
-// L1/shared storage to the L1 cache measured faster (1536 cells: 537 us per outer
-// iteration without an arena against 656 us with the largest one).
-// The exchange vectors of the resident solvers come first, whatever the knob says.
+// Shared-memory arena of a launch, in doubles: at least what the resident solvers need (their
+// exchange vectors and V-cycle vectors come first, whatever the knob says). By default
+// classes of up to 768 cells take half the SM's shared memory; larger ones take no more, and
+// the unified L1/shared storage is left to the L1 cache (measured over the first 400 outer
+// iterations, us each, with the default / 205 KB: 384 cells 125 / 130, 768 cells 217 / 228, 1536
+// cells 347 / 359; general solvers at 1536 cells: 537 without an arena, 656 with the largest).
 int arenaDoublesFor(long wsDoubles, int knobKb, int nmax, long resident) {
     const long shared = static_cast<long>(rq::solveSharedBytes());
     const long optin = maxSmemOptin();

@@ -153,7 +153,7 @@ struct DeviceScope {
             cudaSetDevice(prev);
     }
 };
-// one job on the problem's own workspace: a grid of one CTA of the class's size, the
+// one job on the problem's own workspace: one CTA or cluster of the class's launch shape, the
 // arena the batch path would give the class, queued on the legacy stream and finished
 // by the time the caller copies results back (the problem's mutex held by the caller)
 void runOneJob(rq_problem &p, const rq::DevJob &job);

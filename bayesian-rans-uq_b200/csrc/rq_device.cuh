@@ -1,6 +1,6 @@
 // Device-side data layout of the B200 forward model. One mesh class (mesh,
 // boundary conditions, viscosity, settings, probes, AMG pattern) lives in HBM
-// once; every coefficient draw is a job that one CTA runs from cold start to
+// once; every coefficient draw is a job that one CTA (or one thread-block cluster) runs from cold start to
 // its verdict without leaving the GPU (see rq_solver.cu).
 #pragma once
 #include <cstddef>

@@ -1,5 +1,5 @@
-// The B200 forward model: one CTA runs one SIMPLE + k-omega SST solve, every
-// outer iteration of it, from cold start to its verdict, with all state in
+// The B200 forward model: one CTA (a thread-block cluster for large meshes) runs one
+// SIMPLE + k-omega SST solve, every outer iteration of it, from cold start to its verdict, with all state in
 // HBM/L2 and the CTA's shared memory. Persistent CTAs pull draws from a job
 // queue (atomic counter), so a batch of mixed mesh classes keeps every SM busy
 // until the longest solve ends; a serving loop launches the same kernel per
@@ -7,21 +7,21 @@
 //
 // The loop restates SIMPLESolver::solve (rans-uq/src/SIMPLESolver.cpp:1193-1716)
 // on the structured periodic layout of rq_setup.h. Every face sum is gathered
-// per cell in the reference's face order; dot products are block reductions
-// (warp shuffles, then a fixed-order sum of the warp partials that every
+// per cell; dot products are block reductions (FP64 matrix products add a warp's
+// lanes, then a fixed-order sum of the warp partials that every
 // thread evaluates identically, so control flow stays uniform in the CTA).
 //
 // Inner solvers (core/include/LinearSolver.hpp): right-Jacobi BiCGSTAB
 // (:251-345) for momentum, k and omega; for the pressure correction PCG
 // (:184-246) with Jacobi or with the AMG V-cycle of this project (fixed
 // aggregation from rq_setup.cpp, damped-Jacobi smoothing, Galerkin values
-// refreshed per solve, dense coarsest inverse), or BiCGSTAB.
+// refreshed when it degrades, dense coarsest inverse), or BiCGSTAB. Classes of up to
+// 1536 cells run them in registers (rq_resident.cuh).
 #include "rq_device.cuh"
 #include "rq_kernels.h"
 
 #include <cuda_runtime.h>
 #include <math.h>
-
 
 #include <type_traits>
 
@@ -2843,7 +2843,7 @@ __global__ void __launch_bounds__(NT, ctasPerSM(NT)) serveKernel(ServeQueue q, d
 }
 
 // ---------------------------------------------------------------- allocation-free single solve
-// One job passed by value (no job array, no queue counter), solved by one CTA in
+// One job passed by value (no job array, no queue counter), solved by one CTA or cluster in
 // the scratch array.
 template <int NT, bool Cluster>
 __global__ void __launch_bounds__(NT, ctasPerSM(NT)) solveOneKernel(DevJob job, double *ws, int arenaDoubles) {

@@ -5,7 +5,7 @@
 // (rans-uq/src/ForwardModel.cpp:35-137) looks the nearest one up after the
 // bounds check, solves from it instead of the uniform state, and stores the
 // state of a Converged solve. Here every cached state stays in device memory in
-// the fields layout (11 x n), and the solve reads it directly: one job, one CTA,
+// the fields layout (11 x n), and the solve reads it directly: one job, one CTA or cluster,
 // whose final state lands in a staging buffer that becomes the new entry by a
 // pointer move (no copy, no host round trip). The cache's byte count is the
 // reference's own payload count, so entries are evicted after the same calls.

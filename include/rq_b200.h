@@ -234,7 +234,7 @@ int rq_mesh_save_binary(const rq_mesh_desc *mesh, const char *path);
    aggregation of the matrix, damped-Jacobi V-cycle, dense coarsest inverse. */
 int rq_linear_solve(const rq_ldu *A, double *x, int32_t max_iter, double tol, int32_t kind,
                     rq_solver_result *result);
-/* Many systems in one persistent launch (one CTA per system, largest first).
+/* Many systems in persistent launches (one thread-block cluster per system, largest first).
    x[s]: per-system initial guess in, solution out (host). precision RQ_PREC_MIXED:
    FP32 PCG corrections inside an FP64 residual-refinement loop (AMG and PCG kinds;
    BiCGSTAB stays FP64); result iterations count the inner FP32 iterations. */
