@@ -20,19 +20,21 @@ int maxSmemOptin() {
 }
 
 // Shared-memory arena of a launch, in doubles: at least what the resident solvers need (their
-// exchange vectors and V-cycle vectors come first, whatever the knob says). By default
-// classes of up to 768 cells take half the SM's shared memory; larger ones take no more, and
-// the unified L1/shared storage is left to the L1 cache (measured over the first 400 outer
-// iterations, us each, with the default / 205 KB: 384 cells 125 / 130, 768 cells 217 / 228, 1536
-// cells 347 / 359; general solvers at 1536 cells: 537 without an arena, 656 with the largest).
+// exchange vectors and V-cycle vectors come first, whatever the knob says). By default classes
+// of up to 768 cells and those with resident solvers take 130 KB with the fixed part, just
+// inside the carveout of 132 KB that half the SM would set too; the rest of the SM's storage is
+// L1. Measured on a B200, us per outer iteration over the first 400: 384 cells 84.8 / 82.2 with
+// 114 / 130 KB, 768 cells 154.8 / 152.4, 24 x 16 bump 168.6 / 153.5; with 224 KB 4 % slower than
+// with 114 at all three channel sizes. Larger classes without resident solvers take none (1536
+// cells: 537 without an arena, 656 with the largest).
 int arenaDoublesFor(long wsDoubles, int knobKb, int nmax, long resident) {
     const long shared = static_cast<long>(rq::solveSharedBytes());
     const long optin = maxSmemOptin();
     long bytes;
     if (knobKb >= 0)
         bytes = std::min<long>(knobKb * 1024L, optin - shared);
-    else if (nmax <= 768)
-        bytes = (optin / 2 - 1024) - shared; // half the SM (the whole hot set fits)
+    else if (nmax <= 768 || resident > 0)
+        bytes = 130 * 1024 - shared;
     else
         bytes = 0;
     bytes = std::max<long>(0, std::min(bytes, wsDoubles * 8));
@@ -93,7 +95,8 @@ rq::LaunchShape shapeOf(const rq_problem &p, int block, int arenaKb) {
     if (cluster > 1)
         return {block, static_cast<int>(clusterArena(p.cls)), cluster};
     return {block,
-            arenaDoublesFor(p.cls.wsDoubles, arenaKb, p.mesh.n, rq::residentDoubles(p.cls)), 1};
+            arenaDoublesFor(p.cls.wsDoubles, arenaKb, p.mesh.n,
+                            rq::residentDoubles(p.cls, block)), 1};
 }
 
 int chooseArena(const std::vector<const rq_problem *> &probs) {
@@ -102,7 +105,7 @@ int chooseArena(const std::vector<const rq_problem *> &probs) {
     int nmax = 0;
     long resident = 0;
     for (const auto *p : probs) {
-        resident = std::max(resident, rq::residentDoubles(p->cls));
+        resident = std::max(resident, rq::residentDoubles(p->cls, 512)); // the serving CTAs' size
         ws = std::max(ws, static_cast<long>(p->cls.wsDoubles));
         knob = std::max(knob, p->arenaKb);
         nmax = std::max(nmax, p->mesh.n);

@@ -8,9 +8,9 @@ namespace rq {
 
 size_t solveSharedBytes();   // fixed shared memory of a CTA
 size_t clusterSharedBytes(); // the same of the cluster kernels
-// Doubles at the start of the arena that the resident inner solvers of a class need (0:
-// the class is too large for them, rq_resident.cuh).
-long residentDoubles(const DevClass &C);
+// Doubles at the start of the arena that the resident inner solvers of a class need in CTAs
+// of `block` threads (0: they do not apply, rq_resident.cuh).
+long residentDoubles(const DevClass &C, int block);
 // Launch shape of a solve: CTA size (64, 128, 256, 512, 768 or 1024), shared-memory arena
 // per CTA in doubles for the hot arrays (0 = all global), and CTAs per solve (above 1: a
 // thread-block cluster of 768-thread CTAs whose arena holds the small AMG levels).

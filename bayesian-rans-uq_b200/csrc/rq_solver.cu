@@ -2895,8 +2895,8 @@ size_t solveSharedBytes() { return kSharedBytes; }
 size_t clusterSharedBytes() {
     return reinterpret_cast<size_t>(solveEntry<kClusterThreads, true>(kEntryBytes));
 }
-long residentDoubles(const DevClass &C) {
-    if (C.n > kResCells * kResMaxThreads)
+long residentDoubles(const DevClass &C, int block) {
+    if (C.st.precision != kFP64 || block > kResMaxThreads || C.n > kResCells * block)
         return 0;
     return resExchange(C.n) + (C.resAmg ? (C.amgVecs + 31) / 32 * 32 : 0);
 }
