@@ -7,6 +7,7 @@ runs the CUDA library, which raises if it is missing.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -129,20 +130,24 @@ class LinearBatch:
         N.call("rq_linsys_create", _ldu_array(self.systems), C.c_int32(len(self.systems)),
                C.c_int32(_kind(kind)), C.c_int32(N.PRECISIONS[precision]), C.byref(h))
         self.handle = h
+        self._solving = threading.Lock()
 
     def solve(self, max_iter: int = 500, tol: float = 1e-6, xs=None):
         """From xs (or zero); returns (results, solutions)."""
         out = (N.SolverResult * len(self.systems))()
         if xs is None:
-            # the solutions' pages are touched while the device solves
-            N.call("rq_linsys_solve_device", self.handle, C.c_int32(max_iter), C.c_double(tol),
-                   C.c_void_p(0))
-            sol = [np.full(s.n_cells, 0.0) for s in self.systems]
-            N.call("rq_linsys_results", self.handle, out, _x_pointers(sol))
+            # the solutions' pages are touched while the device solves; one solve at a time,
+            # so that the results read back are this call's
+            with self._solving:
+                N.call("rq_linsys_solve_device", self.handle, C.c_int32(max_iter),
+                       C.c_double(tol), C.c_void_p(0))
+                sol = [np.full(s.n_cells, 0.0) for s in self.systems]
+                N.call("rq_linsys_results", self.handle, out, _x_pointers(sol))
         else:
             sol = xs
-            N.call("rq_linsys_solve", self.handle, C.c_int32(max_iter), C.c_double(tol),
-                   _x_pointers(sol), out)
+            with self._solving:
+                N.call("rq_linsys_solve", self.handle, C.c_int32(max_iter), C.c_double(tol),
+                       _x_pointers(sol), out)
         return [_result(r) for r in out], sol
 
     def solve_device(self, max_iter: int, tol: float, stream: int = 0) -> None:
