@@ -33,16 +33,16 @@ UNIT = "solves/s"
 # (CPU pilot of the compiled reference); used only by the CPU arm's extrapolation
 REF_ITERS = (12460, 58690, 258900)
 BYTES_OUTER, BYTES_KRYLOV, BYTES_PRESSURE = 1600, 360, 400  # algorithmic B/cell (FP64)
-# From one ncu capture of solveKernel<768> solving one 1536-cell draw for 600 outer
-# iterations (profiles/solveKernel768_1536cells_full_ncu.md):
+# From one ncu capture of solveKernel<512> solving one 1536-cell draw for 600 outer
+# iterations (profiles/solveKernel_resident_and_cluster_ncu.md):
 # * DRAM bytes (read + write): the first touch of the mesh class and the workspace;
 #   later iterations hit L2, so the figure does not grow with the iteration count;
 # * L2 bytes (lts__t_sectors x 32 B) per outer iteration: what the solve moves
 #   between its SM and L2 (L1 misses, spills, stores);
 # * the L2's peak: 3 sectors per cycle on each of the 184 slices (ncu's
 #   lts__t_sectors peak_sustained) x 32 B at the 1965 MHz clock.
-DRAM_BYTES_PER_DRAW_1536 = 2_609_408 + 2_304
-L2_BYTES_PER_ITER_1536 = 280_240_249 * 32 / 600
+DRAM_BYTES_PER_DRAW_1536 = 2_587_904 + 256
+L2_BYTES_PER_ITER_1536 = 166_757_762 * 32 / 600
 L2_PEAK_GBS = 3 * 32 * 184 * 1.965
 
 
