@@ -452,17 +452,21 @@ __device__ __forceinline__ void downRes(const Shared &S, int l, const double *fr
         R.r[i] = R.b[i] - rowRes(R.ac, R.av, x, R.aw, i);
     levelSync(S, l);
 }
-// and on the way up: the correction xc of the level below, post-smoothing; the solution in x
+// and on the way up: the correction xc of the level below, post-smoothing; the solution in x.
+// The corrected iterate replaces the pre-smoothed one, each thread its own rows. It must not go
+// to r: on a cluster the level below restricts this level's r in every CTA, with no cluster
+// barrier since, and a CTA that is late would read iterates for residuals.
 template <bool SH>
 __device__ __forceinline__ void upRes(const Shared &S, int l, const double *xc) {
     const ResLevel R = levelOf<SH>(S, l);
     const bool two = S.C.amgSweeps >= 2;
-    const double al = S.C.amgAlpha, *x = two ? R.x : R.xa;
+    const double al = S.C.amgAlpha;
+    double *x = two ? R.x : R.xa;
     const int ts = levelThreads(S, l);
     for (int i = levelTid(S, l); i < R.n; i += ts)
-        R.r[i] = x[i] + al * rowRes(R.pc, R.pv, xc, R.pw, i);
+        x[i] += al * rowRes(R.pc, R.pv, xc, R.pw, i);
     levelSync(S, l);
-    smoothRes<SH>(S, l, R, R.r, two ? R.xa : R.x);
+    smoothRes<SH>(S, l, R, x, two ? R.xa : R.x);
     if (two)
         smoothRes<SH>(S, l, R, R.xa, R.x);
 }

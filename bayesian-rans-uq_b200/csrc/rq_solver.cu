@@ -1031,26 +1031,26 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
     // one level of the up sweep (levels >= 1; level 0 ends in the reduction below):
     // x = x_pre + alpha P x_c, then the post sweeps; the result ends in xb. With a
     // piecewise-constant P (one coarse row per fine row) x is formed inside the first
-    // sweep; with a smoothed P it is formed in a phase of its own (into the level's
-    // residual slot, free by then), so that the sweep over a wide coarse row loads
+    // sweep; with a smoothed P it is formed in a phase of its own, in place of x_pre (not
+    // in the residual's slot: see upRes), so that the sweep over a wide coarse row loads
     // each neighbour's x once instead of re-forming it from P.
     auto up = [&](int l) {
         const DevAmgLevel &Lv = C.lev[l];
         const int n = Lv.n, t0 = levelTid(S, l), ts = levelThreads(S, l);
-        T *b = vb(l), *xa = b + n, *xb = b + 2 * n, *xi = b + 3 * n;
+        T *b = vb(l), *xa = b + n, *xb = b + 2 * n;
         const T *rd = b + 4 * n;
-        const T *xpre = two ? xb : xa;
+        T *xpre = two ? xb : xa;
         T *out = two ? xa : xb;
         const T *val = amgVal + Lv.valOff;
         if (Lv.pw > 1) {
             for (int i = t0; i < n; i += ts)
-                xi[i] = xpre[i] + al * prolong(l, i);
+                xpre[i] += al * prolong(l, i);
             sync(l);
             segPass<T>(n, t0, ts,
                        [&](int i, int j, int seg) {
-                           return ellDot<T>(Lv.ecol, val, xi, Lv.width, i, j, seg);
+                           return ellDot<T>(Lv.ecol, val, xpre, Lv.width, i, j, seg);
                        },
-                       [&](int i, T ax) { out[i] = xi[i] + om * (b[i] - ax) * rd[i]; });
+                       [&](int i, T ax) { out[i] = xpre[i] + om * (b[i] - ax) * rd[i]; });
         } else {
             for (int i = t0; i < n; i += ts) {
                 const T x0 = xpre[i] + al * prolong(l, i);
@@ -1090,27 +1090,27 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
     }
     double rz = 0.0;
     if (L > 1 && (lean || C.lev[0].pw > 1)) { // level 0, smoothed P: x = x_pre + alpha P x_c in a
-        // sweep of its own (into rr, free since the restriction to level 1), then the
+        // sweep of its own (in place of x_pre: see upRes), then the
         // post sweep(s) read it (each x once, not re-formed at every neighbour)
         const int n = C.lev[0].n;
-        const T *xprev = two ? Kxb : Kxa;
+        T *x = two ? Kxb : Kxa;
         T *out = two ? Kxa : Kz;
         if (lean) {
             if constexpr (std::is_same_v<T, double>) {
                 const ResLevel &R = S.RL[0];
                 const double *xc = S.RL[1].x;
                 FOR_OWN(i, n)
-                    Krr[i] = xprev[i] + al * rowRes(R.pc, R.pv, xc, R.pw, i);
+                    x[i] += al * rowRes(R.pc, R.pv, xc, R.pw, i);
             }
         } else {
             FOR_OWN(i, n)
-                Krr[i] = xprev[i] + al * prolong(0, i);
+                x[i] += al * prolong(0, i);
         }
         SYNC();
         double part = 0.0;
         FOR_OWN(i, n) {
-            const T ax = rowDotT(cellOf(C, i), M, Krr, nx);
-            const T zi = Krr[i] + om * (Kr[i] - ax) * Krd[i];
+            const T ax = rowDotT(cellOf(C, i), M, x, nx);
+            const T zi = x[i] + om * (Kr[i] - ax) * Krd[i];
             out[i] = zi;
             if (!two)
                 part += double(Kr[i]) * double(zi);
