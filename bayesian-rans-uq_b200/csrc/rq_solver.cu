@@ -2778,6 +2778,10 @@ __global__ void __launch_bounds__(NT, ctasPerSM(NT)) solveKernel(const DevJob *j
         if (j >= njobs)
             break;
         runJob(S, jobs[j], ws, arena, arenaDoubles);
+        // an inadmissible draw passes no cluster barrier in runJob: without this one rank 0
+        // could store the next job into a CTA whose warps have not read the last one
+        if constexpr (kCluster)
+            SYNC();
     }
 }
 

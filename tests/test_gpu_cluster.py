@@ -29,6 +29,24 @@ def test_equal_draws_and_launches_give_equal_rows(rq, nx, ny, precision):
         np.testing.assert_array_equal(p, first.predictions[0])
 
 
+def test_inadmissible_draws_between_admissible_ones(rq):
+    """An out-of-bounds draw passes no cluster barrier of its solve; the clusters' job queue
+    stays in step over single ones, runs of them, and a batch of nothing else."""
+    case = cases.bump_case(60, 36, max_iter=ITERS)
+    batch = cases.product_batch(rq, case)
+    good, bad = [0.31, 0.09], [0.95, 0.09]
+    alone = batch.evaluate([good])
+    for pattern in ("b", "bbb", "gb", "bg", "bbgbbbbg" * 30, "b" * 200, "g" + "b" * 150 + "g"):
+        rows = batch.evaluate([good if ch == "g" else bad for ch in pattern]).rows
+        for ch, row in zip(pattern, rows):
+            if ch == "g":
+                assert row.result.status == alone.rows[0].result.status
+                np.testing.assert_array_equal(row.result.predictions, alone.predictions[0])
+            else:
+                assert row.result.status == rq.EvaluationStatus.InvalidParameters
+                assert row.result.log_lik == -1e30
+
+
 def test_eight_ctas(rq, checker):
     check_fields(rq, checker, cases.bump_case(260, 128, max_iter=3))
 
