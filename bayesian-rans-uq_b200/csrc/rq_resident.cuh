@@ -9,8 +9,10 @@
 // so neither memory nor the FP64 pipe is near its limit. Cycles per iteration in isolation
 // on a B200, by cells per thread: 384 cells 3147 / 2568 / 2677 / 3033 (1 / 2 / 3 / 4),
 // 1536 cells - / - / 4916 / 5450: few warps make the block sums cheap, and four cells (11
-// doubles of state each) spill out of 128 registers. With the sums on the tensor cores and
-// the branch-free quotients below: 1766 at 384 cells, 2550 at 768, 4234 at 1536.
+// doubles of state each) spill out of 128 registers. With the sums on the tensor cores: 1925
+// at 384 cells, 2869 at 768, 4592 at 1536. (Branch-free quotients from the approximate
+// reciprocal took another 160 to 360 cycles off and were taken back: they gave NaN or zero for
+// infinite, subnormal and extreme divisors. 1.4 to 6 % of a solve.)
 #pragma once
 
 // Threads of the working group, and the zero slot of an exchange vector: entries
@@ -155,12 +157,12 @@ __device__ __noinline__ void bicgstabRes(double *x, double r0n, int maxIter, dou
     int rp = 0;
     sumRes<1>(acc, rp, nw);
     const double bound2 = (tol * r0n) * (tol * r0n);
-    double rhoN = acc[0], rhoInv = 1, alphaOm = 1, omega = 1;
+    double rhoN = acc[0], rho = 1, alphaOm = 1, omega = 1;
     double last = r0n * r0n;
     for (int it = 0; it < maxIter; ++it) {
         if (fabs(rhoN) < 1e-30)
             break;
-        const double beta = (rhoN * rhoInv) * alphaOm;
+        const double beta = (rhoN / (rho + 1e-30)) * alphaOm;
 #pragma unroll
         for (int k = 0; k < kResCells; ++k) {
             p[k] = r[k] + beta * (p[k] - omega * v[k]);
@@ -173,11 +175,10 @@ __device__ __noinline__ void bicgstabRes(double *x, double r0n, int maxIter, dou
             v[k] = A.times(k, p[k] * A.rd[k], e0);
             s1[0] += rh[k] * v[k];
         }
-        rhoInv = recip(rhoN + 1e-30);
         sumRes<1>(s1, rp, nw);
         if (fabs(s1[0]) < 1e-30)
             break;
-        const double alpha = quot(rhoN, s1[0]);
+        const double alpha = rhoN / s1[0];
         double s3[3] = {0.0, 0.0, 0.0};
 #pragma unroll
         for (int k = 0; k < kResCells; ++k) { // r holds s until the iteration's end
@@ -203,7 +204,7 @@ __device__ __noinline__ void bicgstabRes(double *x, double r0n, int maxIter, dou
             res.converged = true;
             break;
         }
-        omega = (s3[0] > 1e-30) ? quot(s3[1], s3[0]) : 0.0;
+        omega = (s3[0] > 1e-30) ? s3[1] / s3[0] : 0.0;
         double s4[2] = {0.0, 0.0};
 #pragma unroll
         for (int k = 0; k < kResCells; ++k) {
@@ -212,7 +213,7 @@ __device__ __noinline__ void bicgstabRes(double *x, double r0n, int maxIter, dou
             s4[0] += r[k] * r[k];
             s4[1] += rh[k] * r[k];
         }
-        alphaOm = quot(alpha, omega + 1e-30);
+        alphaOm = alpha / (omega + 1e-30);
         sumRes<2>(s4, rp, nw);
         last = s4[0];
         if (dropped(s4[0], bound2, r0n, tol)) {
@@ -221,6 +222,7 @@ __device__ __noinline__ void bicgstabRes(double *x, double r0n, int maxIter, dou
         }
         if (fabs(omega) < 1e-30)
             break;
+        rho = rhoN;
         rhoN = s4[1];
     }
 #pragma unroll
@@ -662,7 +664,7 @@ __device__ __noinline__ void pcgRes(double *x, double r0n, int maxIter, double t
                 res.breakdown = true;
                 done = true;
             } else {
-                const double alpha = quot(rz, q[0]);
+                const double alpha = rz / q[0];
                 q[0] = 0.0;
 #pragma unroll
                 for (int k = 0; k < kResCells; ++k) {

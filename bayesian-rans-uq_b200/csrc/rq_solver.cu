@@ -190,24 +190,6 @@ __device__ __forceinline__ void groupSync(int threads) {
     asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
 
-// ---------------------------------------------------------------- arithmetic
-// a / b by Newton-Raphson iteration from the hardware's approximate reciprocal, and one
-// correction of the quotient: within one unit in the last place for operands and quotients
-// of normal size (the solvers' guards keep |b| above 1e-30). Unlike the division operator
-// it has no branch, so its latency overlaps the block sum beside it (85 cycles each, four
-// per BiCGSTAB iteration).
-__device__ __forceinline__ double recip(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    y = fma(y, fma(-b, y, 1.0), y);
-    y = fma(y, fma(-b, y, 1.0), y);
-    return y;
-}
-__device__ __forceinline__ double quot(double a, double b) {
-    const double y = recip(b), q = a * y;
-    return fma(fma(-b, q, a), y, q);
-}
-
 // ---------------------------------------------------------------- reductions
 // D = A B of one FP64 m8n8k4 product: a is this lane's A[lane / 4][lane % 4], b its
 // B[lane % 4][lane / 4]; d0, d1 receive D[lane / 4][2 (lane % 4) + 0, 1].
@@ -418,8 +400,8 @@ __device__ __forceinline__ double limitedCorr(double F, double dphi, double gx, 
                                               double dy) {
     if (!(fabs(dphi) > 1e-300) || F == 0.0)
         return 0.0;
-    const double r = quot(2.0 * (gx * dx + gy * dy), dphi) - 1.0;
-    const double psi = r > 0.0 ? quot(r * r + r, r * r + 1.0) : 0.0;
+    const double r = 2.0 * (gx * dx + gy * dy) / dphi - 1.0;
+    const double psi = r > 0.0 ? (r * r + r) / (r * r + 1.0) : 0.0;
     return 0.5 * psi * (fabs(F) * dphi);
 }
 
@@ -1888,13 +1870,13 @@ __device__ __noinline__ void phClosure(Shared &S, double floorV) {
                 W.S[c] = Sc;
                 const double kc = dmax(W.k[c], 0.0), wc = dmax(W.w[c], 1e-20);
                 const double y = dmax(C.wd[c], 1e-20);
-                const double cd = quot(2.0 * sw2, wc) * (W.gKx[c] * W.gWx[c] + W.gKy[c] * W.gWy[c]);
+                const double cd = 2.0 * sw2 / wc * (W.gKx[c] * W.gWx[c] + W.gKy[c] * W.gWy[c]);
                 W.CD[c] = cd;
                 const double sqk = sqrt(dmax(kc, 0.0)), ws = dmax(wc, 1e-20);
                 const double ys = dmax(y, 1e-20), y2 = ys * ys;
-                const double t1 = quot(sqk, bs * ws * ys);
-                const double t2 = quot(500.0 * nu, y2 * ws);
-                const double t3 = quot(4.0 * sw2 * kc, dmax(cd, 1e-10) * y2);
+                const double t1 = sqk / (bs * ws * ys);
+                const double t2 = 500.0 * nu / (y2 * ws);
+                const double t3 = 4.0 * sw2 * kc / (dmax(cd, 1e-10) * y2);
                 const double arg1 = dmin(dmax(t1, t2), t3);
                 const double F1 = tanh(arg1 * arg1 * arg1 * arg1);
                 W.F1[c] = F1;
@@ -1904,7 +1886,7 @@ __device__ __noinline__ void phClosure(Shared &S, double floorV) {
                 W.F2[c] = F2;
                 double den = dmax(a1 * wc, Sc * F2);
                 den = dmax(den, 1e-20);
-                const double nut = quot(a1 * kc, den);
+                const double nut = a1 * kc / den;
                 const double raw = nut * Sc * Sc;
                 const double lim = 10.0 * bs * dmax(kc, 0.0) * dmax(wc, 1e-20);
                 W.Pk[c] = dmin(raw, lim);
@@ -2001,7 +1983,7 @@ __device__ __noinline__ void phMomentum(Shared &S, int comp, double (&acc)[3]) {
         bsum += C.relax[0] * dsum * Uc; // (1 - alpha) / alpha
         const double dd = dsum * C.relax[1];
         if (comp == 0) {
-            W.aP[c] = fabs(dd) > 1e-30 ? quot(V, dd) : 0.0;
+            W.aP[c] = fabs(dd) > 1e-30 ? V / dd : 0.0;
             const double uy = W.Uy[c];
             acc[2] += dsum * sqrt(Uc * Uc + uy * uy);
         }
@@ -2238,14 +2220,14 @@ __device__ __noinline__ void phTurbAssemble(Shared &S, int eq, double (&acc)[1])
             dsum += bs * wc * V;
         } else {
             const double Sv = W.S[c];
-            const double lim = quot(10.0 * bs * dmax(W.k[c], 0.0) * wc, dmax(nuT, 1e-30));
+            const double lim = 10.0 * bs * dmax(W.k[c], 0.0) * wc / dmax(nuT, 1e-30);
             bsum += blend(al1, al2, F1) * dmin(Sv * Sv, lim) * V;
             dsum += blend(b1, b2, F1) * wc * V;
             bsum += (1.0 - F1) * W.CD[c] * V;
             if (balance) {
                 const double corr = bl + nu * (6 * nu * iB1) * __ldg(C.slap + c) * V;
                 if (corr < 0)
-                    dsum -= quot(corr, wc);
+                    dsum -= corr / wc;
                 else
                     bsum += corr;
             }
