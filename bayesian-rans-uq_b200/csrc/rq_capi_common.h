@@ -7,6 +7,7 @@
 #include "rq_kernels.h"
 #include "rq_lin.cuh"
 #include "rq_linsys.h"
+#include "rq_prefault.h"
 #include "rq_setup.h"
 
 #include <cuda_runtime.h>
@@ -83,16 +84,6 @@ struct DevBuf {
     }
     template <class T> T *as() const { return static_cast<T *>(p); }
 };
-
-// Touches the pages of an output buffer that a copy from the device will fill. Called while
-// the device works: a fresh 56 MB field buffer otherwise costs its page faults (about 7 ms)
-// inside the copy, after the solve.
-inline void prefault(void *p, size_t bytes) {
-    constexpr size_t page = 4096;
-    char *c = static_cast<char *>(p);
-    for (size_t i = 0; i < bytes; i += page)
-        const_cast<volatile char *>(c)[i] = 0;
-}
 
 // The reference's parameter bounds (core/include/InferenceParameters.hpp:147-165).
 inline const double kLower[11] = {0.1, 0.1, 0.01, 0.1, 0.1, 0.1, 0.01, 0.1, 0.01, 0.1, 0.35};
