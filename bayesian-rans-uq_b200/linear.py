@@ -152,8 +152,9 @@ class LinearBatch:
 
     def solve_device(self, max_iter: int, tol: float, stream: int = 0) -> None:
         """Queue a zero-start solve of every system on `stream`; does not wait."""
-        N.call("rq_linsys_solve_device", self.handle, C.c_int32(max_iter), C.c_double(tol),
-               C.c_void_p(stream))
+        with self._solving:  # not between a solve and its results
+            N.call("rq_linsys_solve_device", self.handle, C.c_int32(max_iter), C.c_double(tol),
+                   C.c_void_p(stream))
 
     def results(self, with_x: bool = False):
         out = (N.SolverResult * len(self.systems))()
