@@ -26,20 +26,35 @@ int maxSmemOptin() {
 // L1. Measured on a B200, us per outer iteration over the first 400: 384 cells 84.8 / 82.2 with
 // 114 / 130 KB, 768 cells 154.8 / 152.4, 24 x 16 bump 168.6 / 153.5; with 224 KB 4 % slower than
 // with 114 at all three channel sizes. Larger classes without resident solvers take none (1536
-// cells: 537 without an arena, 656 with the largest).
-int arenaDoublesFor(long wsDoubles, int knobKb, int nmax, long resident) {
+// cells: 537 without an arena, 656 with the largest). CTAs of fewer than 512 threads, of which
+// the registers hold two, take half the SM where there are more solves than SMs, so that two run
+// on each (384 cells, 60 iterations, with 64 / 128 / 256 threads: 148 draws 22.5 / 10.2 / 7.6 ms
+// with 130 KB, 26.6 / 12.5 / 9.2 with half; 296 draws 44.8 / 20.4 / 15.1 against 31.0 / 15.6 / 11.6).
+// The results do not depend on the arena.
+int arenaDoublesFor(long wsDoubles, int knobKb, int nmax, long resident, bool pairs) {
     const long shared = static_cast<long>(rq::solveSharedBytes());
     const long optin = maxSmemOptin();
     long bytes;
     if (knobKb >= 0)
         bytes = std::min<long>(knobKb * 1024L, optin - shared);
-    else if (nmax <= 768 || resident > 0)
-        bytes = 130 * 1024 - shared;
-    else
+    else if (nmax > 768 && resident == 0)
         bytes = 0;
+    else
+        bytes = (pairs ? optin / 2 - 1024 : 130 * 1024) - shared;
     bytes = std::max<long>(0, std::min(bytes, wsDoubles * 8));
     bytes = std::min(std::max(bytes, resident * 8), optin - shared);
     return static_cast<int>(bytes / 8 / 32 * 32);
+}
+
+int smCount() {
+    static thread_local int forDev = -1, v = 1;
+    int dev = 0;
+    check(cudaGetDevice(&dev), "cudaGetDevice");
+    if (dev != forDev) {
+        check(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev), "attribute");
+        forDev = dev;
+    }
+    return v;
 }
 
 void runOneJob(rq_problem &p, const rq::DevJob &job) {
@@ -49,7 +64,7 @@ void runOneJob(rq_problem &p, const rq::DevJob &job) {
     check(cudaMemcpy(p.dJobs.p, &job, sizeof(rq::DevJob), cudaMemcpyHostToDevice), "job");
     check(cudaMemset(p.dCounter.p, 0, sizeof(int)), "counter");
     check(rq::launchSolve(p.dJobs.as<rq::DevJob>(), 1, p.dCounter.as<int>(), p.dWs.as<double>(),
-                          p.cls.wsDoubles, 1, shapeOf(p, p.block, p.arenaKb), nullptr),
+                          p.cls.wsDoubles, 1, shapeOf(p, p.block, p.arenaKb, 1), nullptr),
           "solve launch");
 }
 
@@ -90,13 +105,14 @@ int clusterOf(const rq_problem &p, int block, int arenaKb) {
     return p.mesh.n < 32768 ? 4 : 8;
 }
 
-rq::LaunchShape shapeOf(const rq_problem &p, int block, int arenaKb) {
+rq::LaunchShape shapeOf(const rq_problem &p, int block, int arenaKb, long solves) {
     const int cluster = clusterOf(p, block, arenaKb);
     if (cluster > 1)
         return {block, static_cast<int>(clusterArena(p.cls)), cluster};
     return {block,
             arenaDoublesFor(p.cls.wsDoubles, arenaKb, p.mesh.n,
-                            rq::residentDoubles(p.cls, block)), 1};
+                            rq::residentDoubles(p.cls, block),
+                            block < 512 && solves > smCount()), 1};
 }
 
 int chooseArena(const std::vector<const rq_problem *> &probs) {
@@ -110,7 +126,7 @@ int chooseArena(const std::vector<const rq_problem *> &probs) {
         knob = std::max(knob, p->arenaKb);
         nmax = std::max(nmax, p->mesh.n);
     }
-    return arenaDoublesFor(ws, knob, nmax, resident);
+    return arenaDoublesFor(ws, knob, nmax, resident, false);
 }
 
 } // namespace rqc
@@ -511,11 +527,8 @@ void launchClass(rq_problem &P, const std::vector<int> &rows, const double *thet
         j.clock = clockDev ? clockDev + 12L * r : nullptr;
     }
     const long wsStride = P.cls.wsDoubles;
-    const rq::LaunchShape shape = shapeOf(P, P.block, P.arenaKb);
-    int dev = 0, sms = 1;
-    check(cudaGetDevice(&dev), "cudaGetDevice");
-    check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attribute");
-    const int atOnce = rq::concurrentSolves(shape, sms);
+    const rq::LaunchShape shape = shapeOf(P, P.block, P.arenaKb, n);
+    const int atOnce = rq::concurrentSolves(shape, smCount());
     if (atOnce < 1)
         throw RqError(RQ_E_CUDA, "solve kernel does not fit on an SM with this arena");
     const int grid = std::max(1, std::min(n, atOnce));
@@ -723,7 +736,7 @@ int rq_problem_set_launch(rq_problem *p, const rq_launch_shape *shape) {
         if (shape->arena_kb < -1)
             throw std::invalid_argument("arena_kb must be -1 (default rule), 0 or positive");
         std::lock_guard<std::mutex> lock(p->mu);
-        if (rq::concurrentSolves(shapeOf(*p, shape->block_threads, shape->arena_kb), 1) < 1)
+        if (rq::concurrentSolves(shapeOf(*p, shape->block_threads, shape->arena_kb, 1), 1) < 1)
             throw std::invalid_argument("this launch shape does not fit on an SM");
         p->block = shape->block_threads;
         p->arenaKb = shape->arena_kb;
@@ -793,7 +806,7 @@ int rq_problem_tune(rq_problem *p, const double *theta, int32_t iters,
             c.us_per_iteration = -1.0;
             if (!rq::launchVariantExists(c.block_threads) || c.arena_kb < -1)
                 continue;
-            const rq::LaunchShape shape = shapeOf(*p, c.block_threads, c.arena_kb);
+            const rq::LaunchShape shape = shapeOf(*p, c.block_threads, c.arena_kb, 1);
             if (rq::concurrentSolves(shape, 1) < 1)
                 continue;
             check(cudaMemset(dCounter.p, 0, sizeof(int)), "counter");
@@ -1077,7 +1090,7 @@ int rq_evaluate_noalloc(rq_problem *p, const double *theta_dev, rq_row_out *row_
         job.row = reinterpret_cast<rq::RowOut *>(row_dev);
         job.pred = predictions_dev;
         // the batch path's launch shape of the class
-        check(rq::launchSolveNoAlloc(job, p->noallocScratch, shapeOf(*p, p->block, p->arenaKb),
+        check(rq::launchSolveNoAlloc(job, p->noallocScratch, shapeOf(*p, p->block, p->arenaKb, 1),
                                      static_cast<cudaStream_t>(stream)),
               "allocation-free solve launch");
     });

@@ -149,11 +149,12 @@ struct DeviceScope {
 // by the time the caller copies results back (the problem's mutex held by the caller)
 void runOneJob(rq_problem &p, const rq::DevJob &job);
 int maxSmemOptin();
-// shared-memory arena (doubles) of a launch of these classes
-int arenaDoublesFor(long wsDoubles, int knobKb, int nmax, long resident);
+// shared-memory arena (doubles) of a launch of these classes (pairs: two CTAs per SM)
+int arenaDoublesFor(long wsDoubles, int knobKb, int nmax, long resident, bool pairs);
 int chooseArena(const std::vector<const rq_problem *> &probs);
-// the launch shape of one class for a CTA size and arena knob
-rq::LaunchShape shapeOf(const rq_problem &p, int block, int arenaKb);
+int smCount();
+// the launch shape of one class for a CTA size, an arena knob and a number of solves
+rq::LaunchShape shapeOf(const rq_problem &p, int block, int arenaKb, long solves);
 inline rq_row_out toRow(const rq::RowOut &o) {
     return rq_row_out{o.status, o.iterations, o.stalled, o.converged, o.loglik, o.finalWorst,
                       o.contractionRate};
