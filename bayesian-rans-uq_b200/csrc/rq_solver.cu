@@ -8,7 +8,7 @@
 // The loop restates SIMPLESolver::solve (rans-uq/src/SIMPLESolver.cpp:1193-1716)
 // on the structured periodic layout of rq_setup.h. Every face sum is gathered
 // per cell; dot products are block reductions (FP64 matrix products add a warp's
-// lanes, then a fixed-order sum of the warp partials that every
+// lanes, then shuffles the warp partials, which every
 // thread evaluates identically, so control flow stays uniform in the CTA).
 //
 // Inner solvers (core/include/LinearSolver.hpp): right-Jacobi BiCGSTAB
@@ -144,7 +144,7 @@ struct Shared {
     KW<double> K64;
     KW<float> K32;
     double coeff[11];
-    alignas(16) double red[2][kRedSlots][32];
+    double red[2][kRedSlots][32];
     double cred[2][kRedSlots][kCluster ? kMaxCluster : 1]; // the cluster's CTA sums
     double ring[4][kWindowCap];  // U, k, omega, Q change samples
     int cnt[4];
@@ -201,9 +201,10 @@ __device__ __forceinline__ void mma884(double &d0, double &d1, double a, double 
 
 // Block reductions. A warp adds its lanes with two FP64 matrix products (sumRes); lane 0
 // parks the sum in shared memory, and after one barrier every warp adds the same partials
-// in the same order (eight per lane, then a product) -- so all threads of the CTA hold
-// bit-identical values and branch alike. Partials of warps that the CTA lacks are zero
-// (runJob). 480 cycles with shuffles at 16 warps, 631 at 24.
+// by the same shuffles -- so all threads of the CTA hold bit-identical values and branch
+// alike. (With matrix products for the partials too, which every warp repeats, the solves of
+// the general solvers took 8 to 14 % longer: mixed form, 384 / 768 / 1536 cells 166 / 286 / 448
+// us per outer iteration against 146 / 264 / 416; with shuffles for both 152 / 271 / 425.)
 template <int K>
 __device__ __forceinline__ void blockSum(double (&v)[K], Shared &S, int &rp) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -219,15 +220,13 @@ __device__ __forceinline__ void blockSum(double (&v)[K], Shared &S, int &rp) {
         for (int k = 0; k < K; ++k)
             S.red[rp][k][warp] = v[k];
     __syncthreads();
+    const int nw = blockDim.x >> 5;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        const double2 *r = reinterpret_cast<const double2 *>(&S.red[rp][k][8 * (lane & 3)]);
-        const double2 a = r[0], b = r[1], c = r[2], d = r[3];
-        v[k] = ((a.x + b.x) + (c.x + d.x)) + ((a.y + b.y) + (c.y + d.y));
+        v[k] = lane < nw ? S.red[rp][k][lane] : 0.0;
+        for (int o = 16; o > 0; o >>= 1)
+            v[k] += __shfl_xor_sync(FULL, v[k], o);
     }
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-        mma884(v[k], w[k], v[k], 1.0);
     if constexpr (kCluster) { // every CTA adds the CTA sums in the order of the ranks
         const int nc = ctaCount(), rank = ctaRank();
         if (static_cast<int>(threadIdx.x) < nc)
@@ -2674,8 +2673,6 @@ __device__ void runJob(Shared &S, const DevJob &job, double *ws, double *arena, 
         int *dst = reinterpret_cast<int *>(&S.C);
         for (int t = threadIdx.x; t < words; t += blockDim.x)
             dst[t] = src[t];
-        for (int t = threadIdx.x; t < 2 * kRedSlots * 32; t += blockDim.x)
-            (&S.red[0][0][0])[t] = 0.0;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
