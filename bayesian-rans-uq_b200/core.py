@@ -622,7 +622,7 @@ class ForwardBatch:
 
     def set_launch(self, block_threads: int, arena_kb: int = -1) -> None:
         """Applies a launch shape (rq_problem_set_launch): CTA size and shared-memory
-        arena in KiB (-1 = the default rule, 0 = none)."""
+        arena in KiB (-1 = the default rule, 0 = no more than the solver needs)."""
         shape = N.LaunchShape(int(block_threads), int(arena_kb), 0.0)
         N.call("rq_problem_set_launch", self._problem.handle, C.byref(shape))
 

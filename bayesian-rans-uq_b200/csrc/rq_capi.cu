@@ -74,7 +74,7 @@ void runOneJob(rq_problem &p, const rq::DevJob &job) {
 // (us per outer iteration with 70 / 110 / 150 / 208 KB: 100 x 50 cells 1039 / 1049 / 1045 / 1050,
 // 200 x 100 2437 / 2441 / 2451 / 2502, 400 x 200 7877 / 8002 / 8207 / 8670).
 constexpr long kClusterArenaKb = 112;
-long clusterArena(const rq::DevClass &C) {
+long clusterArena(const rq::DevClass &C, int knobKb) {
     long need = pad32(C.locDoubles);
     auto table = [&](int width, int rows) {
         const long cnt = width * pad32(rows);
@@ -89,30 +89,57 @@ long clusterArena(const rq::DevClass &C) {
     }
     const long m = C.lev[C.nlev - 1].n;
     need += pad32(2 * m * m);
-    return std::max<long>(pad32(C.locDoubles), std::min<long>(need, kClusterArenaKb * 1024 / 8));
+    const long most = maxSmemOptin() - static_cast<long>(rq::clusterSharedBytes());
+    const long limit = std::min(knobKb < 0 ? kClusterArenaKb * 1024 : knobKb * 1024L, most);
+    return std::max<long>(pad32(C.locDoubles), std::min<long>(need, limit / 8 / 32 * 32));
 }
 
-// CTAs per solve, by the class's size alone, so that a row's result does not depend on the
-// batch it is solved in. Classes above 1536 cells at the default CTA size and arena rule
-// take a cluster of 4 (8 from 32768 cells). Measured on a B200, ms per call with 4 / 8 CTAs
-// per solve (one CTA: 92, 171): 8 draws of 100 x 50 cells 45 / 38, 8 draws of 200 x 100
-// 38 / 28, but 32 draws of 200 x 100 51 / 85: 36 clusters of 4 fit the GPU at once, only 14
-// of 8. 400 x 200 cells: 14.5 / 8.8 ms per outer iteration.
-int clusterOf(const rq_problem &p, int block, int arenaKb) {
-    if (p.mesh.n <= 1536 || block != 768 || arenaKb >= 0 ||
-        8 * clusterArena(p.cls) > maxSmemOptin() - static_cast<long>(rq::clusterSharedBytes()))
-        return 1;
-    return p.mesh.n < 32768 ? 4 : 8;
+// CTAs per solve of a class above 1536 cells, in the order of a batch of `solves` draws; the
+// results do not depend on it (solveSlices). A solve takes about 5000 + cells / CTAs units of
+// time (units of 0.2 to 0.3 us per outer iteration), up to 1.9 times that as L2 fills with the
+// solves beside it, and only so many clusters fit the GPU at once. Measured on a B200, ms per outer
+// iteration of the whole batch with 4 / 2 / 1 CTAs:
+//   draws      64 x 40 cells        100 x 50             200 x 100
+//      1   0.60 / 0.72 / 0.85   0.93 / 1.24 / 1.59    2.67 /  4.00 /  6.38
+//     32   0.62 / 0.73 / 0.85   0.97 / 1.25 / 1.59    3.74 /  5.24 /  8.45
+//     64   1.24 / 0.77 / 0.86   1.93 / 1.39 / 1.72    7.24 /  6.42 / 10.55
+//    148   3.02 / 1.52 / 1.03   4.81 / 2.81 / 2.29   16.85 / 13.69 / 13.75
+// and with 8 / 4 / 2 of 400 x 200: 1 draw 7.35 / 11.95 / 21.87, 32 draws 28.0 / 20.3 / 36.2, 148
+// draws 103 / 99 / 83. (One CTA of the former kernel: 148 draws 1.31, 2.95 and 18.1.)
+rq::LaunchShape clusterShape(const rq_problem &p, int block, int arenaKb, long solves) {
+    rq::LaunchShape best{block, static_cast<int>(clusterArena(p.cls, arenaKb)), 0};
+    const int most = rq::solveSlices(p.mesh.n);
+    const double n = p.mesh.n;
+    double least = 0.0;
+    for (int ctas = most; 4 * ctas >= most; ctas /= 2) {
+        rq::LaunchShape sh = best;
+        sh.cluster = ctas;
+        const long atOnce = rq::concurrentSolves(sh, smCount());
+        if (atOnce < 1)
+            continue;
+        auto wave = [&](long m) {
+            return m > 0 ? (5000 + n / ctas) * std::min(1.9, 1 + m * n / 2.5e6) : 0.0;
+        };
+        const double t = static_cast<double>(solves / atOnce) * wave(atOnce) + wave(solves % atOnce);
+        if (best.cluster == 0 || t < least) {
+            best = sh;
+            least = t;
+        }
+        if (solves <= atOnce && ctas == most)
+            break;
+    }
+    if (best.cluster == 0)
+        best.cluster = most; // the caller reports that it does not fit
+    return best;
 }
 
 rq::LaunchShape shapeOf(const rq_problem &p, int block, int arenaKb, long solves) {
-    const int cluster = clusterOf(p, block, arenaKb);
-    if (cluster > 1)
-        return {block, static_cast<int>(clusterArena(p.cls)), cluster};
+    if (p.mesh.n > 1536 && block == 768)
+        return clusterShape(p, block, arenaKb, solves);
     return {block,
             arenaDoublesFor(p.cls.wsDoubles, arenaKb, p.mesh.n,
                             rq::residentDoubles(p.cls, block),
-                            block < 512 && solves > smCount()), 1};
+                            block < 512 && solves > smCount()), 0};
 }
 
 int chooseArena(const std::vector<const rq_problem *> &probs) {

@@ -12,11 +12,18 @@ size_t clusterSharedBytes(); // the same of the cluster kernels
 // of `block` threads (0: they do not apply, rq_resident.cuh).
 long residentDoubles(const DevClass &C, int block);
 // Launch shape of a solve: CTA size (64, 128, 256, 512, 768 or 1024), shared-memory arena
-// per CTA in doubles for the hot arrays (0 = all global), and CTAs per solve (above 1: a
-// thread-block cluster of 768-thread CTAs whose arena holds the small AMG levels).
+// per CTA in doubles for the hot arrays (0 = all global), and the CTAs per solve of the cluster
+// kernels (768 threads; the arena holds the small AMG levels), 0: the kernels of one CTA.
 struct LaunchShape {
     int block, arenaDoubles, cluster;
 };
+// Slices of the sums of a class that the cluster kernels solve: the CTAs of its largest
+// cluster, whatever the number it runs on.
+constexpr int kMaxSlices = 8;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int solveSlices(int n) { return n < 32768 ? 4 : kMaxSlices; }
 // Persistent solves: each pulls job indices from *nextJob (zeroed by the caller)
 // until njobs are taken; ws is solves x wsStride doubles of per-solve workspace.
 cudaError_t launchSolve(const DevJob *jobs, int njobs, int *nextJob, double *ws, long wsStride,

@@ -32,16 +32,17 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 
 // A solve runs on one CTA, or (objects compiled with RQ_CLUSTER) on a thread-block cluster
-// whose CTAs share the workspace in global memory: cells, faces and rows are dealt out
-// over all threads of the cluster, SYNC is its barrier, and block sums end in an exchange
-// of the CTAs' sums through distributed shared memory. Each CTA keeps its own copy of the
-// shared-memory state (Shared) and derives the same values in it.
+// of 1 to 8 CTAs, which share the workspace in global memory: cells, faces and rows are dealt
+// out over all threads of the cluster, SYNC is its barrier, and block sums end in an exchange
+// of partial sums through distributed shared memory. Each CTA keeps its own copy of the
+// shared-memory state (Shared) and derives the same values in it. A class's sums are formed
+// in a fixed number of slices (solveSlices), of which a CTA holds one or several, so the
+// number of CTAs changes no bit of a result.
 #ifdef RQ_CLUSTER
 constexpr bool kCluster = true;
 #else
 constexpr bool kCluster = false;
 #endif
-constexpr int kMaxCluster = 16;
 __device__ __forceinline__ int ctaRank() {
     unsigned r = 0;
     if constexpr (kCluster)
@@ -57,7 +58,7 @@ __device__ __forceinline__ int ctaCount() {
 __device__ __forceinline__ int gTid() { return ctaRank() * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int gThreads() { return ctaCount() * blockDim.x; }
 __device__ __forceinline__ void SYNC() {
-    if constexpr (kCluster)
+    if (kCluster && ctaCount() > 1)
         asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
     else
         __syncthreads();
@@ -73,7 +74,11 @@ __device__ __forceinline__ void putRemote(int *p, int v, int rank) {
     asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\t"
                  "st.shared::cluster.s32 [r], %2;\n\t}" ::"r"(a), "r"(rank), "r"(v) : "memory");
 }
-constexpr int kRedSlots = 8;             // values per block reduction
+constexpr int kRedSlots = 8; // values per block reduction
+constexpr int kSumSlots = 3; // of a sum
+// rows of warp partials: a reduction's values, or a sum's of every slice that a CTA holds
+constexpr int kRedRows = kCluster ? kMaxSlices * kSumSlots : kRedSlots;
+constexpr int kRedWarps = kCluster ? 24 : 32; // the cluster kernels' CTAs have 24 warps
 
 struct Work {
     double *Ux, *Uy, *p, *k, *w, *nuT, *F1, *F2, *Pk, *CD, *S;
@@ -144,8 +149,9 @@ struct Shared {
     KW<double> K64;
     KW<float> K32;
     double coeff[11];
-    double red[2][kRedSlots][32];
-    double cred[2][kRedSlots][kCluster ? kMaxCluster : 1]; // the cluster's CTA sums
+    alignas(16) double red[2][kRedRows][kRedWarps];
+    double cred[2][kRedSlots][kCluster ? kMaxSlices : 1]; // sums of the cluster's slices
+    int slices, ownSlices; // of the class's sums, and of these the CTA's
     double ring[4][kWindowCap];  // U, k, omega, Q change samples
     int cnt[4];
     double q[kMaxProbes], qPrev[kMaxProbes];
@@ -205,9 +211,13 @@ __device__ __forceinline__ void mma884(double &d0, double &d1, double a, double 
 // alike. (With matrix products for the partials too, which every warp repeats, the solves of
 // the general solvers took 8 to 14 % longer: mixed form, 384 / 768 / 1536 cells 166 / 286 / 448
 // us per outer iteration against 146 / 264 / 416; with shuffles for both 152 / 271 / 425.)
+//
+// Slice i of `slices` holds the cells (i + k slices) blockDim + 0 .. blockDim - 1, k = 0, 1, ...
+// CTA r of c CTAs holds the slices r, r + c, ..., which are the cells of its own sweeps
+// (FOR_OWN). Within a slice a thread adds its cells, a warp its threads and the slice its
+// warps, whichever CTA does it, and every thread adds the slices in order.
 template <int K>
-__device__ __forceinline__ void blockSum(double (&v)[K], Shared &S, int &rp) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+__device__ __forceinline__ void parkSums(double (&v)[K], Shared &S, int rp, int slice) {
     double u[K], w[K];
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -215,33 +225,70 @@ __device__ __forceinline__ void blockSum(double (&v)[K], Shared &S, int &rp) {
 #pragma unroll
     for (int k = 0; k < K; ++k)
         mma884(v[k], w[k], u[k] + w[k], 1.0);
-    if (lane == 0)
+    if ((threadIdx.x & 31) == 0)
 #pragma unroll
         for (int k = 0; k < K; ++k)
-            S.red[rp][k][warp] = v[k];
+            S.red[rp][slice * K + k][threadIdx.x >> 5] = v[k];
+}
+__device__ __forceinline__ double addLanes(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        v += __shfl_xor_sync(FULL, v, o);
+    return v;
+}
+// the sums of the parked partials, in every thread; a barrier for what was stored before
+template <int K>
+__device__ __forceinline__ void totalSums(double (&v)[K], Shared &S, int &rp) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     __syncthreads();
-    const int nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        v[k] = lane < nw ? S.red[rp][k][lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1)
-            v[k] += __shfl_xor_sync(FULL, v[k], o);
-    }
-    if constexpr (kCluster) { // every CTA adds the CTA sums in the order of the ranks
-        const int nc = ctaCount(), rank = ctaRank();
-        if (static_cast<int>(threadIdx.x) < nc)
-#pragma unroll
-            for (int k = 0; k < K; ++k)
-                putRemote(&S.cred[rp][k][rank], v[k], threadIdx.x);
+    if constexpr (kCluster) { // a warp per slice and value, the sums to every CTA
+        const int nc = ctaCount(), rank = ctaRank(), rows = S.ownSlices * K;
+        for (int t = warp; t < rows; t += nw) {
+            double w = 0.0, unused; // eight partials per lane, the four lanes by a product
+            if (8 * (lane & 3) < nw) {
+                const double2 *r = reinterpret_cast<const double2 *>(&S.red[rp][t][8 * (lane & 3)]);
+                const double2 a = r[0], b = r[1], c = r[2], d = r[3];
+                w = ((a.x + b.x) + (c.x + d.x)) + ((a.y + b.y) + (c.y + d.y));
+            }
+            mma884(w, unused, w, 1.0);
+            const int slice = t / K, k = t - slice * K;
+            if (lane < nc)
+                putRemote(&S.cred[rp][k][slice * nc + rank], w, lane);
+        }
         SYNC();
+        const int ns = S.slices;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             v[k] = S.cred[rp][k][0];
-            for (int c = 1; c < nc; ++c)
+            for (int c = 1; c < ns; ++c)
                 v[k] += S.cred[rp][k][c];
         }
+    } else { // every warp the same partials
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            v[k] = addLanes(lane < nw ? S.red[rp][k][lane] : 0.0);
     }
     rp ^= 1;
+}
+// add(i) adds item i's terms to v, for the thread's items of 0 .. count - 1; one value of v
+// per slice is parked
+template <int K, typename Add>
+__device__ __forceinline__ void parkOver(double (&v)[K], Shared &S, int rp, int count, Add add) {
+    const int own = kCluster ? S.ownSlices : 1;
+    const int step = (kCluster ? S.slices : 1) * blockDim.x;
+    for (int slice = 0; slice < own; ++slice) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            v[k] = 0.0;
+        for (int i = (slice * ctaCount() + ctaRank()) * blockDim.x + threadIdx.x; i < count; i += step)
+            add(i);
+        parkSums(v, S, rp, slice);
+    }
+}
+template <int K, typename Add>
+__device__ __forceinline__ void sumOver(double (&v)[K], Shared &S, int &rp, int count, Add add) {
+    parkOver(v, S, rp, count, add);
+    totalSums(v, S, rp);
 }
 
 // Maximum over a warp of nonnegative values: their bit patterns are ordered as integers, so
@@ -470,16 +517,15 @@ __device__ __noinline__ LinRes bicgstabT(Shared &S, int &rp, const KW<T> &K, T *
     T *r = K.r, *rh = K.rh, *p = K.pv, *v = K.v, *s = K.s, *t = K.t, *ph = K.ph, *sh = K.sh,
       *rd = K.rd;
     const Mat<T> M = matOf(K);
-    double acc[1] = {0.0};
-    FOR_CELLS(c) {
+    double acc[1];
+    sumOver(acc, S, rp, n, [&](int c) {
         rh[c] = r[c];
         p[c] = T(0);
         v[c] = T(0);
         const T dc = M.d[c];
         rd[c] = (fabs(double(dc)) > 1e-30) ? T(1) / dc : T(1); // jacobiPrecond as a product
         acc[0] += double(r[c]) * double(r[c]);
-    }
-    blockSum<1>(acc, S, rp);
+    });
     double rhoN = acc[0], rho = 1, alpha = 1, omega = 1;
     for (int it = 0; it < maxIter; ++it) {
         if (fabs(rhoN) < 1e-30)
@@ -491,26 +537,24 @@ __device__ __noinline__ LinRes bicgstabT(Shared &S, int &rp, const KW<T> &K, T *
             ph[c] = pc * rd[c];
         }
         SYNC();
-        double a1[1] = {0.0};
-        FOR_CELLS(c) {
+        double a1[1];
+        sumOver(a1, S, rp, n, [&](int c) {
             const Cell q = cellOf(C, c);
             const T vc = rowDotT(q, M, ph, nx);
             v[c] = vc;
             a1[0] += double(rh[c]) * double(vc);
-        }
-        blockSum<1>(a1, S, rp);
+        });
         const double rv = a1[0];
         if (fabs(rv) < 1e-30)
             break;
         alpha = rhoN / rv;
-        double a2[1] = {0.0};
-        FOR_CELLS(c) {
+        double a2[1];
+        sumOver(a2, S, rp, n, [&](int c) {
             const T sc = r[c] - T(alpha) * v[c];
             s[c] = sc;
             sh[c] = sc * rd[c];
             a2[0] += double(sc) * double(sc);
-        }
-        blockSum<1>(a2, S, rp);
+        });
         const double sn = sqrt(a2[0]);
         if (sn / r0n < tol) {
             FOR_CELLS(c) x[c] += T(alpha) * ph[c];
@@ -520,26 +564,24 @@ __device__ __noinline__ LinRes bicgstabT(Shared &S, int &rp, const KW<T> &K, T *
             res.converged = true;
             return res;
         }
-        double a3[2] = {0.0, 0.0};
-        FOR_CELLS(c) {
+        double a3[2];
+        sumOver(a3, S, rp, n, [&](int c) {
             const Cell q = cellOf(C, c);
             const T tc = rowDotT(q, M, sh, nx);
             t[c] = tc;
             a3[0] += double(tc) * double(tc);
             a3[1] += double(tc) * double(s[c]);
-        }
-        blockSum<2>(a3, S, rp);
+        });
         const double tt = a3[0];
         omega = (tt > 1e-30) ? a3[1] / tt : 0.0;
-        double a4[2] = {0.0, 0.0};
-        FOR_CELLS(c) {
+        double a4[2];
+        sumOver(a4, S, rp, n, [&](int c) {
             x[c] += T(alpha) * ph[c] + T(omega) * sh[c];
             const T rc = s[c] - T(omega) * t[c];
             r[c] = rc;
             a4[0] += double(rc) * double(rc);
             a4[1] += double(rh[c]) * double(rc);
-        }
-        blockSum<2>(a4, S, rp);
+        });
         const double rn = sqrt(a4[0]);
         res.iterations = it + 1;
         res.finalRes = rn / r0n;
@@ -870,7 +912,8 @@ __device__ __forceinline__ int segOf(int n, int nt) {
     return seg;
 }
 
-// A pass over the rows of a small level with several threads per row: lane j of a
+// A pass over the rows of a small level with several threads per row (as many as one CTA could
+// give each, so that the partial sums do not depend on the number of CTAs): lane j of a
 // row's segment computes part(i, j, seg), the partial sum of the row's terms j,
 // j + seg, ...; the partials are added by shuffles within the segment (a tree) and
 // the segment's first lane calls use(i, total). Every one of the nt threads takes part, t
@@ -878,7 +921,7 @@ __device__ __forceinline__ int segOf(int n, int nt) {
 // thread per row this is the plain row loop.
 template <typename T, typename Part, typename Use>
 __device__ __forceinline__ void segPass(int n, int t, int nt, Part part, Use use) {
-    const int seg = segOf(n, nt), per = nt / seg;
+    const int seg = segOf(n, blockDim.x), per = nt / seg;
     const int r = t / seg, j = t - r * seg;
     for (int base = 0; base < n; base += per) {
         const int i = base + r;
@@ -1075,7 +1118,6 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
         // post sweep(s) read it (each x once, not re-formed at every neighbour)
         const int n = C.lev[0].n;
         T *x = two ? Kxb : Kxa;
-        T *out = two ? Kxa : Kz;
         if (lean) {
             if constexpr (std::is_same_v<T, double>) {
                 const ResLevel &R = S.RL[0];
@@ -1088,33 +1130,27 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
                 x[i] += al * prolong(0, i);
         }
         SYNC();
-        double part = 0.0;
-        FOR_OWN(i, n) {
-            const T ax = rowDotT(cellOf(C, i), M, x, nx);
-            const T zi = x[i] + om * (Kr[i] - ax) * Krd[i];
-            out[i] = zi;
-            if (!two)
-                part += double(Kr[i]) * double(zi);
-        }
+        auto sweep = [&](const T *from, T *to, int i) { // a damped-Jacobi sweep's row
+            const T ax = rowDotT(cellOf(C, i), M, from, nx);
+            const T zi = from[i] + om * (Kr[i] - ax) * Krd[i];
+            to[i] = zi;
+            return zi;
+        };
+        double a[1];
         if (two) {
+            FOR_OWN(i, n)
+                sweep(x, Kxa, i);
             SYNC();
-            FOR_OWN(i, n) {
-                const T ax = rowDotT(cellOf(C, i), M, Kxa, nx);
-                const T zi = Kxa[i] + om * (Kr[i] - ax) * Krd[i];
-                Kz[i] = zi;
-                part += double(Kr[i]) * double(zi);
-            }
+            sumOver(a, S, rp, n, [&](int i) { a[0] += double(Kr[i]) * double(sweep(Kxa, Kz, i)); });
+        } else {
+            sumOver(a, S, rp, n, [&](int i) { a[0] += double(Kr[i]) * double(sweep(x, Kz, i)); });
         }
-        double a[1] = {part};
-        blockSum<1>(a, S, rp);
         rz = a[0];
     } else if (L > 1) { // level 0, piecewise-constant P: prolongation fused into the
         // first post sweep (then the second)
         const int n = C.lev[0].n;
         const T *xprev = two ? Kxb : Kxa;
-        T *out = two ? Kxa : Kz;
-        double part = 0.0;
-        FOR_OWN(i, n) {
+        auto first = [&](T *to, int i) {
             const T xi = xprev[i] + al * prolong(0, i);
             const Cell q = cellOf(C, i);
             const int c = i;
@@ -1126,31 +1162,31 @@ template <typename T> __device__ __noinline__ double vcycleT(Shared &S, int &rp,
             const T y1 = q.yNfirst ? tN : tS, y2 = q.yNfirst ? tS : tN;
             const T ax = (((M.d[c] * xi + x1) + x2) + y1) + y2;
             const T zi = xi + om * (Kr[i] - ax) * Krd[c];
-            out[i] = zi;
-            if (!two)
-                part += double(Kr[i]) * double(zi);
-        }
+            to[i] = zi;
+            return zi;
+        };
+        double a[1];
         if (two) {
+            FOR_OWN(i, n)
+                first(Kxa, i);
             SYNC();
-            FOR_OWN(i, n) {
+            sumOver(a, S, rp, n, [&](int i) {
                 const T ax = rowDotT(cellOf(C, i), M, Kxa, nx);
                 const T zi = Kxa[i] + om * (Kr[i] - ax) * Krd[i];
                 Kz[i] = zi;
-                part += double(Kr[i]) * double(zi);
-            }
+                a[0] += double(Kr[i]) * double(zi);
+            });
+        } else {
+            sumOver(a, S, rp, n, [&](int i) { a[0] += double(Kr[i]) * double(first(Kz, i)); });
         }
-        double a[1] = {part};
-        blockSum<1>(a, S, rp);
         rz = a[0];
     } else {
         const T *xb = vb(0) + 2 * C.lev[0].n;
-        double part = 0.0;
-        FOR_OWN(i, n0) {
+        double a[1];
+        sumOver(a, S, rp, n0, [&](int i) {
             Kz[i] = xb[i];
-            part += double(Kr[i]) * double(xb[i]);
-        }
-        double a[1] = {part};
-        blockSum<1>(a, S, rp);
+            a[0] += double(Kr[i]) * double(xb[i]);
+        });
         rz = a[0];
     }
     return rz;
@@ -1166,13 +1202,12 @@ template <typename T> __device__ __noinline__ double pcgMatvec(Shared &S, int &r
     const Mat<T> M = matOf(K);
     const T *p = K.pv;
     T *Ap = K.v;
-    double a[1] = {0.0};
-    FOR_CELLS(c) {
+    double a[1];
+    sumOver(a, S, rp, n, [&](int c) {
         const T v = rowDotT(cellOf(C, c), M, p, nx);
         Ap[c] = v;
         a[0] += double(p[c]) * double(v);
-    }
-    blockSum<1>(a, S, rp);
+    });
     return a[0];
 }
 // x += alpha p, r -= alpha Ap; returns (r, r)
@@ -1181,14 +1216,13 @@ __device__ __noinline__ double pcgUpdate(Shared &S, int &rp, const KW<T> &K, T *
     const int n = S.C.n;
     const T *p = K.pv, *Ap = K.v;
     T *r = K.r;
-    double a[1] = {0.0};
-    FOR_CELLS(c) {
+    double a[1];
+    sumOver(a, S, rp, n, [&](int c) {
         x[c] += T(alpha) * p[c];
         const T rc = r[c] - T(alpha) * Ap[c];
         r[c] = rc;
         a[0] += double(rc) * double(rc);
-    }
-    blockSum<1>(a, S, rp);
+    });
     return a[0];
 }
 // z = r / diag; returns (r, z)
@@ -1196,12 +1230,11 @@ template <typename T> __device__ __noinline__ double pcgJacobi(Shared &S, int &r
     const int n = S.C.n;
     const T *r = K.r, *rdv = K.rd;
     T *z = K.z;
-    double a[1] = {0.0};
-    FOR_CELLS(c) {
+    double a[1];
+    sumOver(a, S, rp, n, [&](int c) {
         z[c] = r[c] * rdv[c];
         a[0] += double(r[c]) * double(z[c]);
-    }
-    blockSum<1>(a, S, rp);
+    });
     return a[0];
 }
 // p = z + beta p (beta 0: p = z), then a barrier
@@ -1226,23 +1259,21 @@ __device__ __noinline__ Two pcgUpdateSum(Shared &S, int &rp, const KW<T> &K, T *
     const int n = S.C.n;
     const T *p = K.pv, *Ap = K.v;
     T *r = K.r;
-    double a[2] = {0.0, 0.0};
-    FOR_CELLS(c) {
+    double a[2];
+    sumOver(a, S, rp, n, [&](int c) {
         x[c] += T(alpha) * p[c];
         const T rc = r[c] - T(alpha) * Ap[c];
         r[c] = rc;
         a[0] += double(rc) * double(rc);
         a[1] += double(rc);
-    }
-    blockSum<2>(a, S, rp);
+    });
     return Two{a[0], a[1]};
 }
 // the sum of r (the first residual of a solve)
 template <typename T> __device__ __noinline__ double sumOf(Shared &S, int &rp, const T *r) {
     const int n = S.C.n;
-    double a[1] = {0.0};
-    FOR_CELLS(c) a[0] += double(r[c]);
-    blockSum<1>(a, S, rp);
+    double a[1];
+    sumOver(a, S, rp, n, [&](int c) { a[0] += double(r[c]); });
     return a[0];
 }
 
@@ -1270,14 +1301,13 @@ __device__ __noinline__ Two pcgPrecondF32(Shared &S, int &rp, const KW<T> &K, do
     const double shift = sumR / rowsum0 - double(F.z[0]);
     const T *r = K.r;
     T *z = K.z;
-    double a[2] = {0.0, 0.0};
-    FOR_CELLS(c) {
+    double a[2];
+    sumOver(a, S, rp, n, [&](int c) {
         const T zc = T(double(F.z[c]) + shift);
         a[1] += double(r[c]) * double(z[c]);
         z[c] = zc;
         a[0] += double(r[c]) * double(zc);
-    }
-    blockSum<2>(a, S, rp);
+    });
     return Two{a[0], a[1]};
 }
 
@@ -1422,9 +1452,8 @@ __device__ __noinline__ LinRes mixedSolve(Shared &S, int &rp, double *x64, doubl
     for (int round = 0; round < 8 && out.iterations < maxIter; ++round) {
         // the FP32 solve targets the remaining reduction of the FP64 residual
         const double innerTol = tol * r0n / rn;
-        double an[1] = {0.0};
-        FOR_CELLS(c) an[0] += double(K.r[c]) * double(K.r[c]);
-        blockSum<1>(an, S, rp);
+        double an[1];
+        sumOver(an, S, rp, n, [&](int c) { an[0] += double(K.r[c]) * double(K.r[c]); });
         const double r32n = sqrt(an[0]);
         LinRes in;
         FOR_CELLS(c) K.x[c] = 0.0f;
@@ -1434,15 +1463,14 @@ __device__ __noinline__ LinRes mixedSolve(Shared &S, int &rp, double *x64, doubl
         out.iterations += in.iterations;
         FOR_CELLS(c) x64[c] += double(K.x[c]);
         SYNC();
-        double a[1] = {0.0};
-        FOR_CELLS(c) {
+        double a[1];
+        sumOver(a, S, rp, n, [&](int c) {
             const Cell q = cellOf(C, c);
             const double rc = W.b[c] - rowDot(q, W.d, W.aW, W.aE, W.aS, W.aN, x64, nx);
             W.r[c] = rc;
             K.r[c] = float(rc);
             a[0] += rc * rc;
-        }
-        blockSum<1>(a, S, rp);
+        });
         rn = sqrt(a[0]);
         if (rn / r0n < tol) {
             out.converged = true;
@@ -1942,12 +1970,13 @@ __device__ __noinline__ void phMomentumFaces(Shared &S, int comp) {
 // The momentum rows of one component from the face values of phMomentumFaces (a resolved
 // wall: molecular viscosity, U_b = 0, no flux), summed in the reference's order (x faces, y
 // faces, walls); the row's residual. The x pass leaves V / a_P in aP for the p' equation.
-__device__ __noinline__ void phMomentum(Shared &S, int comp, double (&acc)[3]) {
+__device__ __noinline__ void phMomentum(Shared &S, int comp, int rp) {
     RQ_PRELUDE
     const double *U = comp == 0 ? W.Ux : W.Uy, *gP = comp == 0 ? W.gPx : W.gPy;
     const double *phi = W.phi, *D = W.pCoeff, *tsf = W.phiPred, *ccf = W.fScr;
     const double fb = comp == 0 ? st.fx : st.fy;
-    FOR_CELLS(c) {
+    double acc[3];
+    parkOver(acc, S, rp, n, [&](int c) {
         const Cell q = cellOf(C, c);
         const int fW = q.W, fE = c, fS = n + c, fN = n + c + nx;
         const double FW = phi[fW], FE = phi[fE], DW = D[fW], DE = D[fE];
@@ -1998,19 +2027,20 @@ __device__ __noinline__ void phMomentum(Shared &S, int comp, double (&acc)[3]) {
         W.r[c] = rc;
         acc[0] += fabs(rc);
         acc[1] += rc * rc;
-    }
+    });
 }
 
 // Predicted face flux (stored Rhie-Chow, :1401-1419) and the coefficient of p'. The flux of
 // the velocity at the iteration start is interpolated here, beside the new one, from the
 // same geometry (a sweep of its own in phStart cost a store and ten loads per face).
-__device__ __noinline__ void phPressureFaces(Shared &S, double (&fs)[1]) {
+__device__ __noinline__ void phPressureFaces(Shared &S, int rp) {
     RQ_PRELUDE
     const double relaxCorr = 1.0 - st.aU;
     const double *Ux = W.Ux, *Uy = W.Uy, *Uxp = W.Uxp, *Uyp = W.Uyp, *dP = W.aP, *p = W.p;
     const double *gPx = W.gPx, *gPy = W.gPy, *phi = W.phi;
     double *pred = W.phiPred, *coeff = W.pCoeff;
-    FOR_OWN(f, n + nfy) {
+    double fs[1];
+    parkOver(fs, S, rp, n + nfy, [&](int f) {
         int o, q;
         double ph = 0.0, pc = 0.0;
         if (faceCells(C, f, o, q)) {
@@ -2028,12 +2058,13 @@ __device__ __noinline__ void phPressureFaces(Shared &S, double (&fs)[1]) {
         pred[f] = ph;
         coeff[f] = pc;
         fs[0] += fabs(ph);
-    }
+    });
 }
 
-__device__ __noinline__ void phPressureCells(Shared &S, double (&pacc)[3]) {
+__device__ __noinline__ void phPressureCells(Shared &S, int rp) {
     RQ_PRELUDE
-        FOR_CELLS(c) {
+        double pacc[2];
+        parkOver(pacc, S, rp, n, [&](int c) {
             const Cell q = cellOf(C, c);
             const int fE = c, fW = q.W, fN = n + c + nx, fS = n + c;
             // diagonal: coefficients of internal faces in order
@@ -2081,7 +2112,7 @@ __device__ __noinline__ void phPressureCells(Shared &S, double (&pacc)[3]) {
             W.pp[c] = 0.0;
             pacc[0] += fabs(bsum);
             pacc[1] += bsum * bsum;
-        }
+        });
 }
 
 // Pressure-velocity corrections (:916-940, :1443-1467): U -= grad p' V / aP with
@@ -2168,14 +2199,15 @@ __device__ __noinline__ void phTurbFaces(Shared &S, int eq) {
 // its wall value, its row is decoupled and its neighbours take the value to their right-hand
 // side, so no row reads a wall cell's unknown and it is set here. (The residual as a sweep
 // of its own re-read the five coefficients: 3300 cycles at 384 cells, 8700 at 1536.)
-__device__ __noinline__ void phTurbAssemble(Shared &S, int eq, double (&acc)[1]) {
+__device__ __noinline__ void phTurbAssemble(Shared &S, int eq, int rp) {
     RQ_PRELUDE
     double *X = eq == 0 ? W.k : W.w;
     const double *phi = W.phi, *D = W.pCoeff, *bal = W.phiPred, *ccf = W.fScr;
     const double s1 = eq == 0 ? sk1 : sw1, s2 = eq == 0 ? sk2 : sw2;
     const bool balance = eq == 1 && C.balance;
     const double iB1 = 1.0 / b1, iBeta = 1.0 / S.wallBeta;
-    FOR_CELLS(c) {
+    double acc[1];
+    parkOver(acc, S, rp, n, [&](int c) {
         if (eq == 1) // the bounds of the k just solved (read below at this cell only)
             clampK(S, c);
         const Cell q = cellOf(C, c);
@@ -2263,7 +2295,7 @@ __device__ __noinline__ void phTurbAssemble(Shared &S, int eq, double (&acc)[1])
         W.b[c] = bsum;
         W.r[c] = rc;
         acc[0] += rc * rc;
-    }
+    });
 }
 
 // Change norms; mx[4], mx[5]: squares of the largest |U| and |dU|.
@@ -2396,11 +2428,11 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
                 SYNC();
             }
             double *U = comp == 0 ? W.Ux : W.Uy;
-            double acc[3] = {0.0, 0.0, 0.0};
+            double acc[3];
             phMomentumFaces(S, comp);
             SYNC();
-            phMomentum(S, comp, acc);
-            blockSum<3>(acc, S, rp);
+            phMomentum(S, comp, rp);
+            totalSums(acc, S, rp);
             momRes = comp == 0 ? acc[0] : dmax(momRes, acc[0]);
             if (comp == 0)
                 momScale = acc[2];
@@ -2412,14 +2444,13 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
 
         mark(S, 2);
         // ---- predicted flux (stored Rhie-Chow, :1401-1419) and p' assembly (:717-830)
-        double fs[1] = {0.0};
-        phPressureFaces(S, fs);
-        SYNC();
-        double pacc[3] = {0.0, 0.0, fs[0]};
-        phPressureCells(S, pacc);
-        blockSum<3>(pacc, S, rp);
-        Ls.contScaled = pacc[0] / dmax(pacc[2], 1e-300);
-        Ls.fluxScale = pacc[2];
+        double fs[1], pacc[2];
+        phPressureFaces(S, rp);
+        totalSums(fs, S, rp);
+        phPressureCells(S, rp);
+        totalSums(pacc, S, rp);
+        Ls.contScaled = pacc[0] / dmax(fs[0], 1e-300);
+        Ls.fluxScale = fs[0];
         mark(S, 3);
         LinRes &resP = Ls.resP;
         resP = solvePressure(S, rp, W.pp, sqrt(pacc[1]), st.innerIter, st.innerTol, st.pSolver,
@@ -2442,11 +2473,11 @@ __device__ void runSolve(Shared &S, const DevJob &job) {
             // inside the change norms (each reads only its own cell's value)
             for (int eq = 0; eq < 2; ++eq) { // 0: k, 1: omega
                 double *X = eq == 0 ? W.k : W.w;
-                double acc[1] = {0.0};
+                double acc[1];
                 phTurbFaces(S, eq);
                 SYNC();
-                phTurbAssemble(S, eq, acc);
-                blockSum<1>(acc, S, rp);
+                phTurbAssemble(S, eq, rp);
+                totalSums(acc, S, rp);
                 LinRes &rr = eq == 0 ? resK : resW;
                 solveBicg(S, rp, X, sqrt(acc[0]), st.innerIter, st.innerTol, &rr);
                 if (threadIdx.x == 0)
@@ -2687,6 +2718,8 @@ __device__ void runJob(Shared &S, const DevJob &job, double *ws, double *arena, 
             S.coeff[idx] = v;
         }
         S.admitted = ok;
+        S.slices = kCluster ? solveSlices(S.C.n) : 1;
+        S.ownSlices = S.slices / ctaCount();
         if (ok)
             carve(S, ws, arena, arenaDoubles);
     }
@@ -2900,30 +2933,29 @@ void *pick(int block) { return entryOf(kEntrySolve, block); }
 void *pickServe(int block) { return entryOf(kEntryServe, block); }
 // the function of a launch shape, and its dynamic shared memory
 void *shapeEntry(int kind, const LaunchShape &sh) {
-    if (sh.cluster > 1)
+    if (sh.cluster > 0)
         return sh.block == kClusterThreads ? solveEntry<kClusterThreads, true>(kind) : nullptr;
     return entryOf(kind, sh.block);
 }
 size_t shapeBytes(const LaunchShape &sh) {
-    return (sh.cluster > 1 ? clusterSharedBytes() : solveSharedBytes()) + sizeof(double) * static_cast<size_t>(sh.arenaDoubles);
+    return (sh.cluster > 0 ? clusterSharedBytes() : solveSharedBytes()) +
+           sizeof(double) * static_cast<size_t>(sh.arenaDoubles);
 }
 // The limits are set to the device's own, not to the launch's: they belong to the function, and
 // another thread may be launching it with another arena.
-cudaError_t setAttributes(void *fn, const LaunchShape &sh) {
+cudaError_t setAttributes(void *fn) {
     int dev = 0, optin = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-    if (e == cudaSuccess && sh.cluster > 8)
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
 cudaLaunchConfig_t configOf(const LaunchShape &sh, int solves, cudaStream_t stream,
                             cudaLaunchAttribute *attr) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(solves * sh.cluster);
+    cfg.gridDim = dim3(solves * (sh.cluster > 1 ? sh.cluster : 1));
     cfg.blockDim = dim3(sh.block);
     cfg.dynamicSmemBytes = shapeBytes(sh);
     cfg.stream = stream;
@@ -2950,7 +2982,7 @@ cudaError_t launchSolve(const DevJob *jobs, int njobs, int *nextJob, double *ws,
     void *fn = shapeEntry(kEntrySolve, sh);
     if (!fn)
         return cudaErrorInvalidConfiguration;
-    cudaError_t e = setAttributes(fn, sh);
+    cudaError_t e = setAttributes(fn);
     if (e != cudaSuccess)
         return e;
     cudaLaunchAttribute attr;
@@ -2965,7 +2997,7 @@ cudaError_t launchSolve(const DevJob *jobs, int njobs, int *nextJob, double *ws,
 
 int concurrentSolves(const LaunchShape &sh, int sms) {
     void *fn = shapeEntry(kEntrySolve, sh);
-    if (!fn || setAttributes(fn, sh) != cudaSuccess) {
+    if (!fn || setAttributes(fn) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -2993,7 +3025,7 @@ cudaError_t launchServe(const ServeQueue &q, double *ws, long wsStride, int grid
     void *fn = pickServe(block);
     if (!fn)
         return cudaErrorInvalidConfiguration;
-    cudaError_t e = setAttributes(fn, {block, arenaDoubles, 1});
+    cudaError_t e = setAttributes(fn);
     if (e != cudaSuccess)
         return e;
     ServeQueue qq = q;
@@ -3007,7 +3039,7 @@ cudaError_t launchServe(const ServeQueue &q, double *ws, long wsStride, int grid
 int serveBlocksPerSM(int block, int arenaDoubles) {
     const size_t smem = solveSharedBytes() + sizeof(double) * static_cast<size_t>(arenaDoubles);
     void *fn = pickServe(block);
-    if (!fn || setAttributes(fn, {block, arenaDoubles, 1}) != cudaSuccess)
+    if (!fn || setAttributes(fn) != cudaSuccess)
         return 0;
     int blocks = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, block, smem) != cudaSuccess)
@@ -3039,7 +3071,7 @@ cudaError_t launchSolveNoAlloc(const DevJob &job, double *scratch, const LaunchS
     void *fn = shapeEntry(kEntryOne, sh);
     if (!fn)
         return cudaErrorInvalidConfiguration;
-    cudaError_t e = setAttributes(fn, sh);
+    cudaError_t e = setAttributes(fn);
     if (e != cudaSuccess)
         return e;
     cudaLaunchAttribute attr;

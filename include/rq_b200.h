@@ -164,11 +164,13 @@ int rq_problem_info(const rq_problem *p, int32_t *n_cells, int32_t *n_obs, int32
 int rq_problem_workspace_bytes(const rq_problem *p, uint64_t *bytes);
 
 /* Launch shape of a mesh class: the CTA size of its solves and the shared-memory
-   arena each CTA places the solve's hottest arrays in. */
+   arena in which each CTA places the solve's hottest arrays. */
 typedef struct rq_launch_shape {
     int32_t block_threads;   /* 64, 128, 256, 512, 768 or 1024 */
-    int32_t arena_kb;        /* arena per CTA in KiB; 0 = none; -1 = the default rule (half
-                                the SM's shared memory up to 768 cells, none above) */
+    int32_t arena_kb;        /* arena per CTA in KiB beyond what the solver itself needs; 0 =
+                                only that; -1 = the default rule (130 KB with the fixed part
+                                for the classes whose inner solvers run in registers and those
+                                of up to 768 cells, 112 KB on clusters, else none) */
     double us_per_iteration; /* measured by rq_problem_tune; 0 when not measured */
 } rq_launch_shape;
 
@@ -178,8 +180,10 @@ typedef struct rq_launch_shape {
    `iters` outer iterations with the GPU's own timer, writes the measured time per
    outer iteration into measured[k] (NULL allowed; candidates that do not fit on an SM
    get a negative time), applies the fastest to the problem and returns it in *chosen.
-   Results do not depend on the arena; the CTA size changes only the order of the
-   block sums (agreement to rounding). Blocks until the timings are in. */
+   Results do not depend on the arena, nor on how many CTAs a solve above 1536 cells
+   takes (its cluster grows where draws are few; 768 threads, the default, only); the
+   CTA size changes only the order of the block sums (agreement to rounding). Blocks
+   until the timings are in. */
 int rq_problem_tune(rq_problem *p, const double *theta, int32_t iters,
                     const rq_launch_shape *candidates, int32_t n_candidates,
                     rq_launch_shape *measured, rq_launch_shape *chosen);

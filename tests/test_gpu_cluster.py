@@ -1,5 +1,8 @@
 """Solves on thread-block clusters (classes above 1536 cells).
 
+How many CTAs a solve takes depends on the number of draws; its sums are formed in the same
+slices whatever that number, so rows equal those of a draw alone bit for bit.
+
 The CTAs of a cluster share the level vectors in global memory and run the small AMG levels
 whole, each for itself. A CTA that reads a vector which another has overwritten shows as a row
 that differs between equal draws or between launches, or as fields away from the
@@ -69,3 +72,48 @@ def test_more_cells_than_16_bit_columns(rq, checker):
     one = np.maximum(distance(512), distance(1024))
     assert np.all(one < 1e-3)
     assert np.all(distance(0) <= 10 * one + 1e-9)
+
+
+@pytest.mark.parametrize("solver,precision", [("AMG", "fp64"), ("PCG", "fp64"),
+                                              ("BiCGSTAB", "fp64"), ("AMG", "mixed"),
+                                              ("BiCGSTAB", "mixed")])
+@pytest.mark.parametrize("nx,ny", [(49, 32), (60, 36), (100, 50)])
+def test_rows_do_not_depend_on_the_number_of_draws(rq, nx, ny, solver, precision):
+    case = cases.bump_case(nx, ny, max_iter=8, turb_start=2)
+    batch = cases.product_batch(rq, case, pressure_solver=solver, precision=precision)
+    theta = np.array([[0.29, 0.085], [0.31, 0.09], [0.33, 0.095]])
+    alone = [batch.evaluate_fields(theta[i:i + 1])[1][0] for i in range(3)]
+    for n in (3, 40, 75, 160):  # 4, 2, 1 and 1 CTAs per solve on a B200
+        _, fields, _ = batch.evaluate_fields(np.tile(theta, (n, 1))[:n])
+        for i, f in enumerate(fields):
+            np.testing.assert_array_equal(f, alone[i % 3])
+
+
+@pytest.mark.parametrize("n", [20, 40, 70])  # 8, 4 and 2 CTAs
+def test_rows_of_an_eight_cta_class(rq, n):
+    case = cases.bump_case(260, 128, max_iter=3)
+    batch = cases.product_batch(rq, case)
+    want = batch.evaluate([[0.31, 0.09]]).predictions[0]
+    for row in batch.evaluate(np.repeat([[0.31, 0.09]], n, axis=0)).predictions:
+        np.testing.assert_array_equal(row, want)
+
+
+def test_a_long_queue_fills_the_gpu(rq):
+    """Enough draws for every SM run one per SM, not four or eight SMs each."""
+    import torch
+    from test_gpu_residency import most_at_once
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    batch = cases.product_batch(rq, cases.bump_case(64, 40, max_iter=60))
+    assert most_at_once(rq, batch, sms) >= 0.9 * sms
+
+
+@pytest.mark.parametrize("nx,ny", [(60, 36), (100, 50)])
+def test_results_do_not_depend_on_the_arena(rq, nx, ny):
+    batch = cases.product_batch(rq, cases.bump_case(nx, ny, max_iter=8, turb_start=2))
+    theta = np.array([[0.29, 0.085], [0.31, 0.09]])
+    _, want, _ = batch.evaluate_fields(theta)
+    for arena in (0, 40, 200):
+        batch.set_launch(768, arena)
+        _, got, _ = batch.evaluate_fields(theta)
+        np.testing.assert_array_equal(got, want)
