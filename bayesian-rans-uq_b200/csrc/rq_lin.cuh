@@ -10,8 +10,8 @@ namespace rq {
 
 constexpr int kLinMaxLevels = 16;
 constexpr int kLinThreads = 1024;
-constexpr int kLinMaxCluster = 16;
-constexpr int kLinMaxLocalBytes = 220 * 1024; // shared memory of the local levels' vectors
+constexpr int kLinMaxSlices = 16;   // slices of a system's sums: the CTAs of its largest cluster
+constexpr int kLinMaxLocalBytes = 208 * 1024; // shared memory of the local levels' vectors
 constexpr int kLinLocalRows = 2048; // rows of a level that every CTA of a cluster runs whole
 enum LinKind : int32_t { kLinAmg = 0, kLinPcg = 1, kLinBicgstab = 2 };
 
@@ -39,7 +39,8 @@ struct DevLinLevel {
 
 struct DevLinSys {
     int32_t n, nlev, kind, precision, maxIter, m; // m: rows of the coarsest level
-    int32_t loc, pad; // first level (>= 1) of at most kLinLocalRows rows
+    int32_t loc;      // first level (>= 1) of at most kLinLocalRows rows
+    int32_t slices;   // slices of its sums: a multiple of the CTAs that solve it
     double tol;
     int64_t lvOff;    // doubles: FP64 level vectors (after 8n FP64 Krylov vectors)
     int64_t f32Off;   // doubles: start of the FP32 area (mixed form)

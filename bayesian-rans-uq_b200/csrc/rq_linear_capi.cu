@@ -3,6 +3,9 @@
 // and the persistent linKernel launch (rq_linsolve.cu).
 #include "rq_capi_common.h"
 
+#include <functional>
+#include <queue>
+
 using namespace rqc;
 
 // Standalone LDU systems resident on the device (rq_linsys_*).
@@ -45,16 +48,80 @@ void checkSolveArgs(int maxIter, double tol) {
                                     "cap and positive finite tolerance");
 }
 
-// CTAs per system, by its rows alone (so that its result does not depend on the batch): the
-// smallest power of two that leaves a thread no more than two to four rows, at most 16.
-// Measured on a B200, ms per FP64 AMG solve to 1e-10 of one n x n system with 8 / 4 / 2 rows
-// per thread as the bound: n = 64 1.70 / 1.63 / 1.46, n = 128 3.16 / 2.53 / 2.30, n = 256
-// (16 CTAs in all three) 4.06, n = 512 11.4 (about 260 with one CTA).
-int linCluster(int rows) {
+// Slices of a system's sums, and so the CTAs of its largest cluster: the smallest power of two
+// that leaves a thread fewer than two rows, at most 16.
+int linSlices(int rows) {
     int c = 1;
-    while (c < rq::kLinMaxCluster && 2L * c * rq::kLinThreads <= rows)
+    while (c < rq::kLinMaxSlices && 2L * c * rq::kLinThreads <= rows)
         c *= 2;
     return c;
+}
+
+// How often the clusters of a batch are halved from their largest size (no bit of a result
+// depends on it): the number for which a list of the systems, largest first, ends first on a
+// GPU of which a cluster of c CTAs takes one part in clustersAtOnce(c). A solve takes about
+// 3860 (rows / 4096)^0.3 + rows / c units of time (0.35 us), up to 2.4 times that as the rows
+// in flight outgrow L2. Measured on a B200, ms of FP64 AMG solves to 1e-10, by halvings 0 / 1 /
+// 2 / 3 / 4 (systems of n x n):
+//     1 of 64    1.48 / 1.67 /  1.87            148 of  64    7.21 /  3.51 /  2.95
+//     1 of 128   2.13 / 2.33 /  3.0 / 4.4 / 6.5  32 of 128   10.7 /  6.9 /  4.2 /  5.9 /  8.9
+//                                               148 of 128   46.3 / 23.9 / 18.9 / 15.2 / 15.6
+//     1 of 256   4.1 /  5.5 /  8.2 / 14 / 24     16 of 256   13.1 / 14.0 / 14.2 / 24.5 / 43.6
+//     1 of 512  11.4 / 18.4 / 32.5 / 61 / 113    32 of 512   97 / 98 / 77 / 138 / 255
+// (One 512-thread CTA per system, the former kernel: 148 of 64 about 7, 148 of 128 28.8, one of
+// 512 about 260.)
+template <typename AtOnce>
+int linHalvings(const std::vector<int> &rowsLargestFirst, AtOnce clustersAtOnce) {
+    const int most = rq::kLinMaxSlices;
+    std::vector<double> share(most + 1, -1.0);
+    auto shareOf = [&](int c) {
+        if (share[c] < 0.0) {
+            const int k = clustersAtOnce(c);
+            share[c] = k > 0 ? 1.0 / k : 2.0; // 2: does not fit
+        }
+        return share[c];
+    };
+    struct Run {
+        double end, share, rows;
+        bool operator>(const Run &o) const { return end > o.end; }
+    };
+    int best = -1;
+    double least = 0.0;
+    for (int h = 0; most >> h; ++h) {
+        std::priority_queue<Run, std::vector<Run>, std::greater<Run>> running;
+        double now = 0.0, free = 1.0, rows = 0.0, last = 0.0;
+        bool fits = true, waits = false;
+        for (int n : rowsLargestFirst) {
+            const int c = std::max(1, linSlices(n) >> h);
+            const double part = shareOf(c);
+            if (part > 1.0) {
+                fits = false;
+                break;
+            }
+            while (free < part - 1e-9) {
+                now = running.top().end;
+                free += running.top().share;
+                rows -= running.top().rows;
+                running.pop();
+                waits = true;
+            }
+            free -= part;
+            rows += n;
+            const double t = 3860 * std::pow(n / 4096.0, 0.3) + static_cast<double>(n) / c;
+            const double end = now + t * std::min(2.4, 1 + 0.7e-6 * rows);
+            running.push({end, part, static_cast<double>(n)});
+            last = std::max(last, end);
+        }
+        if (fits && (best < 0 || last < least)) {
+            best = h;
+            least = last;
+        }
+        if (fits && !waits) // smaller clusters only take longer
+            break;
+    }
+    if (best < 0)
+        throw RqError(RQ_E_CUDA, "linear solve kernel does not fit on an SM");
+    return best;
 }
 
 void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int precision) {
@@ -302,8 +369,15 @@ void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int preci
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return L.rows[a] > L.rows[b]; });
     L.sys.clear();
     long wsTotal = 0;
+    std::vector<int> queue(n);
+    for (int k = 0; k < n; ++k)
+        queue[k] = L.rows[order[k]];
+    const size_t localMost = *std::max_element(localOf.begin(), localOf.end());
+    const int halvings =
+        linHalvings(queue, [&](int c) { return rq::linConcurrent(c, localMost); });
     for (int s : order) {
-        const int cluster = linCluster(L.rows[s]);
+        byIndex[s].slices = linSlices(L.rows[s]);
+        const int cluster = std::max(1, byIndex[s].slices >> halvings);
         if (L.groups.empty() || L.groups.back().cluster != cluster) {
             L.groups.emplace_back();
             L.groups.back().first = static_cast<int>(L.sys.size());

@@ -38,8 +38,8 @@ constexpr int NT = kLinThreads;
 
 struct LinShared {
     DevLinSys sys;
-    double red[2][NT / 32];
-    double cred[2][2][kLinMaxCluster]; // the CTAs' sums, in alternating buffers
+    double red[2 * kLinMaxSlices][NT / 32]; // warp sums of each value of the CTA's slices
+    double cred[2][2][kLinMaxSlices];       // the slices' sums, in alternating buffers
     int job;
     int rank, ctas;
 };
@@ -63,44 +63,60 @@ template <typename V> __device__ __forceinline__ void putRemote(V *p, V v, int r
         asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(r), "r"(static_cast<int>(v)) : "memory");
 }
 
-// Sum of K per-thread values over the cluster. Each warp reduces by shuffles, lane 0
-// parks the partial, every warp re-reduces all partials in the same order, and the CTAs'
-// sums are exchanged and added in rank order, so every thread returns the same bits.
-template <int K> __device__ __forceinline__ void blockSum(double (&v)[K], LinShared &S, int &rp) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// Sums over the rows of a system. They are formed in sys.slices slices, whatever the number of
+// CTAs: slice i holds the rows (i + k slices) NT + 0 .. NT - 1, k = 0, 1, ..., and CTA r of c
+// the slices r, r + c, ..., which are the rows of its other passes too. A thread adds its rows
+// of a slice, each warp its threads by shuffles (lane 0 parks the sum), one warp per slice and
+// value the warps, and every thread the slices in order: all threads return the same bits, and
+// so does a cluster of any size.
+__device__ __forceinline__ double addLanes(double v) {
 #pragma unroll
-    for (int k = 0; k < K; ++k)
-        for (int o = 16; o > 0; o >>= 1)
-            v[k] += __shfl_xor_sync(FULL, v[k], o);
-    __syncthreads(); // the previous reduction's readers are done with red
-    if (lane == 0)
+    for (int o = 16; o > 0; o >>= 1)
+        v += __shfl_xor_sync(FULL, v, o);
+    return v;
+}
+// rows(t0, nt) adds the terms of the rows t0, t0 + nt, ... to v
+template <int K, typename Rows>
+__device__ __forceinline__ void parkOver(double (&v)[K], LinShared &S, Rows rows) {
+    const int nt = S.sys.slices * NT, own = S.sys.slices / S.ctas;
+    for (int i = 0; i < own; ++i) {
 #pragma unroll
         for (int k = 0; k < K; ++k)
-            S.red[k][warp] = v[k];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        double s = lane < NT / 32 ? S.red[k][lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1)
-            s += __shfl_xor_sync(FULL, s, o);
-        v[k] = s;
-    }
-    if (S.ctas > 1) {
-        if (static_cast<int>(threadIdx.x) < S.ctas)
-#pragma unroll
-            for (int k = 0; k < K; ++k)
-                putRemote(&S.cred[rp][k][S.rank], v[k], threadIdx.x);
-        gSync(S);
+            v[k] = 0.0;
+        rows((i * S.ctas + S.rank) * NT + static_cast<int>(threadIdx.x), nt);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            v[k] = S.cred[rp][k][0];
-            for (int c = 1; c < S.ctas; ++c)
-                v[k] += S.cred[rp][k][c];
+            const double w = addLanes(v[k]);
+            if ((threadIdx.x & 31) == 0)
+                S.red[i * K + k][threadIdx.x >> 5] = w;
         }
-        rp ^= 1;
     }
 }
-static_assert(NT / 32 <= 32, "blockSum reads one partial per lane");
+// the sums of what parkOver left; a barrier of the cluster for what was stored before
+template <int K> __device__ __forceinline__ void totalSums(double (&v)[K], LinShared &S, int &rp) {
+    const int lane = threadIdx.x & 31, rows = S.sys.slices / S.ctas * K;
+    __syncthreads();
+    for (int t = threadIdx.x >> 5; t < rows; t += NT / 32) {
+        const double w = addLanes(S.red[t][lane]);
+        const int i = t / K, k = t - i * K;
+        if (lane < S.ctas)
+            putRemote(&S.cred[rp][k][i * S.ctas + S.rank], w, lane);
+    }
+    gSync(S);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        v[k] = S.cred[rp][k][0];
+        for (int c = 1; c < S.sys.slices; ++c)
+            v[k] += S.cred[rp][k][c];
+    }
+    rp ^= 1;
+}
+template <int K, typename Rows>
+__device__ __forceinline__ void sumOver(double (&v)[K], LinShared &S, int &rp, Rows rows) {
+    parkOver(v, S, rows);
+    totalSums(v, S, rp);
+}
+static_assert(NT / 32 == 32, "a lane per warp sum");
 
 // one level of the hierarchy in value type T (FP64, or the FP32 copies)
 template <typename T> struct Lv {
@@ -164,24 +180,26 @@ __device__ __forceinline__ Lv<T> levelOf(const DevLinSys &S, int l, void *ws) {
 // broadcast back and the same sweeps after it (a symmetric preconditioner).
 // lvws: the level vectors of levels 1 .. loc - 1; t: a level-0 scratch vector. A level's
 // iterate alternates between x and r; its solution ends in r (the coarsest's in x).
-// Returns this thread's part of (r, z).
+// Parks (r, z) (parkOver).
 template <typename T>
-__device__ double vcycle(LinShared &S, const T *r, T *z, T *t, void *lvws, const T *inv) {
+__device__ void vcycle(LinShared &S, const T *r, T *z, T *t, void *lvws, const T *inv) {
     static_assert(kSweeps == 2, "the buffers alternate for two sweeps");
     const DevLinSys &sys = S.sys;
     const int L = sys.nlev;
     const T w = T(kOmega);
-    double rz = 0.0;
+    double rz[1];
     if (L == 1) { // the whole system is the coarsest level
         const int m = sys.m;
-        for (int i = gTid(S); i < m; i += gThreads(S)) {
-            T s = T(0);
-            for (int j = 0; j < m; ++j)
-                s += inv[i * m + j] * r[j];
-            z[i] = s;
-            rz += double(r[i]) * double(s);
-        }
-        return rz;
+        parkOver(rz, S, [&](int t0, int nt) {
+            for (int i = t0; i < m; i += nt) {
+                T s = T(0);
+                for (int j = 0; j < m; ++j)
+                    s += inv[i * m + j] * r[j];
+                z[i] = s;
+                rz[0] += double(r[i]) * double(s);
+            }
+        });
+        return;
     }
     auto tid = [&](int l) { return l >= sys.loc ? static_cast<int>(threadIdx.x) : gTid(S); };
     auto threads = [&](int l) { return l >= sys.loc ? NT : gThreads(S); };
@@ -255,35 +273,42 @@ __device__ double vcycle(LinShared &S, const T *r, T *z, T *t, void *lvws, const
             x[i] = y[i] + w * res * __ldg(A.rdg + i);
         });
         sync(l);
-        passRows<T>(A, x, t0, nt, [&](int i, T ax) {
+        auto last = [&](int i, T ax) {
             const T res = b[i] - ax;
             const T zi = x[i] + w * res * __ldg(A.rdg + i);
             y[i] = zi;
-            if (l == 0)
-                rz += double(r[i]) * double(zi);
-        });
-        if (l > 0) // level 0: the caller's block sum
+            return zi;
+        };
+        if (l > 0) {
+            passRows<T>(A, x, t0, nt, last);
             sync(l);
+        } else { // the caller's sum ends with a barrier
+            parkOver(rz, S, [&](int s0, int st) {
+                passRows<T>(A, x, s0, st, [&](int i, T ax) {
+                    rz[0] += double(r[i]) * double(last(i, ax));
+                });
+            });
+        }
         xc = y;
     }
-    return rz;
 }
 
 // z = M^-1 r; returns (r, z)
 template <typename T>
 __device__ __forceinline__ double precondition(LinShared &S, int &rp, bool amg, const T *r, T *z,
                                                T *t, void *lvws, const T *inv, const T *rdg0) {
-    double a[1] = {0.0};
-    if (amg) {
-        a[0] = vcycle<T>(S, r, z, t, lvws, inv);
-    } else {
-        for (int i = gTid(S); i < S.sys.n; i += gThreads(S)) {
-            const T zi = r[i] * __ldg(rdg0 + i);
-            z[i] = zi;
-            a[0] += double(r[i]) * double(zi);
-        }
-    }
-    blockSum<1>(a, S, rp);
+    double a[1];
+    if (amg)
+        vcycle<T>(S, r, z, t, lvws, inv);
+    else
+        parkOver(a, S, [&](int t0, int nt) {
+            for (int i = t0; i < S.sys.n; i += nt) {
+                const T zi = r[i] * __ldg(rdg0 + i);
+                z[i] = zi;
+                a[0] += double(r[i]) * double(zi);
+            }
+        });
+    totalSums(a, S, rp);
     return a[0];
 }
 
@@ -305,24 +330,26 @@ __device__ PcgOut pcg(LinShared &S, int &rp, const Lv<T> &A0, T *x, T *r, T *z, 
         p[i] = z[i];
     gSync(S);
     for (int it = 0; it < maxIter; ++it) {
-        double b1[1] = {0.0};
-        passRows<T>(A0, p, gTid(S), gThreads(S), [&](int i, T v) {
-            q[i] = v;
-            b1[0] += double(p[i]) * double(v);
+        double b1[1];
+        sumOver(b1, S, rp, [&](int t0, int nt) {
+            passRows<T>(A0, p, t0, nt, [&](int i, T v) {
+                q[i] = v;
+                b1[0] += double(p[i]) * double(v);
+            });
         });
-        blockSum<1>(b1, S, rp);
         const double pAp = b1[0];
         if (fabs(pAp) < 1e-30)
             break;
         const double alpha = rz / pAp;
-        double b2[1] = {0.0};
-        for (int i = gTid(S); i < n; i += gThreads(S)) {
-            x[i] += T(alpha) * p[i];
-            const T ri = r[i] - T(alpha) * q[i];
-            r[i] = ri;
-            b2[0] += double(ri) * double(ri);
-        }
-        blockSum<1>(b2, S, rp);
+        double b2[1];
+        sumOver(b2, S, rp, [&](int t0, int nt) {
+            for (int i = t0; i < n; i += nt) {
+                x[i] += T(alpha) * p[i];
+                const T ri = r[i] - T(alpha) * q[i];
+                r[i] = ri;
+                b2[0] += double(ri) * double(ri);
+            }
+        });
         o.iterations = it + 1;
         o.finalRes = sqrt(b2[0]) / r0n;
         if (o.finalRes < tol) {
@@ -346,14 +373,15 @@ __device__ PcgOut bicgstab(LinShared &S, int &rp, const Lv<double> &A0, double *
     double *r = ws, *rh = ws + n, *p = ws + 2L * n, *v = ws + 3L * n, *s = ws + 4L * n,
            *t = ws + 5L * n, *ph = ws + 6L * n, *sh = ws + 7L * n;
     PcgOut o{0, false, 0.0};
-    double a[1] = {0.0};
-    for (int i = gTid(S); i < n; i += gThreads(S)) {
-        rh[i] = r[i];
-        p[i] = 0.0;
-        v[i] = 0.0;
-        a[0] += r[i] * r[i];
-    }
-    blockSum<1>(a, S, rp);
+    double a[1];
+    sumOver(a, S, rp, [&](int t0, int nt) {
+        for (int i = t0; i < n; i += nt) {
+            rh[i] = r[i];
+            p[i] = 0.0;
+            v[i] = 0.0;
+            a[0] += r[i] * r[i];
+        }
+    });
     double rhoN = a[0], rho = 1, alpha = 1, omega = 1;
     for (int it = 0; it < maxIter; ++it) {
         if (fabs(rhoN) < 1e-30)
@@ -365,23 +393,25 @@ __device__ PcgOut bicgstab(LinShared &S, int &rp, const Lv<double> &A0, double *
             ph[i] = pi * __ldg(A0.rdg + i);
         }
         gSync(S);
-        double a1[1] = {0.0};
-        passRows<double>(A0, ph, gTid(S), gThreads(S), [&](int i, double vi) {
-            v[i] = vi;
-            a1[0] += rh[i] * vi;
+        double a1[1];
+        sumOver(a1, S, rp, [&](int t0, int nt) {
+            passRows<double>(A0, ph, t0, nt, [&](int i, double vi) {
+                v[i] = vi;
+                a1[0] += rh[i] * vi;
+            });
         });
-        blockSum<1>(a1, S, rp);
         if (fabs(a1[0]) < 1e-30)
             break;
         alpha = rhoN / a1[0];
-        double a2[1] = {0.0};
-        for (int i = gTid(S); i < n; i += gThreads(S)) {
-            const double si = r[i] - alpha * v[i];
-            s[i] = si;
-            sh[i] = si * __ldg(A0.rdg + i);
-            a2[0] += si * si;
-        }
-        blockSum<1>(a2, S, rp);
+        double a2[1];
+        sumOver(a2, S, rp, [&](int t0, int nt) {
+            for (int i = t0; i < n; i += nt) {
+                const double si = r[i] - alpha * v[i];
+                s[i] = si;
+                sh[i] = si * __ldg(A0.rdg + i);
+                a2[0] += si * si;
+            }
+        });
         const double sn = sqrt(a2[0]);
         if (sn / r0n < tol) {
             for (int i = gTid(S); i < n; i += gThreads(S))
@@ -392,23 +422,25 @@ __device__ PcgOut bicgstab(LinShared &S, int &rp, const Lv<double> &A0, double *
             o.converged = true;
             return o;
         }
-        double a3[2] = {0.0, 0.0};
-        passRows<double>(A0, sh, gTid(S), gThreads(S), [&](int i, double ti) {
-            t[i] = ti;
-            a3[0] += ti * ti;
-            a3[1] += ti * s[i];
+        double a3[2];
+        sumOver(a3, S, rp, [&](int t0, int nt) {
+            passRows<double>(A0, sh, t0, nt, [&](int i, double ti) {
+                t[i] = ti;
+                a3[0] += ti * ti;
+                a3[1] += ti * s[i];
+            });
         });
-        blockSum<2>(a3, S, rp);
         omega = a3[0] > 1e-30 ? a3[1] / a3[0] : 0.0;
-        double a4[2] = {0.0, 0.0};
-        for (int i = gTid(S); i < n; i += gThreads(S)) {
-            x[i] += alpha * ph[i] + omega * sh[i];
-            const double ri = s[i] - omega * t[i];
-            r[i] = ri;
-            a4[0] += ri * ri;
-            a4[1] += rh[i] * ri;
-        }
-        blockSum<2>(a4, S, rp);
+        double a4[2];
+        sumOver(a4, S, rp, [&](int t0, int nt) {
+            for (int i = t0; i < n; i += nt) {
+                x[i] += alpha * ph[i] + omega * sh[i];
+                const double ri = s[i] - omega * t[i];
+                r[i] = ri;
+                a4[0] += ri * ri;
+                a4[1] += rh[i] * ri;
+            }
+        });
         o.iterations = it + 1;
         o.finalRes = sqrt(a4[0]) / r0n;
         if (o.finalRes < tol) {
@@ -427,13 +459,14 @@ __device__ PcgOut bicgstab(LinShared &S, int &rp, const Lv<double> &A0, double *
 // r = b - A x in FP64; returns ||r||
 __device__ double residual(LinShared &S, int &rp, const Lv<double> &A0, const double *b,
                            const double *x, double *r) {
-    double a[1] = {0.0};
-    passRows<double>(A0, x, gTid(S), gThreads(S), [&](int i, double ax) {
-        const double ri = b[i] - ax;
-        r[i] = ri;
-        a[0] += ri * ri;
+    double a[1];
+    sumOver(a, S, rp, [&](int t0, int nt) {
+        passRows<double>(A0, x, t0, nt, [&](int i, double ax) {
+            const double ri = b[i] - ax;
+            r[i] = ri;
+            a[0] += ri * ri;
+        });
     });
-    blockSum<1>(a, S, rp);
     return sqrt(a[0]);
 }
 
