@@ -10,6 +10,7 @@ namespace rq {
 
 constexpr int kLinMaxLevels = 16;
 constexpr int kLinThreads = 1024;
+constexpr int kLinSmallThreads = 512; // of the systems of one slice
 constexpr int kLinMaxSlices = 16;   // slices of a system's sums: the CTAs of its largest cluster
 constexpr int kLinMaxLocalBytes = 208 * 1024; // shared memory of the local levels' vectors
 constexpr int kLinLocalRows = 2048; // rows of a level that every CTA of a cluster runs whole
@@ -53,12 +54,17 @@ struct DevLinSys {
     DevLinLevel lev[kLinMaxLevels];
 };
 
-// Persistent clusters of `cluster` CTAs of kLinThreads threads, one system at a time each;
-// *next zeroed by the caller; ws: `slots` workspaces of wsStride doubles, one per cluster;
-// localBytes: shared memory of the local levels' vectors.
+// Threads of a CTA (kLinThreads or kLinSmallThreads), CTAs per system, and shared memory of the
+// local levels' vectors.
+struct LinShape {
+    int threads = kLinThreads, cluster = 1;
+    size_t localBytes = 0;
+};
+// Persistent clusters, one system at a time each; *next zeroed by the caller; ws: `slots`
+// workspaces of wsStride doubles, one per cluster.
 cudaError_t launchLinear(const DevLinSys *systems, int nsys, int *next, double *ws, long wsStride,
-                         int slots, int cluster, size_t localBytes, cudaStream_t stream);
+                         int slots, const LinShape &shape, cudaStream_t stream);
 // Clusters that run at once (0: the shape does not fit).
-int linConcurrent(int cluster, size_t localBytes);
+int linConcurrent(const LinShape &shape);
 
 } // namespace rq

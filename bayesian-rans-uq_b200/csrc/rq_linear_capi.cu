@@ -11,12 +11,12 @@ using namespace rqc;
 // Standalone LDU systems resident on the device (rq_linsys_*).
 struct rq_linsys {
     int nsys = 0, kind = 0, precision = 0, maxLevels = 0;
-    // systems of one cluster size: a range of `sys`, the clusters launched for it with a
+    // systems of one launch shape: a range of `sys`, the clusters launched for it with a
     // workspace each, and a stream beside the caller's (all but the first group)
     struct Group {
-        int first = 0, count = 0, cluster = 1, slots = 1;
+        int first = 0, count = 0, slots = 1;
         long wsStride = 0, wsOff = 0;
-        size_t localBytes = 0;
+        rq::LinShape shape;
         cudaStream_t stream = nullptr;
         cudaEvent_t done = nullptr;
     };
@@ -57,6 +57,12 @@ int linSlices(int rows) {
     return c;
 }
 
+// Threads per CTA, by the rows alone: 512 with 128 registers for the systems of one slice, else
+// 1024 with 64. Measured on a B200, ms of FP64 AMG solves, 1 / 592 systems of n x n, 512 against
+// 1024 threads: n = 16 0.24 / 1.00 against 0.30 / 1.31, n = 24 0.32 / 1.33 against 0.37 / 1.64,
+// n = 32 0.44 / 2.02 against 0.57 / 2.56, n = 45 1.00 / 4.34 against 1.01 / 4.49.
+int linThreads(int rows) { return linSlices(rows) == 1 ? rq::kLinSmallThreads : rq::kLinThreads; }
+
 // How often the clusters of a batch are halved from their largest size (no bit of a result
 // depends on it): the number for which a list of the systems, largest first, ends first on a
 // GPU of which a cluster of c CTAs takes one part in clustersAtOnce(c). A solve takes about
@@ -73,13 +79,14 @@ int linSlices(int rows) {
 template <typename AtOnce>
 int linHalvings(const std::vector<int> &rowsLargestFirst, AtOnce clustersAtOnce) {
     const int most = rq::kLinMaxSlices;
-    std::vector<double> share(most + 1, -1.0);
-    auto shareOf = [&](int c) {
-        if (share[c] < 0.0) {
-            const int k = clustersAtOnce(c);
-            share[c] = k > 0 ? 1.0 / k : 2.0; // 2: does not fit
+    std::vector<double> share(most + 1, -1.0); // by CTAs; 0: one of kLinSmallThreads
+    auto shareOf = [&](int threads, int c) {
+        double &part = share[threads == rq::kLinThreads ? c : 0];
+        if (part < 0.0) {
+            const int k = clustersAtOnce(threads, c);
+            part = k > 0 ? 1.0 / k : 2.0; // 2: does not fit
         }
-        return share[c];
+        return part;
     };
     struct Run {
         double end, share, rows;
@@ -93,7 +100,7 @@ int linHalvings(const std::vector<int> &rowsLargestFirst, AtOnce clustersAtOnce)
         bool fits = true, waits = false;
         for (int n : rowsLargestFirst) {
             const int c = std::max(1, linSlices(n) >> h);
-            const double part = shareOf(c);
+            const double part = shareOf(linThreads(n), c);
             if (part > 1.0) {
                 fits = false;
                 break;
@@ -363,7 +370,7 @@ void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int preci
         byIndex[s].x = L.dX.as<double>() + L.xOff[s];
         byIndex[s].out = L.dOut.as<rq::LinOut>() + s;
     }
-    // queue order: by cluster size, largest systems first (longest-processing-time)
+    // queue order: by launch shape, largest systems first (longest-processing-time)
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return L.rows[a] > L.rows[b]; });
@@ -374,24 +381,28 @@ void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int preci
         queue[k] = L.rows[order[k]];
     const size_t localMost = *std::max_element(localOf.begin(), localOf.end());
     const int halvings =
-        linHalvings(queue, [&](int c) { return rq::linConcurrent(c, localMost); });
+        linHalvings(queue, [&](int threads, int c) {
+            return rq::linConcurrent({threads, c, localMost});
+        });
     for (int s : order) {
         byIndex[s].slices = linSlices(L.rows[s]);
+        const int threads = linThreads(L.rows[s]);
         const int cluster = std::max(1, byIndex[s].slices >> halvings);
-        if (L.groups.empty() || L.groups.back().cluster != cluster) {
+        if (L.groups.empty() || L.groups.back().shape.cluster != cluster ||
+            L.groups.back().shape.threads != threads) {
             L.groups.emplace_back();
             L.groups.back().first = static_cast<int>(L.sys.size());
-            L.groups.back().cluster = cluster;
+            L.groups.back().shape = {threads, cluster, 0};
         }
         rq_linsys::Group &g = L.groups.back();
         ++g.count;
         g.wsStride = std::max(g.wsStride, wsOf[s]);
-        g.localBytes = std::max(g.localBytes, localOf[s]);
+        g.shape.localBytes = std::max(g.shape.localBytes, localOf[s]);
         L.sys.push_back(byIndex[s]);
     }
     for (size_t k = 0; k < L.groups.size(); ++k) {
         rq_linsys::Group &g = L.groups[k];
-        const int atOnce = rq::linConcurrent(g.cluster, g.localBytes);
+        const int atOnce = rq::linConcurrent(g.shape);
         if (atOnce < 1)
             throw RqError(RQ_E_CUDA, "linear solve kernel does not fit on an SM");
         g.slots = std::min(g.count, atOnce);
@@ -409,7 +420,7 @@ void buildLinsys(rq_linsys &L, const rq_ldu *systems, int n, int kind, int preci
     L.dNext.ensure(sizeof(int) * L.groups.size());
 }
 
-// One launch per cluster size, side by side: the first on the caller's stream, the others
+// One launch per shape, side by side: the first on the caller's stream, the others
 // on streams of the handle that fork from it and join it.
 void launchLinsys(rq_linsys &L, int maxIter, double tol, cudaStream_t stream) {
     for (auto &d : L.sys) {
@@ -428,7 +439,7 @@ void launchLinsys(rq_linsys &L, int maxIter, double tol, cudaStream_t stream) {
             check(cudaStreamWaitEvent(st, L.fork, 0), "stream wait");
         check(rq::launchLinear(L.dSys.as<rq::DevLinSys>() + g.first, g.count,
                                L.dNext.as<int>() + k, L.dWs.as<double>() + g.wsOff, g.wsStride,
-                               g.slots, g.cluster, g.localBytes, st), "linear solve launch");
+                               g.slots, g.shape, st), "linear solve launch");
         if (k) {
             check(cudaEventRecord(g.done, st), "event record");
             check(cudaStreamWaitEvent(stream, g.done, 0), "stream wait");

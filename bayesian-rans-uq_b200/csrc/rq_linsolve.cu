@@ -34,22 +34,26 @@ constexpr int kSweeps = 2;     // pre- and post-smoothing sweeps
 constexpr int kMixedRounds = 12;
 constexpr double kMixedInnerTol = 1e-4; // relative drop asked of each FP32 correction
 
-constexpr int NT = kLinThreads;
-
-struct LinShared {
+// NT: threads of a CTA; the smaller ones solve systems of one slice
+template <int NT> struct LinShared {
+    static constexpr bool kOne = NT == kLinSmallThreads;
+    __device__ int nCtas() const { return kOne ? 1 : ctas; }
+    __device__ int nSlices() const { return kOne ? 1 : sys.slices; }
     DevLinSys sys;
-    double red[2 * kLinMaxSlices][NT / 32]; // warp sums of each value of the CTA's slices
-    double cred[2][2][kLinMaxSlices];       // the slices' sums, in alternating buffers
+    double red[kOne ? 4 : 2 * kLinMaxSlices][NT / 32]; // warp sums of the CTA's slices
+    double cred[2][2][kOne ? 1 : kLinMaxSlices]; // the slices' sums, in alternating buffers
     int job;
     int rank, ctas;
 };
 extern __shared__ __align__(16) unsigned char linSmem[]; // vectors of the local levels
 
 // thread index in the cluster and its threads; the cluster's barrier
-__device__ __forceinline__ int gTid(const LinShared &S) { return S.rank * NT + threadIdx.x; }
-__device__ __forceinline__ int gThreads(const LinShared &S) { return S.ctas * NT; }
-__device__ __forceinline__ void gSync(const LinShared &S) {
-    if (S.ctas > 1)
+template <int NT> __device__ __forceinline__ int gTid(const LinShared<NT> &S) {
+    return (S.kOne ? 0 : S.rank * NT) + threadIdx.x;
+}
+template <int NT> __device__ __forceinline__ int gThreads(const LinShared<NT> &S) { return S.nCtas() * NT; }
+template <int NT> __device__ __forceinline__ void gSync(const LinShared<NT> &S) {
+    if (S.nCtas() > 1)
         asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
     else
         __syncthreads();
@@ -68,7 +72,8 @@ template <typename V> __device__ __forceinline__ void putRemote(V *p, V v, int r
 // the slices r, r + c, ..., which are the rows of its other passes too. A thread adds its rows
 // of a slice, each warp its threads by shuffles (lane 0 parks the sum), one warp per slice and
 // value the warps, and every thread the slices in order: all threads return the same bits, and
-// so does a cluster of any size.
+// so does a cluster of any size. (With one slice every warp adds the warps, which saves a
+// barrier; the parked sums alternate between two buffers then.)
 __device__ __forceinline__ double addLanes(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -76,28 +81,38 @@ __device__ __forceinline__ double addLanes(double v) {
     return v;
 }
 // rows(t0, nt) adds the terms of the rows t0, t0 + nt, ... to v
-template <int K, typename Rows>
-__device__ __forceinline__ void parkOver(double (&v)[K], LinShared &S, Rows rows) {
-    const int nt = S.sys.slices * NT, own = S.sys.slices / S.ctas;
+template <int K, int NT, typename Rows>
+__device__ __forceinline__ void parkOver(double (&v)[K], LinShared<NT> &S, int rp, Rows rows) {
+    const int nt = S.nSlices() * NT, own = S.nSlices() / S.nCtas();
+    const int first = S.nSlices() == 1 ? rp * K : 0;
     for (int i = 0; i < own; ++i) {
 #pragma unroll
         for (int k = 0; k < K; ++k)
             v[k] = 0.0;
-        rows((i * S.ctas + S.rank) * NT + static_cast<int>(threadIdx.x), nt);
+        rows(i * S.nCtas() * NT + gTid(S), nt);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const double w = addLanes(v[k]);
             if ((threadIdx.x & 31) == 0)
-                S.red[i * K + k][threadIdx.x >> 5] = w;
+                S.red[first + i * K + k][threadIdx.x >> 5] = w;
         }
     }
 }
 // the sums of what parkOver left; a barrier of the cluster for what was stored before
-template <int K> __device__ __forceinline__ void totalSums(double (&v)[K], LinShared &S, int &rp) {
-    const int lane = threadIdx.x & 31, rows = S.sys.slices / S.ctas * K;
+template <int K, int NT>
+__device__ __forceinline__ void totalSums(double (&v)[K], LinShared<NT> &S, int &rp) {
+    const int lane = threadIdx.x & 31;
     __syncthreads();
+    if (S.nSlices() == 1) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            v[k] = addLanes(lane < NT / 32 ? S.red[rp * K + k][lane] : 0.0);
+        rp ^= 1;
+        return;
+    }
+    const int rows = S.sys.slices / S.ctas * K;
     for (int t = threadIdx.x >> 5; t < rows; t += NT / 32) {
-        const double w = addLanes(S.red[t][lane]);
+        const double w = addLanes(lane < NT / 32 ? S.red[t][lane] : 0.0);
         const int i = t / K, k = t - i * K;
         if (lane < S.ctas)
             putRemote(&S.cred[rp][k][i * S.ctas + S.rank], w, lane);
@@ -111,12 +126,12 @@ template <int K> __device__ __forceinline__ void totalSums(double (&v)[K], LinSh
     }
     rp ^= 1;
 }
-template <int K, typename Rows>
-__device__ __forceinline__ void sumOver(double (&v)[K], LinShared &S, int &rp, Rows rows) {
-    parkOver(v, S, rows);
+template <int K, int NT, typename Rows>
+__device__ __forceinline__ void sumOver(double (&v)[K], LinShared<NT> &S, int &rp, Rows rows) {
+    parkOver(v, S, rp, rows);
     totalSums(v, S, rp);
 }
-static_assert(NT / 32 == 32, "a lane per warp sum");
+static_assert(kLinThreads <= 1024, "a lane per warp sum");
 
 // one level of the hierarchy in value type T (FP64, or the FP32 copies)
 template <typename T> struct Lv {
@@ -181,8 +196,8 @@ __device__ __forceinline__ Lv<T> levelOf(const DevLinSys &S, int l, void *ws) {
 // lvws: the level vectors of levels 1 .. loc - 1; t: a level-0 scratch vector. A level's
 // iterate alternates between x and r; its solution ends in r (the coarsest's in x).
 // Parks (r, z) (parkOver).
-template <typename T>
-__device__ void vcycle(LinShared &S, const T *r, T *z, T *t, void *lvws, const T *inv) {
+template <typename T, int NT>
+__device__ void vcycle(LinShared<NT> &S, int rp, const T *r, T *z, T *t, void *lvws, const T *inv) {
     static_assert(kSweeps == 2, "the buffers alternate for two sweeps");
     const DevLinSys &sys = S.sys;
     const int L = sys.nlev;
@@ -190,7 +205,7 @@ __device__ void vcycle(LinShared &S, const T *r, T *z, T *t, void *lvws, const T
     double rz[1];
     if (L == 1) { // the whole system is the coarsest level
         const int m = sys.m;
-        parkOver(rz, S, [&](int t0, int nt) {
+        parkOver(rz, S, rp, [&](int t0, int nt) {
             for (int i = t0; i < m; i += nt) {
                 T s = T(0);
                 for (int j = 0; j < m; ++j)
@@ -283,7 +298,7 @@ __device__ void vcycle(LinShared &S, const T *r, T *z, T *t, void *lvws, const T
             passRows<T>(A, x, t0, nt, last);
             sync(l);
         } else { // the caller's sum ends with a barrier
-            parkOver(rz, S, [&](int s0, int st) {
+            parkOver(rz, S, rp, [&](int s0, int st) {
                 passRows<T>(A, x, s0, st, [&](int i, T ax) {
                     rz[0] += double(r[i]) * double(last(i, ax));
                 });
@@ -294,14 +309,14 @@ __device__ void vcycle(LinShared &S, const T *r, T *z, T *t, void *lvws, const T
 }
 
 // z = M^-1 r; returns (r, z)
-template <typename T>
-__device__ __forceinline__ double precondition(LinShared &S, int &rp, bool amg, const T *r, T *z,
+template <typename T, int NT>
+__device__ __forceinline__ double precondition(LinShared<NT> &S, int &rp, bool amg, const T *r, T *z,
                                                T *t, void *lvws, const T *inv, const T *rdg0) {
     double a[1];
     if (amg)
-        vcycle<T>(S, r, z, t, lvws, inv);
+        vcycle<T>(S, rp, r, z, t, lvws, inv);
     else
-        parkOver(a, S, [&](int t0, int nt) {
+        parkOver(a, S, rp, [&](int t0, int nt) {
             for (int i = t0; i < S.sys.n; i += nt) {
                 const T zi = r[i] * __ldg(rdg0 + i);
                 z[i] = zi;
@@ -320,8 +335,8 @@ struct PcgOut {
 
 // PCG from x (in T) with r = b - A x already in r and r0n = ||r||; the
 // reference's loop (LinearSolver.hpp:206-245). Vectors r, z, p, q, t: n each.
-template <typename T>
-__device__ PcgOut pcg(LinShared &S, int &rp, const Lv<T> &A0, T *x, T *r, T *z, T *p, T *q, T *t,
+template <typename T, int NT>
+__device__ PcgOut pcg(LinShared<NT> &S, int &rp, const Lv<T> &A0, T *x, T *r, T *z, T *p, T *q, T *t,
                       void *lvws, const T *inv, double r0n, int maxIter, double tol, bool amg) {
     const int n = A0.n;
     PcgOut o{0, false, 0.0};
@@ -367,7 +382,8 @@ __device__ PcgOut pcg(LinShared &S, int &rp, const Lv<T> &A0, T *x, T *r, T *z, 
 }
 
 // Right-Jacobi BiCGSTAB (LinearSolver.hpp:251-345) in FP64; r holds b - A x.
-__device__ PcgOut bicgstab(LinShared &S, int &rp, const Lv<double> &A0, double *x, double *ws,
+template <int NT>
+__device__ PcgOut bicgstab(LinShared<NT> &S, int &rp, const Lv<double> &A0, double *x, double *ws,
                            double r0n, int maxIter, double tol) {
     const int n = A0.n;
     double *r = ws, *rh = ws + n, *p = ws + 2L * n, *v = ws + 3L * n, *s = ws + 4L * n,
@@ -457,7 +473,8 @@ __device__ PcgOut bicgstab(LinShared &S, int &rp, const Lv<double> &A0, double *
 }
 
 // r = b - A x in FP64; returns ||r||
-__device__ double residual(LinShared &S, int &rp, const Lv<double> &A0, const double *b,
+template <int NT>
+__device__ double residual(LinShared<NT> &S, int &rp, const Lv<double> &A0, const double *b,
                            const double *x, double *r) {
     double a[1];
     sumOver(a, S, rp, [&](int t0, int nt) {
@@ -470,7 +487,8 @@ __device__ double residual(LinShared &S, int &rp, const Lv<double> &A0, const do
     return sqrt(a[0]);
 }
 
-__device__ void solveOne(LinShared &S, int &rp, double *ws) {
+template <int NT>
+__device__ void solveOne(LinShared<NT> &S, int &rp, double *ws) {
     const DevLinSys &sys = S.sys;
     const int n = sys.n;
     const bool amg = sys.kind == kLinAmg;
@@ -530,9 +548,10 @@ __device__ void solveOne(LinShared &S, int &rp, double *ws) {
         *sys.out = out;
 }
 
+template <int NT>
 __global__ void __launch_bounds__(NT, 1) linKernel(const DevLinSys *systems, int nsys, int *next,
                                                    double *wsBase, long wsStride) {
-    __shared__ LinShared S;
+    __shared__ LinShared<NT> S;
     if (threadIdx.x == 0) {
         unsigned rank, ctas;
         asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -542,7 +561,7 @@ __global__ void __launch_bounds__(NT, 1) linKernel(const DevLinSys *systems, int
     }
     __syncthreads();
     gSync(S); // every CTA of the cluster has started: its shared memory can be written
-    double *ws = wsBase + wsStride * (blockIdx.x / S.ctas);
+    double *ws = wsBase + wsStride * (blockIdx.x / S.nCtas());
     int rp = 0;
     for (;;) {
         if (gTid(S) == 0) {
@@ -570,21 +589,26 @@ __global__ void __launch_bounds__(NT, 1) linKernel(const DevLinSys *systems, int
 } // namespace
 
 namespace {
-cudaError_t linConfig(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, int slots, int cluster,
-                      size_t localBytes, cudaStream_t stream) {
+const void *kernelOf(const LinShape &sh) {
+    return sh.threads == kLinSmallThreads ? reinterpret_cast<const void *>(&linKernel<kLinSmallThreads>)
+                                          : reinterpret_cast<const void *>(&linKernel<kLinThreads>);
+}
+cudaError_t linConfig(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, int slots,
+                      const LinShape &sh, cudaStream_t stream) {
     // the limit of the largest local levels, not of this launch: it belongs to the function, and
     // another thread may be launching it for other systems
-    cudaError_t e = cudaFuncSetAttribute(linKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const void *fn = kernelOf(sh);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kLinMaxLocalBytes);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(linKernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cfg = cudaLaunchConfig_t{};
-    cfg.gridDim = dim3(slots * cluster);
-    cfg.blockDim = dim3(kLinThreads);
-    cfg.dynamicSmemBytes = localBytes;
+    cfg.gridDim = dim3(slots * sh.cluster);
+    cfg.blockDim = dim3(sh.threads);
+    cfg.dynamicSmemBytes = sh.localBytes;
     cfg.stream = stream;
     attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = cluster;
+    attr.val.clusterDim.x = sh.cluster;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
@@ -593,21 +617,22 @@ cudaError_t linConfig(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, int sl
 } // namespace
 
 cudaError_t launchLinear(const DevLinSys *systems, int nsys, int *next, double *ws, long wsStride,
-                         int slots, int cluster, size_t localBytes, cudaStream_t stream) {
+                         int slots, const LinShape &sh, cudaStream_t stream) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr;
-    cudaError_t e = linConfig(cfg, attr, slots, cluster, localBytes, stream);
+    cudaError_t e = linConfig(cfg, attr, slots, sh, stream);
     if (e != cudaSuccess)
         return e;
-    return cudaLaunchKernelEx(&cfg, linKernel, systems, nsys, next, ws, wsStride);
+    void *args[] = {&systems, &nsys, &next, &ws, &wsStride};
+    return cudaLaunchKernelExC(&cfg, kernelOf(sh), args);
 }
 
-int linConcurrent(int cluster, size_t localBytes) {
+int linConcurrent(const LinShape &sh) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr;
     int count = 0;
-    if (linConfig(cfg, attr, 1, cluster, localBytes, nullptr) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&count, linKernel, &cfg) != cudaSuccess) {
+    if (linConfig(cfg, attr, 1, sh, nullptr) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&count, kernelOf(sh), &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
