@@ -33,3 +33,16 @@ def test_mixed_sizes():
         (r1,), (x1,) = lin.solve_batch([systems[k]], kind="AMG", max_iter=500, tol=1e-10)
         assert results[k].converged and results[k].iterations == r1.iterations
         np.testing.assert_array_equal(xs[k], x1)
+
+
+def test_solutions_of_small_and_large_systems_in_any_order():
+    """Runs of small solutions are read back together, those of 12288 rows and more alone."""
+    sizes = [20, 111, 8, 9, 110, 10, 112, 113, 5, 40]
+    systems = [wl.poisson_system(n, 70 + k) for k, n in enumerate(sizes)]
+    batch = lin.LinearBatch(systems, kind="AMG")
+    _, zero = batch.solve(500, 1e-10)
+    _, start = batch.solve(500, 1e-10, xs=[np.zeros(s.n_cells) for s in systems])
+    for s, x, y in zip(systems, zero, start):
+        (_,), (x1,) = lin.solve_batch([s], kind="AMG", max_iter=500, tol=1e-10)
+        np.testing.assert_array_equal(x, x1)
+        np.testing.assert_array_equal(y, x1)
