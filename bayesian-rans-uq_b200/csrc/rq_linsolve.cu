@@ -1,6 +1,6 @@
 // Standalone batched linear solves on the device: one thread-block cluster per LDU system
-// (1 to 16 CTAs by its rows), persistent clusters pulling systems from a queue (largest
-// first, as the host orders them). The solvers restate core/include/LinearSolver.hpp:
+// (1 to 16 CTAs by its rows and the batch), persistent clusters pulling systems from a queue
+// (largest first, as the host orders them). The solvers restate core/include/LinearSolver.hpp:
 //   PCG (:184-246) with the Jacobi preconditioner or the AMG V-cycle of this
 //   project (damped-Jacobi smoothing, aggregate-sum restriction, aggregate
 //   broadcast prolongation scaled by an over-correction factor, dense coarsest

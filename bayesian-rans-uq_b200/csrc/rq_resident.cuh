@@ -541,8 +541,8 @@ __device__ __forceinline__ void coarseRes(Shared &S, const double *rr0) {
 // holds the finest level in registers; all threads of the CTA run the coarse levels. The
 // caller's next CTA barrier makes x and *out visible.
 // What bounds it: the instructions that each of its 13 to 21 phases issues. Measured on a
-// B200, cycles of the pressure solve per PCG iteration: 19 800 / 39 200 / 62 900 at 384 /
-// 768 / 1536 cells, against 23 900 / 53 500 / 95 000 of pcgT and vcycleT.
+// B200, us of the pressure solve per PCG iteration (the first 400 outer iterations): 8.0 / 15.4 /
+// 25.3 at 384 / 768 / 1536 cells, against 12.2 / 27.2 / 48.3 of pcgT and vcycleT before.
 template <bool AMG>
 __device__ __noinline__ void pcgRes(double *x, double r0n, int maxIter, double tol, LinRes *out) {
     Shared &S = *reinterpret_cast<Shared *>(rqSmem);

@@ -168,7 +168,7 @@ struct Shared {
     LoopState L;                          // the outer loop's scalars (runSolve)
     ResShared R;                          // block sums of the resident solvers
     int resWarps;                         // their working warps, 0: the general solvers
-    int resAmg;                           // the V-cycle too (one sweep per level)
+    int resAmg;                           // the V-cycle too
     double *resInv;                       // the coarsest inverse in coarseRes's order,
     int ownInv;                           // a CTA's own copy in shared memory
     int resDone;                          // a PCG solve has ended
@@ -460,10 +460,6 @@ __device__ __forceinline__ double rowDot(const Cell &q, const double *d, const d
     const double tS = q.south ? aS[c] * x[c - nx] : 0.0;
     const double tN = q.north ? aN[c] * x[c + nx] : 0.0;
     return accum4(q, d[c] * x[c], tW, tE, tS, tN);
-}
-
-__device__ __forceinline__ double jac(double r, double d) {
-    return (fabs(d) > 1e-30) ? r / d : r; // jacobiPrecond, LinearSolver.hpp:173-177
 }
 
 // The cells a thread owns in every per-cell sweep: c = thread, thread + threads, ...
@@ -931,12 +927,6 @@ __device__ __forceinline__ void segPass(int n, int t, int nt, Part part, Use use
         if (j == 0 && i < n)
             use(i, s);
     }
-}
-
-// row i of an ELL level times x, entries in column order
-template <typename T>
-__device__ __forceinline__ T csrRowT(const DevAmgLevel &L, const T *val, const T *x, int i) {
-    return ellDot<T>(L.ecol, val, x, L.width, i);
 }
 
 #include "rq_resident.cuh"
