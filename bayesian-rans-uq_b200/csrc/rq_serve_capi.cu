@@ -85,7 +85,8 @@ struct rq_server {
     std::vector<rq_problem *> problems;
     // every slot runs 512 threads whatever the classes' own CTA sizes, so a request's
     // result does not depend on which other classes the server holds (a batch of a
-    // class above 1024 cells runs 768 threads; its served requests agree to rounding)
+    // class above 1536 cells runs on clusters of 768-thread CTAs; its served requests, one
+    // CTA each, agree to rounding)
     int capacity = 0, thetaStride = 1, predStride = 1, block = 512, grid = 1, arena = 0;
     long long idleNs = 0;
     MappedBuf host; // jobs | theta | rows | predictions | clocks | done | published | closed

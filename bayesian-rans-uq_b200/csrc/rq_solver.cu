@@ -244,7 +244,8 @@ __device__ __forceinline__ void totalSums(double (&v)[K], Shared &S, int &rp) {
     if constexpr (kCluster) { // a warp per slice and value, the sums to every CTA
         const int nc = ctaCount(), rank = ctaRank(), rows = S.ownSlices * K;
         for (int t = warp; t < rows; t += nw) {
-            double w = 0.0, unused; // eight partials per lane, the four lanes by a product
+            double w = 0.0, unused; // eight partials per lane, four lanes by a product: one warp
+                                    // does it, so it costs less than five shuffles here
             if (8 * (lane & 3) < nw) {
                 const double2 *r = reinterpret_cast<const double2 *>(&S.red[rp][t][8 * (lane & 3)]);
                 const double2 a = r[0], b = r[1], c = r[2], d = r[3];

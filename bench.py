@@ -41,8 +41,8 @@ BYTES_OUTER, BYTES_KRYLOV, BYTES_PRESSURE = 1600, 360, 400  # algorithmic B/cell
 #   between its SM and L2 (L1 misses, spills, stores);
 # * the L2's peak: 3 sectors per cycle on each of the 184 slices (ncu's
 #   lts__t_sectors peak_sustained) x 32 B at the 1965 MHz clock.
-DRAM_BYTES_PER_DRAW_1536 = 2_587_904 + 256
-L2_BYTES_PER_ITER_1536 = 166_757_762 * 32 / 600
+DRAM_BYTES_PER_DRAW_1536 = 2_510_848
+L2_BYTES_PER_ITER_1536 = 159_382_903 * 32 / 600
 L2_PEAK_GBS = 3 * 32 * 184 * 1.965
 
 
@@ -656,7 +656,7 @@ def linear_arm(args):
                 "note": "one-shot rq_linear_solve_batch: host set-up, upload, solve, download"},
         "gpu_launches": args.steps,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
-                     "frac": achieved / hbm, "traffic": None, "kernel": "linKernel<512>",
+                     "frac": achieved / hbm, "traffic": None, "kernel": "linKernel",
                      "note": "algorithmic level-0 bytes per AMG-PCG iteration (5 CSR passes + 32 "
                              "vector passes) x iterations; coarse levels not counted"},
         "cpu_baseline": cpu,
