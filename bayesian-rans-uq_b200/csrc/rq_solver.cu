@@ -79,6 +79,9 @@ constexpr int kSumSlots = 3; // of a sum
 // rows of warp partials: a reduction's values, or a sum's of every slice that a CTA holds
 constexpr int kRedRows = kCluster ? kMaxSlices * kSumSlots : kRedSlots;
 constexpr int kRedWarps = kCluster ? 24 : 32; // the cluster kernels' CTAs have 24 warps
+#ifdef RQ_CLUSTER
+static_assert(RQ_CTA == 32 * kRedWarps, "a column per warp");
+#endif
 
 struct Work {
     double *Ux, *Uy, *p, *k, *w, *nuT, *F1, *F2, *Pk, *CD, *S;
@@ -218,6 +221,7 @@ __device__ __forceinline__ void mma884(double &d0, double &d1, double a, double 
 // warps, whichever CTA does it, and every thread adds the slices in order.
 template <int K>
 __device__ __forceinline__ void parkSums(double (&v)[K], Shared &S, int rp, int slice) {
+    static_assert(K <= kSumSlots, "rows of a slice's sums");
     double u[K], w[K];
 #pragma unroll
     for (int k = 0; k < K; ++k)
